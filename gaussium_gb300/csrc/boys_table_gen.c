@@ -18,6 +18,10 @@
  * exponential's rows (GS_BOYS_EXPT: row k = exp(-T_k) / j!, j = 0..6, and a zero): with
  * the factorials folded in, an expansion about T_k is a Horner chain of FMAs in T_k - T.
  *
+ * For FP32 quartets (T below BOYS_TMAX32, their largest asymptotic threshold) it writes
+ * GS_BOYS_F32_<M>: row k = eight floats {hi, lo of F_M(T_k); F_{M+j}(T_k) / j!, j = 1..4;
+ * hi, lo of exp(-T_k)}, hi + lo being the value to twice a float's precision.
+ *
  * usage: boys_table_gen OUT.h
  */
 #include <math.h>
@@ -27,7 +31,14 @@
 #define BOYS_TMAX 80
 #define BOYS_ROWS (BOYS_TMAX * BOYS_INV_H + 1)
 #define BOYS_NCOL 18 /* F_0..F_16 and exp(-T) */
+#define BOYS_TMAX32 50
 #define BOYS_TAYLOR_MMAX 10 /* F_{M+6} is the highest order tabulated */
+
+static void pair32(FILE *f, long double x)
+{
+    const float hi = (float)x;
+    fprintf(f, "%af,%af,", hi, (float)(x - hi));
+}
 
 int main(int argc, char **argv)
 {
@@ -73,7 +84,18 @@ int main(int argc, char **argv)
         for (int j = 0; j <= 6; ++j) fprintf(f, "%a,", (double)(F[k][BOYS_NCOL - 1] / fact[j]));
         fprintf(f, "0x0p+0, \\\n");
     }
-    fprintf(f, "\n");
+    fprintf(f, "\n#define BOYS_TMAX32 %d\n#define BOYS_ROWS32 %d\n", BOYS_TMAX32,
+            BOYS_TMAX32 * BOYS_INV_H + 1);
+    for (int M = 0; M <= BOYS_TAYLOR_MMAX; ++M) {
+        fprintf(f, "#define GS_BOYS_F32_%d \\\n", M);
+        for (int k = 0; k <= BOYS_TMAX32 * BOYS_INV_H; ++k) {
+            pair32(f, F[k][M]);
+            for (int j = 1; j <= 4; ++j) fprintf(f, "%af,", (float)(F[k][M + j] / fact[j]));
+            pair32(f, F[k][BOYS_NCOL - 1]);
+            fprintf(f, " \\\n");
+        }
+        fprintf(f, "\n");
+    }
     fclose(f);
     return 0;
 }

@@ -301,11 +301,11 @@ __global__ void k_boys(int n, const double* __restrict__ t, double* __restrict__
 __device__ __forceinline__ double block_dmax(const double* __restrict__ d, int ns, int a, int b,
                                              int c, int e) {
     double dm = d[a * ns + b];
-    dm = fmax(dm, d[c * ns + e]);
-    dm = fmax(dm, d[a * ns + c]);
-    dm = fmax(dm, d[a * ns + e]);
-    dm = fmax(dm, d[b * ns + c]);
-    dm = fmax(dm, d[b * ns + e]);
+    dm = gs::max_nonneg(dm, d[c * ns + e]);
+    dm = gs::max_nonneg(dm, d[a * ns + c]);
+    dm = gs::max_nonneg(dm, d[a * ns + e]);
+    dm = gs::max_nonneg(dm, d[b * ns + c]);
+    dm = gs::max_nonneg(dm, d[b * ns + e]);
     return dm;
 }
 
@@ -337,7 +337,7 @@ __global__ void k_partition(int ntask, const int2* __restrict__ tasks,
         } else {
             dm = block_dmax(dmax, nshell, B.sa, B.sb, K.sa, K.sb);
         }
-        const double est = (double)B.qmax * (double)K.qmax * dm;
+        const double est = gs::widen(B.qmax) * gs::widen(K.qmax) * dm;
         kind = est < thr ? 0 : (est >= cut ? 1 : 2);
     }
     const unsigned lane = threadIdx.x & 31;

@@ -108,6 +108,8 @@ GS_HD GS_INLINE const double* boys_table() {
 __device__ __align__(16) const double g_boys_taylor[BOYS_ROWS * 8] = {
     GS_BOYS_CAT(GS_BOYS_TAYLOR_, GS_BOYS_ORDER)};
 __device__ __align__(16) const double g_boys_expt[BOYS_ROWS * 8] = {GS_BOYS_EXPT};
+__device__ __align__(16) const float g_boys_f32[BOYS_ROWS32 * 8] = {
+    GS_BOYS_CAT(GS_BOYS_F32_, GS_BOYS_ORDER)};
 constexpr int kBoysOrder = GS_BOYS_ORDER;
 static_assert(kBoysOrder >= 0 && kBoysOrder <= BOYS_TAYLOR_MMAX, "Boys order without rows");
 #else
@@ -122,6 +124,92 @@ template <typename T> GS_HD GS_INLINE T ldg(const T* p) {
 #endif
 }
 
+// ------------------------------------------------------------------ work moved off the FP64 pipe
+// A warp-wide FP64 instruction takes 64 cycles of its scheduler's pipe here (measured: 0.5
+// lanes per clock, the same for one warp and for four), a conversion to or from double 82, a
+// DSETP 64; an integer or FP32 instruction takes one.  These helpers do with a few integer
+// operations on the IEEE words what would otherwise take such an instruction.
+
+// (float)x, rounded to nearest even; the conversion itself outside the normal floats.
+GS_HD GS_INLINE float narrow(double x) {
+#if defined(__CUDA_ARCH__)
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned e = (hi >> 20) & 0x7ffu;
+    if (e - 897u < 253u) {                    // 2^-126 <= |x| < 2^127
+        const unsigned f = ((e - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+        const unsigned rest = lo & 0x1fffffffu;
+        const unsigned up = rest > 0x10000000u - (f & 1u) ? 1u : 0u;
+        return __uint_as_float((hi & 0x80000000u) | (f + up));
+    }
+#endif
+    return (float)x;
+}
+GS_HD GS_INLINE double narrow_to(double, double x) { return x; }
+GS_HD GS_INLINE float narrow_to(float, double x) { return narrow(x); }
+
+// (double)x, exact; the conversion itself for zero, subnormals, infinities and NaN.
+GS_HD GS_INLINE double widen(float x) {
+#if defined(__CUDA_ARCH__)
+    const unsigned b = __float_as_uint(x);
+    if (((b >> 23) & 0xffu) - 1u < 254u)
+        return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)),
+                                (int)(b << 29));
+#endif
+    return (double)x;
+}
+GS_HD GS_INLINE double widen(double x) { return x; }
+
+// 2 x, exact.
+GS_HD GS_INLINE double twice(double x) {
+#if defined(__CUDA_ARCH__)
+    const int hi = __double2hiint(x);
+    if ((((unsigned)hi >> 20) & 0x7ffu) - 1u < 0x7fdu)
+        return __hiloint2double(hi + 0x00100000, __double2loint(x));
+#endif
+    return 2.0 * x;
+}
+GS_HD GS_INLINE float twice(float x) { return 2.0f * x; }
+
+// The larger of two values that are not negative (densities' magnitudes): as integers.
+GS_HD GS_INLINE double max_nonneg(double a, double b) {
+#if defined(__CUDA_ARCH__)
+    return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
+#else
+    return a > b ? a : b;
+#endif
+}
+
+// High word of a whole number n, 1 <= n < 2^20, as a double.
+GS_HD constexpr unsigned whole_hiword(unsigned n) {
+    unsigned e = 0;
+    for (unsigned m = n; m > 1; m >>= 1) ++e;
+    return ((1023u + e) << 20) | ((n << (20 - e)) & 0xfffffu);
+}
+
+// t < n for t >= 0 and a whole number n: false for NaN.
+template <unsigned N> GS_HD GS_INLINE bool below(double t) {
+#if defined(__CUDA_ARCH__)
+    return (unsigned)__double2hiint(t) < whole_hiword(N);
+#else
+    return t < (double)N;
+#endif
+}
+template <unsigned N> GS_HD GS_INLINE bool below(float t) { return t < (float)N; }
+
+// Nearest grid row k of t >= 0 and T_k - t (exact), the rounding by the sum with 1.5 2^52,
+// whose last bit is worth one.  k is held to the table whatever t is.
+GS_HD GS_INLINE int boys_row(double t, double& d) {
+    const double magic = 6755399441055744.0;
+    const double kf = t * BOYS_INV_H + magic;
+    d = (kf - magic) * (1.0 / BOYS_INV_H) - t;
+#if defined(__CUDA_ARCH__)
+    return min((unsigned)__double2loint(kf), (unsigned)(BOYS_ROWS - 1));
+#else
+    const double k = kf - magic;
+    return k >= 0 && k < BOYS_ROWS ? (int)k : BOYS_ROWS - 1;
+#endif
+}
+
 // Boys function below BOYS_TMAX, always in FP64: 7-term Taylor expansion of F_M about the
 // nearest grid point (grid step 1/BOYS_INV_H), then downward recursion
 //   F_{m-1}(t) = (2t F_m(t) + e^{-t}) / (2m - 1),
@@ -132,8 +220,8 @@ GS_HD GS_INLINE void boys_small(double t, double pref, double* __restrict__ F) {
 #if defined(__CUDA_ARCH__) && defined(GS_BOYS_ORDER)
     if constexpr (M == kBoysOrder) {
         // the same expansion and recursion from this order's Taylor rows
-        const int k = __double2int_rn(t * BOYS_INV_H);
-        const double d = fma((double)k, 1.0 / BOYS_INV_H, -t);     // t_k - t, exact
+        double d;                                                  // t_k - t, exact
+        const int k = boys_row(t, d);
         const double2* g = reinterpret_cast<const double2*>(g_boys_taylor) + 4 * k;
         const double2 g01 = __ldg(g), g23 = __ldg(g + 1), g45 = __ldg(g + 2), g67 = __ldg(g + 3);
         double f = fma(g67.x, d, g45.y);
@@ -183,37 +271,66 @@ GS_HD GS_INLINE void boys_small(double t, double pref, double* __restrict__ F) {
     }
 }
 
-// Boys function below the asymptotic threshold for an FP32 quartet: the same grid, the
-// Taylor expansion cut after the d^4 term (its remainder, at most d^5/5! < 3e-10 of F_M
-// for |d| <= 1/32, is far below FP32 rounding) and the downward recursion, all in FP64;
-// each F_m is rounded to float once and then scaled by pref in float.  t - t_k is exact in
-// float (both are multiples of t's ulp and |t - t_k| <= 1/32).
+// The same below an FP32 quartet's threshold, without the FP64 pipe: F_M and exp(-t) as
+// unevaluated sums of two floats.  row: eight floats of grid point T_k (see
+// boys_table_gen.c), d = T_k - t, exact in float (both are multiples of t's last place and
+// |d| <= 1/32).  The leading term of each expansion is a pair, so the float rounding of the
+// rest, |d| of it at most, is 2^-29 of the result; the downward recursion carries pairs with
+// error-free sums and products (Dekker, Numer. Math. 18, 224 (1971)); each F_m is rounded to
+// float once, as from FP64, and scaled.  About 17 FP32 instructions an order, against two
+// FP64 ones and a conversion at 64 and 82 cycles a warp.
+template <int M>
+GS_HD GS_INLINE void boys_pair32(const float* __restrict__ r, float t, float d, float pref,
+                                 float* __restrict__ F) {
+    const float tail = d * fmaf(d, fmaf(d, fmaf(d, r[5], r[4]), r[3]), r[2]);
+    const float fl0 = r[1] + tail;
+    float h = r[0] + fl0;
+    float l = fl0 - (h - r[0]);                          // |r[0]| >= |fl0|
+    F[M] = h * pref;
+    if (M > 0) {
+        const float q = d * fmaf(d, fmaf(d, fmaf(d, 1.0f / 24, 1.0f / 6), 0.5f), 1.0f);
+        const float el0 = fmaf(r[6], q, r[7]);
+        const float eh = r[6] + el0;
+        const float el = el0 - (eh - r[6]);
+        const float t2 = t + t;
+        GS_UNROLL for (int m = M; m >= 1; --m) {
+            const float ph = t2 * h;
+            const float pl = fmaf(t2, l, fmaf(t2, h, -ph));
+            const float a = fmaxf(ph, eh), b = fminf(ph, eh);    // both positive
+            float s = a + b;
+            float z = (b - (s - a)) + (pl + el);
+            if (m > 1) {                                  // times 1 / (2m - 1)
+                const float ch = (float)(1.0 / (2 * m - 1));
+                const float cl = (float)(1.0 / (2 * m - 1) - (double)ch);
+                const float g = s * ch;
+                z = fmaf(z, ch, fmaf(s, cl, fmaf(s, ch, -g)));
+                s = g;
+            }
+            h = s + z;
+            l = z - (h - s);
+            F[m - 1] = h * pref;
+        }
+    }
+}
+
+// Boys function below the asymptotic threshold for an FP32 quartet: from the order's pair
+// rows where the translation unit has them, else from the FP64 grid: the Taylor expansion
+// cut after the d^4 term (its remainder, at most d^5/5! < 3e-10 of F_M for |d| <= 1/32, is
+// far below FP32 rounding) and the downward recursion, all in FP64; each F_m is rounded to
+// float once and then scaled by pref in float.  Per primitive quartet the FP64 form holds
+// the FP64 pipe for 14 + 2.4 M instructions' time, the pair form not at all.
 template <int M>
 GS_HD GS_INLINE void boys_small32(float t, float pref, float* __restrict__ F) {
     static_assert(M + 4 <= BOYS_NCOL - 2, "Taylor terms beyond the tabulated orders");
 #if defined(__CUDA_ARCH__) && defined(GS_BOYS_ORDER)
     if constexpr (M == kBoysOrder) {
-        // this order's Taylor rows, cut after the d^4 term as below
-        const int k = __float2int_rn(t * float(BOYS_INV_H));
-        const double d = (double)((float)k * (1.0f / BOYS_INV_H) - t);
-        const double2* g = reinterpret_cast<const double2*>(g_boys_taylor) + 4 * k;
-        const double2 g01 = __ldg(g), g23 = __ldg(g + 1), g45 = __ldg(g + 2);
-        double Fd[M + 1];
-        double f = fma(g45.x, d, g23.y);
-        f = fma(f, d, g23.x);
-        f = fma(f, d, g01.y);
-        Fd[M] = fma(f, d, g01.x);
-        if (M > 0) {
-            const double2* x = reinterpret_cast<const double2*>(g_boys_expt) + 4 * k;
-            const double2 x01 = __ldg(x), x23 = __ldg(x + 1), x45 = __ldg(x + 2);
-            double e = fma(x45.x, d, x23.y);
-            e = fma(e, d, x23.x);
-            e = fma(e, d, x01.y);
-            const double et = fma(e, d, x01.x);
-            const double t2 = 2.0 * (double)t;
-            GS_UNROLL for (int m = M; m >= 1; --m) Fd[m - 1] = (t2 * Fd[m] + et) * (1.0 / (2 * m - 1));
-        }
-        GS_UNROLL for (int m = 0; m <= M; ++m) F[m] = (float)Fd[m] * pref;
+        const float kf = fmaf(t, float(BOYS_INV_H), 12582912.0f);    // 1.5 2^23: rounds
+        const unsigned k = min(__float_as_uint(kf) & 0x3fffffu, (unsigned)(BOYS_ROWS32 - 1));
+        const float d = (kf - 12582912.0f) * (1.0f / BOYS_INV_H) - t;
+        const float4* g = reinterpret_cast<const float4*>(g_boys_f32) + 2 * k;
+        const float4 g0 = __ldg(g), g1 = __ldg(g + 1);
+        const float r[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+        boys_pair32<M>(r, t, d, pref, F);
         return;
     }
 #endif
@@ -243,8 +360,8 @@ GS_HD GS_INLINE void boys_small32(float t, float pref, float* __restrict__ F) {
 // F_m(T) ~ (2m-1)!! / (2T)^m * sqrt(pi/T) / 2 is within 2^-54 (FP64) or 2^-26 (FP32) of
 // F_m for every m <= M.  Its relative error is the regularised upper incomplete gamma
 // function Q(m + 1/2, T), which grows with m, so the threshold depends on M only.
-constexpr double kBoysAsym64[17] = {36, 40, 43, 46, 49, 52, 54, 57, 59, 61, 64, 66, 68, 70, 72, 74, 76};
-constexpr float kBoysAsym32[17] = {17, 20, 23, 25, 28, 30, 32, 34, 36, 38, 40, 42, 43, 45, 47, 48, 50};
+constexpr unsigned kBoysAsym64[17] = {36, 40, 43, 46, 49, 52, 54, 57, 59, 61, 64, 66, 68, 70, 72, 74, 76};
+constexpr unsigned kBoysAsym32[17] = {17, 20, 23, 25, 28, 30, 32, 34, 36, 38, 40, 42, 43, 45, 47, 48, 50};
 
 // F[m] = pref * F_m(t), m = 0..M.  Below the threshold: the grid expansion and the
 // downward recursion in FP64 (boys_small, or boys_small32 for an FP32 quartet, which
@@ -256,9 +373,9 @@ template <int M, typename T>
 GS_HD GS_INLINE void boys(T t, T pref, T* __restrict__ F) {
     static_assert(M <= 16, "Boys orders beyond the table");
     constexpr bool dbl = sizeof(T) == 8;
-    constexpr T thr = dbl ? T(kBoysAsym64[M]) : T(kBoysAsym32[M]);
-    static_assert(thr <= T(BOYS_TMAX), "asymptotic threshold beyond the grid");
-    if (t < thr) {
+    constexpr unsigned thr = dbl ? kBoysAsym64[M] : kBoysAsym32[M];
+    static_assert(thr <= (dbl ? BOYS_TMAX : BOYS_TMAX32), "asymptotic threshold beyond the grid");
+    if (below<thr>(t)) {
         if constexpr (dbl) boys_small<M>(t, pref, F);
         else boys_small32<M>(t, pref, F);
     } else {
@@ -272,36 +389,68 @@ GS_HD GS_INLINE void boys(T t, T pref, T* __restrict__ F) {
 }
 
 // ------------------------------------------------------------------ one shell quartet
+// Adds one primitive quartet's [e0|f0] targets to the contraction accumulators.
+template <int LA, int LB, int LC, int LD, typename T>
+GS_HD GS_INLINE void eri_primitive(const PrimRec<T>& P, const PrimRec<T>& Q,
+                                   T* __restrict__ acc) {
+    using G = ClassGen<LA, LB, LC, LD>;
+    const T pq = P.p + Q.p;
+    const T PQx = Q.Px - P.Px, PQy = Q.Py - P.Py, PQz = Q.Pz - P.Pz;
+    const T r2 = PQx * PQx + PQy * PQy + PQz * PQz;
+#if defined(__CUDA_ARCH__) && defined(GS_BOYS_ORDER)
+    if constexpr (G::L == 0 && sizeof(T) == 8 && kBoysOrder == 0) {
+        // (ss|ss): with X = p q R^2, T = X / (p + q); far quartets (T >= threshold) need only
+        // 1/sqrt(X), near ones only 1/sqrt(p + q), so one reciprocal square root serves a
+        // warp that holds both, and the far lanes add nothing to the near lanes' work
+        constexpr double thr = kBoysAsym64[0];
+        const T X = P.p * Q.p * r2;
+        const T u = fma(-thr, pq, X);
+        const bool far = __double2hiint(u) >= 0;
+        const T y = gs_rsqrt(far ? X : pq);
+        T f = T(0.88622692545275801365);                 // sqrt(pi)/2
+        if (!far) {
+            double d;
+            const int k = boys_row(X * (y * y), d);
+            const double2* g = reinterpret_cast<const double2*>(g_boys_taylor) + 4 * k;
+            const double2 g01 = __ldg(g), g23 = __ldg(g + 1), g45 = __ldg(g + 2), g67 = __ldg(g + 3);
+            f = fma(fma(fma(fma(fma(fma(g67.x, d, g45.y), d, g45.x), d, g23.y), d, g23.x), d,
+                        g01.y), d, g01.x);
+        }
+        acc[0] = fma(P.Kp * Q.Kp * y, f, acc[0]);
+        return;
+    }
+#endif
+    const T rs = gs_rsqrt(pq);
+    const T ipq = rs * rs;
+    const T wq = Q.p * ipq, wp = P.p * ipq;
+    const T t = P.p * wq * r2;
+    T F[G::L + 1];
+    boys<G::L, T>(t, P.Kp * Q.Kp * rs, F);
+    VrrCoef<T> c;
+    c.PAx = P.PAx; c.PAy = P.PAy; c.PAz = P.PAz;
+    c.WPx = wq * PQx; c.WPy = wq * PQy; c.WPz = wq * PQz;
+    c.QCx = Q.PAx; c.QCy = Q.PAy; c.QCz = Q.PAz;
+    c.WQx = -wp * PQx; c.WQy = -wp * PQy; c.WQz = -wp * PQz;
+    c.i2p = P.i2p; c.i2q = Q.i2p;
+    c.rp2 = wq * P.i2p; c.rq2 = wp * Q.i2p;
+    c.i2pq = T(0.5) * ipq;
+    G::vrr(F, c, acc);
+}
+
 // Contracted Cartesian block of the canonical quartet (bra | ket), in the component
-// order of ClassGen (blk[((ia*NB+ib)*NC+ic)*ND+id]), without per-component scaling.
+// order of ClassGen (blk[((ia*NB+ib)*NC+ic)*ND+id]), without per-component scaling.  The
+// ket's primitives are the outer loop: the lanes of a warp share the bra pair far more often
+// than the ket pair, so the inner loop's loads fall on one line instead of 32.
 template <int LA, int LB, int LC, int LD, typename T>
 GS_HD GS_INLINE void eri_quartet(const PairRec& B, const PairRec& K,
                                  const PrimRec<T>* __restrict__ prims, T* __restrict__ blk) {
     using G = ClassGen<LA, LB, LC, LD>;
     T acc[G::NACC];
     GS_UNROLL for (int i = 0; i < G::NACC; ++i) acc[i] = T(0);
-    for (int i = 0; i < B.nprim; ++i) {
-        const PrimRec<T> P = prims[B.prim_off + i];
-        for (int j = 0; j < K.nprim; ++j) {
-            const PrimRec<T> Q = prims[K.prim_off + j];
-            const T pq = P.p + Q.p;
-            const T rs = gs_rsqrt(pq);
-            const T ipq = rs * rs;
-            const T PQx = Q.Px - P.Px, PQy = Q.Py - P.Py, PQz = Q.Pz - P.Pz;
-            const T wq = Q.p * ipq, wp = P.p * ipq;
-            const T t = P.p * wq * (PQx * PQx + PQy * PQy + PQz * PQz);
-            T F[G::L + 1];
-            boys<G::L, T>(t, P.Kp * Q.Kp * rs, F);
-            VrrCoef<T> c;
-            c.PAx = P.PAx; c.PAy = P.PAy; c.PAz = P.PAz;
-            c.WPx = wq * PQx; c.WPy = wq * PQy; c.WPz = wq * PQz;
-            c.QCx = Q.PAx; c.QCy = Q.PAy; c.QCz = Q.PAz;
-            c.WQx = -wp * PQx; c.WQy = -wp * PQy; c.WQz = -wp * PQz;
-            c.i2p = P.i2p; c.i2q = Q.i2p;
-            c.rp2 = wq * P.i2p; c.rq2 = wp * Q.i2p;
-            c.i2pq = T(0.5) * ipq;
-            G::vrr(F, c, acc);
-        }
+    for (int j = 0; j < K.nprim; ++j) {
+        const PrimRec<T> Q = prims[K.prim_off + j];
+        for (int i = 0; i < B.nprim; ++i)
+            eri_primitive<LA, LB, LC, LD, T>(prims[B.prim_off + i], Q, acc);
     }
     G::hrr(acc, T(B.ABx), T(B.ABy), T(B.ABz), T(K.ABx), T(K.ABy), T(K.ABz), blk);
 }
@@ -313,29 +462,10 @@ template <int LA, int LB, int LC, int LD, typename T>
 GS_HD GS_INLINE void eri_accumulate(const PairRec& B, const PairRec& K,
                                     const PrimRec<T>* __restrict__ prims, T* __restrict__ acc,
                                     int start, int stride) {
-    using G = ClassGen<LA, LB, LC, LD>;
     const int nK = K.nprim, ntot = B.nprim * nK;
-    for (int x = start; x < ntot; x += stride) {
-        const PrimRec<T> P = prims[B.prim_off + x / nK];
-        const PrimRec<T> Q = prims[K.prim_off + x % nK];
-        const T pq = P.p + Q.p;
-        const T rs = gs_rsqrt(pq);
-        const T ipq = rs * rs;
-        const T PQx = Q.Px - P.Px, PQy = Q.Py - P.Py, PQz = Q.Pz - P.Pz;
-        const T wq = Q.p * ipq, wp = P.p * ipq;
-        const T t = P.p * wq * (PQx * PQx + PQy * PQy + PQz * PQz);
-        T F[G::L + 1];
-        boys<G::L, T>(t, P.Kp * Q.Kp * rs, F);
-        VrrCoef<T> c;
-        c.PAx = P.PAx; c.PAy = P.PAy; c.PAz = P.PAz;
-        c.WPx = wq * PQx; c.WPy = wq * PQy; c.WPz = wq * PQz;
-        c.QCx = Q.PAx; c.QCy = Q.PAy; c.QCz = Q.PAz;
-        c.WQx = -wp * PQx; c.WQy = -wp * PQy; c.WQz = -wp * PQz;
-        c.i2p = P.i2p; c.i2q = Q.i2p;
-        c.rp2 = wq * P.i2p; c.rq2 = wp * Q.i2p;
-        c.i2pq = T(0.5) * ipq;
-        G::vrr(F, c, acc);
-    }
+    for (int x = start; x < ntot; x += stride)
+        eri_primitive<LA, LB, LC, LD, T>(prims[B.prim_off + x / nK], prims[K.prim_off + x % nK],
+                                         acc);
 }
 
 // ------------------------------------------------------------------ shell-pair records

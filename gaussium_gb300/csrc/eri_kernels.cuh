@@ -16,6 +16,18 @@ constexpr int kBlock = 128;
 #define GS_THREAD_MINB 1
 #endif
 
+// Whether the component scales of an s or p shell (one per component) are all exactly one,
+// by their words; never claimed for d shells, whose mixed components carry sqrt(3).  Blocks of
+// unit scales skip the scaling products: in the (ps|ss) Fock digestion they are a third of a
+// quartet's FP64 instructions outside the primitive loops.
+template <int L> __device__ __forceinline__ bool unit_scale(const double* __restrict__ cs) {
+    if constexpr (L >= 2) return false;
+    int z = 0;
+    GS_UNROLL for (int i = 0; i < 2 * L + 1; ++i)
+        z |= (__double2hiint(cs[i]) ^ 0x3ff00000) | __double2loint(cs[i]);
+    return z == 0;
+}
+
 // Block write epilogue: the canonical block of `task`, scaled per component, at its
 // original-order position.
 template <int LA, int LB, int LC, int LD, typename T>
@@ -24,21 +36,34 @@ __device__ __forceinline__ void write_block(const WriteArgs& a, const WriteTask&
     using G = ClassGen<LA, LB, LC, LD>;
     long long s[4];
     block_strides(task.code, G::NA, G::NB, G::NC, G::ND, s);
+    const double* cs = a.comp_scale;
+    double* out = a.out + task.off;
+    if constexpr (LA < 2 && LB < 2 && LC < 2 && LD < 2) {
+        if (unit_scale<LA>(cs + 6 * B.sa) && unit_scale<LB>(cs + 6 * B.sb) &&
+            unit_scale<LC>(cs + 6 * K.sa) && unit_scale<LD>(cs + 6 * K.sb)) {
+            GS_UNROLL for (int ia = 0; ia < G::NA; ++ia)
+            GS_UNROLL for (int ib = 0; ib < G::NB; ++ib)
+            GS_UNROLL for (int ic = 0; ic < G::NC; ++ic)
+            GS_UNROLL for (int id = 0; id < G::ND; ++id)
+                out[ia * s[0] + ib * s[1] + ic * s[2] + id * s[3]] =
+                    widen(blk[((ia * G::NB + ib) * G::NC + ic) * G::ND + id]);
+            return;
+        }
+    }
     double sab[G::NA * G::NB], scd[G::NC * G::ND];
     GS_UNROLL for (int i = 0; i < G::NA; ++i)
         GS_UNROLL for (int j = 0; j < G::NB; ++j)
-            sab[i * G::NB + j] = a.comp_scale[6 * B.sa + i] * a.comp_scale[6 * B.sb + j];
+            sab[i * G::NB + j] = cs[6 * B.sa + i] * cs[6 * B.sb + j];
     GS_UNROLL for (int i = 0; i < G::NC; ++i)
         GS_UNROLL for (int j = 0; j < G::ND; ++j)
-            scd[i * G::ND + j] = a.comp_scale[6 * K.sa + i] * a.comp_scale[6 * K.sb + j];
-    double* out = a.out + task.off;
+            scd[i * G::ND + j] = cs[6 * K.sa + i] * cs[6 * K.sb + j];
     GS_UNROLL for (int ia = 0; ia < G::NA; ++ia)
     GS_UNROLL for (int ib = 0; ib < G::NB; ++ib)
     GS_UNROLL for (int ic = 0; ic < G::NC; ++ic)
     GS_UNROLL for (int id = 0; id < G::ND; ++id) {
         const int e = ((ia * G::NB + ib) * G::NC + ic) * G::ND + id;
         out[ia * s[0] + ib * s[1] + ic * s[2] + id * s[3]] =
-            (double)blk[e] * (sab[ia * G::NB + ib] * scd[ic * G::ND + id]);
+            widen(blk[e]) * (sab[ia * G::NB + ib] * scd[ic * G::ND + id]);
     }
 }
 
@@ -94,18 +119,18 @@ __global__ void __launch_bounds__(32 * kSplitWarps) k_eri_write_split(const Writ
 // (always, without screening).
 __device__ __forceinline__ bool jk_keep(const JKArgs& a, const PairRec& B, const PairRec& K) {
     if (a.screen_thr <= 0.0) return true;
-    const double bound = (double)B.qmax * (double)K.qmax;
+    const double bound = widen(B.qmax) * widen(K.qmax);
     double dm;
     if (a.shell_mol) {
         dm = a.mol_dmax[a.shell_mol[B.sa]];
     } else {
         const int ns = a.nshell;
         dm = a.shell_dmax[B.sa * ns + B.sb];
-        dm = fmax(dm, a.shell_dmax[K.sa * ns + K.sb]);
-        dm = fmax(dm, a.shell_dmax[B.sa * ns + K.sa]);
-        dm = fmax(dm, a.shell_dmax[B.sa * ns + K.sb]);
-        dm = fmax(dm, a.shell_dmax[B.sb * ns + K.sa]);
-        dm = fmax(dm, a.shell_dmax[B.sb * ns + K.sb]);
+        dm = max_nonneg(dm, a.shell_dmax[K.sa * ns + K.sb]);
+        dm = max_nonneg(dm, a.shell_dmax[B.sa * ns + K.sa]);
+        dm = max_nonneg(dm, a.shell_dmax[B.sa * ns + K.sb]);
+        dm = max_nonneg(dm, a.shell_dmax[B.sb * ns + K.sa]);
+        dm = max_nonneg(dm, a.shell_dmax[B.sb * ns + K.sb]);
     }
     const double est = bound * dm;
     return !(est < a.screen_thr || est < a.prec_lo || est >= a.prec_hi);
@@ -118,18 +143,31 @@ __device__ __forceinline__ void jk_digest(const JKArgs& a, const int2 task, cons
                                           long long mbase) {
     using G = ClassGen<LA, LB, LC, LD>;
     constexpr int NA = G::NA, NB = G::NB, NC = G::NC, ND = G::ND;
-    const double deg = (B.sa == B.sb ? 0.5 : 1.0) * (K.sa == K.sb ? 0.5 : 1.0) *
-                       (task.x == task.y ? 0.5 : 1.0);
+    const int halves = (B.sa == B.sb) + (K.sa == K.sb) + (task.x == task.y);
+    const T deg = halves == 0 ? T(1) : halves == 1 ? T(0.5) : halves == 2 ? T(0.25) : T(0.125);
     const double* cs = a.comp_scale;
     T sc[NA * NB * NC * ND];
-    {
-        T sab[NA * NB], scd[NC * ND];
+    const bool unit_bra = unit_scale<LA>(cs + 6 * B.sa) && unit_scale<LB>(cs + 6 * B.sb);
+    const bool unit_ket = unit_scale<LC>(cs + 6 * K.sa) && unit_scale<LD>(cs + 6 * K.sb);
+    T sab[NA * NB];
+    if (!unit_bra) {
         GS_UNROLL for (int i = 0; i < NA; ++i)
             GS_UNROLL for (int j = 0; j < NB; ++j)
-                sab[i * NB + j] = (T)(deg * cs[6 * B.sa + i] * cs[6 * B.sb + j]);
+                sab[i * NB + j] = deg * narrow_to(T(0), cs[6 * B.sa + i] * cs[6 * B.sb + j]);
+    } else {
+        GS_UNROLL for (int i = 0; i < NA * NB; ++i) sab[i] = deg;
+    }
+    if (unit_ket) {
+        if (unit_bra && halves == 0) {
+            GS_UNROLL for (int e = 0; e < G::NBLK; ++e) sc[e] = blk[e];
+        } else {
+            GS_UNROLL for (int e = 0; e < G::NBLK; ++e) sc[e] = blk[e] * sab[e / (NC * ND)];
+        }
+    } else {
+        T scd[NC * ND];
         GS_UNROLL for (int i = 0; i < NC; ++i)
             GS_UNROLL for (int j = 0; j < ND; ++j)
-                scd[i * ND + j] = (T)(cs[6 * K.sa + i] * cs[6 * K.sb + j]);
+                scd[i * ND + j] = narrow_to(T(0), cs[6 * K.sa + i] * cs[6 * K.sb + j]);
         GS_UNROLL for (int ab = 0; ab < NA * NB; ++ab)
             GS_UNROLL for (int cd = 0; cd < NC * ND; ++cd)
                 sc[ab * NC * ND + cd] = blk[ab * NC * ND + cd] * (sab[ab] * scd[cd]);
@@ -141,9 +179,9 @@ __device__ __forceinline__ void jk_digest(const JKArgs& a, const int2 task, cons
         double* Jo = a.j + mbase;
         T pab[NA * NB], pcd[NC * ND];
         GS_UNROLL for (int i = 0; i < NA; ++i)
-            GS_UNROLL for (int j = 0; j < NB; ++j) pab[i * NB + j] = (T)P[(fa + i) * n + fb + j];
+            GS_UNROLL for (int j = 0; j < NB; ++j) pab[i * NB + j] = narrow_to(T(0), P[(fa + i) * n + fb + j]);
         GS_UNROLL for (int i = 0; i < NC; ++i)
-            GS_UNROLL for (int j = 0; j < ND; ++j) pcd[i * ND + j] = (T)P[(fc + i) * n + fd + j];
+            GS_UNROLL for (int j = 0; j < ND; ++j) pcd[i * ND + j] = narrow_to(T(0), P[(fc + i) * n + fd + j]);
         T jab[NA * NB], jcd[NC * ND];
         GS_UNROLL for (int i = 0; i < NA * NB; ++i) jab[i] = T(0);
         GS_UNROLL for (int i = 0; i < NC * ND; ++i) jcd[i] = T(0);
@@ -155,23 +193,23 @@ __device__ __forceinline__ void jk_digest(const JKArgs& a, const int2 task, cons
             }
         GS_UNROLL for (int i = 0; i < NA; ++i)
             GS_UNROLL for (int j = 0; j < NB; ++j)
-                atomicAdd(Jo + (fa + i) * n + fb + j, 2.0 * (double)jab[i * NB + j]);
+                atomicAdd(Jo + (fa + i) * n + fb + j, widen(twice(jab[i * NB + j])));
         GS_UNROLL for (int i = 0; i < NC; ++i)
             GS_UNROLL for (int j = 0; j < ND; ++j)
-                atomicAdd(Jo + (fc + i) * n + fd + j, 2.0 * (double)jcd[i * ND + j]);
+                atomicAdd(Jo + (fc + i) * n + fd + j, widen(twice(jcd[i * ND + j])));
     }
     for (int s = 0; s < a.nk; ++s) {
         const double* P = a.pk + (size_t)s * a.mat_stride + mbase;
         double* Kout = a.k + (size_t)s * a.mat_stride + mbase;
         T pbd[NB * ND], pbc[NB * NC], pad[NA * ND], pac[NA * NC];
         GS_UNROLL for (int i = 0; i < NB; ++i)
-            GS_UNROLL for (int j = 0; j < ND; ++j) pbd[i * ND + j] = (T)P[(fb + i) * n + fd + j];
+            GS_UNROLL for (int j = 0; j < ND; ++j) pbd[i * ND + j] = narrow_to(T(0), P[(fb + i) * n + fd + j]);
         GS_UNROLL for (int i = 0; i < NB; ++i)
-            GS_UNROLL for (int j = 0; j < NC; ++j) pbc[i * NC + j] = (T)P[(fb + i) * n + fc + j];
+            GS_UNROLL for (int j = 0; j < NC; ++j) pbc[i * NC + j] = narrow_to(T(0), P[(fb + i) * n + fc + j]);
         GS_UNROLL for (int i = 0; i < NA; ++i)
-            GS_UNROLL for (int j = 0; j < ND; ++j) pad[i * ND + j] = (T)P[(fa + i) * n + fd + j];
+            GS_UNROLL for (int j = 0; j < ND; ++j) pad[i * ND + j] = narrow_to(T(0), P[(fa + i) * n + fd + j]);
         GS_UNROLL for (int i = 0; i < NA; ++i)
-            GS_UNROLL for (int j = 0; j < NC; ++j) pac[i * NC + j] = (T)P[(fa + i) * n + fc + j];
+            GS_UNROLL for (int j = 0; j < NC; ++j) pac[i * NC + j] = narrow_to(T(0), P[(fa + i) * n + fc + j]);
         T kac[NA * NC], kad[NA * ND], kbc[NB * NC], kbd[NB * ND];
         GS_UNROLL for (int i = 0; i < NA * NC; ++i) kac[i] = T(0);
         GS_UNROLL for (int i = 0; i < NA * ND; ++i) kad[i] = T(0);
@@ -189,16 +227,16 @@ __device__ __forceinline__ void jk_digest(const JKArgs& a, const int2 task, cons
         }
         GS_UNROLL for (int i = 0; i < NA; ++i)
             GS_UNROLL for (int j = 0; j < NC; ++j)
-                atomicAdd(Kout + (fa + i) * n + fc + j, (double)kac[i * NC + j]);
+                atomicAdd(Kout + (fa + i) * n + fc + j, widen(kac[i * NC + j]));
         GS_UNROLL for (int i = 0; i < NA; ++i)
             GS_UNROLL for (int j = 0; j < ND; ++j)
-                atomicAdd(Kout + (fa + i) * n + fd + j, (double)kad[i * ND + j]);
+                atomicAdd(Kout + (fa + i) * n + fd + j, widen(kad[i * ND + j]));
         GS_UNROLL for (int i = 0; i < NB; ++i)
             GS_UNROLL for (int j = 0; j < NC; ++j)
-                atomicAdd(Kout + (fb + i) * n + fc + j, (double)kbc[i * NC + j]);
+                atomicAdd(Kout + (fb + i) * n + fc + j, widen(kbc[i * NC + j]));
         GS_UNROLL for (int i = 0; i < NB; ++i)
             GS_UNROLL for (int j = 0; j < ND; ++j)
-                atomicAdd(Kout + (fb + i) * n + fd + j, (double)kbd[i * ND + j]);
+                atomicAdd(Kout + (fb + i) * n + fd + j, widen(kbd[i * ND + j]));
     }
 }
 

@@ -76,11 +76,12 @@ template <int LA, int LB, int LC, int LD, typename T, int VG = 1, int RQ = 1> st
     static constexpr size_t BYTES_JK = (size_t)WARP_JK * sizeof(T) * kWideWarps;
 };
 
-template <typename T>
-__device__ __forceinline__ void wide_setup(const PrimRec<T>& P, const PrimRec<T>& Q, int L,
-                                           T* __restrict__ c, T* __restrict__ F);
-
-template <int M, typename T>
+// Recursion coefficients and scaled Boys values of one primitive quartet.  KB, KK, KX: the
+// largest multiples of 1/2p, 1/2q and 1/2(p+q) that the class's program reads.  The doubled
+// ones are exponent increments (an FP64 product takes 76 cycles of its pipe), and a class of
+// low angular momentum leaves out the multiples it never reads: for (ps|ss) 15 products of
+// about 60 FP64 instructions.
+template <int M, typename T, int KB = 4, int KK = 4, int KX = 4>
 __device__ __forceinline__ void wide_setup_m(const PrimRec<T>& P, const PrimRec<T>& Q,
                                              T* __restrict__ c, T* __restrict__ F) {
     const T pq = P.p + Q.p;
@@ -97,15 +98,17 @@ __device__ __forceinline__ void wide_setup_m(const PrimRec<T>& P, const PrimRec<
     c[3] = wq * PQx; c[4] = wq * PQy; c[5] = wq * PQz;
     c[6] = Q.PAx; c[7] = Q.PAy; c[8] = Q.PAz;
     c[9] = -wp * PQx; c[10] = -wp * PQy; c[11] = -wp * PQz;
-    const T i2p = P.i2p, i2q = Q.i2p, rp2 = wq * P.i2p, rq2 = wp * Q.i2p, i2pq = T(0.5) * ipq;
-#pragma unroll
-    for (int k = 1; k <= 4; ++k) {
-        c[12 + k - 1] = T(k) * i2p;
-        c[16 + k - 1] = -T(k) * rp2;
-        c[20 + k - 1] = T(k) * i2q;
-        c[24 + k - 1] = -T(k) * rq2;
-        c[28 + k - 1] = T(k) * i2pq;
-    }
+    auto multiples = [](T* o, T x, int n) {
+        if (n >= 1) o[0] = x;
+        if (n >= 2) o[1] = twice(x);
+        if (n >= 3) o[2] = T(3) * x;
+        if (n >= 4) o[3] = twice(twice(x));
+    };
+    multiples(c + 12, P.i2p, KB);
+    if (KB >= 1) multiples(c + 16, -(wq * P.i2p), KB);
+    multiples(c + 20, Q.i2p, KK);
+    if (KK >= 1) multiples(c + 24, -(wp * Q.i2p), KK);
+    if (KX >= 1) multiples(c + 28, T(0.5) * ipq, KX);
 }
 
 // One synchronisation step of the VRR node program: the step's records (noff .. noff+cnt)
@@ -248,7 +251,9 @@ __device__ __forceinline__ void wide_contract(const PairRec& B, const PairRec& K
         if (lane < Lay::SB && base + lane < nmine) {
             const PrimRec<T> P = prims[B.prim_off + i / nK];
             const PrimRec<T> Q = prims[K.prim_off + i % nK];
-            wide_setup_m<L, T>(P, Q, sC + lane * kNCoef, sF + lane * (L + 1));
+            wide_setup_m<L, T, (LA + LB > 0 ? LA + LB - 1 : 0), (LC + LD > 0 ? LC + LD - 1 : 0),
+                         (LC + LD > 0 ? LA + LB : 0)>(P, Q, sC + lane * kNCoef,
+                                                      sF + lane * (L + 1));
             sC[lane * kNCoef + kZeroCoef] = T(0);
         }
         __syncwarp();
@@ -451,7 +456,7 @@ __device__ __forceinline__ void wide_write_out(const WriteArgs& a, const WriteTa
         const int id = e % G::ND, ic = (e / G::ND) % G::NC;
         const int ib = (e / (G::ND * G::NC)) % G::NB, ia = e / (G::ND * G::NC * G::NB);
         out[ia * s[0] + ib * s[1] + ic * s[2] + id * s[3]] =
-            (double)(H[__ldg(os + e)] * (sab[ia * G::NB + ib] * scd[ic * G::ND + id]));
+            widen(H[__ldg(os + e)] * (sab[ia * G::NB + ib] * scd[ic * G::ND + id]));
     }
 }
 
@@ -468,6 +473,31 @@ __global__ void __launch_bounds__(32 * kWideWarps, GS_WIDE_MINB) k_wide_write(co
     const PairRec K = a.pairs[task.ket];
     wide_quartet<LA, LB, LC, LD, T, VG, RQ>(B, K, (const PrimRec<T>*)a.prims, sm, lane);
     wide_write_out<LA, LB, LC, LD, T>(a, task, B, K, sm, lane);
+}
+
+// One output vector of the digestion: out(x) += sum_i term(x, i), x < NOUT, i < NIN, for the
+// warp.  A vector of few elements (as K_bd of (dp|ds), 3 sums of 36 terms) spreads each sum
+// over the largest power of two of lanes that fits, so that the warp does not issue NIN
+// multiply-adds for a handful of lanes: for (dp|ds) the six vectors take 40 FP64
+// instructions a quartet instead of 90, at 64 cycles of the pipe each.
+template <int NOUT, int NIN, typename T, typename Term, typename Add>
+__device__ __forceinline__ void warp_sums(int lane, Term term, Add add) {
+    constexpr int S = NOUT * 16 <= 32 && NIN >= 16 ? 16 : NOUT * 8 <= 32 && NIN >= 8 ? 8
+                      : NOUT * 4 <= 32 && NIN >= 4 ? 4 : NOUT * 2 <= 32 && NIN >= 2 ? 2 : 1;
+    const int part = lane % S;
+#pragma unroll
+    for (int x0 = 0; x0 < NOUT; x0 += 32 / S) {
+        const int x = x0 + lane / S;
+        const bool in = x < NOUT;
+        T r = T(0);
+        if (in) {
+#pragma unroll 4
+            for (int i = part; i < NIN; i += S) r = term(x, i, r);
+        }
+#pragma unroll
+        for (int o = S / 2; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        if (in && part == 0) add(x, r);
+    }
 }
 
 // J/K digestion of an evaluated quartet (HRR buffer in sm).
@@ -492,9 +522,10 @@ __device__ __forceinline__ void wide_jk_digest(const JKArgs& a, const int2& task
     T* sab = V + G::NBLK;
     T* scd = sab + NAB;
     for (int x = lane; x < NAB; x += 32)
-        sab[x] = (T)(deg * a.comp_scale[6 * B.sa + x / NB] * a.comp_scale[6 * B.sb + x % NB]);
+        sab[x] = narrow_to(T(0), deg * a.comp_scale[6 * B.sa + x / NB] *
+                                     a.comp_scale[6 * B.sb + x % NB]);
     for (int x = lane; x < NCD; x += 32)
-        scd[x] = (T)(a.comp_scale[6 * K.sa + x / ND] * a.comp_scale[6 * K.sb + x % ND]);
+        scd[x] = narrow_to(T(0), a.comp_scale[6 * K.sa + x / ND] * a.comp_scale[6 * K.sb + x % ND]);
     __syncwarp();
     const unsigned short* __restrict__ os = W::outslot();
     for (int e = lane; e < G::NBLK; e += 32) V[e] = sm[__ldg(os + e)] * (sab[e / NCD] * scd[e % NCD]);
@@ -504,55 +535,59 @@ __device__ __forceinline__ void wide_jk_digest(const JKArgs& a, const int2& task
     if (a.j) {
         const double* P = a.pj + mbase;
         double* Jo = a.j + mbase;
-        for (int ab = lane; ab < NAB; ab += 32) {
-            T r = T(0);
-            for (int cd = 0; cd < NCD; ++cd)
-                r = fma(V[ab * NCD + cd], (T)P[(fc + cd / ND) * n + fd + cd % ND], r);
-            atomicAdd(Jo + (fa + ab / NB) * n + fb + ab % NB, 2.0 * (double)r);
-        }
-        for (int cd = lane; cd < NCD; cd += 32) {
-            T r = T(0);
-            for (int ab = 0; ab < NAB; ++ab)
-                r = fma(V[ab * NCD + cd], (T)P[(fa + ab / NB) * n + fb + ab % NB], r);
-            atomicAdd(Jo + (fc + cd / ND) * n + fd + cd % ND, 2.0 * (double)r);
-        }
+        warp_sums<NAB, NCD, T>(
+            lane,
+            [&](int ab, int cd, T r) {
+                return fma(V[ab * NCD + cd], narrow_to(T(0), P[(fc + cd / ND) * n + fd + cd % ND]), r);
+            },
+            [&](int ab, T r) {
+                atomicAdd(Jo + (fa + ab / NB) * n + fb + ab % NB, widen(twice(r)));
+            });
+        warp_sums<NCD, NAB, T>(
+            lane,
+            [&](int cd, int ab, T r) {
+                return fma(V[ab * NCD + cd], narrow_to(T(0), P[(fa + ab / NB) * n + fb + ab % NB]), r);
+            },
+            [&](int cd, T r) {
+                atomicAdd(Jo + (fc + cd / ND) * n + fd + cd % ND, widen(twice(r)));
+            });
     }
     for (int s = 0; s < a.nk; ++s) {
         const double* P = a.pk + (size_t)s * a.mat_stride + mbase;
         double* Ko = a.k + (size_t)s * a.mat_stride + mbase;
         // K'_ac += sum_bd v P_bd ; K'_ad += sum_bc v P_bc ; K'_bc += sum_ad v P_ad ; K'_bd += sum_ac v P_ac
-        for (int x = lane; x < NA * NC; x += 32) {
-            const int ia = x / NC, ic = x % NC;
-            T r = T(0);
-            for (int ib = 0; ib < NB; ++ib)
-                for (int id = 0; id < ND; ++id)
-                    r = fma(V[((ia * NB + ib) * NC + ic) * ND + id], (T)P[(fb + ib) * n + fd + id], r);
-            atomicAdd(Ko + (fa + ia) * n + fc + ic, (double)r);
-        }
-        for (int x = lane; x < NA * ND; x += 32) {
-            const int ia = x / ND, id = x % ND;
-            T r = T(0);
-            for (int ib = 0; ib < NB; ++ib)
-                for (int ic = 0; ic < NC; ++ic)
-                    r = fma(V[((ia * NB + ib) * NC + ic) * ND + id], (T)P[(fb + ib) * n + fc + ic], r);
-            atomicAdd(Ko + (fa + ia) * n + fd + id, (double)r);
-        }
-        for (int x = lane; x < NB * NC; x += 32) {
-            const int ib = x / NC, ic = x % NC;
-            T r = T(0);
-            for (int ia = 0; ia < NA; ++ia)
-                for (int id = 0; id < ND; ++id)
-                    r = fma(V[((ia * NB + ib) * NC + ic) * ND + id], (T)P[(fa + ia) * n + fd + id], r);
-            atomicAdd(Ko + (fb + ib) * n + fc + ic, (double)r);
-        }
-        for (int x = lane; x < NB * ND; x += 32) {
-            const int ib = x / ND, id = x % ND;
-            T r = T(0);
-            for (int ia = 0; ia < NA; ++ia)
-                for (int ic = 0; ic < NC; ++ic)
-                    r = fma(V[((ia * NB + ib) * NC + ic) * ND + id], (T)P[(fa + ia) * n + fc + ic], r);
-            atomicAdd(Ko + (fb + ib) * n + fd + id, (double)r);
-        }
+        warp_sums<NA * NC, NB * ND, T>(
+            lane,
+            [&](int x, int i, T r) {
+                const int ia = x / NC, ic = x % NC, ib = i / ND, id = i % ND;
+                return fma(V[((ia * NB + ib) * NC + ic) * ND + id],
+                           narrow_to(T(0), P[(fb + ib) * n + fd + id]), r);
+            },
+            [&](int x, T r) { atomicAdd(Ko + (fa + x / NC) * n + fc + x % NC, widen(r)); });
+        warp_sums<NA * ND, NB * NC, T>(
+            lane,
+            [&](int x, int i, T r) {
+                const int ia = x / ND, id = x % ND, ib = i / NC, ic = i % NC;
+                return fma(V[((ia * NB + ib) * NC + ic) * ND + id],
+                           narrow_to(T(0), P[(fb + ib) * n + fc + ic]), r);
+            },
+            [&](int x, T r) { atomicAdd(Ko + (fa + x / ND) * n + fd + x % ND, widen(r)); });
+        warp_sums<NB * NC, NA * ND, T>(
+            lane,
+            [&](int x, int i, T r) {
+                const int ib = x / NC, ic = x % NC, ia = i / ND, id = i % ND;
+                return fma(V[((ia * NB + ib) * NC + ic) * ND + id],
+                           narrow_to(T(0), P[(fa + ia) * n + fd + id]), r);
+            },
+            [&](int x, T r) { atomicAdd(Ko + (fb + x / NC) * n + fc + x % NC, widen(r)); });
+        warp_sums<NB * ND, NA * NC, T>(
+            lane,
+            [&](int x, int i, T r) {
+                const int ib = x / ND, id = x % ND, ia = i / NC, ic = i % NC;
+                return fma(V[((ia * NB + ib) * NC + ic) * ND + id],
+                           narrow_to(T(0), P[(fa + ia) * n + fc + ic]), r);
+            },
+            [&](int x, T r) { atomicAdd(Ko + (fb + x / ND) * n + fd + x % ND, widen(r)); });
     }
 }
 

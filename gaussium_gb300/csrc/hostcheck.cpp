@@ -27,6 +27,26 @@ extern "C" int hc_boys(int M, int prec, double t, double* F) {
     return -1;
 }
 
+// The FP32 pair form below the asymptotic threshold (boys_pair32), its row built from the
+// FP64 grid as boys_table_gen.c builds it from long double.
+extern "C" int hc_boys_pair32(int M, double t, double* F) {
+    double fact = 1.0;
+    const float tf = (float)t, kf = std::nearbyint(tf * float(BOYS_INV_H));
+    const double* g = h_boys_d + (int)kf * BOYS_NCOL;
+    float r[8];
+    r[0] = (float)g[M];
+    r[1] = (float)(g[M] - (double)r[0]);
+    for (int j = 1; j <= 4; ++j) r[1 + j] = (float)(g[M + j] / (fact *= j));
+    r[6] = (float)g[BOYS_NCOL - 1];
+    r[7] = (float)(g[BOYS_NCOL - 1] - (double)r[6]);
+    const float d = kf * (1.0f / BOYS_INV_H) - tf;
+#define GS_B(MM) case MM: { float f[MM + 1]; boys_pair32<MM>(r, tf, d, 1.0f, f); \
+        for (int i = 0; i <= MM; ++i) F[i] = f[i]; return 0; }
+    switch (M) { GS_B(0) GS_B(1) GS_B(2) GS_B(3) GS_B(4) GS_B(5) GS_B(6) GS_B(7) GS_B(8) GS_B(9) }
+#undef GS_B
+    return -1;
+}
+
 // Canonical block of one quartet (bra, ket index into pairs); out gets NA*NB*NC*ND doubles.
 extern "C" int hc_eri_block(int la, int lb, int lc, int ld, int prec, const PairRec* pairs,
                             const void* prims, int bra, int ket, double* out) {

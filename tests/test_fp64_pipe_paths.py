@@ -1,0 +1,81 @@
+"""The paths that keep work off the FP64 pipe: the FP32 Boys function in float pairs, the
+integer conversions of the Fock digestion, and blocks of unit component scales."""
+import numpy as np
+import pytest
+import torch
+
+import hostcheck
+import oracle
+from gaussium_gb300 import autotune, engine
+from gaussium_gb300.basis import ShellBasis
+from gaussium_gb300.workloads import random_shell_quartets
+
+ASYM32 = [17, 20, 23, 25, 28, 30, 32, 34, 36, 38]
+
+
+@pytest.mark.parametrize("m", range(10))
+def test_boys_pair32_rounds_like_fp64(m):
+    """One float rounding (2^-24 relative), plus three float roundings each of the two
+    expansions' remainders, which are at most 1/32 of the leading terms: 1.25 x 2^-24."""
+    L = hostcheck.hc()
+    rng = np.random.default_rng(m)
+    t = np.concatenate([[0.0, 1 / 32, 1 / 16, 3 / 32, np.nextafter(ASYM32[m], 0)],
+                        np.exp(rng.uniform(np.log(1e-4), np.log(ASYM32[m]), 300))])
+    t = t.astype(np.float32).astype(np.float64)
+    t = t[t < ASYM32[m]]
+    F = np.zeros(m + 1)
+    for x in t:
+        assert L.hc_boys_pair32(m, float(x), F.ctypes.data) == 0
+        ex = np.array([oracle.boys_exact(k, float(x)) for k in range(m + 1)])
+        assert np.max(np.abs(F / ex - 1.0)) < 1.25 * 2.0 ** -24, x
+
+
+def _small_basis(seed, scales):
+    sb, _, _ = random_shell_quartets(3, seed=seed, box_angstrom=1.5, lmax=1)
+    cs = np.random.default_rng(seed).uniform(0.5, 2.0, (sb.nshell, 6)) if scales else \
+        np.ones((sb.nshell, 6))
+    return ShellBasis(sb.l, sb.centre, sb.prim_off, sb.expo, sb.coef, cs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", [autotune.THREAD, autotune.WARP])
+def test_component_scales(gpu_lib, form):
+    """Scaled components give the unit-scale result times the scales: J of the scaled basis
+    is s J[s P s] s of the unit one, a few roundings apart."""
+    unit, scaled = _small_basis(3, False), _small_basis(3, True)
+    s = np.concatenate([scaled.comp_scale[i, :n] for i, n in enumerate(scaled.nfunc)])
+    p = np.random.default_rng(0).standard_normal((unit.nbf, unit.nbf))
+    p = p + p.T
+    a, b = engine.JKEngine(unit, schwarz_thr=0.0), engine.JKEngine(scaled, schwarz_thr=0.0)
+    d = lambda x: torch.as_tensor(x).cuda()   # noqa: E731
+    try:
+        for cls, _, _ in a.segments:
+            if form in autotune.forms(cls, 64):
+                autotune.set_form(cls, 64, form)
+        ja, (ka,) = a.jk(d(s[:, None] * p * s), [d(s[:, None] * p * s)])
+        jb, (kb,) = b.jk(d(p), [d(p)])
+    finally:
+        autotune.reset(a.segments)
+    ss = d(np.outer(s, s))
+    for x, y in ((ja, jb), (ka, kb)):
+        assert float((x * ss - y).abs().max()) < 1e-13 * float(y.abs().max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [1.0, 1e-20, 1e-45, 0.0, 1e30])
+def test_fp32_digestion_of_any_density(gpu_lib, scale):
+    """The FP32 digestion's conversions over the floats' range, their subnormals and zero:
+    FP32 J and K are the FP64 ones to FP32 accuracy (1e-5 of the largest); among subnormals
+    each of the about 600 terms of a sum is off by the smallest float (1.4e-45) times an
+    integral of at most about 10."""
+    sb = _small_basis(5, False)
+    eng = engine.JKEngine(sb, schwarz_thr=0.0)
+    p = np.random.default_rng(1).standard_normal((sb.nbf, sb.nbf))
+    p = (p + p.T) * scale
+    p[0, :] = p[:, 0] = 0.0
+    pt = torch.as_tensor(p).cuda()
+    j64, (k64,) = eng.jk(pt, [pt], precision=64)
+    j32, (k32,) = eng.jk(pt, [pt], precision=32)
+    for x, y in ((j64, j32), (k64, k32)):
+        tol = 1e-5 * float(x.abs().max()) + 1e-41
+        assert float((x - y).abs().max()) <= tol
