@@ -15,13 +15,14 @@ import torch
 
 from . import _lib
 from .basis import ShellBasis
-from .engine import (COOP_PRIM_QUARTETS, PAIR_ORDER, PRIM_SCREEN, DeviceShells, HeavyLane, PairSet,
-                     _pc_lut, heavy_threshold, mixed_prefix, split_forms)
+from .engine import (MIXED_LANES, PAIR_ORDER, PRIM_SCREEN, SIDE_STREAMS,
+                     DeviceShells, HeavyLane, MixedWorkspace, PairSet, _pc_lut, launch_plan,
+                     mixed_plan, segment_profiles)
 from .hamiltonian import one_electron
 from .molecules import shell_basis
 
 
-class BatchedRHF:
+class BatchedRHF(MixedWorkspace):
     def __init__(self, molecules, basis="6-31G*", schwarz_thr=1e-12, device="cuda",
                  max_exp=PRIM_SCREEN):
         self.mols = molecules
@@ -108,8 +109,9 @@ class BatchedRHF:
         # (engine.split_forms)
         work = nprim[self.tasks[:, 0].long()] * nprim[self.tasks[:, 1].long()] \
             if self.ntasks else torch.zeros(0, dtype=torch.int64, device=self.dev)
-        self.heavy = [(int((work[s:e] >= heavy_threshold(cls)).sum()),
-                       int((work[s:e] >= COOP_PRIM_QUARTETS).sum())) for cls, s, e in self.segments]
+        prof = segment_profiles([c for c, _, _ in self.segments], work,
+                                [s for _, s, _ in self.segments] + [self.ntasks])
+        self.heavy, self.profiles = [h for h, _ in prof], [p for _, p in prof]
 
     def _padded_setup(self):
         B, N = len(self.sbs), self.nmax
@@ -181,7 +183,6 @@ class BatchedRHF:
     def _jk_launch(self, P, J, K, precision=64, mixed_cut=None, dmax=None, screen_thr=0.0,
                    classes=None):
         L = _lib.lib()
-        st = _lib.stream()
         lane = HeavyLane(self.dev)
         base = self.tasks.data_ptr()
         if mixed_cut is not None or screen_thr > 0:
@@ -189,31 +190,28 @@ class BatchedRHF:
             # kernel runs, FP64/FP32 by the density-weighted bound
             cut = mixed_cut if mixed_cut is not None else 0.0
             thr = screen_thr if screen_thr > 0 else 1e-300
-            need = max(L.gs_fock_jk_mixed_workspace(e - s) for _, s, e in self.segments)
-            if getattr(self, "_ws", None) is None or self._ws.numel() < need:
-                self._ws = torch.empty(int(need), dtype=torch.uint8, device=self.dev)
-            mol_dmax = None
-            for (cls, s, e), heavy in zip(self.segments, self.heavy):
-                if classes is not None and cls not in classes:
-                    continue
-                # the heavy prefix in the split form, one banded launch per precision; the
-                # bound there takes each molecule's largest |P| (at least the block value the
-                # partition uses, so no quartet is screened or demoted that the partition
-                # would keep)
-                h, launches = mixed_prefix(cls, heavy, cut)
-                for prec, form, first, count, lo, hi in launches:
-                    if mol_dmax is None:
-                        mol_dmax = torch.zeros(len(self.mol_n), dtype=torch.float64,
-                                               device=self.dev)
-                        mol_dmax.scatter_reduce_(0, self.block_mol, dmax, "amax",
-                                                 include_self=True)
+            ws, each = self.mixed_workspace(self.dev)
+            segs = [x for x in zip(self.segments, self.heavy, self.profiles)
+                    if classes is None or x[0][0] in classes]
+            # the heavy prefix in the heavy forms, banded launches per precision; the bound
+            # there takes each molecule's largest |P| (at least the block value the partition
+            # uses, so no quartet is screened or demoted that the partition would keep).  It
+            # is ready before any side stream forks.
+            plans = [mixed_plan(self, cls, s, e, heavy, prof, cut)
+                     for (cls, s, e), heavy, prof in segs]
+            mol_dmax = torch.zeros(len(self.mol_n), dtype=torch.float64, device=self.dev)
+            if any(launches for _, launches in plans):
+                mol_dmax.scatter_reduce_(0, self.block_mol, dmax, "amax", include_self=True)
+            for i, (((cls, s, e), _, _), (h, launches)) in enumerate(zip(segs, plans)):
+                for j, (prec, form, first, count, lo, hi) in enumerate(launches):
                     rc = L.gs_fock_jk_batched(
                         *cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
                         _lib.ptr(self.pairs.prims(prec)), _lib.ptr(self.ds.comp_scale),
                         _lib.ptr(self.local_fo), _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base),
                         _lib.ptr(self.mol_n), _lib.ptr(mol_dmax), self.mat_stride, count,
                         base + (s + first) * 8, _lib.ptr(P), _lib.ptr(J), 1, _lib.ptr(P),
-                        _lib.ptr(K), thr, lo, hi, lane.stream())
+                        _lib.ptr(K), thr, lo, hi,
+                        lane.stream(MIXED_LANES - 1 + j % (SIDE_STREAMS + 1 - MIXED_LANES)))
                     _lib.check(rc, f"gs_fock_jk_batched{cls}")
                 rc = L.gs_fock_jk_batched_mixed(
                     *cls, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
@@ -222,7 +220,8 @@ class BatchedRHF:
                     _lib.ptr(dmax), _lib.ptr(self.mol_shell0), _lib.ptr(self.mol_nshell),
                     _lib.ptr(self.mol_sbase), self.mat_stride, e - s - h, base + (s + h) * 8,
                     _lib.ptr(P), _lib.ptr(J), 1,
-                    _lib.ptr(P), _lib.ptr(K), thr, cut, _lib.ptr(self._ws), self._ws.numel(), st)
+                    _lib.ptr(P), _lib.ptr(K), thr, cut, ws + (i % MIXED_LANES) * each, each,
+                    lane.lane(i, MIXED_LANES))
                 _lib.check(rc, f"gs_fock_jk_batched_mixed{cls}")
             lane.join()
             return
@@ -232,24 +231,14 @@ class BatchedRHF:
             runs = [(64, mixed_cut, float("inf")), (32, 0.0, mixed_cut)]
         for prec, lo, hi in runs:
             prims = self.pairs.prims(prec)
-            plan = [(cls, s, e, split_forms(cls, prec, heavy))
-                    for (cls, s, e), heavy in zip(self.segments, self.heavy)
-                    if classes is None or cls in classes]
-            # heavy prefixes first, on side 0; then every class's rest, alternating streams
-            for heavy_pass in (True, False):
-                for i, (cls, s, e, parts) in enumerate(plan):
-                    for k, (form, first, count) in enumerate(parts):
-                        if (k == 0 and len(parts) > 1) != heavy_pass:
-                            continue
-                        m = (e - s - first) if count is None else count
-                        rc = L.gs_fock_jk_batched(
-                            *cls, prec | (form << 8), _lib.ptr(self.pairs.rec), _lib.ptr(prims),
-                            _lib.ptr(self.ds.comp_scale), _lib.ptr(self.local_fo),
-                            _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base), _lib.ptr(self.mol_n),
-                            _lib.ptr(dmax), self.mat_stride, m, base + (s + first) * 8,
-                            _lib.ptr(P), _lib.ptr(J), 1, _lib.ptr(P), _lib.ptr(K), thr, lo, hi,
-                            lane.stream() if heavy_pass else lane.alternate(i))
-                        _lib.check(rc, f"gs_fock_jk_batched{cls}")
+            for i, (cls, first, m, form, _) in enumerate(launch_plan(self, prec, "jk", classes)):
+                rc = L.gs_fock_jk_batched(
+                    *cls, prec | (form << 8), _lib.ptr(self.pairs.rec), _lib.ptr(prims),
+                    _lib.ptr(self.ds.comp_scale), _lib.ptr(self.local_fo),
+                    _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base), _lib.ptr(self.mol_n),
+                    _lib.ptr(dmax), self.mat_stride, m, base + first * 8, _lib.ptr(P),
+                    _lib.ptr(J), 1, _lib.ptr(P), _lib.ptr(K), thr, lo, hi, lane.lane(i))
+                _lib.check(rc, f"gs_fock_jk_batched{cls}")
         lane.join()
 
     def tune(self, precisions=(64, 32), reps=3):

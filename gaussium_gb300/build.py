@@ -25,10 +25,9 @@ LMAX = 2
 # momentum L <= THREAD64_MAX / THREAD32_MAX get the one-thread-per-quartet kernel
 # (csrc/eri_kernels.cuh) in FP64 / FP32, classes with L >= WIDE_PROG_MIN (FP64) or
 # L >= WIDE32_FROM (FP32) the warp-cooperative kernel (csrc/eri_wide.cuh).  Where a class
-# has both, WIDE64_MIN / WIDE32_MIN set the default and gs_set_class_variant (the
-# autotuner) can choose per class at run time.
-WIDE64_MIN = int(os.environ.get("GS_WIDE64_MIN", "3"))
-WIDE32_MIN = int(os.environ.get("GS_WIDE32_MIN", "8"))
+# has both, the engine chooses by the task list (engine.class_plan), a launch that names no
+# form takes eri_launch.cuh's default, and gs_set_class_variant (the autotuner) can choose
+# per class at run time.
 THREAD64_MAX = int(os.environ.get("GS_THREAD64_MAX", "4"))
 THREAD32_MAX = 7
 WIDE32_FROM = 0
@@ -113,14 +112,12 @@ def generate():
         # GS_BOYS_ORDER: the Boys order of this class's kernels, whose Taylor rows the unit
         # embeds (eri_common.cuh)
         code = ('#define GS_BOYS_ORDER %d\n' % L +
-                '#define GS_WIDE64_MIN %d\n#define GS_WIDE32_MIN %d\n#define GS_THREAD64_MAX %d\n'
-                '#define GS_THREAD32_MAX %d\n#define GS_WIDE_FROM %d\n#define GS_WIDE32_FROM %d\n'
+                '#define GS_THREAD64_MAX %d\n#define GS_THREAD32_MAX %d\n#define GS_WIDE_FROM %d\n#define GS_WIDE32_FROM %d\n'
                 '#include "eri_launch.cuh"\n%s'
                 'int gs_launch_%s(int kind, int prec, const void* args, cudaStream_t st) {\n'
                 '    return gs::launch_any<%d, %d, %d, %d>(kind, prec, args, st);\n}\n'
                 'int gs_variants_%s(int prec) { return gs::variants<%d, %d, %d, %d>(prec); }\n'
-                % (max(WIDE64_MIN, WIDE_PROG_MIN), max(WIDE32_MIN, WIDE_PROG_MIN), THREAD64_MAX,
-                   THREAD32_MAX, WIDE_PROG_MIN, max(WIDE32_FROM, WIDE_PROG_MIN), inc, tag, *cls,
+                % (THREAD64_MAX, THREAD32_MAX, WIDE_PROG_MIN, max(WIDE32_FROM, WIDE_PROG_MIN), inc, tag, *cls,
                    tag, *cls))
         if not os.path.exists(path) or open(path).read() != code:
             with open(path, "w") as f:

@@ -456,15 +456,15 @@ GS_HD GS_INLINE void eri_quartet(const PairRec& B, const PairRec& K,
 }
 
 // Contraction accumulators of the quartet over primitive quartets start, start + stride,
-// ... (flat index i * K.nprim + j): the lanes of a warp that shares one quartet's primitive
+// ... (flat index j * B.nprim + i, the order of eri_quartet): the lanes of a warp that shares one quartet's primitive
 // quartets each call this with their own start and stride 32, then sum the accumulators.
 template <int LA, int LB, int LC, int LD, typename T>
 GS_HD GS_INLINE void eri_accumulate(const PairRec& B, const PairRec& K,
                                     const PrimRec<T>* __restrict__ prims, T* __restrict__ acc,
                                     int start, int stride) {
-    const int nK = K.nprim, ntot = B.nprim * nK;
+    const int nB = B.nprim, ntot = nB * K.nprim;
     for (int x = start; x < ntot; x += stride)
-        eri_primitive<LA, LB, LC, LD, T>(prims[B.prim_off + x / nK], prims[K.prim_off + x % nK],
+        eri_primitive<LA, LB, LC, LD, T>(prims[B.prim_off + x % nB], prims[K.prim_off + x / nB],
                                          acc);
 }
 

@@ -237,8 +237,8 @@ __device__ __forceinline__ void wide_contract(const PairRec& B, const PairRec& K
     T* sC = sm;
     T* sF = sm + Lay::SC;
     T* node = sm + Lay::SC + Lay::SF;
-    const int nK = K.nprim;
-    const int nmine = first < B.nprim * nK ? (B.nprim * nK - first + stride - 1) / stride : 0;
+    const int nB = B.nprim, ntot = nB * K.nprim;
+    const int nmine = first < ntot ? (ntot - first + stride - 1) / stride : 0;
     // the node program: waves of at most 32 nodes (one per lane), or of 32/VG nodes for the
     // grouped form (one per lane group of VG primitive quartets)
     constexpr int NVS = Lay::NVS;
@@ -249,8 +249,9 @@ __device__ __forceinline__ void wide_contract(const PairRec& B, const PairRec& K
     for (int base = 0; base < nmine; base += Lay::SB) {
         const int i = first + (base + lane) * stride;
         if (lane < Lay::SB && base + lane < nmine) {
-            const PrimRec<T> P = prims[B.prim_off + i / nK];
-            const PrimRec<T> Q = prims[K.prim_off + i % nK];
+            const int j = i / nB;                        // bra inner, as in eri_quartet
+            const PrimRec<T> P = prims[B.prim_off + i - j * nB];
+            const PrimRec<T> Q = prims[K.prim_off + j];
             wide_setup_m<L, T, (LA + LB > 0 ? LA + LB - 1 : 0), (LC + LD > 0 ? LC + LD - 1 : 0),
                          (LC + LD > 0 ? LA + LB : 0)>(P, Q, sC + lane * kNCoef,
                                                       sF + lane * (L + 1));
@@ -735,6 +736,111 @@ __global__ void __launch_bounds__(32 * kCoopMaxWarps) k_wide_jk_coop(const JKArg
         wide_jk_digest<LA, LB, LC, LD, T>(a, task, B, K, base, lane);
 }
 
+// Cluster form for the heaviest quartets of a list that is too short to fill the GPU with one
+// block each: a cluster of kClusterBlocks cooperative blocks, on as many SMs, per quartet.
+// Warp w of block r takes primitive quartets r + kClusterBlocks w, ... (one stride over all
+// warps of the cluster); each block adds its warps' partial sums, the cluster meets at its
+// barrier, block 0 adds the blocks' sums in rank order out of their shared memory and runs
+// the HRR and the epilogue.  One block holds four FP64 pipes, and a warp-wide FP64
+// instruction takes 64 cycles of one whatever runs beside it: a (dd|dd) quartet of 500
+// primitive quartets takes 0.9 ms in one block, an eighth of that in eight.
+constexpr int kClusterBlocks = 8;                  // the portable cluster size
+
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
+                 ::: "memory");
+}
+// The element at `local` of block `rank`'s shared memory.
+__device__ __forceinline__ double cluster_load(const double* local, unsigned rank) {
+    unsigned at = (unsigned)__cvta_generic_to_shared(local), to;
+    double v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(at), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(to) : "memory");
+    return v;
+}
+__device__ __forceinline__ float cluster_load(const float* local, unsigned rank) {
+    unsigned at = (unsigned)__cvta_generic_to_shared(local), to;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(at), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(to) : "memory");
+    return v;
+}
+
+// Contract the quartet over the cluster; true in warp 0 of block 0, whose region then holds
+// the HRR buffer.  Every thread of the cluster takes part in both barriers.
+template <int LA, int LB, int LC, int LD, typename T, bool JK>
+__device__ __forceinline__ bool cluster_quartet(const PairRec& B, const PairRec& K,
+                                                const PrimRec<T>* __restrict__ prims,
+                                                T* __restrict__ base, int lane, int warp) {
+    using CL = CoopLayout<LA, LB, LC, LD, T, JK>;
+    constexpr int NACC = CL::NACC;
+    constexpr int NACCW = (NACC + 31) / 32;
+    const unsigned rank = cluster_rank();
+    T* sm = CL::region(base, warp);
+    T acc[NACCW];
+#pragma unroll
+    for (int k = 0; k < NACCW; ++k) acc[k] = T(0);
+    wide_contract<LA, LB, LC, LD, T, 1>(B, K, prims, sm, lane, (int)rank + kClusterBlocks * warp,
+                                        kClusterBlocks * CL::WARPS, acc);
+#pragma unroll
+    for (int k = 0; k < NACCW; ++k) {
+        const int t = lane + 32 * k;
+        if (t < NACC) sm[t] = acc[k];
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < NACC; t += 32 * CL::WARPS) {
+        T v = base[t];
+        for (int w = 1; w < CL::WARPS; ++w) v += CL::region(base, w)[t];
+        base[t] = v;
+    }
+    cluster_sync();                                // the blocks' sums are in place
+    if (rank == 0) {
+        for (int t = threadIdx.x; t < NACC; t += 32 * CL::WARPS) {
+            T v = base[t];
+            for (unsigned r = 1; r < (unsigned)kClusterBlocks; ++r) v += cluster_load(base + t, r);
+            base[t] = v;
+        }
+    }
+    cluster_sync();                                // and read: the other blocks may leave
+    if (rank != 0 || warp != 0) return false;
+    wide_hrr<LA, LB, LC, LD, T>(B, K, base, lane);
+    return true;
+}
+
+template <int LA, int LB, int LC, int LD, typename T>
+__global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(32 * kCoopMaxWarps)
+k_wide_write_cluster(const WriteArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T* base = reinterpret_cast<T*>(smem_raw);
+    const WriteTask task = a.tasks[blockIdx.x / kClusterBlocks];   // the grid is whole clusters
+    const PairRec B = a.pairs[task.bra];
+    const PairRec K = a.pairs[task.ket];
+    if (cluster_quartet<LA, LB, LC, LD, T, false>(B, K, (const PrimRec<T>*)a.prims, base, lane,
+                                                  warp))
+        wide_write_out<LA, LB, LC, LD, T>(a, task, B, K, base, lane);
+}
+
+template <int LA, int LB, int LC, int LD, typename T>
+__global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(32 * kCoopMaxWarps)
+k_wide_jk_cluster(const JKArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T* base = reinterpret_cast<T*>(smem_raw);
+    const int2 task = a.tasks[blockIdx.x / kClusterBlocks];
+    const PairRec B = a.pairs[task.x];
+    const PairRec K = a.pairs[task.y];
+    if (!jk_keep(a, B, K)) return;                 // uniform over the cluster
+    if (cluster_quartet<LA, LB, LC, LD, T, true>(B, K, (const PrimRec<T>*)a.prims, base, lane,
+                                                 warp))
+        wide_jk_digest<LA, LB, LC, LD, T>(a, task, B, K, base, lane);
+}
+
 // Raise a kernel's dynamic shared-memory limit once (the first launch happens before any
 // stream capture, so later launches inside a captured graph make no attribute call).
 template <auto Kernel>
@@ -800,6 +906,31 @@ int launch_wide_coop(int kind, const void* args, cudaStream_t st) {
         if (a.ntask_dev) return GS_ERR_ARG;
         if (set_smem<k_wide_jk_coop<LA, LB, LC, LD, T>>(CL::BYTES)) return GS_ERR_CUDA;
         k_wide_jk_coop<LA, LB, LC, LD, T><<<a.ntask, 32 * CL::WARPS, CL::BYTES, st>>>(a);
+    } else {
+        return GS_ERR_ARG;
+    }
+    return cudaGetLastError() == cudaSuccess ? 0 : GS_ERR_CUDA;
+}
+
+// The cluster form (host task counts only).
+template <int LA, int LB, int LC, int LD, int PREC>
+int launch_wide_cluster(int kind, const void* args, cudaStream_t st) {
+    using T = typename std::conditional<PREC == 64, double, float>::type;
+    if (kind == GS_KIND_WRITE) {
+        using CL = CoopLayout<LA, LB, LC, LD, T, false>;
+        const WriteArgs& a = *(const WriteArgs*)args;
+        if (a.ntask <= 0) return 0;
+        if (set_smem<k_wide_write_cluster<LA, LB, LC, LD, T>>(CL::BYTES)) return GS_ERR_CUDA;
+        k_wide_write_cluster<LA, LB, LC, LD, T>
+            <<<a.ntask * kClusterBlocks, 32 * CL::WARPS, CL::BYTES, st>>>(a);
+    } else if (kind == GS_KIND_JK) {
+        using CL = CoopLayout<LA, LB, LC, LD, T, true>;
+        const JKArgs& a = *(const JKArgs*)args;
+        if (a.ntask <= 0) return 0;
+        if (a.ntask_dev) return GS_ERR_ARG;
+        if (set_smem<k_wide_jk_cluster<LA, LB, LC, LD, T>>(CL::BYTES)) return GS_ERR_CUDA;
+        k_wide_jk_cluster<LA, LB, LC, LD, T>
+            <<<a.ntask * kClusterBlocks, 32 * CL::WARPS, CL::BYTES, st>>>(a);
     } else {
         return GS_ERR_ARG;
     }

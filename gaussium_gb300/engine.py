@@ -42,7 +42,7 @@ HEAVY_PRIM_QUARTETS = 32
 # sums added in shared memory before one HRR.  The class's time would otherwise have a floor at its heaviest quartet,
 # walked by one warp while the other warps of the launch have finished.
 COOP_PRIM_QUARTETS = 128
-THREAD_FORM, WARP_FORM, GROUPED_FORM, SPLIT_FORM, COOP_FORM, STACKED_FORM = 1, 2, 3, 4, 5, 6
+THREAD_FORM, WARP_FORM, GROUPED_FORM, SPLIT_FORM, COOP_FORM, STACKED_FORM, CLUSTER_FORM = range(1, 8)
 # (class, precision) pairs whose heavy quartets stay on the class's own form (set by the
 # autotuner where that measured faster)
 SPLIT_OFF = set()
@@ -89,6 +89,167 @@ def split_forms(cls, precision, heavy):
     return [(hform, 0, h), (form, h, None)]
 
 
+# ---------------------------------------------------------------------- launch plans
+# Times here are in slots of 64 cycles, what a warp-wide FP64 instruction holds its scheduler's
+# pipe for (measured: the same for one warp as for four, so a scheduler has no more FP64
+# throughput than one busy warp uses).
+WORK_LEVELS = 18          # thresholds 1, 2, 4, ... 2^17 of a work profile
+COOP_LEVEL = COOP_PRIM_QUARTETS.bit_length() - 1     # one warp alone takes fewer than that
+_LEVELS = 1 << np.arange(WORK_LEVELS, dtype=np.int64)
+MIN_LATENCY = 600.0       # slots (20 us) below which a long quartet is not worth splitting
+LATENCY_SHARE = 0.15      # of a call's whole work that one lane or warp may take alone
+
+
+def work_profile(work_desc):
+    """(sum, counts) of a segment's primitive-quartet counts, sorted in descending order:
+    counts[k] tasks have at least 2^k."""
+    w = -np.asarray(work_desc, dtype=np.int64)
+    return -int(w.sum()), np.searchsorted(w, -_LEVELS, side="right").tolist()
+
+
+def segment_profiles(cls_list, work_desc, bounds):
+    """(heavy_counts, work_profile) of every segment [bounds[i], bounds[i+1]) of a device
+    tensor of primitive-quartet counts, descending within each segment, in one transfer."""
+    dev = work_desc.device
+    rows = []
+    for cls, s, e in zip(cls_list, bounds[:-1], bounds[1:]):
+        w = work_desc[s:e]
+        lv = torch.as_tensor(np.concatenate([[heavy_threshold(cls), COOP_PRIM_QUARTETS],
+                                             _LEVELS])).to(dev, non_blocking=True)
+        rows.append(torch.cat([w.sum().view(1), torch.searchsorted(-w, -lv, right=True)]))
+    out = []
+    for r in (torch.stack(rows).tolist() if rows else []):
+        out.append(((r[1], r[2]), (r[0], r[3:])))
+    return out
+
+
+def class_sizes(cls):
+    """(accumulators of the [e0|f0] set, integrals of a block)."""
+    la, lb, lc, ld = cls
+    ne = sum((x + 1) * (x + 2) // 2 for x in range(la, la + lb + 1))
+    nf = sum((x + 1) * (x + 2) // 2 for x in range(lc, lc + ld + 1))
+    return ne * nf, int(np.prod(NCART[list(cls)]))
+
+
+def class_costs(cls, precision):
+    """Slots per primitive quartet: of a lane in a full GPU, of a lone warp of the thread form
+    (whose spills nothing hides), and of a warp of the warp forms.  The vertical recursion
+    has about 11 operations per accumulator; the set-up and Boys function about 50."""
+    n = class_sizes(cls)[0]
+    if precision == 64:
+        lane = 50 + 7.0 * n
+        return lane, lane * min(3.0, 1.5 + n / 24), 10 + 0.3 * n
+    return (100 + 12.0 * n) / 64, 30 + n * (0.5 if n <= 256 else 1.25), 10 + 0.1 * n
+
+
+def total_slots(segments, profiles, precision, kind, schedulers):
+    """Slots of a whole call on every scheduler of the GPU, all lanes busy."""
+    t = 0.0
+    for (cls, s, e), (work, _) in zip(segments, profiles):
+        per = (40 + 6 * class_sizes(cls)[1]) if kind == "jk" else (10 + 3 * class_sizes(cls)[1])
+        t += work * class_costs(cls, precision)[0] + (e - s) * per / (1 if precision == 64 else 30)
+    return t / (32 * schedulers)
+
+
+def class_plan(cls, precision, kind, n, profile, limit, built):
+    """[(form, first, count, latency)] for a class segment of n tasks sorted by descending
+    primitive-quartet count w, when no form has been chosen for the class.  Tasks of a tier
+    take at most ``limit`` slots in its form, so that no lane, warp or block walks its
+    primitive quartets while the rest of the GPU has finished; ``latency`` is the tier's
+    longest task's.  The lightest tier runs one thread per quartet where the class's
+    accumulators allow it, else one warp per quartet; heavier ones a warp (thread code, or
+    the warp forms), a block of eight warps, and a cluster of eight blocks per quartet.
+    Thresholds are powers of two (the profile's)."""
+    nacc = class_sizes(cls)[0]
+    lane, alone, warp = class_costs(cls, precision)
+    has = lambda form: bool(built & (1 << (form - 1)))   # noqa: E731
+    most = (496 if precision == 32 else 96 if cls[3] == 0 else 54) if kind == "jk" else \
+        (96 if precision == 32 else 27)
+    # (form, slots per primitive quartet, fixed slots), lightest tier first
+    tiers = []
+    if has(THREAD_FORM) and nacc <= most:
+        tiers.append((THREAD_FORM, alone, 0.0))
+        if nacc <= 27:
+            tiers.append((SPLIT_FORM, alone / 32, 10.0 * nacc))
+    if not tiers or nacc > 27:
+        for form in ((GROUPED_FORM,) if nacc <= 96 else ()) + (STACKED_FORM, WARP_FORM):
+            if has(form):
+                tiers.append((form, warp, 0.0))
+                break
+        if has(COOP_FORM):
+            tiers.append((COOP_FORM, warp / 4, 0.0))
+        if has(CLUSTER_FORM):
+            tiers.append((CLUSTER_FORM, warp / 32, 0.0))
+    if not tiers:
+        return [(0, 0, n, 0.0)]
+    counts = profile[1]
+    top = max([k for k in range(WORK_LEVELS) if counts[k]], default=0)    # w < 2^(top+1)
+    out, end = [], n
+    for i, (form, slots, fixed) in enumerate(tiers):
+        if i + 1 == len(tiers):
+            k = WORK_LEVELS
+        else:
+            k = max(1, int(np.floor(np.log2(max(2.0, limit / slots)))))
+            if form in (GROUPED_FORM, STACKED_FORM, WARP_FORM):
+                k = min(k, COOP_LEVEL)
+        first = counts[k] if k < WORK_LEVELS else 0
+        if first < end:
+            out.append((form, first, end - first, fixed + slots * 2.0 ** min(k, top + 1)))
+            end = first
+    return out[::-1]
+
+
+def launch_plan(engine_like, precision, kind, classes=None, share=1.0):
+    """[(class, first task, count, form, latency)] of one call, longest latency first: the
+    launches go to several streams, so the few long blocks run beside the rest.  Classes
+    with a chosen form (gs_set_class_variant, the autotuner) follow split_forms."""
+    e = engine_like
+    L = _lib.lib()
+    key = (precision, kind)
+    plans = e.__dict__.setdefault("_plans", {})
+    if key not in plans:
+        sch = 4 * torch.cuda.get_device_properties(e.tasks.device).multi_processor_count
+        slots = {p: total_slots(e.segments, e.profiles, p, kind, sch) for p in (64, 32)}
+        plans[key] = (slots, {})
+    slots, cached = plans[key]
+    limit = max(MIN_LATENCY, LATENCY_SHARE * share * slots[precision])
+    out = []
+    for (cls, s, t), heavy, prof in zip(e.segments, e.heavy, e.profiles):
+        if classes is not None and cls not in classes:
+            continue
+        if L.gs_class_variant(*cls, precision) or (cls, precision) in SPLIT_OFF:
+            parts = [(form, first, (t - s - first) if count is None else count,
+                      float("inf") if count is not None else 0.0)
+                     for form, first, count in split_forms(cls, precision, heavy)]
+        else:
+            if (cls, limit) not in cached:
+                cached[cls, limit] = class_plan(cls, precision, kind, t - s, prof, limit,
+                                                L.gs_class_variants(*cls, precision))
+            parts = cached[cls, limit]
+        out += [(cls, s + first, count, form, lat) for form, first, count, lat in parts if count > 0]
+    return sorted(out, key=lambda x: -x[4])
+
+
+def mixed_plan(engine_like, cls, s, t, heavy, prof, mixed_cut):
+    """mixed_prefix for a class segment whose forms were not chosen: the tiers above the
+    lightest of either precision's plan (class_plan) as banded launches over the same
+    prefix, the partitioned launch taking the rest."""
+    e = engine_like
+    L = _lib.lib()
+    if any(L.gs_class_variant(*cls, p) or (cls, p) in SPLIT_OFF for p in (64, 32)):
+        return mixed_prefix(cls, heavy, mixed_cut)
+    plans = {p: [(form, first - s, count) for c, first, count, form, _ in
+                 launch_plan(e, p, "jk", [cls], 0.5)] for p in (64, 32)}
+    h = max((first for p in plans.values() for _, first, _ in p), default=0)
+    out = []
+    for p, lo, hi in ((64, mixed_cut, float("inf")), (32, 0.0, mixed_cut)):
+        for form, first, count in plans[p]:
+            c = min(count, h - first)
+            if c > 0 and hi > 0.0:
+                out.append((p, form, first, c, lo, hi))
+    return h, out
+
+
 def mixed_prefix(cls, heavy, mixed_cut):
     """The heavy prefix of a class segment in a mixed-precision build, whose partitioned
     launch (gs_fock_jk_mixed) evaluates every quartet in the class's configured form.
@@ -112,23 +273,24 @@ def mixed_prefix(cls, heavy, mixed_cut):
     return h, out
 
 
+SIDE_STREAMS = 5
 _SIDE = {}
 
 
 class HeavyLane:
     """Side streams of a build, forked from the caller's stream before their first launch
-    and joined back by ``join``.  Side 0 takes the heavy prefixes of the classes: their few
-    long blocks then run beside the class launches instead of leaving most SMs idle while
-    they finish.  Side 1 takes every other class's launch of a plain (unpartitioned)
-    build, so that one class's last partial wave overlaps the next class's first."""
+    and joined back by ``join``.  A build's launches go round the caller's stream and the
+    sides (``lane``): the few long blocks of the heavy tiers then run beside the class
+    launches instead of leaving most SMs idle while they finish, and one class's last
+    partial wave overlaps the next class's first."""
 
     def __init__(self, device, stream=None):
         d = indexed_device(device)
         self.main = stream or torch.cuda.current_stream(d)
         if d not in _SIDE:
-            _SIDE[d] = (torch.cuda.Stream(device=d), torch.cuda.Stream(device=d))
+            _SIDE[d] = tuple(torch.cuda.Stream(device=d) for _ in range(SIDE_STREAMS))
         self.sides = _SIDE[d]
-        self.forked = [False, False]
+        self.forked = [False] * SIDE_STREAMS
 
     def stream(self, k=0):
         """Side stream k (as the C ABI takes it), forked on first use."""
@@ -137,12 +299,13 @@ class HeavyLane:
             self.forked[k] = True
         return _lib.stream(self.sides[k])
 
-    def alternate(self, i):
-        """The stream of the i-th class launch of a plain build: the caller's or side 1."""
-        return _lib.stream(self.main) if i % 2 == 0 else self.stream(1)
+    def lane(self, i, lanes=SIDE_STREAMS + 1):
+        """The stream of the i-th launch of a build over ``lanes`` streams."""
+        i %= lanes
+        return _lib.stream(self.main) if i == 0 else self.stream(i - 1)
 
     def join(self):
-        for k in (0, 1):
+        for k in range(SIDE_STREAMS):
             if self.forked[k]:
                 self.main.wait_stream(self.sides[k])
                 self.forked[k] = False
@@ -480,6 +643,7 @@ class QuartetBatch:
         self.sorted_ket_nprim = nk[order]
         work = self.sorted_bra_nprim * self.sorted_ket_nprim
         self.heavy = [heavy_counts(cls, work[s:e]) for cls, s, e in self.segments]
+        self.profiles = [work_profile(work[s:e]) for _, s, e in self.segments]
 
     def _plan_device(self, ds, quartets, want32, max_exp):
         dev = ds.device
@@ -525,19 +689,16 @@ class QuartetBatch:
         scls = cls[order]
         ws = w[order]
         nper = torch.bincount(scls, minlength=36).cpu().numpy()
-        hs = torch.zeros(36, dtype=torch.int64, device=dev).index_add_(
-            0, scls, (ws >= lut["thr"][scls]).long())
-        hc = torch.zeros(36, dtype=torch.int64, device=dev).index_add_(
-            0, scls, (ws >= COOP_PRIM_QUARTETS).long())
-        hs, hc = hs.cpu().numpy(), hc.cpu().numpy()
-        self.segments, self.heavy = [], []
+        self.segments = []
         start = 0
         for c in range(36):
             if nper[c]:
                 (la, lb), (lc, ld) = PAIR_ORDER[c // 6], PAIR_ORDER[c % 6]
                 self.segments.append(((la, lb, lc, ld), start, start + int(nper[c])))
-                self.heavy.append((int(hs[c]), int(hc[c])))
                 start += int(nper[c])
+        prof = segment_profiles([c for c, _, _ in self.segments], ws,
+                                [s for _, s, _ in self.segments] + [n])
+        self.heavy, self.profiles = [h for h, _ in prof], [p for _, p in prof]
         self._sorted_dev = (nb[order], nk[order])
 
     def __getattr__(self, name):
@@ -557,38 +718,23 @@ class QuartetBatch:
         return {cls: e - s for cls, s, e in self.segments}
 
     def launch_count(self, precision=64):
-        """Kernel launches one ``run`` makes with the current kernel forms: one per class,
-        and one more for a class whose heavy prefix runs in its own form."""
-        n = 0
-        for (cls, s, e), heavy in zip(self.segments, self.heavy):
-            for form, first, count in split_forms(cls, precision, heavy):
-                n += ((e - s - first) if count is None else count) > 0
-        return n
+        """Kernel launches one ``run`` makes with the current kernel forms: one per class
+        and tier of primitive work."""
+        return len(launch_plan(self, precision, "write"))
 
     def run(self, out, precision=64, stream=None, classes=None):
         _check_device_tensor(out, self.ds.device, "output buffer")
         if out.numel() < self.total:
             raise ValueError(f"output buffer holds {out.numel()} doubles, the blocks need {self.total}")
         L = _lib.lib()
-        st = _lib.stream(stream)
         lane = HeavyLane(self.ds.device, stream)
         base = self.tasks.data_ptr()
         prims = self.pairs.prims(precision)
-        plan = [(cls, s, e, split_forms(cls, precision, heavy))
-                for (cls, s, e), heavy in zip(self.segments, self.heavy)
-                if classes is None or cls in classes]
-        # heavy prefixes first, on side 0; then every class's rest, alternating streams
-        for heavy_pass in (True, False):
-            for i, (cls, s, e, parts) in enumerate(plan):
-                for k, (form, first, count) in enumerate(parts):
-                    if (k == 0 and len(parts) > 1) != heavy_pass:
-                        continue
-                    n = (e - s - first) if count is None else count
-                    rc = L.gs_eri_blocks(*cls, precision | (form << 8), _lib.ptr(self.pairs.rec),
-                                         _lib.ptr(prims), _lib.ptr(self.ds.comp_scale), n,
-                                         base + (s + first) * WRITE_TASK, _lib.ptr(out),
-                                         lane.stream() if heavy_pass else lane.alternate(i))
-                    _lib.check(rc, f"gs_eri_blocks{cls}")
+        for i, (cls, first, n, form, _) in enumerate(launch_plan(self, precision, "write", classes)):
+            rc = L.gs_eri_blocks(*cls, precision | (form << 8), _lib.ptr(self.pairs.rec),
+                                 _lib.ptr(prims), _lib.ptr(self.ds.comp_scale), n,
+                                 base + first * WRITE_TASK, _lib.ptr(out), lane.lane(i))
+            _lib.check(rc, f"gs_eri_blocks{cls}")
         lane.join()
         return out
 
@@ -603,7 +749,24 @@ def eri_blocks(sb: ShellBasis, quartets, precision=64, device="cuda"):
 
 
 # ---------------------------------------------------------------------- Fock (J/K) engine
-class JKEngine:
+# streams of the partitioned launches of a mixed-precision build, each with its own workspace
+# (one class's lists at a time); the heavy tiers take the remaining side streams
+MIXED_LANES = 4
+
+
+class MixedWorkspace:
+    """The partition workspace of an engine with ``segments``: one region per stream of the
+    partitioned launches."""
+
+    def mixed_workspace(self, dev):
+        need = max(_lib.lib().gs_fock_jk_mixed_workspace(e - s) for _, s, e in self.segments)
+        need = -(-int(need) // 256) * 256
+        if getattr(self, "_ws", None) is None or self._ws.numel() < MIXED_LANES * need:
+            self._ws = torch.empty(MIXED_LANES * need, dtype=torch.uint8, device=dev)
+        return self._ws.data_ptr(), need
+
+
+class JKEngine(MixedWorkspace):
     """Integral-direct Coulomb/exchange builder over all unique shell quartets of one
     basis, with Schwarz screening (task list built once per geometry) and optional
     density-weighted screening / precision selection per call."""
@@ -642,7 +805,8 @@ class JKEngine:
         nprim = torch.as_tensor(self.pairs.nprim).to(dev)
         self.segments = []
         self.heavy = []           # heavy_counts of each segment
-        chunks = []
+        self.profiles = []        # work_profile of each segment
+        chunks, work = [], []
         ntot = 0
         thr = self.schwarz_thr
         pc = torch.as_tensor(self.pair_class).to(dev)
@@ -682,13 +846,16 @@ class JKEngine:
                 t = torch.stack([bra[o], ket[o]], dim=1).to(torch.int32)
                 (la, lb), (lc, ld) = PAIR_ORDER[cb], PAIR_ORDER[ck]
                 self.segments.append(((la, lb, lc, ld), ntot, ntot + total))
-                self.heavy.append((int((key >= heavy_threshold((la, lb, lc, ld)) * 4096).sum()),
-                                   int((key >= COOP_PRIM_QUARTETS * 4096).sum())))
+                work.append(key // 4096)
                 chunks.append(t)
                 ntot += total
         self.tasks = torch.cat(chunks, 0).contiguous() if chunks else \
             torch.zeros((1, 2), dtype=torch.int32, device=dev)
         self.ntasks = ntot
+        if chunks:
+            prof = segment_profiles([c for c, _, _ in self.segments], torch.cat(work),
+                                    [s for _, s, _ in self.segments] + [ntot])
+            self.heavy, self.profiles = [h for h, _ in prof], [p for _, p in prof]
 
     def shell_dmax(self, mats):
         """max |P_ij| over each (shell, shell) block, over all given matrices."""
@@ -732,54 +899,44 @@ class JKEngine:
         else:
             thr = 0.0
         L = _lib.lib()
-        st = _lib.stream(stream)
         lane = HeavyLane(dev, stream)
         base = self.tasks.data_ptr()
         if mixed_cut is not None:
-            need = max(L.gs_fock_jk_mixed_workspace(e - s) for _, s, e in self.segments)
-            if getattr(self, "_ws", None) is None or self._ws.numel() < need:
-                self._ws = torch.empty(int(need), dtype=torch.uint8, device=dev)
-            for (cls, s, e), heavy in zip(self.segments, self.heavy):
-                if classes is not None and cls not in classes:
-                    continue
+            ws, each = self.mixed_workspace(dev)
+            segs = [x for x in zip(self.segments, self.heavy, self.profiles)
+                    if classes is None or x[0][0] in classes]
+            for i, ((cls, s, e), heavy, prof) in enumerate(segs):
                 # the heavy prefix in the heavy forms: banded launches per precision (the
                 # same density-weighted bound and cut as the partition)
-                h, launches = mixed_prefix(cls, heavy, mixed_cut)
-                for prec, form, first, count, lo, hi in launches:
+                h, launches = mixed_plan(self, cls, s, e, heavy, prof, mixed_cut)
+                for j, (prec, form, first, count, lo, hi) in enumerate(launches):
                     rc = L.gs_fock_jk(*cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
                                       _lib.ptr(self.pairs.prims(prec)),
                                       _lib.ptr(self.ds.comp_scale), _lib.ptr(self.ds.func_off),
                                       self.sb.nshell, n, count, base + (s + first) * 8,
                                       _lib.ptr(pj_c), _lib.ptr(jbuf), nk, _lib.ptr(pk_c),
-                                      _lib.ptr(kbuf), _lib.ptr(dmax), thr, lo, hi, lane.stream())
+                                      _lib.ptr(kbuf), _lib.ptr(dmax), thr, lo, hi,
+                                      lane.stream(MIXED_LANES - 1 + j % (SIDE_STREAMS + 1 - MIXED_LANES)))
                     _lib.check(rc, f"gs_fock_jk{cls}")
                 rc = L.gs_fock_jk_mixed(*cls, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
                                         _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale),
                                         _lib.ptr(self.ds.func_off), self.sb.nshell, n, e - s - h,
                                         base + (s + h) * 8, _lib.ptr(pj_c), _lib.ptr(jbuf), nk,
                                         _lib.ptr(pk_c), _lib.ptr(kbuf), _lib.ptr(dmax), thr,
-                                        mixed_cut, _lib.ptr(self._ws), self._ws.numel(), st)
+                                        mixed_cut, ws + (i % MIXED_LANES) * each, each,
+                                        lane.lane(i, MIXED_LANES))
                 _lib.check(rc, f"gs_fock_jk_mixed{cls}")
             runs = []
         for prec, lo, hi in runs:
             prims = self.pairs.prims(prec)
-            plan = [(cls, s, e, split_forms(cls, prec, heavy))
-                    for (cls, s, e), heavy in zip(self.segments, self.heavy)
-                    if classes is None or cls in classes]
-            # heavy prefixes first, on side 0; then every class's rest, alternating streams
-            for heavy_pass in (True, False):
-                for i, (cls, s, e, parts) in enumerate(plan):
-                    for k, (form, first, count) in enumerate(parts):
-                        if (k == 0 and len(parts) > 1) != heavy_pass:
-                            continue
-                        m = (e - s - first) if count is None else count
-                        rc = L.gs_fock_jk(*cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
-                                          _lib.ptr(prims), _lib.ptr(self.ds.comp_scale),
-                                          _lib.ptr(self.ds.func_off), self.sb.nshell, n, m,
-                                          base + (s + first) * 8, _lib.ptr(pj_c), _lib.ptr(jbuf),
-                                          nk, _lib.ptr(pk_c), _lib.ptr(kbuf), _lib.ptr(dmax), thr,
-                                          lo, hi, lane.stream() if heavy_pass else lane.alternate(i))
-                        _lib.check(rc, f"gs_fock_jk{cls}")
+            for i, (cls, first, m, form, _) in enumerate(launch_plan(self, prec, "jk", classes)):
+                rc = L.gs_fock_jk(*cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
+                                  _lib.ptr(prims), _lib.ptr(self.ds.comp_scale),
+                                  _lib.ptr(self.ds.func_off), self.sb.nshell, n, m,
+                                  base + first * 8, _lib.ptr(pj_c), _lib.ptr(jbuf), nk,
+                                  _lib.ptr(pk_c), _lib.ptr(kbuf), _lib.ptr(dmax), thr, lo, hi,
+                                  lane.lane(i))
+                _lib.check(rc, f"gs_fock_jk{cls}")
         lane.join()
         J = (jbuf + jbuf.T) if jbuf is not None else None
         K = [kbuf[s] + kbuf[s].T for s in range(nk)]

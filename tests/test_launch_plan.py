@@ -1,0 +1,120 @@
+"""Launch plans: the tiers of a class segment, and the cluster form they use for the heaviest
+quartets."""
+import numpy as np
+import pytest
+import torch
+
+from gaussium_gb300 import engine
+
+ALL = [(0, 0, 0, 0), (1, 0, 0, 0), (1, 1, 1, 0), (1, 1, 1, 1), (2, 0, 2, 0), (2, 1, 2, 0),
+       (2, 1, 1, 1), (2, 2, 2, 1), (2, 2, 2, 2)]
+
+
+@pytest.mark.parametrize("kind", ["jk", "write"])
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("cls", ALL)
+def test_tiers_tile_the_segment(cls, precision, kind):
+    """Whatever the work, the tiers cover [0, n) once, lightest last; only forms that are built;
+    no thread tier where the limit leaves no primitive quartet to it."""
+    rng = np.random.default_rng(sum(cls))
+    built = 0b1111111 if sum(cls) <= 5 or precision == 32 else 0b1110110
+    for n, top, limit in ((1, 1, 600.0), (7, 1296, 600.0), (5000, 40, 600.0), (5000, 1296, 1e5),
+                          (300, 0, 600.0), (4096, 200, 1.0)):
+        w = np.sort(rng.integers(0, top + 1, n))[::-1]
+        plan = engine.class_plan(cls, precision, kind, n, engine.work_profile(w), limit, built)
+        at = 0
+        for form, first, count, latency in plan:
+            assert first == at and count > 0 and latency >= 0
+            assert form == 0 or built & (1 << (form - 1))
+            at += count
+        assert at == n
+        forms = [p[0] for p in plan]
+        assert len(set(forms)) == len(forms)
+
+
+def test_segment_profiles_match_host():
+    rng = np.random.default_rng(1)
+    segs = [np.sort(rng.integers(0, t, n))[::-1] for t, n in ((1300, 500), (1, 3), (200000, 40), (9, 1))]
+    bounds = np.concatenate([[0], np.cumsum([len(x) for x in segs])]).tolist()
+    cls = [(0, 0, 0, 0), (1, 1, 1, 1), (2, 2, 2, 2), (2, 0, 0, 0)]
+    got = engine.segment_profiles(cls, torch.as_tensor(np.concatenate(segs).copy()), bounds)
+    for c, w, (heavy, prof) in zip(cls, segs, got):
+        assert heavy == engine.heavy_counts(c, w)
+        assert prof == engine.work_profile(w)
+
+
+def test_mixed_plan_bands(monkeypatch):
+    """Both precisions' heavy tiers cover the same prefix, FP64 at or above the cut and FP32
+    below it; without a cut (screening only) there is no FP32 band."""
+    plans = {64: [((2, 2, 2, 2), 10, 2, 7, 9.0), ((2, 2, 2, 2), 12, 5, 5, 5.0), ((2, 2, 2, 2), 17, 83, 6, 1.0)],
+             32: [((2, 2, 2, 2), 10, 3, 5, 2.0), ((2, 2, 2, 2), 13, 87, 1, 1.0)]}
+
+    class Stub:
+        def gs_class_variant(self, *a):
+            return 0
+    monkeypatch.setattr(engine._lib, "lib", lambda: Stub())
+    monkeypatch.setattr(engine, "launch_plan", lambda e, p, *a: plans[p])
+    inf = float("inf")
+    h, out = engine.mixed_plan(None, (2, 2, 2, 2), 10, 100, None, None, 1e-3)
+    assert h == 7 and out == [(64, 7, 0, 2, 1e-3, inf), (64, 5, 2, 5, 1e-3, inf),
+                              (32, 5, 0, 3, 0.0, 1e-3), (32, 1, 3, 4, 0.0, 1e-3)]
+    h, out = engine.mixed_plan(None, (2, 2, 2, 2), 10, 100, None, None, 0.0)
+    assert h == 7 and [x[0] for x in out] == [64, 64]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,tol", [(64, 1e-13), (32, 1e-5)])
+def test_cluster_form_matches_warp_form(gpu_lib, precision, tol):
+    """Blocks and J/K of every class built with the cluster form, for quartets of one to 1,296
+    primitive quartets (fewer than, and not a multiple of, the cluster's 64 warps)."""
+    from gaussium_gb300 import _lib, build
+    from gaussium_gb300.basis import ShellBasis
+    rng = np.random.default_rng(0)
+    shells = []
+    for l in range(3):
+        for k in (1, 2, 6):
+            shells.append(dict(l=l, centre=rng.uniform(-1, 1, 3), expo=np.exp(rng.uniform(-2, 3, k)),
+                               coef=rng.uniform(0.2, 1.0, k)))
+    sb = ShellBasis.from_shell_dicts(shells)
+    eng = engine.JKEngine(sb, schwarz_thr=0.0, max_exp=0.0)
+    p = rng.standard_normal((sb.nbf, sb.nbf))
+    pt = torch.as_tensor(p + p.T).cuda()
+    n = sb.nbf
+    seen = 0
+    for cls, s, e in eng.segments:
+        if not gpu_lib.gs_class_variants(*cls, precision) & 64:
+            continue
+        seen += 1
+        got = {}
+        for form in (engine.WARP_FORM, engine.CLUSTER_FORM):
+            j = torch.zeros((n, n), dtype=torch.float64, device="cuda")
+            k = torch.zeros_like(j)
+            rc = gpu_lib.gs_fock_jk(
+                *cls, precision | (form << 8), _lib.ptr(eng.pairs.rec),
+                _lib.ptr(eng.pairs.prims(precision)), _lib.ptr(eng.ds.comp_scale),
+                _lib.ptr(eng.ds.func_off), sb.nshell, n, e - s, eng.tasks.data_ptr() + 8 * s,
+                _lib.ptr(pt), _lib.ptr(j), 1, _lib.ptr(pt), _lib.ptr(k), None, 0.0, 0.0, 0.0,
+                _lib.stream())
+            _lib.check(rc, "gs_fock_jk")
+            got[form] = (j, k)
+        for x, y in zip(got[engine.WARP_FORM], got[engine.CLUSTER_FORM]):
+            assert float((x - y).abs().max()) <= tol * float(x.abs().max()), cls
+    assert seen == len([c for c in build.classes() if sum(c) >= 3])
+    # the same quartets as blocks, the heavy ones through the plan's cluster tier
+    tri = np.array([[a, b, c, d] for a in range(9) for b in range(a + 1) for c in range(9)
+                    for d in range(c + 1)])
+    batch = engine.QuartetBatch(eng.ds, tri, want32=precision == 32)
+    plan = engine.launch_plan(batch, precision, "write")
+    assert any(form == engine.CLUSTER_FORM for _, _, _, form, _ in plan)
+    out = torch.full((batch.total,), float("nan"), dtype=torch.float64, device="cuda")
+    batch.run(out, precision)
+    from gaussium_gb300 import autotune
+    ref = torch.full_like(out, float("nan"))
+    try:
+        for cls, _, _ in batch.segments:
+            autotune.set_form(cls, precision, autotune.WARP)
+            engine.SPLIT_OFF.add((cls, precision))
+        batch.run(ref, precision)
+    finally:
+        autotune.reset(batch.segments)
+    assert float((out - ref).abs().max()) <= tol * float(ref.abs().max())
