@@ -56,6 +56,10 @@ _SIGS = {
     "gs_spin_expand": (I, [P, I, I, P, P]),
     "gs_spin_expand_max_orbitals": (I, []),
     "gs_basis_on_grid": (I, [P, P, P, P, P, P, P, I, I, ctypes.c_longlong, P, P, P]),
+    "gs_xc_lda_max_functions": (I, []),
+    "gs_xc_lda_workspace": (ctypes.c_longlong, [ctypes.c_longlong, I]),
+    "gs_xc_lda": (I, [ctypes.c_longlong, I, P, P, P, D, I, D, D, D, D, P, P, P, ctypes.c_longlong,
+                      P]),
     "gs_lda_xc": (I, [ctypes.c_longlong, P, P, D, I, D, D, D, D, P, P, P]),
     "gs_symmetry_zero": (I, [I, I, P, P, P, P, P, P]),
     "gs_dense_expand": (I, [ctypes.c_longlong, P, P, P, P, P, I, P, P]),

@@ -16,9 +16,9 @@ function by function at each point.  Here the quadrature is a fixed grid built o
 
 The grid is centred where the reference centres it, the origin (``centre`` moves it).
 Per evaluation: basis values on the grid (``gs_basis_on_grid``, cached across SCF
-iterations), rho = diag(Phi P Phi^T) (one GEMM), the functionals per point
-(``gs_lda_xc``), V = Phi^T diag(w v) Phi (one GEMM) and E = sum w rho eps.  The GEMMs are
-cuBLAS through torch.matmul.
+iterations), rho = diag(Phi P Phi^T), the functionals per point, V = Phi^T diag(w v) Phi and
+E = sum w rho eps (``gs_xc_lda``).  Above ``gs_xc_lda_max_functions`` functions the two
+contractions are cuBLAS GEMMs through torch.matmul with ``gs_lda_xc`` between them.
 """
 import numpy as np
 import torch
@@ -128,6 +128,24 @@ class ExchangeCorrelationGPU:
     def evaluate_device(self, p):
         """(V_xc matrix, E_xc) for a device density matrix."""
         phi = self.phi()
+        n = self.sb.nbf
+        L = _lib.lib()
+        if isinstance(p, torch.Tensor) and p.shape == (n, n) and p.dtype == torch.float64 and \
+                p.device == phi.device and 0 < n <= L.gs_xc_lda_max_functions():
+            # the library's build (half the multiply-adds of the two GEMMs); a larger basis,
+            # whose tiles exceed the shared memory, and anything torch would refuse go below
+            p = p.detach().contiguous()
+            npts = phi.shape[0]
+            need = L.gs_xc_lda_workspace(npts, n)
+            ws = torch.empty(need, dtype=torch.uint8, device=self.device)
+            v = torch.empty((n, n), dtype=torch.float64, device=self.device)
+            e = torch.empty((), dtype=torch.float64, device=self.device)
+            a, x0, b, c = self.vwn if self.vwn is not None else (0.0, 0.0, 0.0, 1.0)
+            _lib.check(L.gs_xc_lda(npts, n, _lib.ptr(phi), _lib.ptr(p), _lib.ptr(self.weights),
+                                   self.alpha, int(self.vwn is not None), a, x0, b, c,
+                                   _lib.ptr(v), _lib.ptr(e), _lib.ptr(ws), need, _lib.stream()),
+                       "gs_xc_lda")
+            return v, e
         rho = ((phi @ p) * phi).sum(dim=1).contiguous()
         wv, we = self.functionals(rho, self.weights)
         v = phi.transpose(0, 1) @ (phi * wv[:, None])

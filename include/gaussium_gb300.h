@@ -356,6 +356,20 @@ int gs_lda_xc(long long npts, const double* rho, const double* weights, double s
               int vwn, double vwn_a, double vwn_x0, double vwn_b, double vwn_c,
               double* weighted_potential, double* weighted_energy, void* stream);
 
+/* A whole exchange-correlation build (ExchangeCorrelation.integrate_potential for every (i, j)
+ * and integrate_energy, kohnsham/integration.py:14-40) for one density: basis values phi
+ * (npts x nbf, row-major, device), density (nbf x nbf; its symmetric part counts) and
+ * quadrature weights to the symmetric matrix phi^T diag(w v) phi and the energy sum w rho eps,
+ * the functionals as in gs_lda_xc.  Sums run in a fixed order: the same inputs give the same
+ * bits.  workspace: gs_xc_lda_workspace(npts, nbf) bytes on the device, 16-byte aligned (0: npts
+ * or nbf out of range).  At most gs_xc_lda_max_functions functions, else GS_ERR_LIMIT. */
+int gs_xc_lda_max_functions(void);
+long long gs_xc_lda_workspace(long long npts, int nbf);
+int gs_xc_lda(long long npts, int nbf, const double* phi, const double* density,
+              const double* weights, double slater_alpha, int vwn, double vwn_a, double vwn_x0,
+              double vwn_b, double vwn_c, double* matrix, double* energy, void* workspace,
+              long long ws_bytes, void* stream);
+
 /* Point-group zero screening of a dense n^4 tensor (row-major, device), in place: every
  * element Symmetry.none_zero_integral (common/symmetry.py:18-47) declares zero is set to
  * 0.  Tables of a non-C1 group with nops operations besides the identity:
