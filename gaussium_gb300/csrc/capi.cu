@@ -49,13 +49,14 @@ inline int pv(int la, int lb, int lc, int ld, int prec) {
 
 // The precision argument of the launch entry points: 64 or 32, optionally with an explicit
 // kernel form in bits 8.. (1 thread, 2 warp, 3 grouped warp, 4 split, 5 cooperative, 6
-// stacked, 7 cluster; 0 = the class's configured form).  Returns the launcher's precision-and-form word, or -1 if invalid or not built.
+// stacked, 7 cluster; 0 = the class's configured form) and, in bits 16.., the tasks a warp of
+// the warp forms takes (up to 8; 0 = one).  Returns the launcher's precision-and-form word, or -1 if invalid or not built.
 int decode_precision(int la, int lb, int lc, int ld, int precision) {
-    const int prec = precision & 0xff, form = precision >> 8;
-    if ((prec != 64 && prec != 32) || form < 0 || form > 7) return -1;
-    if (form == 0) return pv(la, lb, lc, ld, prec);
+    const int prec = precision & 0xff, form = (precision >> 8) & 0xff, per = precision >> 16;
+    if ((prec != 64 && prec != 32) || form > 7 || per < 0 || per > 8) return -1;
+    if (form == 0) return pv(la, lb, lc, ld, prec) | (per << 16);
     if (!(find_variants(la, lb, lc, ld, prec) & (1 << (form - 1)))) return -1;
-    return prec | (form << 8);
+    return prec | (form << 8) | (per << 16);
 }
 
 inline cudaStream_t S(void* s) { return (cudaStream_t)s; }

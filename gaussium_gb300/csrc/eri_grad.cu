@@ -45,7 +45,9 @@ extern "C" int gs_eri_grad_band(int la, int lb, int lc, int ld, int form, int pr
                                 const int* tasks, int nbf, int natom, const double* density,
                                 int nshell, const double* shell_dmax, double screen_thr,
                                 double prec_lo, double prec_hi, double* grad, void* stream) {
-    if (ntask < 0 || nbf <= 0 || natom <= 0 || !pair_rec || !prim || !comp_scale || !func_off ||
+    const int per = form >> 8;
+    if (form >= 0) form &= 0xff;
+    if (per > 8 || ntask < 0 || nbf <= 0 || natom <= 0 || !pair_rec || !prim || !comp_scale || !func_off ||
         !shell_atom || (ntask > 0 && !tasks) || !density || !grad || form < 0 || form > 3 ||
         (precision != 64 && precision != 32) || (screen_thr > 0 && (!shell_dmax || nshell <= 0)))
         return GS_ERR_ARG;
@@ -75,6 +77,7 @@ extern "C" int gs_eri_grad_band(int la, int lb, int lc, int ld, int form, int pr
     a.screen_thr = screen_thr;
     a.prec_lo = prec_lo;
     a.prec_hi = prec_hi;
+    a.per = per;
     cudaStream_t st = (cudaStream_t)stream;
 #define GS_GL(A, B, C, D) \
     if (la == A && lb == B && lc == C && ld == D) return gs_grad_launch_##A##B##C##D(a, form, st);

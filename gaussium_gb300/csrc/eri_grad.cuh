@@ -35,6 +35,7 @@ struct GradArgs {
     const double* shell_dmax;
     int nshell;
     double screen_thr, prec_lo, prec_hi;
+    int per;                        // tasks a warp of the warp form takes
 };
 
 __device__ __forceinline__ bool grad_keep(const GradArgs& a, const PairRec& B, const PairRec& K) {
@@ -42,12 +43,12 @@ __device__ __forceinline__ bool grad_keep(const GradArgs& a, const PairRec& B, c
     const int ns = a.nshell;
     const double* d = a.shell_dmax;
     double dm = d[B.sa * ns + B.sb];
-    dm = fmax(dm, d[K.sa * ns + K.sb]);
-    dm = fmax(dm, d[B.sa * ns + K.sa]);
-    dm = fmax(dm, d[B.sa * ns + K.sb]);
-    dm = fmax(dm, d[B.sb * ns + K.sa]);
-    dm = fmax(dm, d[B.sb * ns + K.sb]);
-    const double est = (double)B.qmax * (double)K.qmax * dm;
+    dm = max_nonneg(dm, d[K.sa * ns + K.sb]);
+    dm = max_nonneg(dm, d[B.sa * ns + K.sa]);
+    dm = max_nonneg(dm, d[B.sa * ns + K.sb]);
+    dm = max_nonneg(dm, d[B.sb * ns + K.sa]);
+    dm = max_nonneg(dm, d[B.sb * ns + K.sb]);
+    const double est = widen(B.qmax) * widen(K.qmax) * dm;
     return !(est < a.screen_thr || est < a.prec_lo || est >= a.prec_hi);
 }
 
@@ -70,160 +71,104 @@ template <int LA, int LB, int LC, int LD> struct GradLayout {
     static constexpr int SC = kSetupBatch * kNCoefG;
     static constexpr int SF = kSetupBatch * (W::L + 1);
     static constexpr int VRR = ACC + SC + SF + W::NVSLOT;
-    static constexpr int WARP = VRR > W::HSIZE ? VRR : W::HSIZE;
+    // several quartets a warp: the set-up buffers outlive a quartet's HRR, which takes the
+    // node buffer's place
+    static constexpr int MANY = SC + SF + (W::NVSLOT > W::HSIZE ? W::NVSLOT : W::HSIZE);
+    static constexpr int WARP = !SMEM_ACC ? MANY : VRR > W::HSIZE ? VRR : W::HSIZE;
     // two warps per block while they fit the 227 KB a block may use, else one
     static constexpr int WARPS = (size_t)WARP * sizeof(double) * kGradWarps <= 227 * 1024 ? kGradWarps : 1;
     static constexpr size_t BYTES = (size_t)WARP * sizeof(double) * WARPS;
     static_assert((size_t)WARP * sizeof(double) <= 227 * 1024, "gradient class buffer exceeds shared memory");
 };
 
-__device__ __forceinline__ int g_ncart(int l) { return (l + 1) * (l + 2) / 2; }
-
-__device__ __forceinline__ void g_comp(int l, int k, int& x, int& y, int& z) {
-    if (l == 0) { x = y = z = 0; return; }
-    if (l == 1) { x = k == 0; y = k == 1; z = k == 2; return; }
-    if (l == 2) {
-        const int t[6][3] = {{2, 0, 0}, {0, 2, 0}, {0, 0, 2}, {1, 1, 0}, {1, 0, 1}, {0, 1, 1}};
-        x = t[k][0]; y = t[k][1]; z = t[k][2]; return;
-    }
-    int c = 0;
-    for (int lx = l; lx >= 0; --lx)
-        for (int ly = l - lx; ly >= 0; --ly) {
-            if (c == k) { x = lx; y = ly; z = l - lx - ly; return; }
-            ++c;
-        }
-}
-
-__device__ __forceinline__ int g_index(int x, int y, int z) {
-    const int l = x + y + z;
-    if (l == 0) return 0;
-    if (l == 1) return x ? 0 : (y ? 1 : 2);
-    if (l == 2) {
-        if (x == 2) return 0;
-        if (y == 2) return 1;
-        if (z == 2) return 2;
-        if (x && y) return 3;
-        if (x && z) return 4;
-        return 5;
-    }
-    int c = 0;
-    for (int lx = l; lx >= 0; --lx)
-        for (int ly = l - lx; ly >= 0; --ly) {
-            if (lx == x && ly == y) return c;
-            ++c;
-        }
-    return -1;
-}
-
+// VRR of the set-up primitive quartets j0 .. j0 + nb and their weighted accumulation: target
+// lane + 32 k is added to acc[k] (slot | kind << 16 in ent[k], kind 255: none), or to the
+// shared accumulators at their HRR positions, which fill [0, NACC).
 template <int LA, int LB, int LC, int LD>
-__global__ void __launch_bounds__(32 * kGradWarps) k_eri_grad(const GradArgs a) {
+__device__ __forceinline__ void grad_items(const double* __restrict__ sC,
+                                           const double* __restrict__ sF, double* node, int j0,
+                                           int nb, int lane, double* acc, const unsigned* ent,
+                                           double* shared_acc) {
     using W = GradProg<LA, LB, LC, LD>;
     using Lay = GradLayout<LA, LB, LC, LD>;
     constexpr int L = W::L;
-    constexpr bool SMEM_ACC = Lay::SMEM_ACC;
-    constexpr int NACCW = SMEM_ACC ? 1 : (W::NACC + 31) / 32;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double* sm = reinterpret_cast<double*>(smem_raw) + (size_t)warp * Lay::WARP;
-    const int t = blockIdx.x * Lay::WARPS + warp;
-    if (t >= a.ntask) return;
-    const int2 task = a.tasks[t];
-    const PairRec B = a.pairs[task.x];
-    const PairRec K = a.pairs[task.y];
-    if (!grad_keep(a, B, K)) return;               // warp-uniform
-    double acc[NACCW];
-    int accs[NACCW], acck[NACCW];
-#pragma unroll
-    for (int k = 0; k < NACCW; ++k) {
-        acc[k] = 0.0;
-        const int q = lane + 32 * k;
-        const unsigned e = q < W::NACC ? __ldg(W::acc() + q) : 0u;
-        accs[k] = e & 0xffff;
-        acck[k] = q < W::NACC ? (int)(e >> 16) : -1;
-    }
-    if constexpr (SMEM_ACC) {
-        // accumulators at their HRR positions H[accpos[q]], which fill [0, NACC)
-        for (int q = lane; q < W::NACC; q += 32) sm[q] = 0.0;
-    }
-    double* sC = sm + Lay::ACC;
-    double* sF = sC + Lay::SC;
-    double* node = sF + Lay::SF;
-    const int nK = K.nprim;
-    const int ntot = B.nprim * nK;
+    constexpr int NACCW = Lay::SMEM_ACC ? 1 : (W::NACC + 31) / 32;
     const uint4* __restrict__ vrec = W::vrec();
     const int* __restrict__ vseg = W::vseg();
-    for (int base = 0; base < ntot; base += kSetupBatch) {
-        const int i = base + lane;
-        if (lane < kSetupBatch && i < ntot) {
-            const PrimRec<double> P = a.prims[B.prim_off + i / nK];
-            const PrimRec<double> Q = a.prims[K.prim_off + i % nK];
-            double* c = sC + lane * kNCoefG;
-            wide_setup_m<L, double>(P, Q, c, sF + lane * (L + 1));
-            c[32] = 2.0 * P.pad;               // 2 alpha (first bra shell)
-            c[33] = 2.0 * (P.p - P.pad);       // 2 beta
-            c[34] = 2.0 * Q.pad;               // 2 gamma (first ket shell)
-            c[35] = 5.0 * c[28];               // 5/(2(p+q)), raised (dd|..) classes
+    for (int j = j0; j < j0 + nb; ++j) {
+        const double* __restrict__ c = sC + j * kNCoefG;
+        if (lane <= L) node[lane] = sF[j * (L + 1) + lane];
+        __syncwarp();
+        for (int s = 0; s < W::NVSEG; ++s) {
+            const int noff = __ldg(vseg + 4 * s), cnt = __ldg(vseg + 4 * s + 1);
+            const int nt = __ldg(vseg + 4 * s + 2), sync = __ldg(vseg + 4 * s + 3);
+            if (sync && s > 0) __syncwarp();
+            int n = lane;
+            uint4 ra = make_uint4(0, 0, 0, 0), rb = ra;
+            if (n < cnt) {
+                ra = __ldg(vrec + 2 * (noff + n));
+                rb = __ldg(vrec + 2 * (noff + n) + 1);
+            }
+            for (; n < cnt; n += 32) {
+                const uint4 x = ra, y = rb;
+                if (n + 32 < cnt) {
+                    ra = __ldg(vrec + 2 * (noff + n + 32));
+                    rb = __ldg(vrec + 2 * (noff + n + 32) + 1);
+                }
+                double r = c[x.y >> 16] * node[x.y & 0xffff];
+                r = fma(c[x.z >> 16], node[x.z & 0xffff], r);
+                if (nt > 2) r = fma(c[x.w >> 16], node[x.w & 0xffff], r);
+                if (nt > 3) r = fma(c[y.x >> 16], node[y.x & 0xffff], r);
+                if (nt > 4) r = fma(c[y.y >> 16], node[y.y & 0xffff], r);
+                node[x.x & 0xffff] = r;
+            }
         }
         __syncwarp();
-        const int nb = min(kSetupBatch, ntot - base);
-        for (int j = 0; j < nb; ++j) {
-            const double* __restrict__ c = sC + j * kNCoefG;
-            if (lane <= L) node[lane] = sF[j * (L + 1) + lane];
-            __syncwarp();
-            for (int s = 0; s < W::NVSEG; ++s) {
-                const int noff = __ldg(vseg + 4 * s), cnt = __ldg(vseg + 4 * s + 1);
-                const int nt = __ldg(vseg + 4 * s + 2), sync = __ldg(vseg + 4 * s + 3);
-                if (sync && s > 0) __syncwarp();
-                int n = lane;
-                uint4 ra = make_uint4(0, 0, 0, 0), rb = ra;
-                if (n < cnt) {
-                    ra = __ldg(vrec + 2 * (noff + n));
-                    rb = __ldg(vrec + 2 * (noff + n) + 1);
-                }
-                for (; n < cnt; n += 32) {
-                    const uint4 x = ra, y = rb;
-                    if (n + 32 < cnt) {
-                        ra = __ldg(vrec + 2 * (noff + n + 32));
-                        rb = __ldg(vrec + 2 * (noff + n + 32) + 1);
-                    }
-                    double r = c[x.y >> 16] * node[x.y & 0xffff];
-                    r = fma(c[x.z >> 16], node[x.z & 0xffff], r);
-                    if (nt > 2) r = fma(c[x.w >> 16], node[x.w & 0xffff], r);
-                    if (nt > 3) r = fma(c[y.x >> 16], node[y.x & 0xffff], r);
-                    if (nt > 4) r = fma(c[y.y >> 16], node[y.y & 0xffff], r);
-                    node[x.x & 0xffff] = r;
-                }
+        if constexpr (Lay::SMEM_ACC) {
+            for (int q = lane; q < W::NACC; q += 32) {
+                const unsigned e = __ldg(W::acc() + q);
+                const int kind = (int)(e >> 16);
+                const double w = kind == 0 ? 1.0 : c[31 + kind];
+                const int pos = __ldg(W::accpos() + q);
+                shared_acc[pos] = fma(w, node[e & 0xffff], shared_acc[pos]);
             }
-            __syncwarp();
-            if constexpr (SMEM_ACC) {
-                for (int q = lane; q < W::NACC; q += 32) {
-                    const unsigned e = __ldg(W::acc() + q);
-                    const int kind = (int)(e >> 16);
+        } else {
+#pragma unroll
+            for (int k = 0; k < NACCW; ++k) {
+                const unsigned kind = ent[k] >> 16;
+                if (kind != 255u) {
                     const double w = kind == 0 ? 1.0 : c[31 + kind];
-                    const int pos = __ldg(W::accpos() + q);
-                    sm[pos] = fma(w, node[e & 0xffff], sm[pos]);
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < NACCW; ++k) {
-                    if (acck[k] >= 0) {
-                        const double w = acck[k] == 0 ? 1.0 : c[31 + acck[k]];
-                        acc[k] = fma(w, node[accs[k]], acc[k]);
-                    }
+                    acc[k] = fma(w, node[ent[k] & 0xffff], acc[k]);
                 }
             }
-            __syncwarp();
         }
+        __syncwarp();
     }
-    double* H = sm;
-    if constexpr (!SMEM_ACC) {
-#pragma unroll
-        for (int k = 0; k < NACCW; ++k) {
-            const int q = lane + 32 * k;
-            if (q < W::NACC) H[__ldg(W::accpos() + q)] = acc[k];
-        }
-    }
-    __syncwarp();
+}
+
+// Set-up of the primitive quartet (P, Q) into slot x of a round.
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ void grad_setup_slot(const PrimRec<double>& P, const PrimRec<double>& Q,
+                                                double* __restrict__ sC, double* __restrict__ sF,
+                                                int x) {
+    constexpr int L = GradProg<LA, LB, LC, LD>::L;
+    double* c = sC + x * kNCoefG;
+    wide_setup_m<L, double>(P, Q, c, sF + x * (L + 1));
+    c[32] = twice(P.pad);               // 2 alpha (first bra shell)
+    c[33] = twice(P.p - P.pad);         // 2 beta
+    c[34] = twice(Q.pad);               // 2 gamma (first ket shell)
+    c[35] = 5.0 * c[28];                // 5/(2(p+q)), raised (dd|..) classes
+}
+
+// HRR of the accumulators at H, contraction with the density weights and the atomic adds.
+// The raised and lowered slots of every (element, centre, direction) come from the class's
+// table (gen_grad.contraction_table): worked out in the kernel they were 90,000 instructions
+// for one (dd|dd) quartet.  The nine sums over the lanes are reduced by halves (14 FP64
+// additions instead of 45), which leaves each in its own lanes for the atomics.
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ void grad_tail(const GradArgs& a, const int2& task, const PairRec& B,
+                                          const PairRec& K, double* H, int lane) {
+    using W = GradProg<LA, LB, LC, LD>;
     const unsigned int* __restrict__ hop = W::hop();
     const int* __restrict__ hlev = W::hlev();
     const double dv0 = B.ABx, dv1 = B.ABy, dv2 = B.ABz, dv3 = K.ABx, dv4 = K.ABy, dv5 = K.ABz;
@@ -237,64 +182,172 @@ __global__ void __launch_bounds__(32 * kGradWarps) k_eri_grad(const GradArgs a) 
         }
         __syncwarp();
     }
-    // contraction with the density weights
-    const int sh[4] = {B.sa, B.sb, K.sa, K.sb};
-    const int ls[4] = {LA, LB, LC, LD};
-    const int n[4] = {g_ncart(LA), g_ncart(LB), g_ncart(LC), g_ncart(LD)};
-    const int fo[4] = {a.func_off[B.sa], a.func_off[B.sb], a.func_off[K.sa], a.func_off[K.sb]};
+    constexpr int NB = (LB + 1) * (LB + 2) / 2, NC = (LC + 1) * (LC + 2) / 2;
+    constexpr int ND = (LD + 1) * (LD + 2) / 2, NBLK = (LA + 1) * (LA + 2) / 2 * NB * NC * ND;
+    const int fa = a.func_off[B.sa], fb = a.func_off[B.sb];
+    const int fc = a.func_off[K.sa], fd = a.func_off[K.sb];
     double w = 8.0;
     if (B.sa == B.sb) w *= 0.5;
     if (K.sa == K.sb) w *= 0.5;
     if (task.x == task.y) w *= 0.5;
     const int nbf = a.nbf;
-    const double* Pm = a.P;
-    const unsigned short* __restrict__ out = W::out();
+    const double* __restrict__ Pm = a.P;
+    const double* __restrict__ cs = a.comp_scale;
+    const unsigned* __restrict__ con = W::con();
     double g[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) g[k] = 0.0;
-    const int nblk = n[0] * n[1] * n[2] * n[3];
-    for (int e = lane; e < nblk; e += 32) {
-        int idx[4] = {e / (n[1] * n[2] * n[3]), (e / (n[2] * n[3])) % n[1], (e / n[3]) % n[2], e % n[3]};
-        const int pa = fo[0] + idx[0], pb = fo[1] + idx[1], pc = fo[2] + idx[2], pd = fo[3] + idx[3];
+    for (int e = lane; e < NBLK; e += 32) {
+        const int ia = e / (NB * NC * ND), ib = e / (NC * ND) % NB, ic = e / ND % NC, id = e % ND;
+        const int pa = fa + ia, pb = fb + ib, pc = fc + ic, pd = fd + id;
         const double gam = w * (0.5 * Pm[pa * nbf + pb] * Pm[pc * nbf + pd] -
                                 0.125 * (Pm[pa * nbf + pc] * Pm[pb * nbf + pd] +
                                          Pm[pa * nbf + pd] * Pm[pb * nbf + pc]));
         // the HRR blocks are unscaled: the element carries the component scales of all four
         // functions (not 1 for the xy, xz, yz components of a d shell)
-        const double s = gam * a.comp_scale[6 * sh[0] + idx[0]] * a.comp_scale[6 * sh[1] + idx[1]] *
-                         a.comp_scale[6 * sh[2] + idx[2]] * a.comp_scale[6 * sh[3] + idx[3]];
-        for (int cen = 0; cen < 3; ++cen) {
-            int ex[3];
-            g_comp(ls[cen], idx[cen], ex[0], ex[1], ex[2]);
-            for (int x = 0; x < 3; ++x) {
-                int up[3] = {ex[0], ex[1], ex[2]};
-                up[x] += 1;
-                int ii[4] = {idx[0], idx[1], idx[2], idx[3]};
-                int nn[4] = {n[0], n[1], n[2], n[3]};
-                ii[cen] = g_index(up[0], up[1], up[2]);
-                nn[cen] = g_ncart(ls[cen] + 1);
-                double v = H[out[__ldg(W::out_off() + cen) + ((ii[0] * nn[1] + ii[1]) * nn[2] + ii[2]) * nn[3] + ii[3]]];
-                if (ex[x] > 0) {
-                    int dn[3] = {ex[0], ex[1], ex[2]};
-                    dn[x] -= 1;
-                    ii[cen] = g_index(dn[0], dn[1], dn[2]);
-                    nn[cen] = g_ncart(ls[cen] - 1);
-                    v -= ex[x] * H[out[__ldg(W::out_off() + 3 + cen) + ((ii[0] * nn[1] + ii[1]) * nn[2] + ii[2]) * nn[3] + ii[3]]];
-                }
-                g[3 * cen + x] = fma(s, v, g[3 * cen + x]);
-            }
+        const double s = gam * cs[6 * B.sa + ia] * cs[6 * B.sb + ib] * cs[6 * K.sa + ic] *
+                         cs[6 * K.sb + id];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const unsigned u = __ldg(con + k * NBLK + e);
+            const unsigned dn = (u >> 16) & 0x7fffu;
+            double v = H[u & 0xffffu];
+            if (dn != 0x7fffu) v = fma(u >> 31 ? -2.0 : -1.0, H[dn], v);
+            g[k] = fma(s, v, g[k]);
         }
     }
+    constexpr unsigned ALL = 0xffffffffu;
+    double last = g[8];
 #pragma unroll
-    for (int k = 0; k < 9; ++k)
+    for (int o = 16; o > 0; o >>= 1) last += __shfl_xor_sync(ALL, last, o);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) g[k] += __shfl_xor_sync(0xffffffffu, g[k], o);
-    if (lane == 0) {
-        for (int cen = 0; cen < 3; ++cen)
-            for (int x = 0; x < 3; ++x) {
-                atomicAdd(a.grad + 3 * a.shell_atom[sh[cen]] + x, g[3 * cen + x]);
-                atomicAdd(a.grad + 3 * a.shell_atom[sh[3]] + x, -g[3 * cen + x]);
+    for (int o = 16, n = 4; n > 0; o >>= 1, n >>= 1) {
+        const bool hi = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const double send = hi ? g[i] : g[i + n], keep = hi ? g[i + n] : g[i];
+            g[i] = keep + __shfl_xor_sync(ALL, send, o);
+        }
+    }
+    double v = g[0];
+    v += __shfl_xor_sync(ALL, v, 2);
+    v += __shfl_xor_sync(ALL, v, 1);
+    // lanes 4 k (k < 8) hold component k's sum, lane 1 the last
+    const int k = lane == 1 ? 8 : lane >> 2;
+    if (lane == 1) v = last;
+    if (lane == 1 || (lane & 3) == 0) {
+        const int cen = k / 3, x = k - 3 * cen;
+        const int shell = cen == 0 ? B.sa : cen == 1 ? B.sb : K.sa;
+        atomicAdd(a.grad + 3 * a.shell_atom[shell] + x, v);
+        atomicAdd(a.grad + 3 * a.shell_atom[K.sb] + x, -v);
+    }
+}
+
+// a.per consecutive tasks a warp (one for the classes with shared accumulators), their
+// primitive quartets set up together as in wide_many.
+template <int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__(32 * kGradWarps) k_eri_grad(const GradArgs a) {
+    using W = GradProg<LA, LB, LC, LD>;
+    using Lay = GradLayout<LA, LB, LC, LD>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double* sm = reinterpret_cast<double*>(smem_raw) + (size_t)warp * Lay::WARP;
+    double* sC = sm + Lay::ACC;
+    double* sF = sC + Lay::SC;
+    double* node = sF + Lay::SF;
+    if constexpr (Lay::SMEM_ACC) {
+        const int t = blockIdx.x * Lay::WARPS + warp;
+        if (t >= a.ntask) return;
+        const int2 task = a.tasks[t];
+        const PairRec B = a.pairs[task.x];
+        const PairRec K = a.pairs[task.y];
+        if (!grad_keep(a, B, K)) return;               // warp-uniform
+        for (int q = lane; q < W::NACC; q += 32) sm[q] = 0.0;
+        const int nK = K.nprim, ntot = B.nprim * nK;
+        for (int base = 0; base < ntot; base += kSetupBatch) {
+            const int i = base + lane;
+            if (lane < kSetupBatch && i < ntot)
+                grad_setup_slot<LA, LB, LC, LD>(a.prims[B.prim_off + i / nK],
+                                                a.prims[K.prim_off + i % nK], sC, sF, lane);
+            __syncwarp();
+            grad_items<LA, LB, LC, LD>(sC, sF, node, 0, min(kSetupBatch, ntot - base), lane,
+                                       nullptr, nullptr, sm);
+        }
+        grad_tail<LA, LB, LC, LD>(a, task, B, K, sm, lane);
+    } else {
+        constexpr int NACCW = (W::NACC + 31) / 32;
+        constexpr unsigned ALL = 0xffffffffu;
+        const int per = a.per;
+        const int t0 = (blockIdx.x * Lay::WARPS + warp) * per;
+        const int nq = min(per, a.ntask - t0);
+        if (nq <= 0) return;
+        int w = 0, bo = 0, ko = 0, kn = 1;
+        if (lane < nq) {
+            const int2 task = a.tasks[t0 + lane];
+            const PairRec& B = a.pairs[task.x];
+            const PairRec& K = a.pairs[task.y];
+            bo = B.prim_off;
+            ko = K.prim_off;
+            kn = K.nprim;
+            w = grad_keep(a, B, K) ? B.nprim * kn : 0;
+        }
+        int end = w;
+#pragma unroll
+        for (int o = 1; o < kManyTasks; o <<= 1) {
+            const int y = __shfl_up_sync(ALL, end, o);
+            if (lane >= o) end += y;
+        }
+        const int total = __shfl_sync(ALL, end, kManyTasks - 1);
+        double acc[NACCW];
+        unsigned ent[NACCW];
+#pragma unroll
+        for (int k = 0; k < NACCW; ++k) {
+            acc[k] = 0.0;
+            const int q = lane + 32 * k;
+            ent[k] = q < W::NACC ? __ldg(W::acc() + q) : 255u << 16;
+        }
+        int q = 0, left = __shfl_sync(ALL, w, 0);
+        auto close = [&]() {                             // ends quartet q, moves to the next
+            if (__shfl_sync(ALL, w, q) > 0) {
+#pragma unroll
+                for (int k = 0; k < NACCW; ++k) {
+                    const int t = lane + 32 * k;
+                    if (t < W::NACC) node[__ldg(W::accpos() + t)] = acc[k];
+                    acc[k] = 0.0;
+                }
+                __syncwarp();
+                const int2 task = a.tasks[t0 + q];
+                const PairRec B = a.pairs[task.x];
+                const PairRec K = a.pairs[task.y];
+                grad_tail<LA, LB, LC, LD>(a, task, B, K, node, lane);
+                __syncwarp();
             }
+            ++q;
+            left = __shfl_sync(ALL, w, q & 31);
+        };
+        for (int base = 0; base < total; base += kSetupBatch) {
+            const int x = base + lane;
+            int mine = 0;
+#pragma unroll
+            for (int k = 0; k < kManyTasks - 1; ++k) mine += __shfl_sync(ALL, end, k) <= x;
+            const int start = __shfl_sync(ALL, end - w, mine), nK = __shfl_sync(ALL, kn, mine);
+            const int po = __shfl_sync(ALL, bo, mine), qo = __shfl_sync(ALL, ko, mine);
+            if (lane < kSetupBatch && x < total) {
+                const int i = x - start, j = i / nK;
+                grad_setup_slot<LA, LB, LC, LD>(a.prims[po + j], a.prims[qo + i - j * nK], sC, sF,
+                                                lane);
+            }
+            __syncwarp();
+            const int nb = min(kSetupBatch, total - base);
+            for (int j = 0; j < nb;) {
+                while (left == 0) close();
+                const int run = min(left, nb - j);
+                grad_items<LA, LB, LC, LD>(sC, sF, node, j, run, lane, acc, ent, nullptr);
+                j += run;
+                left -= run;
+            }
+        }
+        while (q < nq) close();
     }
 }
 
@@ -512,7 +565,10 @@ int launch_grad(const GradArgs& a, cudaStream_t st) {
     using Lay = GradLayout<LA, LB, LC, LD>;
     auto k = k_eri_grad<LA, LB, LC, LD>;
     if (set_smem<k_eri_grad<LA, LB, LC, LD>>(Lay::BYTES)) return GS_ERR_CUDA;
-    k<<<(a.ntask + Lay::WARPS - 1) / Lay::WARPS, 32 * Lay::WARPS, Lay::BYTES, st>>>(a);
+    GradArgs b = a;
+    if (Lay::SMEM_ACC || b.per < 1) b.per = 1;
+    const int tasks = b.per * Lay::WARPS;
+    k<<<(b.ntask + tasks - 1) / tasks, 32 * Lay::WARPS, Lay::BYTES, st>>>(b);
     return cudaGetLastError() == cudaSuccess ? 0 : GS_ERR_CUDA;
 }
 

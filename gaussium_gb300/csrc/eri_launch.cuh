@@ -8,7 +8,7 @@
 // 2 = warp, 3 = grouped warp, 4 = split: thread code, one warp per quartet, 5 = cooperative:
 // warp code, up to eight warps per quartet, 6 = stacked: warp code, several primitive
 // quartets per lane, 7 = cluster: cooperative blocks on eight SMs per quartet) wins, else the
-// default (default_form).  On GB300 a warp-wide FP64 instruction holds the pipe for the same
+// default (default_form).  Bits 16.. give the tasks a warp of the warp forms takes (0: one).  On GB300 a warp-wide FP64 instruction holds the pipe for the same
 // time whatever its active lanes, so narrow recursion levels are filled with several
 // primitive quartets, and the thread form, whose lanes are all busy, is the better one
 // wherever its accumulators stay near the register file and enough quartets fill the GPU.
@@ -97,7 +97,7 @@ int variants(int prec) {
 }
 
 template <int LA, int LB, int LC, int LD, int PREC>
-int launch_prec(int kind, int variant, const void* args, cudaStream_t st) {
+int launch_prec(int kind, int variant, int per, const void* args, cudaStream_t st) {
     using F = ClassForms<LA, LB, LC, LD>;
     constexpr bool thread = PREC == 64 ? F::thread64 : F::thread32;
     constexpr bool wide = PREC == 64 ? F::wide64 : F::wide32;
@@ -140,14 +140,14 @@ int launch_prec(int kind, int variant, const void* args, cudaStream_t st) {
     if constexpr (stacked) {
         using T = typename std::conditional<PREC == 64, double, float>::type;
         if (v == 6 && kind != GS_KIND_SCHWARZ)
-            return launch_wide<LA, LB, LC, LD, PREC, 1, kStack<T>>(kind, args, st);
+            return launch_wide<LA, LB, LC, LD, PREC, 1, kStack<T>>(kind, args, st, per);
     }
     if (v == 6) v = 2;
     if constexpr (grouped) {
-        if (v == 3) return launch_wide<LA, LB, LC, LD, PREC, F::VG>(kind, args, st);
+        if (v == 3) return launch_wide<LA, LB, LC, LD, PREC, F::VG>(kind, args, st, per);
     }
     if constexpr (wide) {
-        if (v >= 2 || !thread) return launch_wide<LA, LB, LC, LD, PREC>(kind, args, st);
+        if (v >= 2 || !thread) return launch_wide<LA, LB, LC, LD, PREC>(kind, args, st, per);
     }
     if constexpr (thread) return launch_class<LA, LB, LC, LD, PREC>(kind, args, st);
     return GS_ERR_CLASS;
@@ -155,11 +155,11 @@ int launch_prec(int kind, int variant, const void* args, cudaStream_t st) {
 
 template <int LA, int LB, int LC, int LD>
 int launch_any(int kind, int prec_variant, const void* args, cudaStream_t st) {
-    const int variant = prec_variant >> 8;
+    const int variant = (prec_variant >> 8) & 0xff, per = prec_variant >> 16;
     int prec = prec_variant & 0xff;
     if (kind == GS_KIND_SCHWARZ) prec = 64;
-    if (prec == 64) return launch_prec<LA, LB, LC, LD, 64>(kind, variant, args, st);
-    return launch_prec<LA, LB, LC, LD, 32>(kind, variant, args, st);
+    if (prec == 64) return launch_prec<LA, LB, LC, LD, 64>(kind, variant, per, args, st);
+    return launch_prec<LA, LB, LC, LD, 32>(kind, variant, per, args, st);
 }
 
 }  // namespace gs

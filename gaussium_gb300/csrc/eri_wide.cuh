@@ -72,8 +72,15 @@ template <int LA, int LB, int LC, int LD, typename T, int VG = 1, int RQ = 1> st
     static constexpr int HR_JK = W::HSIZE + G::NBLK + G::NA * G::NB + G::NC * G::ND;
     static constexpr int WARP_W = VRR > HR_W ? VRR : HR_W;       // elements of T per warp
     static constexpr int WARP_JK = VRR > HR_JK ? VRR : HR_JK;
-    static constexpr size_t BYTES_W = (size_t)WARP_W * sizeof(T) * kWideWarps;
-    static constexpr size_t BYTES_JK = (size_t)WARP_JK * sizeof(T) * kWideWarps;
+    // several quartets a warp (wide_many): the set-up buffers outlive a quartet's HRR and
+    // epilogue, which share the node buffers' place.  Up to total angular momentum 6; above,
+    // a quartet's recursion is 20 times its set-up and the buffers are large
+    static constexpr bool MANY = G::L <= 6;
+    static constexpr int NODE = VG * RQ * NVS;
+    static constexpr int MANY_W = MANY ? SC + SF + (NODE > HR_W ? NODE : HR_W) : WARP_W;
+    static constexpr int MANY_JK = MANY ? SC + SF + (NODE > HR_JK ? NODE : HR_JK) : WARP_JK;
+    static constexpr size_t BYTES_W = (size_t)MANY_W * sizeof(T) * kWideWarps;
+    static constexpr size_t BYTES_JK = (size_t)MANY_JK * sizeof(T) * kWideWarps;
 };
 
 // Recursion coefficients and scaled Boys values of one primitive quartet.  KB, KK, KX: the
@@ -220,13 +227,12 @@ __device__ __forceinline__ void vrr_step_rq(const uint4* __restrict__ vrec, int 
     }
 }
 
-// Contracted [e0|f0] targets of primitive quartets first, first + stride, ... of the
-// quartet (set up Lay::SB at a time): target lane + 32 k is added to acc[k].
-template <int LA, int LB, int LC, int LD, typename T, int VG, int RQ = 1>
-__device__ __forceinline__ void wide_contract(const PairRec& B, const PairRec& K,
-                                              const PrimRec<T>* __restrict__ prims,
-                                              T* __restrict__ sm, int lane, int first, int stride,
-                                              T* __restrict__ acc) {
+// The VRR of primitive quartets j0 .. j0 + nb of a set-up round (coefficients sC, Boys values
+// sF): target lane + 32 k is added to acc[k], in order.
+template <int LA, int LB, int LC, int LD, typename T, int VG, int RQ>
+__device__ __forceinline__ void wide_items(const T* __restrict__ sC, const T* __restrict__ sF,
+                                           T* __restrict__ node, int j0, int nb, int lane,
+                                           T* __restrict__ acc) {
     static_assert(VG == 1 || RQ == 1, "grouped and stacked forms are separate");
     using G = ClassGen<LA, LB, LC, LD>;
     using W = WideProg<LA, LB, LC, LD>;
@@ -234,129 +240,163 @@ __device__ __forceinline__ void wide_contract(const PairRec& B, const PairRec& K
     constexpr int L = G::L;
     constexpr int NACC = G::NACC;
     constexpr int NACCW = (NACC + 31) / 32;
+    // the node program: waves of at most 32 nodes (one per lane), or of 32/VG nodes for the
+    // grouped form (one per lane group of VG primitive quartets)
+    constexpr int NVS = Lay::NVS;
+    constexpr int NVSEG = VG == 1 ? W::NVSEG : W::NVSEG_G;
+    // VG (grouped) or RQ (stacked) primitive quartets at a time, each with its own node
+    // buffer; the accumulators add them in order, so the sums match the one-at-a-time form.
+    // Grouped: lane = (quartet g, record j of a wave of 32/VG); stacked: lane j runs record j
+    // of every wave on all of them.
+    constexpr int STEP = VG * RQ;
+    constexpr int WAVE = 32 / VG;
+    const uint4* __restrict__ vrec = VG == 1 ? W::vrec() : W::vrec_g();
+    const int* __restrict__ vseg = VG == 1 ? W::vseg() : W::vseg_g();
+    const unsigned short* __restrict__ vtgt = VG == 1 ? W::vtgt() : W::vtgt_g();
+    const int g = lane / WAVE, jw = lane - g * WAVE;
+    for (int j = j0; j < j0 + nb; j += STEP) {
+        const int ng = min(STEP, j0 + nb - j);
+        if constexpr (STEP == 1) {
+            if (lane <= L) node[lane] = sF[j * (L + 1) + lane];
+        } else {
+            for (int x = lane; x < ng * (L + 1); x += 32) {
+                const int q = x / (L + 1), m = x - q * (L + 1);
+                node[q * NVS + m] = sF[(j + q) * (L + 1) + m];
+            }
+        }
+        __syncwarp();
+        int noff = __ldg(vseg), cnt = __ldg(vseg + 1);
+        for (int s = 0; s < NVSEG; ++s) {
+            int noff_n = 0, cnt_n = 0;
+            if (s + 1 < NVSEG) {                             // next step's header, early
+                noff_n = __ldg(vseg + 4 * (s + 1));
+                cnt_n = __ldg(vseg + 4 * (s + 1) + 1);
+            }
+            if (s > 0) __syncwarp();
+            if constexpr (RQ > 1)
+                vrr_step_rq<RQ, NVS, T>(vrec, noff, cnt, ng, sC + j * kNCoef, node, lane);
+            else
+                vrr_step<WAVE, T>(vrec, noff, cnt, g < ng, sC + (j + g) * kNCoef, node + g * NVS,
+                                  jw);
+            noff = noff_n;
+            cnt = cnt_n;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < NACCW; ++k) {
+            const int t = lane + 32 * k;
+            if (t < NACC) {
+                const int v = __ldg(vtgt + t);
+                for (int q = 0; q < ng; ++q) acc[k] += node[q * NVS + v];
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// Set-up of the primitive quartet (P, Q) into slot x of a round.
+template <int LA, int LB, int LC, int LD, typename T>
+__device__ __forceinline__ void wide_setup_slot(const PrimRec<T>& P, const PrimRec<T>& Q,
+                                                T* __restrict__ sC, T* __restrict__ sF, int x) {
+    constexpr int L = ClassGen<LA, LB, LC, LD>::L;
+    wide_setup_m<L, T, (LA + LB > 0 ? LA + LB - 1 : 0), (LC + LD > 0 ? LC + LD - 1 : 0),
+                 (LC + LD > 0 ? LA + LB : 0)>(P, Q, sC + x * kNCoef, sF + x * (L + 1));
+    sC[x * kNCoef + kZeroCoef] = T(0);
+}
+
+// Contracted [e0|f0] targets of primitive quartets first, first + stride, ... of the
+// quartet (set up Lay::SB at a time): target lane + 32 k is added to acc[k].
+template <int LA, int LB, int LC, int LD, typename T, int VG, int RQ = 1>
+__device__ __forceinline__ void wide_contract(const PairRec& B, const PairRec& K,
+                                              const PrimRec<T>* __restrict__ prims,
+                                              T* __restrict__ sm, int lane, int first, int stride,
+                                              T* __restrict__ acc) {
+    using Lay = WideLayout<LA, LB, LC, LD, T, VG, RQ>;
     T* sC = sm;
     T* sF = sm + Lay::SC;
     T* node = sm + Lay::SC + Lay::SF;
     const int nB = B.nprim, ntot = nB * K.nprim;
     const int nmine = first < ntot ? (ntot - first + stride - 1) / stride : 0;
-    // the node program: waves of at most 32 nodes (one per lane), or of 32/VG nodes for the
-    // grouped form (one per lane group of VG primitive quartets)
-    constexpr int NVS = Lay::NVS;
-    constexpr int NVSEG = VG == 1 ? W::NVSEG : W::NVSEG_G;
-    const uint4* __restrict__ vrec = VG == 1 ? W::vrec() : W::vrec_g();
-    const int* __restrict__ vseg = VG == 1 ? W::vseg() : W::vseg_g();
-    const unsigned short* __restrict__ vtgt = VG == 1 ? W::vtgt() : W::vtgt_g();
     for (int base = 0; base < nmine; base += Lay::SB) {
         const int i = first + (base + lane) * stride;
         if (lane < Lay::SB && base + lane < nmine) {
             const int j = i / nB;                        // bra inner, as in eri_quartet
-            const PrimRec<T> P = prims[B.prim_off + i - j * nB];
-            const PrimRec<T> Q = prims[K.prim_off + j];
-            wide_setup_m<L, T, (LA + LB > 0 ? LA + LB - 1 : 0), (LC + LD > 0 ? LC + LD - 1 : 0),
-                         (LC + LD > 0 ? LA + LB : 0)>(P, Q, sC + lane * kNCoef,
-                                                      sF + lane * (L + 1));
-            sC[lane * kNCoef + kZeroCoef] = T(0);
+            wide_setup_slot<LA, LB, LC, LD, T>(prims[B.prim_off + i - j * nB],
+                                               prims[K.prim_off + j], sC, sF, lane);
         }
         __syncwarp();
-        const int nb = min(Lay::SB, nmine - base);
-        if constexpr (RQ > 1) {
-        // RQ primitive quartets at a time, each with its own node buffer; lane j runs record
-        // j of every wave on all of them.  The accumulators add the quartets in order, so
-        // the sums match the one-at-a-time form.
-        for (int j0 = 0; j0 < nb; j0 += RQ) {
-            const int ng = min(RQ, nb - j0);
-            for (int x = lane; x < ng * (L + 1); x += 32) {
-                const int q = x / (L + 1), m = x - q * (L + 1);
-                node[q * NVS + m] = sF[(j0 + q) * (L + 1) + m];
-            }
-            __syncwarp();
-            int noff = __ldg(vseg), cnt = __ldg(vseg + 1);
-            for (int s = 0; s < NVSEG; ++s) {
-                int noff_n = 0, cnt_n = 0;
-                if (s + 1 < NVSEG) {
-                    noff_n = __ldg(vseg + 4 * (s + 1));
-                    cnt_n = __ldg(vseg + 4 * (s + 1) + 1);
-                }
-                if (s > 0) __syncwarp();
-                vrr_step_rq<RQ, NVS, T>(vrec, noff, cnt, ng, sC + j0 * kNCoef, node, lane);
-                noff = noff_n;
-                cnt = cnt_n;
-            }
-            __syncwarp();
+        wide_items<LA, LB, LC, LD, T, VG, RQ>(sC, sF, node, 0, min(Lay::SB, nmine - base), lane,
+                                              acc);
+    }
+}
+
+// Several quartets by one warp, at most kManyTasks (nq of them): lane q < nq brings quartet
+// q's pairs (rec) and primitive-quartet count w (0: nothing to contract).  A set-up round
+// takes primitive quartets across the quartets' boundaries, so that its 110 FP64
+// instructions serve 32 of them and not the two to sixteen of one quartet ((H2O)16/6-31G*:
+// three for (dp|ds)); the quartets' sums and their order are those of one at a time.
+// finish(q) runs after quartet q's last primitive quartet with the accumulators in the HRR
+// region at `hrr` (the node buffers' place).
+constexpr int kManyTasks = 8;
+
+template <int LA, int LB, int LC, int LD, typename T, int VG, int RQ, typename Finish>
+__device__ __forceinline__ void wide_many(int nq, int w, int bra_off, int bra_n, int ket_off,
+                                          const PrimRec<T>* __restrict__ prims,
+                                          T* __restrict__ sm, int lane, Finish finish) {
+    using Lay = WideLayout<LA, LB, LC, LD, T, VG, RQ>;
+    constexpr int NACC = ClassGen<LA, LB, LC, LD>::NACC;
+    constexpr int NACCW = (NACC + 31) / 32;
+    constexpr unsigned ALL = 0xffffffffu;
+    T* sC = sm;
+    T* sF = sm + Lay::SC;
+    T* node = sm + Lay::SC + Lay::SF;
+    if (lane >= nq) w = 0;
+    int end = w;                                     // primitive quartets up to quartet `lane`
 #pragma unroll
-            for (int k = 0; k < NACCW; ++k) {
-                const int t = lane + 32 * k;
-                if (t < NACC) {
-                    const int v = __ldg(vtgt + t);
-                    for (int q = 0; q < ng; ++q) acc[k] += node[q * NVS + v];
-                }
-            }
-            __syncwarp();
-        }
-        } else if constexpr (VG == 1) {
-        for (int j = 0; j < nb; ++j) {
-            const T* __restrict__ c = sC + j * kNCoef;
-            if (lane <= L) node[lane] = sF[j * (L + 1) + lane];
-            __syncwarp();
-            int noff = __ldg(vseg), cnt = __ldg(vseg + 1);
-            for (int s = 0; s < NVSEG; ++s) {
-                int noff_n = 0, cnt_n = 0;
-                if (s + 1 < NVSEG) {                         // next step's header, early
-                    noff_n = __ldg(vseg + 4 * (s + 1));
-                    cnt_n = __ldg(vseg + 4 * (s + 1) + 1);
-                }
-                if (s > 0) __syncwarp();
-                vrr_step<32, T>(vrec, noff, cnt, true, c, node, lane);
-                noff = noff_n;
-                cnt = cnt_n;
-            }
-            __syncwarp();
+    for (int o = 1; o < kManyTasks; o <<= 1) {
+        const int y = __shfl_up_sync(ALL, end, o);
+        if (lane >= o) end += y;
+    }
+    const int total = __shfl_sync(ALL, end, kManyTasks - 1);
+    T acc[NACCW];
 #pragma unroll
-            for (int k = 0; k < NACCW; ++k) {
-                const int t = lane + 32 * k;
-                if (t < NACC) acc[k] += node[__ldg(vtgt + t)];
-            }
-            __syncwarp();
-        }
-        } else {
-        // VG primitive quartets at a time: lane = (quartet g, record j of a wave of 32/VG);
-        // quartet g has its own node buffer.  The accumulators add the quartets in order,
-        // so the sums match the one-at-a-time form.
-        constexpr int WAVE = 32 / VG;
-        const int g = lane / WAVE, jw = lane - g * WAVE;
-        for (int j0 = 0; j0 < nb; j0 += VG) {
-            const int ng = min(VG, nb - j0);
-            for (int x = lane; x < ng * (L + 1); x += 32) {
-                const int gg = x / (L + 1), m = x - gg * (L + 1);
-                node[gg * NVS + m] = sF[(j0 + gg) * (L + 1) + m];
-            }
-            __syncwarp();
-            int noff = __ldg(vseg), cnt = __ldg(vseg + 1);
-            for (int s = 0; s < NVSEG; ++s) {
-                int noff_n = 0, cnt_n = 0;
-                if (s + 1 < NVSEG) {
-                    noff_n = __ldg(vseg + 4 * (s + 1));
-                    cnt_n = __ldg(vseg + 4 * (s + 1) + 1);
-                }
-                if (s > 0) __syncwarp();
-                vrr_step<WAVE, T>(vrec, noff, cnt, g < ng, sC + (j0 + g) * kNCoef,
-                                  node + g * NVS, jw);
-                noff = noff_n;
-                cnt = cnt_n;
-            }
-            __syncwarp();
+    for (int k = 0; k < NACCW; ++k) acc[k] = T(0);
+    int q = 0, left = __shfl_sync(ALL, w, 0);        // the quartet in progress
+    auto close = [&]() {                             // ends quartet q and moves to the next
 #pragma unroll
-            for (int k = 0; k < NACCW; ++k) {
-                const int t = lane + 32 * k;
-                if (t < NACC) {
-                    const int v = __ldg(vtgt + t);
-                    for (int gg = 0; gg < ng; ++gg) acc[k] += node[gg * NVS + v];
-                }
-            }
-            __syncwarp();
+        for (int k = 0; k < NACCW; ++k) {
+            const int t = lane + 32 * k;
+            if (t < NACC) node[t] = acc[k];
+            acc[k] = T(0);
         }
+        __syncwarp();
+        finish(q, node);
+        __syncwarp();
+        ++q;
+        left = __shfl_sync(ALL, w, q & 31);
+    };
+    for (int base = 0; base < total; base += Lay::SB) {
+        const int x = base + lane;
+        int mine = 0;
+#pragma unroll
+        for (int k = 0; k < kManyTasks - 1; ++k) mine += __shfl_sync(ALL, end, k) <= x;
+        const int start = __shfl_sync(ALL, end - w, mine), nB = __shfl_sync(ALL, bra_n, mine);
+        const int po = __shfl_sync(ALL, bra_off, mine), qo = __shfl_sync(ALL, ket_off, mine);
+        if (lane < Lay::SB && x < total) {
+            const int i = x - start, j = i / nB;
+            wide_setup_slot<LA, LB, LC, LD, T>(prims[po + i - j * nB], prims[qo + j], sC, sF, lane);
+        }
+        __syncwarp();
+        const int nb = min(Lay::SB, total - base);
+        for (int j = 0; j < nb;) {
+            while (left == 0) close();
+            const int run = min(left, nb - j);
+            wide_items<LA, LB, LC, LD, T, VG, RQ>(sC, sF, node, j, run, lane, acc);
+            j += run;
+            left -= run;
         }
     }
+    while (q < nq) close();
 }
 
 // Horizontal recursion in shared memory from the contracted targets in sm[0 .. NACC); on
@@ -462,18 +502,43 @@ __device__ __forceinline__ void wide_write_out(const WriteArgs& a, const WriteTa
 }
 
 template <int LA, int LB, int LC, int LD, typename T, int VG, int RQ = 1>
-__global__ void __launch_bounds__(32 * kWideWarps, GS_WIDE_MINB) k_wide_write(const WriteArgs a) {
+__global__ void __launch_bounds__(32 * kWideWarps, GS_WIDE_MINB) k_wide_write(const WriteArgs a,
+                                                                             int per_warp) {
     using Lay = WideLayout<LA, LB, LC, LD, T, VG, RQ>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    T* sm = reinterpret_cast<T*>(smem_raw) + (size_t)warp * Lay::WARP_W;
-    const int t = blockIdx.x * kWideWarps + warp;
-    if (t >= a.ntask) return;
-    const WriteTask task = a.tasks[t];
-    const PairRec B = a.pairs[task.bra];
-    const PairRec K = a.pairs[task.ket];
-    wide_quartet<LA, LB, LC, LD, T, VG, RQ>(B, K, (const PrimRec<T>*)a.prims, sm, lane);
-    wide_write_out<LA, LB, LC, LD, T>(a, task, B, K, sm, lane);
+    T* sm = reinterpret_cast<T*>(smem_raw) + (size_t)warp * Lay::MANY_W;
+    if constexpr (Lay::MANY) {
+        const int t0 = (blockIdx.x * kWideWarps + warp) * per_warp;
+        const int nq = min(per_warp, a.ntask - t0);
+        if (nq <= 0) return;
+        int w = 0, bo = 0, bn = 1, ko = 0;
+        if (lane < nq) {
+            const WriteTask task = a.tasks[t0 + lane];
+            const PairRec& B = a.pairs[task.bra];
+            const PairRec& K = a.pairs[task.ket];
+            bo = B.prim_off;
+            bn = B.nprim;
+            ko = K.prim_off;
+            w = bn * K.nprim;
+        }
+        wide_many<LA, LB, LC, LD, T, VG, RQ>(
+            nq, w, bo, bn, ko, (const PrimRec<T>*)a.prims, sm, lane, [&](int q, T* hrr) {
+                const WriteTask task = a.tasks[t0 + q];
+                const PairRec B = a.pairs[task.bra];
+                const PairRec K = a.pairs[task.ket];
+                wide_hrr<LA, LB, LC, LD, T>(B, K, hrr, lane);
+                wide_write_out<LA, LB, LC, LD, T>(a, task, B, K, hrr, lane);
+            });
+    } else {
+        const int t = blockIdx.x * kWideWarps + warp;
+        if (t >= a.ntask) return;
+        const WriteTask task = a.tasks[t];
+        const PairRec B = a.pairs[task.bra];
+        const PairRec K = a.pairs[task.ket];
+        wide_quartet<LA, LB, LC, LD, T, VG, RQ>(B, K, (const PrimRec<T>*)a.prims, sm, lane);
+        wide_write_out<LA, LB, LC, LD, T>(a, task, B, K, sm, lane);
+    }
 }
 
 // One output vector of the digestion: out(x) += sum_i term(x, i), x < NOUT, i < NIN, for the
@@ -602,17 +667,42 @@ __device__ __forceinline__ void wide_jk_task(const JKArgs& a, int t, T* __restri
     wide_jk_digest<LA, LB, LC, LD, T>(a, task, B, K, sm, lane);
 }
 
-// One warp per task; with a task count on the device (after a partition) the grid is
-// capped and each warp strides over the tasks.
+// per_warp tasks a warp; with a task count on the device (after a partition) the grid is
+// capped and each warp strides over the tasks, per_warp at a time.
 template <int LA, int LB, int LC, int LD, typename T, int VG, int RQ = 1>
-__global__ void __launch_bounds__(32 * kWideWarps, GS_WIDE_MINB) k_wide_jk(const JKArgs a) {
+__global__ void __launch_bounds__(32 * kWideWarps, GS_WIDE_MINB) k_wide_jk(const JKArgs a,
+                                                                          int per_warp) {
     using Lay = WideLayout<LA, LB, LC, LD, T, VG, RQ>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    T* sm = reinterpret_cast<T*>(smem_raw) + (size_t)warp * Lay::WARP_JK;
+    T* sm = reinterpret_cast<T*>(smem_raw) + (size_t)warp * Lay::MANY_JK;
     const int ntask = a.ntask_dev ? *a.ntask_dev : a.ntask;
-    for (int t = blockIdx.x * kWideWarps + warp; t < ntask; t += gridDim.x * kWideWarps) {
-        wide_jk_task<LA, LB, LC, LD, T, VG, RQ>(a, t, sm, lane);
+    const int step = gridDim.x * kWideWarps * per_warp;
+    for (int t0 = (blockIdx.x * kWideWarps + warp) * per_warp; t0 < ntask; t0 += step) {
+        if constexpr (Lay::MANY) {
+            const int nq = min(per_warp, ntask - t0);
+            int w = 0, bo = 0, bn = 1, ko = 0;
+            if (lane < nq) {
+                const int2 task = a.tasks[t0 + lane];
+                const PairRec& B = a.pairs[task.x];
+                const PairRec& K = a.pairs[task.y];
+                bo = B.prim_off;
+                bn = B.nprim;
+                ko = K.prim_off;
+                w = jk_keep(a, B, K) ? bn * K.nprim : 0;
+            }
+            wide_many<LA, LB, LC, LD, T, VG, RQ>(
+                nq, w, bo, bn, ko, (const PrimRec<T>*)a.prims, sm, lane, [&](int q, T* hrr) {
+                    if (__shfl_sync(0xffffffffu, w, q) == 0) return;     // dropped, or no integral
+                    const int2 task = a.tasks[t0 + q];
+                    const PairRec B = a.pairs[task.x];
+                    const PairRec K = a.pairs[task.y];
+                    wide_hrr<LA, LB, LC, LD, T>(B, K, hrr, lane);
+                    wide_jk_digest<LA, LB, LC, LD, T>(a, task, B, K, hrr, lane);
+                });
+        } else {
+            wide_jk_task<LA, LB, LC, LD, T, VG, RQ>(a, t0, sm, lane);
+        }
         __syncwarp();
     }
 }
@@ -853,33 +943,40 @@ int set_smem(size_t sh) {
     return 0;
 }
 
+// per: tasks a warp takes (0: one, or two where the count is on the device and may be far
+// below its bound); one for the classes that run a quartet at a time.
 template <int LA, int LB, int LC, int LD, int PREC, int VG = 1, int RQ = 1>
-int launch_wide(int kind, const void* args, cudaStream_t st) {
+int launch_wide(int kind, const void* args, cudaStream_t st, int per) {
     using T = typename std::conditional<PREC == 64, double, float>::type;
     using Lay = WideLayout<LA, LB, LC, LD, T, VG, RQ>;
     constexpr int TPB = 32 * kWideWarps;
+    if (!Lay::MANY) per = 1;
+    if (per > kManyTasks) return GS_ERR_ARG;
     if (kind == GS_KIND_WRITE) {
         const WriteArgs& a = *(const WriteArgs*)args;
         if (a.ntask <= 0) return 0;
+        if (per < 1) per = 1;
         auto k = k_wide_write<LA, LB, LC, LD, T, VG, RQ>;
         if (set_smem<k_wide_write<LA, LB, LC, LD, T, VG, RQ>>(Lay::BYTES_W)) return GS_ERR_CUDA;
-        k<<<(a.ntask + kWideWarps - 1) / kWideWarps, TPB, Lay::BYTES_W, st>>>(a);
+        k<<<(a.ntask + per * kWideWarps - 1) / (per * kWideWarps), TPB, Lay::BYTES_W, st>>>(a, per);
     } else if (kind == GS_KIND_JK) {
         const JKArgs& a = *(const JKArgs*)args;
         if (a.ntask <= 0) return 0;
         auto k = k_wide_jk<LA, LB, LC, LD, T, VG, RQ>;
         if (set_smem<k_wide_jk<LA, LB, LC, LD, T, VG, RQ>>(Lay::BYTES_JK)) return GS_ERR_CUDA;
-        int grid = (a.ntask + kWideWarps - 1) / kWideWarps;
+        if (per < 1) per = a.ntask_dev ? 2 : 1;
+        int grid = (a.ntask + per * kWideWarps - 1) / (per * kWideWarps);
         if (a.ntask_dev && grid > kWideDeviceCountBlocksPerSM * sm_count())
             grid = kWideDeviceCountBlocksPerSM * sm_count();
-        k<<<grid, TPB, Lay::BYTES_JK, st>>>(a);
+        k<<<grid, TPB, Lay::BYTES_JK, st>>>(a, per);
     } else if (kind == GS_KIND_SCHWARZ) {
         if constexpr (LA == LC && LB == LD && PREC == 64 && VG == 1 && RQ == 1) {
             const SchwarzArgs& a = *(const SchwarzArgs*)args;
             if (a.npair <= 0) return 0;
             auto k = k_wide_schwarz<LA, LB, double>;
-            if (set_smem<k_wide_schwarz<LA, LB, double>>(Lay::BYTES_W)) return GS_ERR_CUDA;
-            k<<<(a.npair + kWideWarps - 1) / kWideWarps, TPB, Lay::BYTES_W, st>>>(a);
+            constexpr size_t bytes = (size_t)Lay::WARP_W * sizeof(T) * kWideWarps;
+            if (set_smem<k_wide_schwarz<LA, LB, double>>(bytes)) return GS_ERR_CUDA;
+            k<<<(a.npair + kWideWarps - 1) / kWideWarps, TPB, bytes, st>>>(a);
         } else {
             return GS_ERR_CLASS;
         }

@@ -209,6 +209,40 @@ def grad_program(cls):
                 regions=[(w, len(es), len(fs)) for w, es, fs in regions])
 
 
+NO_LOWERED = 0x7fff
+
+
+def contraction_table(cls, outs):
+    """Per derivative component 3 cen + x and block element e the HRR slots of the raised and
+    the lowered integral: up | dn << 16 (dn = NO_LOWERED: none), bit 31 set where the lowered
+    one counts twice (e_x = 2).  Component-major, so that a warp's lanes read consecutive
+    words."""
+    ls = list(cls)
+    n = [ncart(x) for x in ls]
+    table = []
+    for cen in range(3):
+        carts = cart(ls[cen])
+        raised = {c: i for i, c in enumerate(cart(ls[cen] + 1))}
+        lowered = {c: i for i, c in enumerate(cart(ls[cen] - 1))} if ls[cen] else {}
+        for x in range(3):
+            for e in range(n[0] * n[1] * n[2] * n[3]):
+                idx = [e // (n[1] * n[2] * n[3]), e // (n[2] * n[3]) % n[1], e // n[3] % n[2],
+                       e % n[3]]
+                lmn = list(carts[idx[cen]])
+
+                def at(which, comps, step):
+                    c = list(lmn)
+                    c[x] += step
+                    ii, nn = list(idx), list(n)
+                    ii[cen], nn[cen] = comps[tuple(c)], len(comps)
+                    return outs[which][((ii[0] * nn[1] + ii[1]) * nn[2] + ii[2]) * nn[3] + ii[3]]
+                word = at(cen, raised, 1)
+                dn = at(3 + cen, lowered, -1) if lmn[x] else NO_LOWERED
+                assert word < 65536 and (dn < NO_LOWERED or not lmn[x]) and lmn[x] <= 2
+                table.append(word | dn << 16 | (1 << 31 if lmn[x] == 2 else 0))
+    return table
+
+
 def emit_grad(cls):
     p = grad_program(cls)
     tag = "".join(map(str, cls))
@@ -220,11 +254,6 @@ def emit_grad(cls):
     segs = [x for s in p["vseg"] for x in (s[0], s[2], s[3], s[5])]
     hop = [x for o in p["hops"] for x in (o[0] | (o[1] << 16), o[2] | (o[3] << 16))]
     acc = [s | (k << 16) for s, k in zip(p["acc_slot"], p["acc_kind"])]
-    out_all, out_off = [], []
-    for o in p["outs"]:
-        out_off.append(len(out_all) if o is not None else -1)
-        if o is not None:
-            out_all.extend(o)
     lines = [f"// generated by gen_grad.py -- gradient warp program of class ({la}{lb}|{lc}{ld})",
              "#pragma once", "namespace gs {",
              arr("unsigned int __align__(16)", f"g{tag}_vrec", p["vrec"]),
@@ -233,20 +262,18 @@ def emit_grad(cls):
              arr("unsigned short", f"g{tag}_accpos", p["acc_pos"]),
              arr("unsigned int", f"g{tag}_hop", hop),
              arr("int", f"g{tag}_hlev", p["hlev"]),
-             arr("unsigned short", f"g{tag}_out", out_all),
-             arr("int", f"g{tag}_outoff", out_off),
+             arr("unsigned int", f"g{tag}_con", contraction_table(cls, p["outs"])),
              f"template <> struct GradProg<{la}, {lb}, {lc}, {ld}> {{",
              f"  static constexpr int L = {p['L']}, NACC = {p['nacc']}, NVSLOT = {p['nvslot']};",
              f"  static constexpr int NVSEG = {len(p['vseg'])}, HSIZE = {p['hsize']}, "
              f"NHLEV = {len(p['hlev']) - 1};",
-             f"  static __device__ const int* out_off() {{ return g{tag}_outoff; }}",
              f"  static __device__ const uint4* vrec() {{ return reinterpret_cast<const uint4*>(g{tag}_vrec); }}",
              f"  static __device__ const int* vseg() {{ return g{tag}_vseg; }}",
              f"  static __device__ const unsigned int* acc() {{ return g{tag}_acc; }}",
              f"  static __device__ const unsigned short* accpos() {{ return g{tag}_accpos; }}",
              f"  static __device__ const unsigned int* hop() {{ return g{tag}_hop; }}",
              f"  static __device__ const int* hlev() {{ return g{tag}_hlev; }}",
-             f"  static __device__ const unsigned short* out() {{ return g{tag}_out; }}",
+             f"  static __device__ const unsigned int* con() {{ return g{tag}_con; }}",
              "};", "}  // namespace gs", ""]
     return "\n".join(lines), p
 

@@ -94,6 +94,13 @@ def split_forms(cls, precision, heavy):
 # pipe for (measured: the same for one warp as for four, so a scheduler has no more FP64
 # throughput than one busy warp uses).
 WORK_LEVELS = 18          # thresholds 1, 2, 4, ... 2^17 of a work profile
+# quartets of fewer than 2^MANY_LEVEL primitive quartets share a warp's set-up, MANY_TASKS at
+# most, in classes up to total angular momentum MANY_LMAX (csrc/eri_wide.cuh)
+MANY_LEVEL, MANY_TASKS, MANY_LMAX = 4, 8, 6
+# and as long as this many warps a scheduler remain: block writing brings up to 15 primitive
+# quartets a quartet, the adjoint and Fock digestion of molecules one to five ((H2O)6/6-31G*
+# gradient 10.4 ms with 4, 10.9 with 16; 300,000 random quartets' blocks 12.9 and 12.7)
+MANY_WARPS = {"jk": 4, "write": 16}
 COOP_LEVEL = COOP_PRIM_QUARTETS.bit_length() - 1     # one warp alone takes fewer than that
 _LEVELS = 1 << np.arange(WORK_LEVELS, dtype=np.int64)
 MIN_LATENCY = 600.0       # slots (20 us) below which a long quartet is not worth splitting
@@ -151,47 +158,51 @@ def total_slots(segments, profiles, precision, kind, schedulers):
     return t / (32 * schedulers)
 
 
-def class_plan(cls, precision, kind, n, profile, limit, built):
+def class_plan(cls, precision, kind, n, profile, limit, built, schedulers=608):
     """[(form, first, count, latency)] for a class segment of n tasks sorted by descending
     primitive-quartet count w, when no form has been chosen for the class.  Tasks of a tier
     take at most ``limit`` slots in its form, so that no lane, warp or block walks its
     primitive quartets while the rest of the GPU has finished; ``latency`` is the tier's
     longest task's.  The lightest tier runs one thread per quartet where the class's
-    accumulators allow it, else one warp per quartet; heavier ones a warp (thread code, or
-    the warp forms), a block of eight warps, and a cluster of eight blocks per quartet.
-    Thresholds are powers of two (the profile's)."""
+    accumulators allow it, else one warp per quartet (several quartets of few primitive
+    quartets: form | per << 8); heavier ones a warp (thread code, or the warp forms), a block
+    of eight warps, and a cluster of eight blocks per quartet.  Thresholds are powers of two
+    (the profile's)."""
     nacc = class_sizes(cls)[0]
     lane, alone, warp = class_costs(cls, precision)
     has = lambda form: bool(built & (1 << (form - 1)))   # noqa: E731
     most = (496 if precision == 32 else 96 if cls[3] == 0 else 54) if kind == "jk" else \
         (96 if precision == 32 else 27)
-    # (form, slots per primitive quartet, fixed slots), lightest tier first
+    # (form, slots per primitive quartet, fixed slots, largest level), lightest tier first
     tiers = []
     if has(THREAD_FORM) and nacc <= most:
-        tiers.append((THREAD_FORM, alone, 0.0))
+        tiers.append((THREAD_FORM, alone, 0.0, WORK_LEVELS))
         if nacc <= 27:
-            tiers.append((SPLIT_FORM, alone / 32, 10.0 * nacc))
+            tiers.append((SPLIT_FORM, alone / 32, 10.0 * nacc, WORK_LEVELS))
     if not tiers or nacc > 27:
         for form in ((GROUPED_FORM,) if nacc <= 96 else ()) + (STACKED_FORM, WARP_FORM):
             if has(form):
-                tiers.append((form, warp, 0.0))
+                if sum(cls) <= MANY_LMAX:
+                    # several light quartets a warp, as long as enough warps remain
+                    per = min(MANY_TASKS, n // (MANY_WARPS[kind] * schedulers))
+                    if per > 1:
+                        tiers.append((form | (per << 8), per * warp, 0.0, MANY_LEVEL))
+                tiers.append((form, warp, 0.0, COOP_LEVEL))
                 break
         if has(COOP_FORM):
-            tiers.append((COOP_FORM, warp / 4, 0.0))
+            tiers.append((COOP_FORM, warp / 4, 0.0, WORK_LEVELS))
         if has(CLUSTER_FORM):
-            tiers.append((CLUSTER_FORM, warp / 32, 0.0))
+            tiers.append((CLUSTER_FORM, warp / 32, 0.0, WORK_LEVELS))
     if not tiers:
         return [(0, 0, n, 0.0)]
     counts = profile[1]
     top = max([k for k in range(WORK_LEVELS) if counts[k]], default=0)    # w < 2^(top+1)
     out, end = [], n
-    for i, (form, slots, fixed) in enumerate(tiers):
+    for i, (form, slots, fixed, most) in enumerate(tiers):
         if i + 1 == len(tiers):
             k = WORK_LEVELS
         else:
-            k = max(1, int(np.floor(np.log2(max(2.0, limit / slots)))))
-            if form in (GROUPED_FORM, STACKED_FORM, WARP_FORM):
-                k = min(k, COOP_LEVEL)
+            k = min(most, max(1, int(np.floor(np.log2(max(2.0, limit / slots))))))
         first = counts[k] if k < WORK_LEVELS else 0
         if first < end:
             out.append((form, first, end - first, fixed + slots * 2.0 ** min(k, top + 1)))
@@ -210,8 +221,8 @@ def launch_plan(engine_like, precision, kind, classes=None, share=1.0):
     if key not in plans:
         sch = 4 * torch.cuda.get_device_properties(e.tasks.device).multi_processor_count
         slots = {p: total_slots(e.segments, e.profiles, p, kind, sch) for p in (64, 32)}
-        plans[key] = (slots, {})
-    slots, cached = plans[key]
+        plans[key] = (slots, sch, {})
+    slots, sch, cached = plans[key]
     limit = max(MIN_LATENCY, LATENCY_SHARE * share * slots[precision])
     out = []
     for (cls, s, t), heavy, prof in zip(e.segments, e.heavy, e.profiles):
@@ -224,7 +235,7 @@ def launch_plan(engine_like, precision, kind, classes=None, share=1.0):
         else:
             if (cls, limit) not in cached:
                 cached[cls, limit] = class_plan(cls, precision, kind, t - s, prof, limit,
-                                                L.gs_class_variants(*cls, precision))
+                                                L.gs_class_variants(*cls, precision), sch)
             parts = cached[cls, limit]
         out += [(cls, s + first, count, form, lat) for form, first, count, lat in parts if count > 0]
     return sorted(out, key=lambda x: -x[4])

@@ -19,7 +19,8 @@ import torch
 
 from . import _lib, scf
 from .basis import ShellBasis
-from .engine import DeviceShells, HeavyLane, JKEngine, QuartetBatch
+from .engine import (MANY_LEVEL, MANY_TASKS, MANY_WARPS, SIDE_STREAMS, DeviceShells, HeavyLane,
+                     JKEngine, QuartetBatch)
 from .fock import FockMatrixRestrictedGPU
 from .hamiltonian import one_electron
 from .molecules import Molecule, shell_basis
@@ -136,8 +137,16 @@ def tune_eri_gradient(sb, engine: JKEngine, shell_atom, P, natom, reps=3):
 
 def one_electron_gradient_kernel(sb, mol, shell_atom, P, W, device="cuda"):
     """The one-electron gradient terms in one launch (gs_one_electron_grad)."""
-    ds = DeviceShells(sb, device)
-    dev = ds.device
+    grad, _ = _one_electron_launch(DeviceShells(sb, device), mol, shell_atom, P, W)
+    return grad.view(-1, 3).cpu().numpy()
+
+
+def _one_electron_launch(ds, mol, shell_atom, P, W, lane=None):
+    """The launch of one_electron_gradient_kernel: its 3 natom results on the device and the
+    buffers that it reads.  With ``lane`` (a HeavyLane) it goes to the lane's last side
+    stream, which forks from the caller's after the uploads; the buffers are then to be held
+    until the lane's join."""
+    dev, sb = ds.device, ds.host
     i, j = np.tril_indices(sb.nshell)
     t = lambda a, dt: torch.as_tensor(np.ascontiguousarray(a, dtype=dt)).to(dev)
     pairs = t(np.stack([i, j], 1), np.int32)
@@ -151,9 +160,10 @@ def one_electron_gradient_kernel(sb, mol, shell_atom, P, W, device="cuda"):
                                       _lib.ptr(ds.expo), _lib.ptr(ds.coef), _lib.ptr(ds.comp_scale),
                                       _lib.ptr(ds.func_off), _lib.ptr(sa_d), len(i), _lib.ptr(pairs),
                                       sb.nbf, len(mol.symbols), _lib.ptr(xyz_d), _lib.ptr(z_d),
-                                      _lib.ptr(p_d), _lib.ptr(w_d), _lib.ptr(grad), _lib.stream()),
+                                      _lib.ptr(p_d), _lib.ptr(w_d), _lib.ptr(grad),
+                                      lane.stream(SIDE_STREAMS - 1) if lane else _lib.stream()),
                "gs_one_electron_grad")
-    return grad.view(-1, 3).cpu().numpy()
+    return grad, (ds, pairs, sa_d, xyz_d, z_d, p_d, w_d)
 
 
 def nuclear_repulsion_gradient(mol):
@@ -194,26 +204,41 @@ def eri_gradient(sb, engine: JKEngine, shell_atom, P, natom, classes=None, host=
     base = engine.tasks.data_ptr()
     lane = HeavyLane(dev)
     inf = float("inf")
-    for (cls, s, e), heavy in zip(engine.segments, engine.heavy):
+    launches = []
+    schedulers = 4 * torch.cuda.get_device_properties(dev).multi_processor_count
+    for (cls, s, e), heavy, (_, counts) in zip(engine.segments, engine.heavy, engine.profiles):
         if classes is not None and cls not in classes:
             continue
-        thread = L.gs_eri_grad_class_form(*cls) == 1
-        # a thread-form class's quartets with many primitive quartets (the task list's
-        # prefix) in the split form, on the side stream beside the other launches
-        h = heavy[0] if GRAD_SPLIT and thread else 0
-        bands = [(64, mixed_cut, inf), (32, 0.0, mixed_cut)] \
-            if (mixed_cut is not None and thread) else [(64, 0.0, inf)]
+        n = e - s
+        if L.gs_eri_grad_class_form(*cls) != 1:
+            # warp form: quartets of few primitive quartets share a warp's set-up
+            h = counts[MANY_LEVEL]
+            per = max(1, min(MANY_TASKS, (n - h) // (MANY_WARPS["jk"] * schedulers)))
+            parts = [(0, 0, h), (per << 8, h, n - h)]
+            bands = [(64, 0.0, inf)]
+        else:
+            # a thread-form class's quartets with many primitive quartets (the task list's
+            # prefix) in the split form
+            h = heavy[0] if GRAD_SPLIT else 0
+            parts = [(3, 0, h), (0, h, n - h)]
+            bands = [(64, mixed_cut, inf), (32, 0.0, mixed_cut)] if mixed_cut is not None else \
+                [(64, 0.0, inf)]
         for prec, lo, hi in bands:
             prims = engine.pairs.p64 if prec == 64 else engine.pairs.p32
-            for form, first, count, side in ((3, 0, h, True), (0, h, e - s - h, False)):
-                if count <= 0:
-                    continue
-                _lib.check(L.gs_eri_grad_band(
-                    *cls, form, prec, _lib.ptr(engine.pairs.rec), _lib.ptr(prims),
-                    _lib.ptr(engine.ds.comp_scale), _lib.ptr(engine.ds.func_off), _lib.ptr(sa),
-                    count, base + (s + first) * 8, sb.nbf, natom, _lib.ptr(pt), sb.nshell,
-                    _lib.ptr(dmax), thr, lo, hi, _lib.ptr(grad),
-                    lane.stream() if side else _lib.stream()), f"gs_eri_grad_band{cls}")
+            for form, first, count in parts:
+                if count > 0:
+                    launches.append((cls, form, prec, prims, first + s, count, lo, hi))
+    # largest angular momenta first: a warp of theirs walks its quartet's primitives the
+    # longest, with few quartets to fill the GPU, so the launches of the smaller classes run
+    # beside them on the other streams
+    launches.sort(key=lambda x: -sum(x[0]))
+    for i, (cls, form, prec, prims, first, count, lo, hi) in enumerate(launches):
+        _lib.check(L.gs_eri_grad_band(
+            *cls, form, prec, _lib.ptr(engine.pairs.rec), _lib.ptr(prims),
+            _lib.ptr(engine.ds.comp_scale), _lib.ptr(engine.ds.func_off), _lib.ptr(sa),
+            count, base + first * 8, sb.nbf, natom, _lib.ptr(pt), sb.nshell,
+            _lib.ptr(dmax), thr, lo, hi, _lib.ptr(grad), lane.lane(i)),
+            f"gs_eri_grad_band{cls}")
     lane.join()
     return grad.view(natom, 3).cpu().numpy() if host else grad.view(natom, 3)
 
@@ -313,11 +338,14 @@ def gradient_from_state(st: RHFState, screen_thr=GRAD_SCREEN_THR, mixed_cut=GRAD
     ``screen_thr`` / ``mixed_cut``: density screening and FP32 recursions for the quartets
     with small density-weighted bounds (eri_gradient; 0.0 / None: every quartet in FP64)."""
     sa = shell_atoms(st.mol, st.sb)
-    g = one_electron_gradient_kernel(st.sb, st.mol, sa, st.P, st.W)
-    g += eri_gradient(st.sb, st.engine, sa, st.P, len(st.mol.symbols), screen_thr=screen_thr,
-                      mixed_cut=mixed_cut)
-    g += nuclear_repulsion_gradient(st.mol)
-    return g
+    lane = HeavyLane(st.engine.dev)
+    # the one-electron kernel on a side stream, beside the adjoint kernels
+    one, held = _one_electron_launch(st.engine.ds, st.mol, sa, st.P, st.W, lane)
+    g = eri_gradient(st.sb, st.engine, sa, st.P, len(st.mol.symbols), host=False,
+                     screen_thr=screen_thr, mixed_cut=mixed_cut)
+    lane.join()
+    del held
+    return (one.view(-1, 3) + g).cpu().numpy() + nuclear_repulsion_gradient(st.mol)
 
 
 def rhf_energy_gradient(mol, basis="6-31G", threshold=1e-12, schwarz_thr=1e-14,

@@ -83,7 +83,10 @@ int gs_class_variant(int la, int lb, int lc, int ld, int precision);
  * quartets (the heavy prefix of a class's task list, sorted by descending primitive work)
  * in the split form where the class runs one thread per quartet, and in the cooperative
  * form where it runs one warp per quartet (warp, grouped or stacked), the heaviest in the
- * cluster form.  The cooperative and cluster forms take host task counts only.  Negative status on a bad class or precision.  No reference counterpart. */
+ * cluster form.  The cooperative and cluster forms take host task counts only.  Bits 16.. give
+ * the number of consecutive tasks a warp of the warp, grouped and stacked forms takes (1-8, 0 =
+ * one; classes of total angular momentum above 6 always one): for tasks of few primitive
+ * quartets, whose set-up then fills the warp's lanes.  Negative status on a bad class or precision.  No reference counterpart. */
 int gs_class_form(int la, int lb, int lc, int ld, int precision);
 
 /* K0 shell-pair builder.  Replaces the per-primitive-quartet prologue of
@@ -270,8 +273,10 @@ int gs_eri_grad(int la, int lb, int lc, int ld, const void* pair_rec, const void
 /* gs_eri_grad with an explicit kernel form for this call: 0 = the class's configured form,
  * 1 = one thread per quartet, 2 = one warp per quartet, 3 = split (the thread code with one
  * warp per quartet over its primitive quartets, for quartets with many of them); forms 1
- * and 3 exist for classes of total angular momentum <= 3 (else GS_ERR_ARG).  No reference
- * counterpart (see gs_eri_grad_contract). */
+ * and 3 exist for classes of total angular momentum <= 3 (else GS_ERR_ARG).  Bits 8.. of form
+ * give the consecutive tasks a warp of the warp form takes (1-8, 0 = one; one for the classes
+ * whose accumulators live in shared memory).  No reference counterpart (see
+ * gs_eri_grad_contract). */
 int gs_eri_grad_form(int la, int lb, int lc, int ld, int form, const void* pair_rec,
                      const void* prim64, const double* comp_scale, const int* func_off,
                      const int* shell_atom, int ntask, const int* tasks, int nbf, int natom,

@@ -25,7 +25,8 @@ def test_tiers_tile_the_segment(cls, precision, kind):
         at = 0
         for form, first, count, latency in plan:
             assert first == at and count > 0 and latency >= 0
-            assert form == 0 or built & (1 << (form - 1))
+            assert form == 0 or built & (1 << ((form & 255) - 1))
+            assert form >> 8 in range(engine.MANY_TASKS + 1)
             at += count
         assert at == n
         forms = [p[0] for p in plan]
@@ -118,3 +119,85 @@ def test_cluster_form_matches_warp_form(gpu_lib, precision, tol):
     finally:
         autotune.reset(batch.segments)
     assert float((out - ref).abs().max()) <= tol * float(ref.abs().max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+def test_many_quartets_a_warp(gpu_lib, precision):
+    """Blocks are the same bits with one to eight quartets a warp, J/K the same sums up to the
+    atomics' order: tasks of zero (screened out) to 36 primitive quartets, counts that are no
+    multiple of the warp's, screened tasks among them."""
+    from gaussium_gb300 import _lib
+    from gaussium_gb300.workloads import random_shell_quartets
+    sb, _, _ = random_shell_quartets(8, seed=11, box_angstrom=6.0, kmax=3)
+    ns = sb.nshell
+    q = np.random.default_rng(4).integers(0, ns, (3001, 4))
+    ds = engine.DeviceShells(sb)
+    batch = engine.QuartetBatch(ds, q, want32=True, max_exp=engine.PRIM_SCREEN)
+    assert any(prof[1][0] < e - s for (_, s, e), prof in zip(batch.segments, batch.profiles))
+    eng = engine.JKEngine(sb, schwarz_thr=0.0, max_exp=engine.PRIM_SCREEN)
+    n = sb.nbf
+    p = np.random.default_rng(5).standard_normal((n, n))
+    pt = torch.as_tensor(p + p.T).cuda()
+    dmax = eng.shell_dmax([pt])
+    for form in (engine.WARP_FORM, engine.GROUPED_FORM, engine.STACKED_FORM):
+        ref = None
+        for per in (0, 1, 2, 5, 8):
+            out = torch.full((batch.total,), float("nan"), dtype=torch.float64, device="cuda")
+            j = torch.zeros((n, n), dtype=torch.float64, device="cuda")
+            k = torch.zeros_like(j)
+            for cls, s, e in batch.segments:
+                f = form if gpu_lib.gs_class_variants(*cls, precision) & (1 << (form - 1)) else \
+                    engine.WARP_FORM
+                _lib.check(gpu_lib.gs_eri_blocks(
+                    *cls, precision | f << 8 | per << 16, _lib.ptr(batch.pairs.rec),
+                    _lib.ptr(batch.pairs.prims(precision)), _lib.ptr(ds.comp_scale), e - s,
+                    batch.tasks.data_ptr() + s * engine.WRITE_TASK, _lib.ptr(out),
+                    _lib.stream()), "gs_eri_blocks")
+            for cls, s, e in eng.segments:
+                f = form if gpu_lib.gs_class_variants(*cls, precision) & (1 << (form - 1)) else \
+                    engine.WARP_FORM
+                _lib.check(gpu_lib.gs_fock_jk(
+                    *cls, precision | f << 8 | per << 16, _lib.ptr(eng.pairs.rec),
+                    _lib.ptr(eng.pairs.prims(precision)), _lib.ptr(eng.ds.comp_scale),
+                    _lib.ptr(eng.ds.func_off), ns, n, e - s, eng.tasks.data_ptr() + 8 * s,
+                    _lib.ptr(pt), _lib.ptr(j), 1, _lib.ptr(pt), _lib.ptr(k), _lib.ptr(dmax), 1e-6,
+                    1e-5, float("inf"), _lib.stream()), "gs_fock_jk")
+            got = (out, j, k)
+            if ref is None:
+                ref = got
+                assert not bool(torch.isnan(out).any())
+            assert torch.equal(out, ref[0]), (form, per)
+            for x, y in zip(got[1:], ref[1:]):
+                assert float((x - y).abs().max()) <= 1e-13 * float(y.abs().max())
+    assert gpu_lib.gs_eri_blocks(0, 0, 0, 0, precision | 2 << 8 | 9 << 16, _lib.ptr(batch.pairs.rec),
+                                 _lib.ptr(batch.pairs.p64), _lib.ptr(ds.comp_scale), 0, None,
+                                 _lib.ptr(ref[0]), None) == 1
+
+
+@pytest.mark.gpu
+def test_gradient_tasks_a_warp(gpu_lib):
+    """The warp form of the adjoint with one to eight quartets a warp, screened ones among
+    them: the same gradient up to the atomics' order."""
+    from gaussium_gb300 import _lib
+    from gaussium_gb300.molecules import shell_basis, water_cluster
+    mol = water_cluster(2, seed=1)
+    sb = shell_basis(mol, "6-31G*")
+    eng = engine.JKEngine(sb, schwarz_thr=1e-12)
+    from gaussium_gb300.gradient import shell_atoms
+    sa = torch.as_tensor(shell_atoms(mol, sb).astype(np.int32)).cuda()
+    p = np.random.default_rng(2).standard_normal((sb.nbf, sb.nbf)) * 0.1
+    pt = torch.as_tensor(p + p.T).cuda()
+    dmax = eng.shell_dmax([pt])
+    ref = None
+    for per in (0, 1, 3, 8):
+        g = torch.zeros(18, dtype=torch.float64, device="cuda")
+        for cls, s, e in eng.segments:
+            _lib.check(gpu_lib.gs_eri_grad_band(
+                *cls, 2 | per << 8, 64, _lib.ptr(eng.pairs.rec), _lib.ptr(eng.pairs.p64),
+                _lib.ptr(eng.ds.comp_scale), _lib.ptr(eng.ds.func_off), _lib.ptr(sa), e - s,
+                eng.tasks.data_ptr() + 8 * s, sb.nbf, 6, _lib.ptr(pt), sb.nshell, _lib.ptr(dmax),
+                1e-7, 0.0, float("inf"), _lib.ptr(g), _lib.stream()), "gs_eri_grad_band")
+        ref = g if ref is None else ref
+        assert float((g - ref).abs().max()) <= 1e-12 * float(ref.abs().max())
+    assert abs(float(g.view(6, 3).sum())) < 1e-10          # translational invariance
