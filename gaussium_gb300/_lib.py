@@ -42,6 +42,7 @@ _SIGS = {
     "gs_class_variant": (I, [I, I, I, I, I]),
     "gs_set_class_variant": (I, [I, I, I, I, I, I]),
     "gs_boys_eval": (I, [I, I, I, P, P, P]),
+    "gs_rsqrt_eval": (I, [I, P, P, P]),
     "gs_fma_probe": (I, [I, I, I, I, P, P]),
     "gs_fma_probe_lanes": (I, [I, I, I, I, I, P, P]),
     "gs_one_electron": (I, [P, P, P, P, P, P, P, I, P, I, I, P, P, P, P, P, P]),

@@ -294,6 +294,11 @@ __global__ void k_boys(int n, const double* __restrict__ t, double* __restrict__
     for (int m = 0; m <= M; ++m) F[(size_t)i * (M + 1) + m] = (double)f[m];
 }
 
+__global__ void k_rsqrt(int n, const double* __restrict__ x, double* __restrict__ y) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) y[i] = gs::gs_rsqrt(x[i]);
+}
+
 // Split a class's quartet tasks by their density-weighted Schwarz estimate
 //   est = qmax_bra * qmax_ket * max |P| over the quartet's six shell blocks
 // into an FP64 list (est >= cut), an FP32 list (thr <= est < cut) and dropped (est < thr).
@@ -751,6 +756,13 @@ int gs_boys_eval(int m, int precision, int n, const double* t, double* F, void* 
         default: return GS_ERR_ARG;
     }
 #undef GS_BM
+    return check_launch();
+}
+
+int gs_rsqrt_eval(int n, const double* x, double* y, void* stream) {
+    if (n < 0 || !x || !y) return GS_ERR_ARG;
+    if (n == 0) return GS_OK;
+    k_rsqrt<<<(n + 127) / 128, 128, 0, S(stream)>>>(n, x, y);
     return check_launch();
 }
 

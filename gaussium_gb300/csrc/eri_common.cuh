@@ -59,8 +59,69 @@ template <typename T> struct VrrCoef {
 template <int LA, int LB, int LC, int LD> struct ClassGen;
 
 // ------------------------------------------------------------------ math helpers
+// FP64 sums and products as fused multiply-adds.  On this part a DADD or a DMUL holds the FP64
+// pipe 19 % longer than a DFMA (79.5 against 67 cycles a warp instruction, eight independent
+// chains), so a + b is fma(a, 1, b) and a b is fma(a, b, 0), the same roundings (only the sign
+// of an exact zero product is lost).  The one and the zero come from constant memory, which
+// the compiler cannot fold back and the instruction takes as an operand.
+#if defined(__CUDACC__)
+static __constant__ double gs_one_zero[2] = {1.0, 0.0};
+#endif
+GS_HD GS_INLINE double gs_fma(double a, double b, double c) {
+#if defined(__CUDA_ARCH__)
+    return fma(a, b, c);
+#else
+    return a * b + c;
+#endif
+}
+GS_HD GS_INLINE double gs_add(double a, double b) {
+#if defined(__CUDA_ARCH__)
+    return fma(a, gs_one_zero[0], b);
+#else
+    return a + b;
+#endif
+}
+GS_HD GS_INLINE double gs_sub(double a, double b) {
+#if defined(__CUDA_ARCH__)
+    return fma(-b, gs_one_zero[0], a);
+#else
+    return a - b;
+#endif
+}
+GS_HD GS_INLINE double gs_mul(double a, double b) {
+#if defined(__CUDA_ARCH__)
+    return fma(a, b, gs_one_zero[1]);
+#else
+    return a * b;
+#endif
+}
+GS_HD GS_INLINE float gs_fma(float a, float b, float c) {
+#if defined(__CUDA_ARCH__)
+    return fmaf(a, b, c);
+#else
+    return a * b + c;
+#endif
+}
+GS_HD GS_INLINE float gs_add(float a, float b) { return a + b; }
+GS_HD GS_INLINE float gs_sub(float a, float b) { return a - b; }
+GS_HD GS_INLINE float gs_mul(float a, float b) { return a * b; }
+GS_HD GS_INLINE double norm2(double x, double y, double z) {
+    return gs_fma(z, z, gs_fma(y, y, gs_mul(x, x)));
+}
+GS_HD GS_INLINE float norm2(float x, float y, float z) { return x * x + y * y + z * z; }
+
+// 1 / sqrt(x): the hardware's 20-bit approximation y and one step of Householder's method of
+// second order, y (1 + r/2 + 3/8 r^2) with r = 1 - x y^2, whose error is 5/16 r^3 < 2^-58
+// before rounding; five FP64 instructions.  Zero, subnormal and non-finite x, and negative
+// ones, go to the library's function.
 GS_HD GS_INLINE double gs_rsqrt(double x) {
 #if defined(__CUDA_ARCH__)
+    if ((unsigned)__double2hiint(x) - 0x00100000u < 0x7fe00000u) {
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+        const double r = fma(-gs_mul(x, y), y, 1.0);
+        return fma(gs_mul(y, r), fma(0.375, r, 0.5), y);
+    }
     return rsqrt(x);
 #else
     return 1.0 / std::sqrt(x);
@@ -200,8 +261,8 @@ template <unsigned N> GS_HD GS_INLINE bool below(float t) { return t < (float)N;
 // whose last bit is worth one.  k is held to the table whatever t is.
 GS_HD GS_INLINE int boys_row(double t, double& d) {
     const double magic = 6755399441055744.0;
-    const double kf = t * BOYS_INV_H + magic;
-    d = (kf - magic) * (1.0 / BOYS_INV_H) - t;
+    const double kf = gs_fma(t, BOYS_INV_H, magic);
+    d = gs_fma(gs_sub(kf, magic), 1.0 / BOYS_INV_H, -t);
 #if defined(__CUDA_ARCH__)
     return min((unsigned)__double2loint(kf), (unsigned)(BOYS_ROWS - 1));
 #else
@@ -229,7 +290,7 @@ GS_HD GS_INLINE void boys_small(double t, double pref, double* __restrict__ F) {
         f = fma(f, d, g23.y);
         f = fma(f, d, g23.x);
         f = fma(f, d, g01.y);
-        F[M] = fma(f, d, g01.x) * pref;
+        F[M] = gs_mul(fma(f, d, g01.x), pref);
         if (M > 0) {
             const double2* x = reinterpret_cast<const double2*>(g_boys_expt) + 4 * k;
             const double2 x01 = __ldg(x), x23 = __ldg(x + 1), x45 = __ldg(x + 2), x67 = __ldg(x + 3);
@@ -238,9 +299,12 @@ GS_HD GS_INLINE void boys_small(double t, double pref, double* __restrict__ F) {
             e = fma(e, d, x23.y);
             e = fma(e, d, x23.x);
             e = fma(e, d, x01.y);
-            const double et = fma(e, d, x01.x) * pref;
-            const double t2 = t + t;
-            GS_UNROLL for (int m = M; m >= 1; --m) F[m - 1] = (t2 * F[m] + et) * (1.0 / (2 * m - 1));
+            const double et = gs_mul(fma(e, d, x01.x), pref);
+            const double t2 = twice(t);
+            GS_UNROLL for (int m = M; m >= 1; --m) {
+                const double x = fma(t2, F[m], et);
+                F[m - 1] = m == 1 ? x : gs_mul(x, 1.0 / (2 * m - 1));
+            }
         }
         return;
     }
@@ -380,10 +444,11 @@ GS_HD GS_INLINE void boys(T t, T pref, T* __restrict__ F) {
         else boys_small32<M>(t, pref, F);
     } else {
         const T rs = gs_rsqrt(t);
-        F[0] = pref * T(0.88622692545275801365) * rs;   // sqrt(pi)/2
+        F[0] = gs_mul(gs_mul(pref, T(0.88622692545275801365)), rs);   // sqrt(pi)/2
         if (M > 0) {
-            const T hit = T(0.5) * rs * rs;
-            GS_UNROLL for (int m = 0; m < M; ++m) F[m + 1] = (T(2 * m + 1) * hit) * F[m];
+            const T hit = gs_mul(gs_mul(T(0.5), rs), rs);
+            GS_UNROLL for (int m = 0; m < M; ++m)
+                F[m + 1] = gs_mul(m == 0 ? hit : gs_mul(T(2 * m + 1), hit), F[m]);
         }
     }
 }
@@ -394,46 +459,46 @@ template <int LA, int LB, int LC, int LD, typename T>
 GS_HD GS_INLINE void eri_primitive(const PrimRec<T>& P, const PrimRec<T>& Q,
                                    T* __restrict__ acc) {
     using G = ClassGen<LA, LB, LC, LD>;
-    const T pq = P.p + Q.p;
-    const T PQx = Q.Px - P.Px, PQy = Q.Py - P.Py, PQz = Q.Pz - P.Pz;
-    const T r2 = PQx * PQx + PQy * PQy + PQz * PQz;
+    const T pq = gs_add(P.p, Q.p);
+    const T PQx = gs_sub(Q.Px, P.Px), PQy = gs_sub(Q.Py, P.Py), PQz = gs_sub(Q.Pz, P.Pz);
+    const T r2 = norm2(PQx, PQy, PQz);
 #if defined(__CUDA_ARCH__) && defined(GS_BOYS_ORDER)
     if constexpr (G::L == 0 && sizeof(T) == 8 && kBoysOrder == 0) {
         // (ss|ss): with X = p q R^2, T = X / (p + q); far quartets (T >= threshold) need only
         // 1/sqrt(X), near ones only 1/sqrt(p + q), so one reciprocal square root serves a
         // warp that holds both, and the far lanes add nothing to the near lanes' work
         constexpr double thr = kBoysAsym64[0];
-        const T X = P.p * Q.p * r2;
+        const T X = gs_mul(gs_mul(P.p, Q.p), r2);
         const T u = fma(-thr, pq, X);
         const bool far = __double2hiint(u) >= 0;
         const T y = gs_rsqrt(far ? X : pq);
         T f = T(0.88622692545275801365);                 // sqrt(pi)/2
         if (!far) {
             double d;
-            const int k = boys_row(X * (y * y), d);
+            const int k = boys_row(gs_mul(X, gs_mul(y, y)), d);
             const double2* g = reinterpret_cast<const double2*>(g_boys_taylor) + 4 * k;
             const double2 g01 = __ldg(g), g23 = __ldg(g + 1), g45 = __ldg(g + 2), g67 = __ldg(g + 3);
             f = fma(fma(fma(fma(fma(fma(g67.x, d, g45.y), d, g45.x), d, g23.y), d, g23.x), d,
                         g01.y), d, g01.x);
         }
-        acc[0] = fma(P.Kp * Q.Kp * y, f, acc[0]);
+        acc[0] = fma(gs_mul(gs_mul(P.Kp, Q.Kp), y), f, acc[0]);
         return;
     }
 #endif
     const T rs = gs_rsqrt(pq);
-    const T ipq = rs * rs;
-    const T wq = Q.p * ipq, wp = P.p * ipq;
-    const T t = P.p * wq * r2;
+    const T ipq = gs_mul(rs, rs);
+    const T wq = gs_mul(Q.p, ipq), wp = gs_mul(P.p, ipq);
+    const T t = gs_mul(gs_mul(P.p, wq), r2);
     T F[G::L + 1];
-    boys<G::L, T>(t, P.Kp * Q.Kp * rs, F);
+    boys<G::L, T>(t, gs_mul(gs_mul(P.Kp, Q.Kp), rs), F);
     VrrCoef<T> c;
     c.PAx = P.PAx; c.PAy = P.PAy; c.PAz = P.PAz;
-    c.WPx = wq * PQx; c.WPy = wq * PQy; c.WPz = wq * PQz;
+    c.WPx = gs_mul(wq, PQx); c.WPy = gs_mul(wq, PQy); c.WPz = gs_mul(wq, PQz);
     c.QCx = Q.PAx; c.QCy = Q.PAy; c.QCz = Q.PAz;
-    c.WQx = -wp * PQx; c.WQy = -wp * PQy; c.WQz = -wp * PQz;
+    c.WQx = gs_mul(-wp, PQx); c.WQy = gs_mul(-wp, PQy); c.WQz = gs_mul(-wp, PQz);
     c.i2p = P.i2p; c.i2q = Q.i2p;
-    c.rp2 = wq * P.i2p; c.rq2 = wp * Q.i2p;
-    c.i2pq = T(0.5) * ipq;
+    c.rp2 = gs_mul(wq, P.i2p); c.rq2 = gs_mul(wp, Q.i2p);
+    c.i2pq = gs_mul(T(0.5), ipq);
     G::vrr(F, c, acc);
 }
 

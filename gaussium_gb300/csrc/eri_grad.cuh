@@ -115,7 +115,7 @@ __device__ __forceinline__ void grad_items(const double* __restrict__ sC,
                     ra = __ldg(vrec + 2 * (noff + n + 32));
                     rb = __ldg(vrec + 2 * (noff + n + 32) + 1);
                 }
-                double r = c[x.y >> 16] * node[x.y & 0xffff];
+                double r = gs_mul(c[x.y >> 16], node[x.y & 0xffff]);
                 r = fma(c[x.z >> 16], node[x.z & 0xffff], r);
                 if (nt > 2) r = fma(c[x.w >> 16], node[x.w & 0xffff], r);
                 if (nt > 3) r = fma(c[y.x >> 16], node[y.x & 0xffff], r);
@@ -186,10 +186,8 @@ __device__ __forceinline__ void grad_tail(const GradArgs& a, const int2& task, c
     constexpr int ND = (LD + 1) * (LD + 2) / 2, NBLK = (LA + 1) * (LA + 2) / 2 * NB * NC * ND;
     const int fa = a.func_off[B.sa], fb = a.func_off[B.sb];
     const int fc = a.func_off[K.sa], fd = a.func_off[K.sb];
-    double w = 8.0;
-    if (B.sa == B.sb) w *= 0.5;
-    if (K.sa == K.sb) w *= 0.5;
-    if (task.x == task.y) w *= 0.5;
+    const int halves = (B.sa == B.sb) + (K.sa == K.sb) + (task.x == task.y);
+    const double w8 = halves == 0 ? 1.0 : halves == 1 ? 0.5 : halves == 2 ? 0.25 : 0.125;
     const int nbf = a.nbf;
     const double* __restrict__ Pm = a.P;
     const double* __restrict__ cs = a.comp_scale;
@@ -200,13 +198,15 @@ __device__ __forceinline__ void grad_tail(const GradArgs& a, const int2& task, c
     for (int e = lane; e < NBLK; e += 32) {
         const int ia = e / (NB * NC * ND), ib = e / (NC * ND) % NB, ic = e / ND % NC, id = e % ND;
         const int pa = fa + ia, pb = fb + ib, pc = fc + ic, pd = fd + id;
-        const double gam = w * (0.5 * Pm[pa * nbf + pb] * Pm[pc * nbf + pd] -
-                                0.125 * (Pm[pa * nbf + pc] * Pm[pb * nbf + pd] +
-                                         Pm[pa * nbf + pd] * Pm[pb * nbf + pc]));
+        // w (P_ab P_cd / 2 - (P_ac P_bd + P_ad P_bc) / 8), w8 = w / 8
+        const double x = fma(Pm[pa * nbf + pc], Pm[pb * nbf + pd],
+                             gs_mul(Pm[pa * nbf + pd], Pm[pb * nbf + pc]));
+        const double gam = gs_mul(w8, fma(twice(twice(Pm[pa * nbf + pb])), Pm[pc * nbf + pd], -x));
         // the HRR blocks are unscaled: the element carries the component scales of all four
         // functions (not 1 for the xy, xz, yz components of a d shell)
-        const double s = gam * cs[6 * B.sa + ia] * cs[6 * B.sb + ib] * cs[6 * K.sa + ic] *
-                         cs[6 * K.sb + id];
+        const double s = gs_mul(gs_mul(gam, cs[6 * B.sa + ia]),
+                                gs_mul(gs_mul(cs[6 * B.sb + ib], cs[6 * K.sa + ic]),
+                                       cs[6 * K.sb + id]));
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
             const unsigned u = __ldg(con + k * NBLK + e);
@@ -219,19 +219,19 @@ __device__ __forceinline__ void grad_tail(const GradArgs& a, const int2& task, c
     constexpr unsigned ALL = 0xffffffffu;
     double last = g[8];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) last += __shfl_xor_sync(ALL, last, o);
+    for (int o = 16; o > 0; o >>= 1) last = gs_add(__shfl_xor_sync(ALL, last, o), last);
 #pragma unroll
     for (int o = 16, n = 4; n > 0; o >>= 1, n >>= 1) {
         const bool hi = lane & o;
 #pragma unroll
         for (int i = 0; i < n; ++i) {
             const double send = hi ? g[i] : g[i + n], keep = hi ? g[i + n] : g[i];
-            g[i] = keep + __shfl_xor_sync(ALL, send, o);
+            g[i] = gs_add(__shfl_xor_sync(ALL, send, o), keep);
         }
     }
     double v = g[0];
-    v += __shfl_xor_sync(ALL, v, 2);
-    v += __shfl_xor_sync(ALL, v, 1);
+    v = gs_add(__shfl_xor_sync(ALL, v, 2), v);
+    v = gs_add(__shfl_xor_sync(ALL, v, 1), v);
     // lanes 4 k (k < 8) hold component k's sum, lane 1 the last
     const int k = lane == 1 ? 8 : lane >> 2;
     if (lane == 1) v = last;
@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(32 * kGradSplitWarps) k_eri_grad_split(const G
 #pragma unroll
     for (int k = 0; k < W::NACC; ++k)
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) H[k] += __shfl_xor_sync(0xffffffffu, H[k], o);
+        for (int o = 16; o > 0; o >>= 1) H[k] = gs_add(__shfl_xor_sync(0xffffffffu, H[k], o), H[k]);
     if (lane == 0) grad_finish<LA, LB, LC, LD>(a, task, B, K, H, a.grad, false);
 }
 

@@ -63,7 +63,7 @@ __device__ __forceinline__ void write_block(const WriteArgs& a, const WriteTask&
     GS_UNROLL for (int id = 0; id < G::ND; ++id) {
         const int e = ((ia * G::NB + ib) * G::NC + ic) * G::ND + id;
         out[ia * s[0] + ib * s[1] + ic * s[2] + id * s[3]] =
-            widen(blk[e]) * (sab[ia * G::NB + ib] * scd[ic * G::ND + id]);
+            gs_mul(widen(blk[e]), gs_mul(sab[ia * G::NB + ib], scd[ic * G::ND + id]));
     }
 }
 
@@ -91,7 +91,7 @@ __device__ __forceinline__ bool split_accumulate(const PairRec& B, const PairRec
     GS_UNROLL for (int i = 0; i < G::NACC; ++i) acc[i] = T(0);
     eri_accumulate<LA, LB, LC, LD, T>(B, K, prims, acc, lane, 32);
     GS_UNROLL for (int i = 0; i < G::NACC; ++i)
-        GS_UNROLL for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+        GS_UNROLL for (int o = 16; o > 0; o >>= 1) acc[i] = gs_add(__shfl_xor_sync(0xffffffffu, acc[i], o), acc[i]);
     return lane == 0;
 }
 
@@ -161,7 +161,7 @@ __device__ __forceinline__ void jk_digest(const JKArgs& a, const int2 task, cons
         if (unit_bra && halves == 0) {
             GS_UNROLL for (int e = 0; e < G::NBLK; ++e) sc[e] = blk[e];
         } else {
-            GS_UNROLL for (int e = 0; e < G::NBLK; ++e) sc[e] = blk[e] * sab[e / (NC * ND)];
+            GS_UNROLL for (int e = 0; e < G::NBLK; ++e) sc[e] = gs_mul(blk[e], sab[e / (NC * ND)]);
         }
     } else {
         T scd[NC * ND];
@@ -170,7 +170,7 @@ __device__ __forceinline__ void jk_digest(const JKArgs& a, const int2 task, cons
                 scd[i * ND + j] = narrow_to(T(0), cs[6 * K.sa + i] * cs[6 * K.sb + j]);
         GS_UNROLL for (int ab = 0; ab < NA * NB; ++ab)
             GS_UNROLL for (int cd = 0; cd < NC * ND; ++cd)
-                sc[ab * NC * ND + cd] = blk[ab * NC * ND + cd] * (sab[ab] * scd[cd]);
+                sc[ab * NC * ND + cd] = gs_mul(blk[ab * NC * ND + cd], gs_mul(sab[ab], scd[cd]));
     }
     const int fa = a.func_off[B.sa], fb = a.func_off[B.sb];
     const int fc = a.func_off[K.sa], fd = a.func_off[K.sb];
@@ -183,13 +183,14 @@ __device__ __forceinline__ void jk_digest(const JKArgs& a, const int2 task, cons
         GS_UNROLL for (int i = 0; i < NC; ++i)
             GS_UNROLL for (int j = 0; j < ND; ++j) pcd[i * ND + j] = narrow_to(T(0), P[(fc + i) * n + fd + j]);
         T jab[NA * NB], jcd[NC * ND];
-        GS_UNROLL for (int i = 0; i < NA * NB; ++i) jab[i] = T(0);
+        const T nil = gs_mul(T(0), T(0));
+        GS_UNROLL for (int i = 0; i < NA * NB; ++i) jab[i] = nil;
         GS_UNROLL for (int i = 0; i < NC * ND; ++i) jcd[i] = T(0);
         GS_UNROLL for (int ab = 0; ab < NA * NB; ++ab)
             GS_UNROLL for (int cd = 0; cd < NC * ND; ++cd) {
                 const T v = sc[ab * NC * ND + cd];
-                jab[ab] += v * pcd[cd];
-                jcd[cd] += v * pab[ab];
+                jab[ab] = gs_fma(v, pcd[cd], jab[ab]);
+                jcd[cd] = gs_fma(v, pab[ab], jcd[cd]);
             }
         GS_UNROLL for (int i = 0; i < NA; ++i)
             GS_UNROLL for (int j = 0; j < NB; ++j)
@@ -220,10 +221,10 @@ __device__ __forceinline__ void jk_digest(const JKArgs& a, const int2 task, cons
         GS_UNROLL for (int ic = 0; ic < NC; ++ic)
         GS_UNROLL for (int id = 0; id < ND; ++id) {
             const T v = sc[((ia * NB + ib) * NC + ic) * ND + id];
-            kac[ia * NC + ic] += v * pbd[ib * ND + id];
-            kad[ia * ND + id] += v * pbc[ib * NC + ic];
-            kbc[ib * NC + ic] += v * pad[ia * ND + id];
-            kbd[ib * ND + id] += v * pac[ia * NC + ic];
+            kac[ia * NC + ic] = gs_fma(v, pbd[ib * ND + id], kac[ia * NC + ic]);
+            kad[ia * ND + id] = gs_fma(v, pbc[ib * NC + ic], kad[ia * ND + id]);
+            kbc[ib * NC + ic] = gs_fma(v, pad[ia * ND + id], kbc[ib * NC + ic]);
+            kbd[ib * ND + id] = gs_fma(v, pac[ia * NC + ic], kbd[ib * ND + id]);
         }
         GS_UNROLL for (int i = 0; i < NA; ++i)
             GS_UNROLL for (int j = 0; j < NC; ++j)

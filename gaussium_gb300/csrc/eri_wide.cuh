@@ -91,31 +91,31 @@ template <int LA, int LB, int LC, int LD, typename T, int VG = 1, int RQ = 1> st
 template <int M, typename T, int KB = 4, int KK = 4, int KX = 4>
 __device__ __forceinline__ void wide_setup_m(const PrimRec<T>& P, const PrimRec<T>& Q,
                                              T* __restrict__ c, T* __restrict__ F) {
-    const T pq = P.p + Q.p;
+    const T pq = gs_add(P.p, Q.p);
     const T rs = gs_rsqrt(pq);
-    const T ipq = rs * rs;
-    const T PQx = Q.Px - P.Px, PQy = Q.Py - P.Py, PQz = Q.Pz - P.Pz;
-    const T wq = Q.p * ipq, wp = P.p * ipq;
-    const T t = P.p * wq * (PQx * PQx + PQy * PQy + PQz * PQz);
+    const T ipq = gs_mul(rs, rs);
+    const T PQx = gs_sub(Q.Px, P.Px), PQy = gs_sub(Q.Py, P.Py), PQz = gs_sub(Q.Pz, P.Pz);
+    const T wq = gs_mul(Q.p, ipq), wp = gs_mul(P.p, ipq);
+    const T t = gs_mul(gs_mul(P.p, wq), norm2(PQx, PQy, PQz));
     T f[M + 1];
-    boys<M, T>(t, P.Kp * Q.Kp * rs, f);
+    boys<M, T>(t, gs_mul(gs_mul(P.Kp, Q.Kp), rs), f);
 #pragma unroll
     for (int m = 0; m <= M; ++m) F[m] = f[m];
     c[0] = P.PAx; c[1] = P.PAy; c[2] = P.PAz;
-    c[3] = wq * PQx; c[4] = wq * PQy; c[5] = wq * PQz;
+    c[3] = gs_mul(wq, PQx); c[4] = gs_mul(wq, PQy); c[5] = gs_mul(wq, PQz);
     c[6] = Q.PAx; c[7] = Q.PAy; c[8] = Q.PAz;
-    c[9] = -wp * PQx; c[10] = -wp * PQy; c[11] = -wp * PQz;
+    c[9] = gs_mul(-wp, PQx); c[10] = gs_mul(-wp, PQy); c[11] = gs_mul(-wp, PQz);
     auto multiples = [](T* o, T x, int n) {
         if (n >= 1) o[0] = x;
         if (n >= 2) o[1] = twice(x);
-        if (n >= 3) o[2] = T(3) * x;
+        if (n >= 3) o[2] = gs_mul(T(3), x);
         if (n >= 4) o[3] = twice(twice(x));
     };
     multiples(c + 12, P.i2p, KB);
-    if (KB >= 1) multiples(c + 16, -(wq * P.i2p), KB);
+    if (KB >= 1) multiples(c + 16, -gs_mul(wq, P.i2p), KB);
     multiples(c + 20, Q.i2p, KK);
-    if (KK >= 1) multiples(c + 24, -(wp * Q.i2p), KK);
-    if (KX >= 1) multiples(c + 28, T(0.5) * ipq, KX);
+    if (KK >= 1) multiples(c + 24, -gs_mul(wp, Q.i2p), KK);
+    if (KX >= 1) multiples(c + 28, gs_mul(T(0.5), ipq), KX);
 }
 
 // One synchronisation step of the VRR node program: the step's records (noff .. noff+cnt)
@@ -151,7 +151,7 @@ __device__ __forceinline__ void vrr_step(const uint4* __restrict__ vrec, int nof
     }
     for (int w = 0; w < nw; ++w) {
         const int nt = a.x >> 16;
-        T r = c0 * v0;
+        T r = gs_mul(c0, v0);
         r = fma(c1, v1, r);
         if (nt > 2) r = fma(c2, v2, r);
         if (nt > 3) r = fma(c3, v3, r);
@@ -209,7 +209,7 @@ __device__ __forceinline__ void vrr_step_rq(const uint4* __restrict__ vrec, int 
             if (q < ng) {
                 const T* __restrict__ cq = c + q * kNCoef;
                 const T* vq = nd + q * NVS;
-                T v = cq[k0] * vq[s0];
+                T v = gs_mul(cq[k0], vq[s0]);
                 v = fma(cq[k1], vq[s1], v);
                 if (nt > 2) v = fma(cq[k2], vq[s2], v);
                 if (nt > 3) v = fma(cq[k3], vq[s3], v);
@@ -287,7 +287,7 @@ __device__ __forceinline__ void wide_items(const T* __restrict__ sC, const T* __
             const int t = lane + 32 * k;
             if (t < NACC) {
                 const int v = __ldg(vtgt + t);
-                for (int q = 0; q < ng; ++q) acc[k] += node[q * NVS + v];
+                for (int q = 0; q < ng; ++q) acc[k] = gs_add(node[q * NVS + v], acc[k]);
             }
         }
         __syncwarp();
@@ -497,7 +497,7 @@ __device__ __forceinline__ void wide_write_out(const WriteArgs& a, const WriteTa
         const int id = e % G::ND, ic = (e / G::ND) % G::NC;
         const int ib = (e / (G::ND * G::NC)) % G::NB, ia = e / (G::ND * G::NC * G::NB);
         out[ia * s[0] + ib * s[1] + ic * s[2] + id * s[3]] =
-            widen(H[__ldg(os + e)] * (sab[ia * G::NB + ib] * scd[ic * G::ND + id]));
+            widen(gs_mul(H[__ldg(os + e)], gs_mul(sab[ia * G::NB + ib], scd[ic * G::ND + id])));
     }
 }
 
@@ -561,7 +561,7 @@ __device__ __forceinline__ void warp_sums(int lane, Term term, Add add) {
             for (int i = part; i < NIN; i += S) r = term(x, i, r);
         }
 #pragma unroll
-        for (int o = S / 2; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        for (int o = S / 2; o > 0; o >>= 1) r = gs_add(__shfl_xor_sync(0xffffffffu, r, o), r);
         if (in && part == 0) add(x, r);
     }
 }
@@ -594,7 +594,7 @@ __device__ __forceinline__ void wide_jk_digest(const JKArgs& a, const int2& task
         scd[x] = narrow_to(T(0), a.comp_scale[6 * K.sa + x / ND] * a.comp_scale[6 * K.sb + x % ND]);
     __syncwarp();
     const unsigned short* __restrict__ os = W::outslot();
-    for (int e = lane; e < G::NBLK; e += 32) V[e] = sm[__ldg(os + e)] * (sab[e / NCD] * scd[e % NCD]);
+    for (int e = lane; e < G::NBLK; e += 32) V[e] = gs_mul(sm[__ldg(os + e)], gs_mul(sab[e / NCD], scd[e % NCD]));
     __syncwarp();
     const int fa = a.func_off[B.sa], fb = a.func_off[B.sb];
     const int fc = a.func_off[K.sa], fd = a.func_off[K.sb];

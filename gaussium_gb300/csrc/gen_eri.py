@@ -88,6 +88,7 @@ class VrrGen:
         self.coefs = set()
         self.count = 0
         self.struct = []      # per node: list of (coefficient name, operand)
+        self.events = []      # ("node", name, terms) and ("acc", index, operand) in order
         self.e_targets = [e for L in range(self.la, self.la + self.lb + 1) for e in cart(L)]
         self.f_targets = [f for L in range(self.lc, self.lc + self.ld + 1) for f in cart(L)]
 
@@ -146,9 +147,7 @@ class VrrGen:
                 terms.append((self.coef("i2pq", e[i]), self.node(shift(e, i, -1), f1, m + 1)))
         name = f"v{self.count}"
         self.count += 1
-        expr = " + ".join(f"{c} * {x}" if not c.startswith("-") else f"-{c[1:]} * {x}"
-                          for c, x in terms).replace("+ -", "- ")
-        self.em.line(f"    const T {name} = {expr};")
+        self.events.append(("node", name, terms))
         self.em.flops += 1 + 2 * (len(terms) - 1)
         self.names[key] = name
         self.struct.append(terms)
@@ -159,9 +158,46 @@ class VrrGen:
         for ie, e in enumerate(self.e_targets):
             for jf, f in enumerate(self.f_targets):
                 x = self.node(e, f, 0)
-                self.em.line(f"    acc[{ie * nf + jf}] += {x};")
+                self.events.append(("acc", ie * nf + jf, x))
                 self.em.flops += 1
+        self.emit()
         return self
+
+    def emit(self):
+        """Straight-line code of the events.  FP64: every term a fused multiply-add (a plain
+        product or sum holds the pipe longer), and a target that no other node reads is added to
+        its accumulator term by term, one instruction less.  FP32, which that pipe does not
+        bound: plain sums of products, a target rounded at the accumulator's size once."""
+        used = {x for kind, _, terms in self.events if kind == "node" for _, x in terms}
+        leaf = {x: None for kind, _, x in self.events if kind == "acc" and x not in used}
+
+        def chain(first, terms):
+            for c, x in terms:
+                first = f"gs_fma({c}, {x}, {first})"
+            return first
+
+        def plain(terms):
+            return " + ".join(f"{c} * {x}" if not c.startswith("-") else f"-{c[1:]} * {x}"
+                              for c, x in terms).replace("+ -", "- ")
+
+        def define(name, terms):
+            expr = chain("gs_mul({}, {})".format(*terms[0]), terms[1:])
+            self.em.line(f"    T {name};")
+            self.em.line(f"    if constexpr (sizeof(T) == 8) {name} = {expr};")
+            self.em.line(f"    else {name} = {plain(terms)};")
+        for kind, key, val in self.events:
+            if kind == "node":
+                if key in leaf:
+                    leaf[key] = val
+                else:
+                    define(key, val)
+            elif leaf.get(val):
+                terms = leaf[val]
+                self.em.line(f"    if constexpr (sizeof(T) == 8) acc[{key}] = "
+                             f"{chain(f'acc[{key}]', terms)};")
+                self.em.line(f"    else {{ const T {val} = {plain(terms)}; acc[{key}] += {val}; }}")
+            else:
+                self.em.line(f"    acc[{key}] = gs_add({val}, acc[{key}]);")
 
 
 class HrrGen:
@@ -202,7 +238,7 @@ class HrrGen:
         self.count += 1
         self.em.line(f"    T {name}[{self.nf}];")
         self.em.line(f"    GS_UNROLL for (int k = 0; k < {self.nf}; ++k) "
-                     f"{name}[k] = {x}[k] + AB{XYZ[i]} * {y}[k];")
+                     f"{name}[k] = gs_fma(AB{XYZ[i]}, {y}[k], {x}[k]);")
         self.em.flops += 2 * self.nf
         self.bra_names[(a, b)] = name
         self.bra_ops.append((name, x, y, i))
@@ -245,7 +281,7 @@ class HrrGen:
                 return f"{n}[k]"
             self.em.line(f"    T {name}[{nab}];")
             self.em.line(f"    GS_UNROLL for (int k = 0; k < {nab}; ++k) "
-                         f"{name}[k] = {ref(x)} + CD{XYZ[i]} * {ref(y)};")
+                         f"{name}[k] = gs_fma(CD{XYZ[i]}, {ref(y)}, {ref(x)});")
             self.em.flops += 2 * nab
             kn[(c, d)] = name
             self.ket_ops.append((name, x, y, i))
@@ -297,7 +333,8 @@ def gen_class(cls):
         src.append(f"    const T {name} = c.{name}; (void){name};")
     for kind, k in sorted(v.coefs):
         if k != 1:
-            src.append(f"    const T {kind}_{k} = T({k}) * {kind};")
+            times = {2: f"twice({kind})", 4: f"twice(twice({kind}))"}.get(k, f"gs_mul(T({k}), {kind})")
+            src.append(f"    const T {kind}_{k} = {times};")
     src.extend(v.em.lines)
     src.append("  }")
     src.append("  template <typename T>")

@@ -281,11 +281,13 @@ def emit_grad(cls):
 THREAD_LMAX = 3       # classes with la+lb+lc+ld <= this also get a thread-per-quartet form
 
 
-def emit_grad_thread(cls, p=None):
+def emit_grad_thread(cls, p=None, mul="{} * {}", add="{} + {}"):
     """Straight-line thread-per-quartet form of the same program: per primitive quartet the
     VRR node program and the weighted accumulation into H[0 .. NACC), then the six HRR
     sub-programs on H and the contraction with the density weights, all with
-    compile-time indices so that the node values and accumulators live in registers."""
+    compile-time indices so that the node values and accumulators live in registers.
+    ``mul`` and ``add`` are the forms of the VRR's plain products and sums (the library's are
+    fused multiply-adds, eri_common.cuh)."""
     p = p or grad_program(cls)
     la, lb, lc, ld = cls
     tag = "".join(map(str, cls))
@@ -297,14 +299,14 @@ def emit_grad_thread(cls, p=None):
         w = vr[8 * r: 8 * r + 8]
         out, nt = w[0] & 0xffff, w[0] >> 16
         terms = [(x >> 16, x & 0xffff) for x in w[1:1 + nt]]
-        e = f"c[{terms[0][0]}] * n[{terms[0][1]}]"
+        e = mul.format(f"c[{terms[0][0]}]", f"n[{terms[0][1]}]")
         for cid, sl in terms[1:]:
             e = f"fma(c[{cid}], n[{sl}], {e})"
         body.append(f"    n[{out}] = {e};")
     acc = []
     for k, (sl, kind, pos) in enumerate(zip(p["acc_slot"], p["acc_kind"], p["acc_pos"])):
         if kind == 0:
-            acc.append(f"    H[{pos}] += n[{sl}];")
+            acc.append(f"    H[{pos}] = " + add.format(f"n[{sl}]", f"H[{pos}]") + ";")
         else:
             acc.append(f"    H[{pos}] = fma(c[{31 + kind}], n[{sl}], H[{pos}]);")
     hrr = [f"    H[{d}] = fma(dv[{dd}], H[{y}], H[{x}]);" for d, x, y, dd in p["hops"]]
@@ -374,7 +376,7 @@ def main():
             with open(path, "w") as f:
                 f.write(code)
         if sum(cls) <= THREAD_LMAX:
-            code = emit_grad_thread(cls, prog)
+            code = emit_grad_thread(cls, prog, "gs_mul({}, {})", "gs_add({}, {})")
             path = os.path.join(out, "eri_gradt_%s.h" % "".join(map(str, cls)))
             if not os.path.exists(path) or open(path).read() != code:
                 with open(path, "w") as f:

@@ -422,6 +422,10 @@ int gs_dense_expand(long long nq, const int* quartets, const long long* offsets,
                     const double* vals, const int* l, const int* func_off, int n, double* out,
                     void* stream);
 
+/* y[i] = 1 / sqrt(x[i]) as the kernels evaluate it (test hook; device arrays): two units in the
+ * last place over the normal range.  No reference counterpart. */
+int gs_rsqrt_eval(int n, const double* x, double* y, void* stream);
+
 /* FMA throughput probe (FP64 or FP32) used to measure the roofline peaks; sink must hold
  * blocks*threads elements of the chosen type.  No reference counterpart. */
 int gs_fma_probe(int precision, int blocks, int threads, int iters, void* sink, void* stream);

@@ -79,3 +79,24 @@ def test_fp32_digestion_of_any_density(gpu_lib, scale):
     for x, y in ((j64, j32), (k64, k32)):
         tol = 1e-5 * float(x.abs().max()) + 1e-41
         assert float((x - y).abs().max()) <= tol
+
+
+@pytest.mark.gpu
+def test_rsqrt(gpu_lib):
+    """Two units in the last place (the step's error under 2^-58 and five roundings) from the
+    smallest to the largest normal number; the library's values outside."""
+    from gaussium_gb300 import _lib
+    rng = np.random.default_rng(3)
+    x = np.concatenate([np.exp(rng.uniform(np.log(2.3e-308), np.log(1.7e308), 200000)),
+                        rng.uniform(1.0, 4.0, 200000),
+                        [2.2250738585072014e-308, 1.7976931348623157e308, 1.0, 2.0, 4.0]])
+    d = torch.as_tensor(x).cuda()
+    y = torch.empty_like(d)
+    _lib.check(gpu_lib.gs_rsqrt_eval(len(x), _lib.ptr(d), _lib.ptr(y), _lib.stream()), "rsqrt")
+    exact = 1.0 / np.sqrt(x.astype(np.longdouble))
+    assert float(np.max(np.abs(y.cpu().numpy() / exact - 1.0))) <= 2 * 2.0 ** -52
+    odd = torch.tensor([0.0, -0.0, 5e-324, 1e-310, float("inf"), float("nan"), -1.0],
+                       dtype=torch.float64, device="cuda")
+    got = torch.empty_like(odd)
+    _lib.check(gpu_lib.gs_rsqrt_eval(7, _lib.ptr(odd), _lib.ptr(got), _lib.stream()), "rsqrt")
+    assert torch.allclose(got, torch.rsqrt(odd), rtol=1e-15, equal_nan=True)
