@@ -159,20 +159,31 @@ GS_HD GS_INLINE const double* boys_table() {
 #endif
 }
 
+// Start of the asymptotic branch for orders 0..M: the smallest T (rounded up) at which
+// F_m(T) ~ (2m-1)!! / (2T)^m * sqrt(pi/T) / 2 is within 2^-54 (FP64) or 2^-26 (FP32) of
+// F_m for every m <= M.  Its relative error is the regularised upper incomplete gamma
+// function Q(m + 1/2, T), which grows with m, so the threshold depends on M only.
+constexpr unsigned kBoysAsym64[17] = {36, 40, 43, 46, 49, 52, 54, 57, 59, 61, 64, 66, 68, 70, 72, 74, 76};
+constexpr unsigned kBoysAsym32[17] = {17, 20, 23, 25, 28, 30, 32, 34, 36, 38, 40, 42, 43, 45, 47, 48, 50};
+
 // Taylor rows of the one Boys order the kernels of a translation unit evaluate most
-// (GS_BOYS_ORDER, defined by the generated class and gradient units): row k holds
-// F_{M+j}(T_k) / j!, j = 0..6, and the exponential's row exp(-T_k) / j!, so that an
-// expansion about T_k is a Horner chain of FMAs in T_k - T.  Other orders use the grid.
+// (GS_BOYS_ORDER, defined by the generated class and gradient units): see boys_table_gen.c.
+// Other orders use the grid.
+struct alignas(32) BoysRow64 {
+    double c[4], e[4];      // F_{M+j}(T_k) / j! and exp(-T_k) / j!, j = 0..3
+    float f[4], x[4];       // the same, j = 4..6
+};
+template <int M> constexpr int kBoysRows64 = (int)(kBoysAsym64[M] + 1) * BOYS_INV_H64 + 1;
 #if defined(__CUDACC__) && defined(GS_BOYS_ORDER)
 #define GS_BOYS_CAT2(a, b) a##b
 #define GS_BOYS_CAT(a, b) GS_BOYS_CAT2(a, b)
-__device__ __align__(16) const double g_boys_taylor[BOYS_ROWS * 8] = {
-    GS_BOYS_CAT(GS_BOYS_TAYLOR_, GS_BOYS_ORDER)};
-__device__ __align__(16) const double g_boys_expt[BOYS_ROWS * 8] = {GS_BOYS_EXPT};
+__device__ const BoysRow64 g_boys_row64[] = {GS_BOYS_CAT(GS_BOYS_ROW64_, GS_BOYS_ORDER)};
 __device__ __align__(16) const float g_boys_f32[BOYS_ROWS32 * 8] = {
     GS_BOYS_CAT(GS_BOYS_F32_, GS_BOYS_ORDER)};
 constexpr int kBoysOrder = GS_BOYS_ORDER;
 static_assert(kBoysOrder >= 0 && kBoysOrder <= BOYS_TAYLOR_MMAX, "Boys order without rows");
+static_assert(sizeof(g_boys_row64) == kBoysRows64<kBoysOrder> * sizeof(BoysRow64),
+              "rows of another threshold");
 #else
 constexpr int kBoysOrder = -1;
 #endif
@@ -257,55 +268,58 @@ template <unsigned N> GS_HD GS_INLINE bool below(double t) {
 }
 template <unsigned N> GS_HD GS_INLINE bool below(float t) { return t < (float)N; }
 
-// Nearest grid row k of t >= 0 and T_k - t (exact), the rounding by the sum with 1.5 2^52,
-// whose last bit is worth one.  k is held to the table whatever t is.
-GS_HD GS_INLINE int boys_row(double t, double& d) {
+// Nearest row k of the half-step grid of t >= 0 and T_k - t (exact), the rounding by the sum
+// with 1.5 2^52, whose last bit is worth one.  k is held to the table whatever t is.
+template <int M> GS_HD GS_INLINE int boys_row(double t, double& d) {
     const double magic = 6755399441055744.0;
-    const double kf = gs_fma(t, BOYS_INV_H, magic);
-    d = gs_fma(gs_sub(kf, magic), 1.0 / BOYS_INV_H, -t);
+    const double kf = gs_fma(t, BOYS_INV_H64, magic);
+    const double kd = gs_sub(kf, magic);
+    d = gs_fma(kd, 1.0 / BOYS_INV_H64, -t);
 #if defined(__CUDA_ARCH__)
-    return min((unsigned)__double2loint(kf), (unsigned)(BOYS_ROWS - 1));
+    return min((unsigned)__double2loint(kf), (unsigned)(kBoysRows64<M> - 1));
 #else
-    const double k = kf - magic;
-    return k >= 0 && k < BOYS_ROWS ? (int)k : BOYS_ROWS - 1;
+    return kd >= 0 && kd < kBoysRows64<M> ? (int)kd : kBoysRows64<M> - 1;
 #endif
 }
 
-// Boys function below BOYS_TMAX, always in FP64: 7-term Taylor expansion of F_M about the
-// nearest grid point (grid step 1/BOYS_INV_H), then downward recursion
+// The seven-term expansion about a row, |d| <= 1/64: the three smallest terms, under 2^-28 of
+// the sum, in float (df = d), four multiply-adds in FP64 instead of six.  (ss|ss) to (pp|ss)
+// spend a quarter of a primitive quartet's FP64 instructions here.
+GS_HD GS_INLINE double boys_horner(const double* c, const float* f, double d, float df) {
+    const float tail = gs_fma(df, gs_fma(df, f[2], f[1]), f[0]);
+    return gs_fma(gs_fma(gs_fma(gs_fma(widen(tail), d, c[3]), d, c[2]), d, c[1]), d, c[0]);
+}
+
+// F[m] = pref F_m(t), m = 0..M, from row r of order M: F_M and exp(-t) expanded about T_k,
+// then the downward recursion of boys_small.
+template <int M>
+GS_HD GS_INLINE void boys_from_row(const BoysRow64& r, double t, double d, double pref,
+                                   double* __restrict__ F) {
+    const float df = narrow(d);
+    F[M] = gs_mul(boys_horner(r.c, r.f, d, df), pref);
+    if (M > 0) {
+        const double et = gs_mul(boys_horner(r.e, r.x, d, df), pref);
+        const double t2 = twice(t);
+        GS_UNROLL for (int m = M; m >= 1; --m) {
+            const double x = gs_fma(t2, F[m], et);
+            F[m - 1] = m == 1 ? x : gs_mul(x, 1.0 / (2 * m - 1));
+        }
+    }
+}
+
+// Boys function below BOYS_TMAX, always in FP64: Taylor expansion of F_M about the
+// nearest grid point, then downward recursion
 //   F_{m-1}(t) = (2t F_m(t) + e^{-t}) / (2m - 1),
 // stable downwards; e^{-t} comes from the tabulated e^{-t_k} times the Taylor series of
-// e^{-(t - t_k)}.  F[m] = pref * F_m(t).
+// e^{-(t - t_k)}.  F[m] = pref * F_m(t).  Orders without rows expand 7 terms on the grid of
+// step 1/BOYS_INV_H.
 template <int M>
 GS_HD GS_INLINE void boys_small(double t, double pref, double* __restrict__ F) {
 #if defined(__CUDA_ARCH__) && defined(GS_BOYS_ORDER)
     if constexpr (M == kBoysOrder) {
-        // the same expansion and recursion from this order's Taylor rows
-        double d;                                                  // t_k - t, exact
-        const int k = boys_row(t, d);
-        const double2* g = reinterpret_cast<const double2*>(g_boys_taylor) + 4 * k;
-        const double2 g01 = __ldg(g), g23 = __ldg(g + 1), g45 = __ldg(g + 2), g67 = __ldg(g + 3);
-        double f = fma(g67.x, d, g45.y);
-        f = fma(f, d, g45.x);
-        f = fma(f, d, g23.y);
-        f = fma(f, d, g23.x);
-        f = fma(f, d, g01.y);
-        F[M] = gs_mul(fma(f, d, g01.x), pref);
-        if (M > 0) {
-            const double2* x = reinterpret_cast<const double2*>(g_boys_expt) + 4 * k;
-            const double2 x01 = __ldg(x), x23 = __ldg(x + 1), x45 = __ldg(x + 2), x67 = __ldg(x + 3);
-            double e = fma(x67.x, d, x45.y);
-            e = fma(e, d, x45.x);
-            e = fma(e, d, x23.y);
-            e = fma(e, d, x23.x);
-            e = fma(e, d, x01.y);
-            const double et = gs_mul(fma(e, d, x01.x), pref);
-            const double t2 = twice(t);
-            GS_UNROLL for (int m = M; m >= 1; --m) {
-                const double x = fma(t2, F[m], et);
-                F[m - 1] = m == 1 ? x : gs_mul(x, 1.0 / (2 * m - 1));
-            }
-        }
+        double d;
+        const int k = boys_row<M>(t, d);
+        boys_from_row<M>(g_boys_row64[k], t, d, pref, F);
         return;
     }
 #endif
@@ -420,13 +434,6 @@ GS_HD GS_INLINE void boys_small32(float t, float pref, float* __restrict__ F) {
     GS_UNROLL for (int m = 0; m <= M; ++m) F[m] = (float)Fd[m] * pref;
 }
 
-// Start of the asymptotic branch for orders 0..M: the smallest T (rounded up) at which
-// F_m(T) ~ (2m-1)!! / (2T)^m * sqrt(pi/T) / 2 is within 2^-54 (FP64) or 2^-26 (FP32) of
-// F_m for every m <= M.  Its relative error is the regularised upper incomplete gamma
-// function Q(m + 1/2, T), which grows with m, so the threshold depends on M only.
-constexpr unsigned kBoysAsym64[17] = {36, 40, 43, 46, 49, 52, 54, 57, 59, 61, 64, 66, 68, 70, 72, 74, 76};
-constexpr unsigned kBoysAsym32[17] = {17, 20, 23, 25, 28, 30, 32, 34, 36, 38, 40, 42, 43, 45, 47, 48, 50};
-
 // F[m] = pref * F_m(t), m = 0..M.  Below the threshold: the grid expansion and the
 // downward recursion in FP64 (boys_small, or boys_small32 for an FP32 quartet, which
 // rounds the FP64 values to float once).  Above it: F_0 = sqrt(pi/t)/2 and the upward
@@ -475,11 +482,8 @@ GS_HD GS_INLINE void eri_primitive(const PrimRec<T>& P, const PrimRec<T>& Q,
         T f = T(0.88622692545275801365);                 // sqrt(pi)/2
         if (!far) {
             double d;
-            const int k = boys_row(gs_mul(X, gs_mul(y, y)), d);
-            const double2* g = reinterpret_cast<const double2*>(g_boys_taylor) + 4 * k;
-            const double2 g01 = __ldg(g), g23 = __ldg(g + 1), g45 = __ldg(g + 2), g67 = __ldg(g + 3);
-            f = fma(fma(fma(fma(fma(fma(g67.x, d, g45.y), d, g45.x), d, g23.y), d, g23.x), d,
-                        g01.y), d, g01.x);
+            const int k = boys_row<0>(gs_mul(X, gs_mul(y, y)), d);
+            f = boys_horner(g_boys_row64[k].c, g_boys_row64[k].f, d, narrow(d));
         }
         acc[0] = fma(gs_mul(gs_mul(P.Kp, Q.Kp), y), f, acc[0]);
         return;

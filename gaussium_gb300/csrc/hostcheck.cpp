@@ -47,6 +47,19 @@ extern "C" int hc_boys_pair32(int M, double t, double* F) {
     return -1;
 }
 
+// The FP64 row form below the asymptotic threshold (boys_from_row) on the rows of order M.
+#define GS_R(MM) static const BoysRow64 h_rows##MM[] = {GS_BOYS_ROW64_##MM};
+GS_R(0) GS_R(1) GS_R(2) GS_R(3) GS_R(4) GS_R(5) GS_R(6) GS_R(7) GS_R(8) GS_R(9) GS_R(10)
+#undef GS_R
+extern "C" int hc_boys_row64(int M, double t, double* F) {
+    double d;
+#define GS_B(MM) case MM: { const int k = boys_row<MM>(t, d); \
+        boys_from_row<MM>(h_rows##MM[k], t, d, 1.0, F); return 0; }
+    switch (M) { GS_B(0) GS_B(1) GS_B(2) GS_B(3) GS_B(4) GS_B(5) GS_B(6) GS_B(7) GS_B(8) GS_B(9) GS_B(10) }
+#undef GS_B
+    return -1;
+}
+
 // Canonical block of one quartet (bra, ket index into pairs); out gets NA*NB*NC*ND doubles.
 extern "C" int hc_eri_block(int la, int lb, int lc, int ld, int prec, const PairRec* pairs,
                             const void* prims, int bra, int ket, double* out) {

@@ -21,6 +21,7 @@ def hc():
         L.hc_make_pairs.argtypes = [I] + [V] * 10
         L.hc_eri_block.argtypes = [I] * 5 + [V, V, I, I, V]
         L.hc_boys.argtypes = [I, I, ctypes.c_double, V]
+        L.hc_boys_row64.argtypes = [I, ctypes.c_double, V]
         L.hc_boys_pair32.argtypes = [I, ctypes.c_double, V]
         _hc = L
     return _hc

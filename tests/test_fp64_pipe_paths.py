@@ -30,6 +30,27 @@ def test_boys_pair32_rounds_like_fp64(m):
         assert np.max(np.abs(F / ex - 1.0)) < 1.25 * 2.0 ** -24, x
 
 
+ASYM64 = [36, 40, 43, 46, 49, 52, 54, 57, 59, 61, 64]
+
+
+@pytest.mark.parametrize("m", range(11))
+def test_boys_row64(m):
+    """The expansions' error (2^-52.6 from the float terms, 2^-54 from the terms left out, a
+    rounding of 2^-53 at each of two multiply-adds of full size) and 2^-53 for each of the two
+    operations an order of the downward recursion: (4 + 2 m) 2^-53, as much again for the
+    reference's own rounding."""
+    L = hostcheck.hc()
+    rng = np.random.default_rng(m)
+    t = np.concatenate([[0.0, 1 / 64, 1 / 32, 3 / 64, np.nextafter(1 / 64, 1), np.nextafter(ASYM64[m], 0)],
+                        np.exp(rng.uniform(np.log(1e-6), np.log(ASYM64[m]), 400)),
+                        rng.uniform(0, ASYM64[m], 400)])
+    F = np.zeros(m + 1)
+    for x in t:
+        assert L.hc_boys_row64(m, float(x), F.ctypes.data) == 0
+        ex = np.array([oracle.boys_exact(k, float(x)) for k in range(m + 1)])
+        assert np.max(np.abs(F / ex - 1.0)) < 2 * (4 + 2 * m) * 2.0 ** -53, x
+
+
 def _small_basis(seed, scales):
     sb, _, _ = random_shell_quartets(3, seed=seed, box_angstrom=1.5, lmax=1)
     cs = np.random.default_rng(seed).uniform(0.5, 2.0, (sb.nshell, 6)) if scales else \
