@@ -42,6 +42,7 @@ _SIGS = {
     "gs_class_variant": (I, [I, I, I, I, I]),
     "gs_set_class_variant": (I, [I, I, I, I, I, I]),
     "gs_boys_eval": (I, [I, I, I, P, P, P]),
+    "gs_task_keys": (I, [ctypes.c_longlong, P, P, P, P, P, P, P]),
     "gs_rsqrt_eval": (I, [I, P, P, P]),
     "gs_fma_probe": (I, [I, I, I, I, P, P]),
     "gs_fma_probe_lanes": (I, [I, I, I, I, I, P, P]),
@@ -50,6 +51,8 @@ _SIGS = {
     "gs_eri_grad": (I, [I, I, I, I, P, P, P, P, P, I, P, I, I, P, P, P]),
     "gs_eri_grad_form": (I, [I, I, I, I, I, P, P, P, P, P, I, P, I, I, P, P, P]),
     "gs_eri_grad_band": (I, [I, I, I, I, I, I, P, P, P, P, P, I, P, I, I, P, I, P, D, D, D, P, P]),
+    "gs_eri_grad_mixed": (I, [I, I, I, I, I, P, P, P, P, P, P, I, P, I, I, P, I, P, D, D, P, P,
+                              ctypes.c_longlong, P]),
     "gs_eri_grad_class_form": (I, [I, I, I, I]),
     "gs_eri_grad_variants": (I, [I, I, I, I]),
     "gs_set_eri_grad_variant": (I, [I, I, I, I, I]),

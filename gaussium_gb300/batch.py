@@ -15,9 +15,9 @@ import torch
 
 from . import _lib
 from .basis import ShellBasis
-from .engine import (MIXED_LANES, PAIR_ORDER, PRIM_SCREEN, SIDE_STREAMS,
-                     DeviceShells, HeavyLane, MixedWorkspace, PairSet, _pc_lut, launch_plan,
-                     mixed_plan, segment_profiles)
+from .engine import (MIXED_LANES, PAIR_ORDER, PRIM_SCREEN, SIDE_STREAMS, DeviceShells, HeavyLane,
+                     MixedWorkspace, PairSet, _pc_lut, launch_plan, mixed_plan, segment_profiles,
+                     task_keys)
 from .hamiltonian import one_electron
 from .molecules import shell_basis
 
@@ -102,7 +102,7 @@ class BatchedRHF(MixedWorkspace):
         pc_d = torch.as_tensor(np.asarray(pc, dtype=np.int64)).to(self.dev)
         pm_d = torch.as_tensor(np.asarray(pair_mol, dtype=np.int64)).to(self.dev)
         self.segments, self.tasks = batched_task_list(q, pc_d, pm_d, nprim, thr, len(PAIR_ORDER),
-                                                      len(self.sbs))
+                                                      len(self.sbs), self.pairs)
         self.ntasks = int(self.tasks.shape[0])
         # tasks of each segment with many primitive quartets (prefixes: the segments are
         # sorted by descending primitive work); they run in the split or cooperative form
@@ -372,13 +372,14 @@ class BatchedRHF(MixedWorkspace):
         return (energies + e_nuc).cpu().numpy(), it
 
 
-def batched_task_list(q, pair_class, pair_mol, nprim, thr, nclass, nmol):
+def batched_task_list(q, pair_class, pair_mol, nprim, thr, nclass, nmol, pairs=None):
     """Unique shell-quartet tasks (bra pair, ket pair) of many molecules, on the device of
     the inputs: for every class pair (cb >= ck) and every molecule, the pairs of that
     molecule with q_bra q_ket >= thr (bra >= ket within one class), quartets never
     crossing molecules.  Each class segment is ordered by primitive-quartet count, largest
-    first, then (primitive pairs of the bra, of the ket), molecule by molecule otherwise.  Returns [((la, lb, lc, ld), start, end)]
-    and the [ntask, 2] int32 task array."""
+    first, then (primitive pairs of the bra, of the ket), then, with the PairSet ``pairs``, by
+    distance (engine.task_keys), molecule by molecule otherwise.  Returns
+    [((la, lb, lc, ld), start, end)] and the [ntask, 2] int32 task array."""
     dev = q.device
     key = pair_mol * nclass + pair_class
     order = torch.argsort(key, stable=True)
@@ -407,8 +408,9 @@ def batched_task_list(q, pair_class, pair_mol, nprim, thr, nclass, nmol):
             if bra.numel() == 0:
                 continue
             # most primitive quartets first, equal (K_bra, K_ket) together
-            perm = torch.argsort((nprim[bra] * nprim[ket]) * 4096 + nprim[bra] * 64 + nprim[ket],
-                                 descending=True, stable=True)
+            key = (nprim[bra] * nprim[ket]) * 4096 + nprim[bra] * 64 + nprim[ket] \
+                if pairs is None else task_keys(pairs, bra, ket)
+            perm = torch.argsort(key, descending=True, stable=True)
             tk = torch.stack([bra[perm], ket[perm]], 1).to(torch.int32)
             (la, lb), (lc, ld) = PAIR_ORDER[cb], PAIR_ORDER[ck]
             segs.append(((la, lb, lc, ld), n, n + tk.shape[0]))

@@ -5,6 +5,8 @@
 #include "eri_grad.cuh"
 #include "eri_grad_list.h"
 
+extern "C" long long gs_fock_jk_mixed_workspace(int ntask);
+
 #define GS_GDECL(A, B, C, D) \
     int gs_grad_launch_##A##B##C##D(const gs::GradArgs&, int, cudaStream_t);
 GS_FOR_EACH_GRAD(GS_GDECL)
@@ -84,6 +86,54 @@ extern "C" int gs_eri_grad_band(int la, int lb, int lc, int ld, int form, int pr
     GS_FOR_EACH_GRAD(GS_GL)
 #undef GS_GL
     return GS_ERR_CLASS;
+}
+
+extern "C" int gs_eri_grad_mixed(int la, int lb, int lc, int ld, int form, const void* pair_rec,
+                                 const void* prim64, const void* prim32, const double* comp_scale,
+                                 const int* func_off, const int* shell_atom, int ntask,
+                                 const int* tasks, int nbf, int natom, const double* density,
+                                 int nshell, const double* shell_dmax, double screen_thr,
+                                 double mixed_cut, double* grad, void* workspace,
+                                 long long ws_bytes, void* stream) {
+    if (ntask < 0 || nbf <= 0 || natom <= 0 || nshell <= 0 || !pair_rec || !prim64 || !prim32 ||
+        !comp_scale || !func_off || !shell_atom || (ntask > 0 && !tasks) || !density || !grad ||
+        !shell_dmax || !workspace || (form != 1 && form != 3))
+        return GS_ERR_ARG;
+    if (!valid_class(la, lb, lc, ld)) return GS_ERR_CLASS;
+    if (!has_thread(la, lb, lc, ld)) return GS_ERR_ARG;
+    if (ntask == 0) return GS_OK;
+    if (ws_bytes < gs_fock_jk_mixed_workspace(ntask)) return GS_ERR_NOMEM;
+    cudaStream_t st = (cudaStream_t)stream;
+    int* counts = (int*)workspace;
+    int2* l64 = (int2*)((char*)workspace + 256);
+    int2* l32 = l64 + ntask;
+    if (gs::partition_tasks(ntask, (const int2*)tasks, (const gs::PairRec*)pair_rec, shell_dmax,
+                            nshell, screen_thr, mixed_cut, l64, l32, counts, st))
+        return GS_ERR_CUDA;
+    gs::GradArgs a{};
+    a.pairs = (const gs::PairRec*)pair_rec;
+    a.prims = (const gs::PrimRec<double>*)prim64;
+    a.prims32 = (const gs::PrimRec<float>*)prim32;
+    a.comp_scale = comp_scale;
+    a.func_off = func_off;
+    a.shell_atom = shell_atom;
+    a.ntask = ntask;
+    a.nbf = nbf;
+    a.P = density;
+    a.grad = grad;
+    a.natom = natom;
+    for (int k = 0; k < 2; ++k) {
+        a.fp32 = k == 1;
+        a.tasks = k ? l32 : l64;
+        a.ntask_dev = counts + k;
+        int rc = GS_ERR_CLASS;
+#define GS_GL(A, B, C, D) \
+        if (la == A && lb == B && lc == C && ld == D) rc = gs_grad_launch_##A##B##C##D(a, form, st);
+        GS_FOR_EACH_GRAD(GS_GL)
+#undef GS_GL
+        if (rc) return rc;
+    }
+    return GS_OK;
 }
 
 extern "C" int gs_eri_grad_form(int la, int lb, int lc, int ld, int form, const void* pair_rec,

@@ -36,6 +36,7 @@ struct GradArgs {
     int nshell;
     double screen_thr, prec_lo, prec_hi;
     int per;                        // tasks a warp of the warp form takes
+    const int* ntask_dev;           // if set, the task count (thread and split forms; ntask: bound)
 };
 
 __device__ __forceinline__ bool grad_keep(const GradArgs& a, const PairRec& B, const PairRec& K) {
@@ -479,36 +480,52 @@ __device__ __forceinline__ void grad_accumulate(const GradArgs& a, const PairRec
     for (int k = 0; k < W::NACC; ++k) H[k] = (double)acc[k];
 }
 
+// Copies of the block's gradient sums: two a warp, by the lanes' parity, while they are small
+// (a shared FP64 addition is a compare-and-swap loop, and lanes that share an atom repeat it).
+constexpr int kGradCopies = 2 * kGradThreads / 32;
+__host__ __device__ inline int grad_copies(int natom) {
+    return natom <= kGradSmemAtoms / kGradCopies ? kGradCopies : 1;
+}
+
 template <int LA, int LB, int LC, int LD, typename T>
 __global__ void __launch_bounds__(kGradThreads) k_eri_grad_thread(const GradArgs a) {
     using W = GradThread<LA, LB, LC, LD>;
     extern __shared__ double sg[];
+    const int ntask = a.ntask_dev ? *a.ntask_dev : a.ntask;
+    if (blockIdx.x * blockDim.x >= ntask) return;          // block-uniform
     const bool shared_sum = a.natom > 0 && a.natom <= kGradSmemAtoms;
+    const int copies = grad_copies(a.natom), n3 = 3 * a.natom;
     if (shared_sum) {
-        for (int i = threadIdx.x; i < 3 * a.natom; i += blockDim.x) sg[i] = 0.0;
+        for (int i = threadIdx.x; i < copies * n3; i += blockDim.x) sg[i] = 0.0;
         __syncthreads();
     }
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < a.ntask) {
+    if (t < ntask) {
         const int2 task = a.tasks[t];
         const PairRec B = a.pairs[task.x];
         const PairRec K = a.pairs[task.y];
         if (grad_keep(a, B, K)) {
             double H[W::HSIZE];
             grad_accumulate<LA, LB, LC, LD, T>(a, B, K, H, 0, 1);
-            grad_finish<LA, LB, LC, LD>(a, task, B, K, H, shared_sum ? sg : a.grad, true);
+            const int copy = copies > 1 ? 2 * (threadIdx.x >> 5) + (threadIdx.x & 1) : 0;
+            grad_finish<LA, LB, LC, LD>(a, task, B, K, H, shared_sum ? sg + copy * n3 : a.grad,
+                                        true);
         }
     }
     if (shared_sum) {
         __syncthreads();
-        for (int i = threadIdx.x; i < 3 * a.natom; i += blockDim.x)
-            if (sg[i] != 0.0) atomicAdd(a.grad + i, sg[i]);
+        for (int i = threadIdx.x; i < n3; i += blockDim.x) {
+            double v = sg[i];
+            for (int c = 1; c < copies; ++c) v += sg[c * n3 + i];
+            if (v != 0.0) atomicAdd(a.grad + i, v);
+        }
     }
 }
 
 template <int LA, int LB, int LC, int LD, typename T>
 int launch_grad_thread_t(const GradArgs& a, cudaStream_t st) {
-    const size_t sh = (a.natom > 0 && a.natom <= kGradSmemAtoms) ? 3 * sizeof(double) * a.natom : 0;
+    const size_t sh = (a.natom > 0 && a.natom <= kGradSmemAtoms)
+                          ? 3 * sizeof(double) * a.natom * grad_copies(a.natom) : 0;
     if (set_smem<k_eri_grad_thread<LA, LB, LC, LD, T>>(3 * sizeof(double) * kGradSmemAtoms))
         return GS_ERR_CUDA;
     k_eri_grad_thread<LA, LB, LC, LD, T><<<(a.ntask + kGradThreads - 1) / kGradThreads,
@@ -534,7 +551,7 @@ __global__ void __launch_bounds__(32 * kGradSplitWarps) k_eri_grad_split(const G
     using W = GradThread<LA, LB, LC, LD>;
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * kGradSplitWarps + (threadIdx.x >> 5);
-    if (t >= a.ntask) return;                      // warp-uniform
+    if (t >= (a.ntask_dev ? *a.ntask_dev : a.ntask)) return;       // warp-uniform
     const int2 task = a.tasks[t];
     const PairRec B = a.pairs[task.x];
     const PairRec K = a.pairs[task.y];

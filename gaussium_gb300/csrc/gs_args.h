@@ -79,4 +79,10 @@ struct SchwarzArgs {
     int npair;
     double* q;                  // [npairs total] output
 };
+
+// Splits ntask tasks by their density-weighted bound (capi.cu, k_partition): an FP64 list at
+// l64 (bound >= cut), an FP32 list at l32 (thr <= bound < cut), their lengths at counts[0], [1].
+int partition_tasks(int ntask, const int2* tasks, const PairRec* pairs, const double* shell_dmax,
+                    int nshell, double thr, double cut, int2* l64, int2* l32, int* counts,
+                    cudaStream_t st);
 }  // namespace gs

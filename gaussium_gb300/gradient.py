@@ -220,25 +220,40 @@ def eri_gradient(sb, engine: JKEngine, shell_atom, P, natom, classes=None, host=
             # a thread-form class's quartets with many primitive quartets (the task list's
             # prefix) in the split form
             h = heavy[0] if GRAD_SPLIT else 0
-            parts = [(3, 0, h), (0, h, n - h)]
-            bands = [(64, mixed_cut, inf), (32, 0.0, mixed_cut)] if mixed_cut is not None else \
-                [(64, 0.0, inf)]
+            parts = [(3, 0, h), (1, h, n - h)]
+            # with a cut: partitioned lists, one launch a precision (prec 0)
+            bands = [(0, mixed_cut, inf)] if mixed_cut is not None else [(64, 0.0, inf)]
         for prec, lo, hi in bands:
-            prims = engine.pairs.p64 if prec == 64 else engine.pairs.p32
             for form, first, count in parts:
                 if count > 0:
-                    launches.append((cls, form, prec, prims, first + s, count, lo, hi))
+                    launches.append((cls, form, prec, first + s, count, lo, hi))
     # largest angular momenta first: a warp of theirs walks its quartet's primitives the
     # longest, with few quartets to fill the GPU, so the launches of the smaller classes run
     # beside them on the other streams
     launches.sort(key=lambda x: -sum(x[0]))
-    for i, (cls, form, prec, prims, first, count, lo, hi) in enumerate(launches):
-        _lib.check(L.gs_eri_grad_band(
-            *cls, form, prec, _lib.ptr(engine.pairs.rec), _lib.ptr(prims),
-            _lib.ptr(engine.ds.comp_scale), _lib.ptr(engine.ds.func_off), _lib.ptr(sa),
-            count, base + first * 8, sb.nbf, natom, _lib.ptr(pt), sb.nshell,
-            _lib.ptr(dmax), thr, lo, hi, _lib.ptr(grad), lane.lane(i)),
-            f"gs_eri_grad_band{cls}")
+    lanes = SIDE_STREAMS + 1
+    # each stream's partitions share one workspace, a launch's lists at a time
+    need = [0] * lanes
+    for i, x in enumerate(launches):
+        if x[2] == 0:
+            need[i % lanes] = max(need[i % lanes], int(L.gs_fock_jk_mixed_workspace(x[4])))
+    ws = [torch.empty(b, dtype=torch.uint8, device=dev) for b in need]
+    for i, (cls, form, prec, first, count, lo, hi) in enumerate(launches):
+        if prec == 0:
+            w = ws[i % lanes]
+            rc = L.gs_eri_grad_mixed(
+                *cls, form, _lib.ptr(engine.pairs.rec), _lib.ptr(engine.pairs.p64),
+                _lib.ptr(engine.pairs.p32), _lib.ptr(engine.ds.comp_scale),
+                _lib.ptr(engine.ds.func_off), _lib.ptr(sa), count, base + first * 8, sb.nbf, natom,
+                _lib.ptr(pt), sb.nshell, _lib.ptr(dmax), thr, lo, _lib.ptr(grad), _lib.ptr(w),
+                w.numel(), lane.lane(i, lanes))
+        else:
+            rc = L.gs_eri_grad_band(
+                *cls, form, prec, _lib.ptr(engine.pairs.rec), _lib.ptr(engine.pairs.p64),
+                _lib.ptr(engine.ds.comp_scale), _lib.ptr(engine.ds.func_off), _lib.ptr(sa),
+                count, base + first * 8, sb.nbf, natom, _lib.ptr(pt), sb.nshell,
+                _lib.ptr(dmax), thr, lo, hi, _lib.ptr(grad), lane.lane(i, lanes))
+        _lib.check(rc, f"eri_gradient{cls}")
     lane.join()
     return grad.view(natom, 3).cpu().numpy() if host else grad.view(natom, 3)
 

@@ -296,6 +296,18 @@ int gs_eri_grad_band(int la, int lb, int lc, int ld, int form, int precision,
                      const double* shell_dmax, double screen_thr, double prec_lo,
                      double prec_hi, double* grad, void* stream);
 
+/* Mixed-precision form of gs_eri_grad_form for the thread (1) and split (3) forms: a partition
+ * kernel splits the tasks by their density-weighted bound (as gs_fock_jk_mixed does) into an
+ * FP64 list (bound >= mixed_cut) and an FP32 list (screen_thr <= bound < mixed_cut), and one
+ * launch each evaluates them, as gs_eri_grad_band's bands do, on full warps.  workspace: at
+ * least gs_fock_jk_mixed_workspace(ntask) bytes on the device.  No reference counterpart. */
+int gs_eri_grad_mixed(int la, int lb, int lc, int ld, int form, const void* pair_rec,
+                      const void* prim64, const void* prim32, const double* comp_scale,
+                      const int* func_off, const int* shell_atom, int ntask, const int* tasks,
+                      int nbf, int natom, const double* density, int nshell,
+                      const double* shell_dmax, double screen_thr, double mixed_cut, double* grad,
+                      void* workspace, long long ws_bytes, void* stream);
+
 /* The form (1 thread, 2 warp) a gs_eri_grad launch of that class uses: the configured
  * variant or the default; negative status on a class without gradient kernels.  No
  * reference counterpart. */
@@ -421,6 +433,14 @@ int gs_fock_jk_batched_persistent(const void* pair_rec, const void* prim64, cons
 int gs_dense_expand(long long nq, const int* quartets, const long long* offsets,
                     const double* vals, const int* l, const int* func_off, int n, double* out,
                     void* stream);
+
+/* Sort keys (to be sorted descending) of n Fock tasks (bra[i], ket[i]): primitive-quartet count,
+ * the pairs' primitive counts, and the pairs' distance in coarse steps, so that neighbouring
+ * tasks take the same loop counts and the same branch of the Boys function.  nprim: kept
+ * primitive pairs per pair; key >> 18 is the primitive-quartet count.  Device arrays.  No
+ * reference counterpart. */
+int gs_task_keys(long long n, const long long* bra, const long long* ket, const int* nprim,
+                 const void* pair_rec, const void* prim64, long long* keys, void* stream);
 
 /* y[i] = 1 / sqrt(x[i]) as the kernels evaluate it (test hook; device arrays): two units in the
  * last place over the normal range.  No reference counterpart. */

@@ -201,3 +201,60 @@ def test_gradient_tasks_a_warp(gpu_lib):
         ref = g if ref is None else ref
         assert float((g - ref).abs().max()) <= 1e-12 * float(ref.abs().max())
     assert abs(float(g.view(6, 3).sum())) < 1e-10          # translational invariance
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", [1, 3])
+def test_gradient_partition_matches_bands(gpu_lib, form):
+    """The partitioned adjoint evaluates the quartets of the two bands, each in its precision:
+    the same gradient up to the order of the sums."""
+    from gaussium_gb300 import _lib
+    from gaussium_gb300.gradient import shell_atoms
+    from gaussium_gb300.molecules import shell_basis, water_cluster
+    mol = water_cluster(2, seed=2)
+    sb = shell_basis(mol, "6-31G*")
+    eng = engine.JKEngine(sb, schwarz_thr=1e-12)
+    sa = torch.as_tensor(shell_atoms(mol, sb).astype(np.int32)).cuda()
+    p = np.random.default_rng(3).standard_normal((sb.nbf, sb.nbf)) * 0.1
+    pt = torch.as_tensor(p + p.T).cuda()
+    dmax = eng.shell_dmax([pt])
+    ws = torch.empty(gpu_lib.gs_fock_jk_mixed_workspace(eng.ntasks), dtype=torch.uint8, device="cuda")
+    inf = float("inf")
+    for cls, s, e in eng.segments:
+        if sum(cls) > 3:
+            continue
+        tail = (_lib.ptr(eng.ds.comp_scale), _lib.ptr(eng.ds.func_off), _lib.ptr(sa), e - s,
+                eng.tasks.data_ptr() + 8 * s, sb.nbf, 6, _lib.ptr(pt), sb.nshell, _lib.ptr(dmax))
+        a, b = (torch.zeros(18, dtype=torch.float64, device="cuda") for _ in range(2))
+        for prec, prims, lo, hi in ((64, eng.pairs.p64, 1e-3, inf), (32, eng.pairs.p32, 0.0, 1e-3)):
+            _lib.check(gpu_lib.gs_eri_grad_band(
+                *cls, form, prec, _lib.ptr(eng.pairs.rec), _lib.ptr(prims), *tail, 1e-9, lo, hi,
+                _lib.ptr(a), _lib.stream()), "gs_eri_grad_band")
+        call = (*cls, form, _lib.ptr(eng.pairs.rec), _lib.ptr(eng.pairs.p64),
+                _lib.ptr(eng.pairs.p32), *tail, 1e-9, 1e-3, _lib.ptr(b), _lib.ptr(ws))
+        _lib.check(gpu_lib.gs_eri_grad_mixed(*call, ws.numel(), _lib.stream()), "gs_eri_grad_mixed")
+        assert float((a - b).abs().max()) <= 1e-12 * float(a.abs().max()), cls
+        assert gpu_lib.gs_eri_grad_mixed(*call, 256, None) == 5
+
+
+@pytest.mark.gpu
+def test_task_keys(gpu_lib):
+    """Key fields against their definition: counts exactly, the distance bin to a rounding."""
+    from gaussium_gb300.workloads import random_shell_quartets
+    sb, _, _ = random_shell_quartets(4, seed=9, box_angstrom=8.0)
+    eng = engine.JKEngine(sb, schwarz_thr=0.0)
+    n = eng.npairs
+    rng = np.random.default_rng(0)
+    bra, ket = (torch.as_tensor(rng.integers(0, n, 4000)).cuda() for _ in range(2))
+    keys = engine.task_keys(eng.pairs, bra, ket).cpu().numpy()
+    b, k = bra.cpu().numpy(), ket.cpu().numpy()
+    nprim = eng.pairs.nprim
+    assert np.array_equal(keys >> 6, nprim[b] * nprim[k] * 4096 + nprim[b] * 64 + nprim[k])
+    assert np.array_equal(keys // engine.KEY_WORK, nprim[b] * nprim[k])
+    rec = eng.pairs.p64.cpu().numpy().view(np.float64).reshape(-1, 10)
+    at = eng.pairs.prim_start.cpu().numpy() + np.maximum(nprim - 1, 0)
+    d2 = ((rec[at[b], 2:5] - rec[at[k], 2:5]) ** 2).sum(1) + 0.25
+    want = np.where(nprim[b] * nprim[k] > 0, np.clip(np.floor(2 * np.log2(d2)) + 4, 0, 63), 0)
+    both = np.abs((keys & 63) - want)
+    assert both.max() <= 1          # steps are sqrt(2) or 3/2 and 4/3: not quite the logarithm's
+    assert np.mean(both) < 0.2
