@@ -42,6 +42,7 @@ _SIGS = {
     "gs_class_variant": (I, [I, I, I, I, I]),
     "gs_set_class_variant": (I, [I, I, I, I, I, I]),
     "gs_boys_eval": (I, [I, I, I, P, P, P]),
+    "gs_product_tasks": (I, [ctypes.c_longlong, I, P, P, P, P, P, P]),
     "gs_task_keys": (I, [ctypes.c_longlong, P, P, P, P, P, P, P]),
     "gs_rsqrt_eval": (I, [I, P, P, P]),
     "gs_fma_probe": (I, [I, I, I, I, P, P]),

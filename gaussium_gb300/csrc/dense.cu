@@ -50,9 +50,68 @@ k_dense_expand(long long nq, const int4* __restrict__ quartets,
     }
 }
 
+// Unique quartets as products of ranges of a pair list: range r holds the quartets (bra pair
+// b, ket pair k) with b in [bra, bra + nbra) and k in [ket, ket + nket), or, for nket = 0, the
+// pairs k <= b of [bra, bra + nbra) with themselves.  Its quartets are numbers first[r] ..
+// first[r + 1]; their blocks have size[r] elements from base[r] on.
+struct QuartetRange {
+    long long first, base;
+    int bra, nbra, ket, nket, size, pad;
+};
+
+__global__ void __launch_bounds__(256)
+k_product_tasks(long long n, int nranges, const QuartetRange* __restrict__ ranges,
+                const int2* __restrict__ pair_shells, int* __restrict__ tasks,
+                int4* __restrict__ quartets, long long* __restrict__ offsets) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    int lo = 0, hi = nranges - 1;                  // the last range that starts at or before t
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (ranges[mid].first <= t) lo = mid; else hi = mid - 1;
+    }
+    const QuartetRange r = ranges[lo];
+    const long long x = t - r.first;
+    int b, k;
+    if (r.nket > 0) {
+        b = r.bra + (int)(x / r.nket);
+        k = r.ket + (int)(x % r.nket);
+    } else {                                       // row i of the triangle holds i + 1 pairs
+        long long i = (long long)((sqrt(8.0 * (double)x + 1.0) - 1.0) * 0.5);
+        while (i * (i + 1) / 2 > x) --i;
+        while ((i + 1) * (i + 2) / 2 <= x) ++i;
+        b = r.bra + (int)i;
+        k = r.bra + (int)(x - i * (i + 1) / 2);
+    }
+    const long long off = r.base + x * r.size;
+    int* w = tasks + 6 * t;                        // WriteTask: bra, ket, code, pad, offset
+    w[0] = b;
+    w[1] = k;
+    w[2] = 0;
+    w[3] = 0;
+    *reinterpret_cast<long long*>(w + 4) = off;
+    const int2 B = pair_shells[b], K = pair_shells[k];
+    quartets[t] = make_int4(B.x, B.y, K.x, K.y);
+    offsets[t] = off;
+}
+
 }  // namespace
 
 extern "C" {
+
+int gs_product_tasks(long long n, int nranges, const void* ranges, const int* pair_shells,
+                     void* tasks, int* quartets, long long* offsets, void* stream) {
+    if (n < 0 || nranges < 0 ||
+        (n > 0 && (nranges == 0 || !ranges || !pair_shells || !tasks || !quartets || !offsets)))
+        return GS_ERR_ARG;
+    if (n == 0) return GS_OK;
+    const long long blocks = (n + 255) / 256;
+    if (blocks > 0x7fffffffLL) return GS_ERR_ARG;
+    k_product_tasks<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
+        n, nranges, (const QuartetRange*)ranges, (const int2*)pair_shells, (int*)tasks,
+        (int4*)quartets, offsets);
+    return cudaGetLastError() == cudaSuccess ? GS_OK : GS_ERR_CUDA;
+}
 
 int gs_dense_expand(long long nq, const int* quartets, const long long* offsets,
                     const double* vals, const int* l, const int* func_off, int n, double* out,

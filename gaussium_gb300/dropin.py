@@ -70,20 +70,26 @@ def unique_shell_quartets(nshell):
 
 def dense_eri(sb: ShellBasis, device="cuda", precision=64):
     """Dense N^4 ERI tensor (torch f64 on the device) from unique shell quartets."""
-    ds = engine.DeviceShells(sb, device)
-    q = unique_shell_quartets(sb.nshell)
-    batch = engine.QuartetBatch(ds, q, want32=precision == 32)
     n = sb.nbf
     if n ** 4 * 8 > 64 * 2 ** 30:
         raise MemoryError(f"dense ERI tensor of {n} functions does not fit")
-    vals = torch.zeros(max(1, batch.total), dtype=torch.float64, device=ds.device)
-    batch.run(vals, precision)
+    ds = engine.DeviceShells(sb, device)
     dev = ds.device
+    try:
+        batch = engine.UniqueQuartets(ds, want32=precision == 32)
+        nq, qt, offs = batch.n, batch.quartets, batch.block_offsets
+    except ValueError:
+        # very many different contractions: a task per quartet, planned on the host
+        q = unique_shell_quartets(sb.nshell)
+        batch = engine.QuartetBatch(ds, q, want32=precision == 32)
+        nq = len(q)
+        qt = torch.as_tensor(np.ascontiguousarray(q, dtype=np.int32)).to(dev)
+        offs = torch.as_tensor(np.ascontiguousarray(batch.offsets[:-1], dtype=np.int64)).to(dev)
+    vals = torch.empty(max(1, batch.total), dtype=torch.float64, device=dev)
+    batch.run(vals, precision)
     # the 8-fold expansion on the device (gs_dense_expand): one warp per unique block
-    qt = torch.as_tensor(np.ascontiguousarray(q, dtype=np.int32)).to(dev)
-    offs = torch.as_tensor(np.ascontiguousarray(batch.offsets[:-1], dtype=np.int64)).to(dev)
     t = torch.empty((n, n, n, n), dtype=torch.float64, device=dev)
-    _lib.check(_lib.lib().gs_dense_expand(len(q), _lib.ptr(qt), _lib.ptr(offs), _lib.ptr(vals),
+    _lib.check(_lib.lib().gs_dense_expand(nq, _lib.ptr(qt), _lib.ptr(offs), _lib.ptr(vals),
                                           _lib.ptr(ds.l), _lib.ptr(ds.func_off), n, _lib.ptr(t),
                                           _lib.stream()), "gs_dense_expand")
     return t

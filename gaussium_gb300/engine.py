@@ -13,6 +13,8 @@ Layout in HBM (all owned by torch tensors):
                 longest blocks), equal primitive counts together (a warp's threads run
                 the same loop trip counts).
 """
+import functools
+
 import numpy as np
 import torch
 
@@ -48,6 +50,7 @@ THREAD_FORM, WARP_FORM, GROUPED_FORM, SPLIT_FORM, COOP_FORM, STACKED_FORM, CLUST
 SPLIT_OFF = set()
 
 
+@functools.lru_cache(maxsize=None)
 def heavy_threshold(cls):
     """Primitive quartets from which a quartet of class ``cls`` is run in the split form."""
     la, lb, lc, ld = cls
@@ -130,6 +133,7 @@ def segment_profiles(cls_list, work_desc, bounds):
     return out
 
 
+@functools.lru_cache(maxsize=None)
 def class_sizes(cls):
     """(accumulators of the [e0|f0] set, integrals of a block)."""
     la, lb, lc, ld = cls
@@ -138,6 +142,7 @@ def class_sizes(cls):
     return ne * nf, int(np.prod(NCART[list(cls)]))
 
 
+@functools.lru_cache(maxsize=None)
 def class_costs(cls, precision):
     """Slots per primitive quartet: of a lane in a full GPU, of a lone warp of the thread form
     (whose spills nothing hides), and of a warp of the warp forms.  The vertical recursion
@@ -355,6 +360,32 @@ def _check_device_tensor(t, device, what, shape=None):
         raise ValueError(f"{what} must be contiguous")
 
 
+PACK_BYTES = 1 << 20
+
+
+def upload(device, *arrays):
+    """numpy arrays as tensors on the device.  Small sets travel as one block, of which the
+    tensors are views (a copy from pageable memory costs 10 us or more whatever its size)."""
+    arrays = [np.ascontiguousarray(a) for a in arrays]
+    offs, total = [], 0
+    for a in arrays:
+        offs.append(total)
+        total += -(-a.nbytes // 256) * 256
+    if len(arrays) < 2 or total > PACK_BYTES:
+        return [torch.as_tensor(a).to(device) for a in arrays]
+    block = np.zeros(total, dtype=np.uint8)
+    for a, o in zip(arrays, offs):
+        block[o:o + a.nbytes] = a.reshape(-1).view(np.uint8)
+    dev = torch.from_numpy(block).to(device)
+    typed, out = {}, []
+    for a, o in zip(arrays, offs):
+        if a.dtype not in typed:
+            typed[a.dtype] = dev.view(torch.from_numpy(np.empty(0, a.dtype)).dtype)
+        strides = [x // a.itemsize for x in a.strides]
+        out.append(typed[a.dtype].as_strided(a.shape, strides, o // a.itemsize))
+    return out
+
+
 class DeviceShells:
     """A ShellBasis copied to the device."""
 
@@ -362,17 +393,13 @@ class DeviceShells:
         self.host = sb
         self.device = indexed_device(device)
 
-        def t(a, dt):
-            return torch.as_tensor(np.ascontiguousarray(a), dtype=dt).to(self.device)
-
-        self.centre = t(sb.centre, torch.float64)
-        self.l = t(sb.l, torch.int32)
-        self.prim_off = t(sb.prim_off, torch.int32)
-        self.expo = t(sb.expo, torch.float64)
-        self.coef = t(sb.coef, torch.float64)
-        self.comp_scale = t(sb.comp_scale, torch.float64)
-        self.func_off = t(sb.func_off, torch.int32)
-        self.nprim = t(sb.nprim, torch.int64)          # primitives per shell (device planning)
+        # nprim: primitives per shell (device planning)
+        (self.centre, self.l, self.prim_off, self.expo, self.coef, self.comp_scale, self.func_off,
+         self.nprim) = upload(
+            self.device, sb.centre.astype(np.float64, copy=False), sb.l.astype(np.int32, copy=False),
+            sb.prim_off.astype(np.int32, copy=False), sb.expo.astype(np.float64, copy=False),
+            sb.coef.astype(np.float64, copy=False), sb.comp_scale.astype(np.float64, copy=False),
+            sb.func_off.astype(np.int32, copy=False), sb.nprim.astype(np.int64))
         self.nshell = sb.nshell
         self.nbf = sb.nbf
 
@@ -423,7 +450,10 @@ def check_shell_indices(idx, nshell, what):
 class PairSet:
     """Shell pairs (la >= lb inside each pair) with their primitive-pair records."""
 
-    def __init__(self, ds: DeviceShells, pair_shells, want32=True, stream=None, max_exp=0.0):
+    def __init__(self, ds: DeviceShells, pair_shells, want32=True, stream=None, max_exp=0.0,
+                 count=True):
+        """``count=False``: leave the kept primitive pairs per pair on the device (``nprim`` then
+        holds all of them)."""
         ps = np.ascontiguousarray(pair_shells, dtype=np.int32).reshape(-1, 2)
         sb = ds.host
         check_shell_indices(ps, sb.nshell, "shell pairs")
@@ -441,21 +471,21 @@ class PairSet:
         self.la = sb.l[ps[:, 0]] if len(ps) else np.zeros(0, np.int32)
         self.lb = sb.l[ps[:, 1]] if len(ps) else np.zeros(0, np.int32)
         dev = ds.device
-        self.shells = torch.as_tensor(ps).to(dev)
-        self.prim_start = torch.as_tensor(off[:-1].astype(np.int32)).to(dev)
+        # groups: consecutive pairs packed into warps of at most 32 primitive pairs (the build)
+        self.shells, self.prim_start, self.groups = upload(dev, ps, off[:-1].astype(np.int32),
+                                                           pair_groups(npp))
         self.rec = torch.empty(max(1, self.n) * PAIR_REC, dtype=torch.uint8, device=dev)
         total = max(1, int(off[-1]))
         self.p64 = torch.empty(total * PRIM64, dtype=torch.uint8, device=dev)
         self.p32 = torch.empty(total * PRIM32, dtype=torch.uint8, device=dev) if want32 else None
         self.nprim_pairs = int(off[-1])
         self.max_exp = max_exp
-        # consecutive pairs packed into warps of at most 32 primitive pairs (the pair build)
-        self.groups = torch.as_tensor(pair_groups(npp)).to(dev)
         self.ngroups = int(self.groups.numel()) - 1
         self.kept = torch.zeros(max(1, self.n), dtype=torch.int32, device=dev)
         self.build(stream)
         # primitive pairs kept per shell pair (the work per pair after screening)
-        self.nprim = self.kept[:self.n].cpu().numpy().astype(np.int64)
+        if count:
+            self.nprim = self.kept[:self.n].cpu().numpy().astype(np.int64)
 
     def build(self, stream=None, want32=True):
         """(Re)compute the pair records (kernel K0) from the device shells; with
@@ -748,6 +778,98 @@ class QuartetBatch:
             _lib.check(rc, f"gs_eri_blocks{cls}")
         lane.join()
         return out
+
+
+RANGE_DTYPE = np.dtype([("first", "<i8"), ("base", "<i8"), ("bra", "<i4"), ("nbra", "<i4"),
+                        ("ket", "<i4"), ("nket", "<i4"), ("size", "<i4"), ("pad", "<i4")])
+MAX_RANGES = 1 << 15
+
+
+def unique_pair_ranges(pair_class, nprim):
+    """The unique quartets of pairs sorted by class and, in a class, by descending primitive
+    count, as ranges (RANGE_DTYPE) of constant class and primitive-quartet count, each
+    class segment by descending count: (ranges, counts w per range, segments), or None if
+    they are too many (bases with hundreds of different contractions)."""
+    key = pair_class.astype(np.int64) << 32 | (2 ** 31 - nprim.astype(np.int64))
+    start = np.flatnonzero(np.diff(key, prepend=-1))
+    end = np.append(start[1:], len(key))
+    groups = [[] for _ in PAIR_ORDER]                  # per class: (first pair, pairs, nprim)
+    for s, e in zip(start.tolist(), end.tolist()):
+        groups[int(pair_class[s])].append((s, e - s, int(nprim[s])))
+    if sum(len(g) for g in groups) ** 2 > 2 * MAX_RANGES:
+        return None
+    rows, work, segments = [], [], []
+    first = base = 0
+    for cb in range(len(PAIR_ORDER)):
+        for ck in range(cb + 1):
+            cls = PAIR_ORDER[cb] + PAIR_ORDER[ck]
+            size = class_sizes(cls)[1]
+            found = []
+            for i, (b, nb, wb) in enumerate(groups[cb]):
+                for j, (k, nk, wk) in enumerate(groups[ck]):
+                    if cb != ck or j < i:
+                        found.append((wb * wk, b, nb, k, nk, nb * nk))
+                    elif j == i:
+                        found.append((wb * wk, b, nb, 0, 0, nb * (nb + 1) // 2))
+            begin = first
+            for w, b, nb, k, nk, count in sorted(found, key=lambda x: -x[0]):
+                rows.append((first, base, b, nb, k, nk, size, 0))
+                work.append((w, count))
+                first += count
+                base += count * size
+            if first > begin:
+                segments.append((cls, begin, first))
+    return np.array(rows, dtype=RANGE_DTYPE), work, segments
+
+
+class UniqueQuartets:
+    """Blocks of every unique shell quartet of a basis, each in canonical shell order (bra
+    pair class >= ket pair class, la >= lb), for the dense tensor: one record per shell pair,
+    and tasks expanded on the device (``gs_product_tasks``) from a few ranges of pairs.
+    Blocks go through QuartetBatch.run."""
+
+    def __init__(self, ds: DeviceShells, want32=False):
+        sb = ds.host
+        i, j = np.tril_indices(sb.nshell)
+        swap = sb.l[i] < sb.l[j]
+        a, b = np.where(swap, j, i), np.where(swap, i, j)
+        pc = _pc_lut[sb.l[a], sb.l[b]]
+        npp = sb.nprim[a].astype(np.int64) * sb.nprim[b]
+        order = np.lexsort((-npp, pc))                 # every primitive pair is kept (no screen)
+        plan = unique_pair_ranges(pc[order], npp[order])
+        if plan is None:
+            raise ValueError("too many ranges")
+        ranges, work, self.segments = plan
+        self.ds = ds
+        self.pairs = PairSet(ds, np.stack([a, b], 1)[order], want32=want32, count=False)
+        self.n = self.segments[-1][2] if self.segments else 0
+        last = ranges[-1] if len(ranges) else None
+        self.total = 0 if last is None else int(last["base"] + work[-1][1] * last["size"])
+        at = 0
+        self.heavy, self.profiles = [], []
+        for cls, s, e in self.segments:
+            mine = []
+            while at < len(work) and ranges["first"][at] < e:
+                mine.append(work[at])
+                at += 1
+            w, c = np.array(mine, dtype=np.int64).T    # w descending
+            upto = np.concatenate([[0], np.cumsum(c)])
+            ge = upto[np.searchsorted(-w, -np.concatenate(
+                [[heavy_threshold(cls), COOP_PRIM_QUARTETS], _LEVELS]), side="right")].tolist()
+            self.heavy.append((ge[0], ge[1]))
+            self.profiles.append((int((w * c).sum()), ge[2:]))
+        dev = ds.device
+        r = torch.as_tensor(ranges.view(np.uint8)).to(dev)
+        self.tasks = torch.empty(max(1, self.n) * WRITE_TASK, dtype=torch.uint8, device=dev)
+        self.quartets = torch.empty((max(1, self.n), 4), dtype=torch.int32, device=dev)
+        self.block_offsets = torch.empty(max(1, self.n), dtype=torch.int64, device=dev)
+        _lib.check(_lib.lib().gs_product_tasks(self.n, len(ranges), _lib.ptr(r),
+                                               _lib.ptr(self.pairs.shells), _lib.ptr(self.tasks),
+                                               _lib.ptr(self.quartets),
+                                               _lib.ptr(self.block_offsets), _lib.stream()),
+                   "gs_product_tasks")
+
+    run = QuartetBatch.run
 
 
 def eri_blocks(sb: ShellBasis, quartets, precision=64, device="cuda"):

@@ -425,6 +425,17 @@ int gs_fock_jk_batched_persistent(const void* pair_rec, const void* prim64, cons
                                   double* k, double screen_thr, double mixed_cut,
                                   void* workspace, long long ws_bytes, void* stream);
 
+/* Block tasks of unique shell quartets given as products of ranges of a canonical pair list
+ * (pair_shells[2 p], la >= lb): each of nranges 40-byte records {int64 first quartet, int64
+ * first block offset, int32 first bra pair, bra pairs, first ket pair, ket pairs, elements of
+ * a block, 0} stands for the quartets of its bra pairs with its ket pairs, or, with 0 ket
+ * pairs, of its bra pairs with themselves, ket <= bra; records in order of their first
+ * quartet.  Writes n tasks (gs_eri_blocks), the quartets' shells (4 each) and their block
+ * offsets (gs_dense_expand).  Device arrays.  Replaces the key enumeration of
+ * create_repulsion_matrix (matrixelements/electron_repulsion_matrix.py:28-42). */
+int gs_product_tasks(long long n, int nranges, const void* ranges, const int* pair_shells,
+                     void* tasks, int* quartets, long long* offsets, void* stream);
+
 /* Dense N^4 ERI tensor from unique shell-quartet blocks: the 8-fold expansion of
  * TwoElectronRepulsion.create_repulsion_matrix (matrixelements/electron_repulsion_matrix.py:
  * 43-45).  quartets[4*q..4*q+3] = shells (A, B, C, D) of block q; its n_A n_B n_C n_D values

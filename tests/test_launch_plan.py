@@ -258,3 +258,56 @@ def test_task_keys(gpu_lib):
     both = np.abs((keys & 63) - want)
     assert both.max() <= 1          # steps are sqrt(2) or 3/2 and 4/3: not quite the logarithm's
     assert np.mean(both) < 0.2
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_unique_pair_ranges(seed):
+    """The ranges hold every unique pair of pairs once, bra class >= ket class, and each class
+    segment is one run of them by descending primitive-quartet count."""
+    rng = np.random.default_rng(seed)
+    n = [1, 7, 40, 91][seed]
+    pc = np.sort(rng.integers(0, 6, n))
+    npp = rng.choice([1, 3, 6, 9, 18, 36], n)
+    order = np.lexsort((-npp, pc))
+    pc, npp = pc[order], npp[order]
+    ranges, work, segs = engine.unique_pair_ranges(pc, npp)
+    seen, at = set(), 0
+    for r, (w, count) in zip(ranges, work):
+        assert r["first"] == at
+        at += count
+        b = range(r["bra"], r["bra"] + r["nbra"])
+        mine = [(x, y) for x in b for y in range(r["ket"], r["ket"] + r["nket"])] if r["nket"] else \
+            [(x, y) for x in b for y in range(r["bra"], x + 1)]
+        assert len(mine) == count
+        for x, y in mine:
+            assert pc[x] >= pc[y] and npp[x] * npp[y] == w
+            assert (max(x, y), min(x, y)) not in seen
+            seen.add((max(x, y), min(x, y)))
+    assert len(seen) == n * (n + 1) // 2 == at == segs[-1][2]
+    for cls, s, e in segs:
+        w = [x[0] for r, x in zip(ranges, work) if s <= r["first"] < e]
+        assert w == sorted(w, reverse=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("basis,waters", [("STO-3G", 1), ("6-31G*", 2)])
+def test_dense_tensor_from_ranges(gpu_lib, basis, waters, monkeypatch):
+    """The dense tensor from pair ranges against the one from a host list of quartets."""
+    from gaussium_gb300 import dropin
+    from gaussium_gb300.molecules import shell_basis, water_cluster
+    sb = shell_basis(water_cluster(waters, seed=3), basis)
+    a = dropin.dense_eri(sb)
+    monkeypatch.setattr(engine, "MAX_RANGES", 0)
+    b = dropin.dense_eri(sb)
+    assert float((a - b).abs().max()) <= 1e-14 * float(b.abs().max())
+    for perm in ((1, 0, 2, 3), (0, 1, 3, 2), (2, 3, 0, 1)):
+        assert torch.equal(a, a.permute(perm))
+
+
+def test_upload_views():
+    arrays = [np.arange(5, dtype=np.int32), np.zeros((0, 2), np.float64), np.ones((3, 2)),
+              np.arange(3, dtype=np.int64)]
+    got = engine.upload("cpu", *arrays)
+    for a, t in zip(arrays, got):
+        assert t.numpy().dtype == a.dtype and np.array_equal(t.numpy(), a)
+        assert t.data_ptr() % 8 == 0
