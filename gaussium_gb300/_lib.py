@@ -34,6 +34,11 @@ _SIGS = {
                                           P, I, P, P, P, I, P, P, D, D, P, ctypes.c_longlong, P]),
     "gs_fock_jk_mixed": (I, [I, I, I, I, P, P, P, P, P, I, I, I, P, P, P, I, P, P, P, D, D, P,
                              ctypes.c_longlong, P]),
+    "gs_fock_jk_mixed_forms": (I, [I, I, I, I, I, I, P, P, P, P, P, I, I, I, P, P, P, I, P, P, P, D,
+                                   D, P, ctypes.c_longlong, P]),
+    "gs_fock_jk_batched_mixed_forms": (I, [I, I, I, I, I, I, P, P, P, P, P, P, P, P, P, P, P, P,
+                                           ctypes.c_longlong, I, P, P, P, I, P, P, D, D, P,
+                                           ctypes.c_longlong, P]),
     "gs_fock_jk_mixed_noalloc": (I, [I, I, I, I, P, P, P, P, P, I, I, I, P, P, P, I, P, P, P, D,
                                      D, P]),
     "gs_fock_jk_mixed_noalloc_max_tasks": (I, []),

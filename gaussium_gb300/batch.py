@@ -15,7 +15,7 @@ import torch
 
 from . import _lib
 from .basis import ShellBasis
-from .engine import (MIXED_LANES, PAIR_ORDER, PRIM_SCREEN, SIDE_STREAMS, DeviceShells, HeavyLane,
+from .engine import (MIXED_LANES, PAIR_ORDER, PRIM_SCREEN, DeviceShells, HeavyLane,
                      MixedWorkspace, PairSet, _pc_lut, launch_plan, mixed_plan, segment_profiles,
                      task_keys)
 from .hamiltonian import one_electron
@@ -190,39 +190,33 @@ class BatchedRHF(MixedWorkspace):
             # kernel runs, FP64/FP32 by the density-weighted bound
             cut = mixed_cut if mixed_cut is not None else 0.0
             thr = screen_thr if screen_thr > 0 else 1e-300
-            ws, each = self.mixed_workspace(self.dev)
-            segs = [x for x in zip(self.segments, self.heavy, self.profiles)
-                    if classes is None or x[0][0] in classes]
-            # the heavy prefix in the heavy forms, banded launches per precision; the bound
-            # there takes each molecule's largest |P| (at least the block value the partition
-            # uses, so no quartet is screened or demoted that the partition would keep).  It
-            # is ready before any side stream forks.
-            plans = [mixed_plan(self, cls, s, e, heavy, prof, cut)
-                     for (cls, s, e), heavy, prof in segs]
+            banded, tiers = mixed_plan(self, classes, cut)
+            ws, each = self.mixed_workspace(self.dev, tiers)
+            # the bound of the banded launches takes each molecule's largest |P| (at least the
+            # block value the partition uses, so no quartet is screened or demoted that the
+            # partition would keep).  It is ready before any side stream forks.
             mol_dmax = torch.zeros(len(self.mol_n), dtype=torch.float64, device=self.dev)
-            if any(launches for _, launches in plans):
+            if banded:
                 mol_dmax.scatter_reduce_(0, self.block_mol, dmax, "amax", include_self=True)
-            for i, (((cls, s, e), _, _), (h, launches)) in enumerate(zip(segs, plans)):
-                for j, (prec, form, first, count, lo, hi) in enumerate(launches):
-                    rc = L.gs_fock_jk_batched(
-                        *cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
-                        _lib.ptr(self.pairs.prims(prec)), _lib.ptr(self.ds.comp_scale),
-                        _lib.ptr(self.local_fo), _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base),
-                        _lib.ptr(self.mol_n), _lib.ptr(mol_dmax), self.mat_stride, count,
-                        base + (s + first) * 8, _lib.ptr(P), _lib.ptr(J), 1, _lib.ptr(P),
-                        _lib.ptr(K), thr, lo, hi,
-                        lane.stream(MIXED_LANES - 1 + j % (SIDE_STREAMS + 1 - MIXED_LANES)))
-                    _lib.check(rc, f"gs_fock_jk_batched{cls}")
-                rc = L.gs_fock_jk_batched_mixed(
-                    *cls, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
+            for i, (cls, first, prec, form, count, lo, hi) in enumerate(banded):
+                rc = L.gs_fock_jk_batched(
+                    *cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
+                    _lib.ptr(self.pairs.prims(prec)), _lib.ptr(self.ds.comp_scale),
+                    _lib.ptr(self.local_fo), _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base),
+                    _lib.ptr(self.mol_n), _lib.ptr(mol_dmax), self.mat_stride, count,
+                    base + first * 8, _lib.ptr(P), _lib.ptr(J), 1, _lib.ptr(P), _lib.ptr(K), thr,
+                    lo, hi, lane.lane(i + 1))
+                _lib.check(rc, f"gs_fock_jk_batched{cls}")
+            for i, (cls, first, count, f64, f32) in enumerate(tiers):
+                rc = L.gs_fock_jk_batched_mixed_forms(
+                    *cls, f64, f32, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
                     _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale), _lib.ptr(self.local_fo),
                     _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base), _lib.ptr(self.mol_n),
                     _lib.ptr(dmax), _lib.ptr(self.mol_shell0), _lib.ptr(self.mol_nshell),
-                    _lib.ptr(self.mol_sbase), self.mat_stride, e - s - h, base + (s + h) * 8,
-                    _lib.ptr(P), _lib.ptr(J), 1,
-                    _lib.ptr(P), _lib.ptr(K), thr, cut, ws + (i % MIXED_LANES) * each, each,
-                    lane.lane(i, MIXED_LANES))
-                _lib.check(rc, f"gs_fock_jk_batched_mixed{cls}")
+                    _lib.ptr(self.mol_sbase), self.mat_stride, count, base + first * 8,
+                    _lib.ptr(P), _lib.ptr(J), 1, _lib.ptr(P), _lib.ptr(K), thr, cut,
+                    ws + (i % MIXED_LANES) * each, each, lane.lane(i, MIXED_LANES))
+                _lib.check(rc, f"gs_fock_jk_batched_mixed_forms{cls}")
             lane.join()
             return
         thr = 0.0

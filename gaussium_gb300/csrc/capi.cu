@@ -625,10 +625,13 @@ int fock_jk_mixed_impl(int la, int lb, int lc, int ld, const void* pair_rec, con
                        int nshell, int nbf, int ntask, const int* tasks, const double* pj,
                        double* j, int nk, const double* pk, double* k,
                        const double* shell_dmax, double screen_thr, double mixed_cut,
-                       void* workspace, long long ws_bytes, void* stream) {
+                       void* workspace, long long ws_bytes, void* stream, int form64 = 0,
+                       int form32 = 0) {
     launch_fn f = find_class(la, lb, lc, ld);
     if (!f) return GS_ERR_CLASS;
-    if (ntask < 0 || nbf <= 0 || nk < 0 || !pair_rec || !prim64 || !prim32 || !comp_scale ||
+    const int pf64 = decode_precision(la, lb, lc, ld, form64 < 0 ? -1 : 64 | form64 << 8);
+    const int pf32 = decode_precision(la, lb, lc, ld, form32 < 0 ? -1 : 32 | form32 << 8);
+    if (pf64 < 0 || pf32 < 0 || ntask < 0 || nbf <= 0 || nk < 0 || !pair_rec || !prim64 || !prim32 || !comp_scale ||
         !func_off || (ntask > 0 && !tasks) || (!!pj != !!j) || (nk > 0 && (!pk || !k)) ||
         !shell_dmax || !workspace)
         return GS_ERR_ARG;
@@ -664,12 +667,12 @@ int fock_jk_mixed_impl(int la, int lb, int lc, int ld, const void* pair_rec, con
     a.prims = prim64;
     a.tasks = l64;
     a.ntask_dev = counts;
-    int rc = f(GS_KIND_JK, pv(la, lb, lc, ld, 64), &a, S(stream));
+    int rc = f(GS_KIND_JK, pf64, &a, S(stream));
     if (rc) return rc;
     a.prims = prim32;
     a.tasks = l32;
     a.ntask_dev = counts + 1;
-    return f(GS_KIND_JK, pv(la, lb, lc, ld, 32), &a, S(stream));
+    return f(GS_KIND_JK, pf32, &a, S(stream));
 }
 }  // namespace
 
@@ -682,6 +685,18 @@ int gs_fock_jk_mixed(int la, int lb, int lc, int ld, const void* pair_rec, const
     return fock_jk_mixed_impl(la, lb, lc, ld, pair_rec, prim64, prim32, comp_scale, func_off,
                               nshell, nbf, ntask, tasks, pj, j, nk, pk, k, shell_dmax, screen_thr,
                               mixed_cut, workspace, ws_bytes, stream);
+}
+
+int gs_fock_jk_mixed_forms(int la, int lb, int lc, int ld, int form64, int form32,
+                           const void* pair_rec, const void* prim64, const void* prim32,
+                           const double* comp_scale, const int* func_off, int nshell, int nbf,
+                           int ntask, const int* tasks, const double* pj, double* j, int nk,
+                           const double* pk, double* k, const double* shell_dmax,
+                           double screen_thr, double mixed_cut, void* workspace,
+                           long long ws_bytes, void* stream) {
+    return fock_jk_mixed_impl(la, lb, lc, ld, pair_rec, prim64, prim32, comp_scale, func_off,
+                              nshell, nbf, ntask, tasks, pj, j, nk, pk, k, shell_dmax, screen_thr,
+                              mixed_cut, workspace, ws_bytes, stream, form64, form32);
 }
 
 // ---------------------------------------------------------------------- no-allocation form
@@ -720,7 +735,9 @@ int gs_fock_jk_mixed_noalloc(int la, int lb, int lc, int ld, const void* pair_re
                               mixed_cut, ws, (long long)sizeof(g_noalloc_ws), stream);
 }
 
-int gs_fock_jk_batched_mixed(int la, int lb, int lc, int ld, const void* pair_rec,
+namespace {
+int fock_jk_batched_mixed_impl(int la, int lb, int lc, int ld, int form64, int form32,
+                               const void* pair_rec,
                              const void* prim64, const void* prim32, const double* comp_scale,
                              const int* func_off, const int* shell_mol, const long long* mol_base,
                              const int* mol_n, const double* mol_dmax, const int* mol_shell0,
@@ -730,7 +747,9 @@ int gs_fock_jk_batched_mixed(int la, int lb, int lc, int ld, const void* pair_re
                              double mixed_cut, void* workspace, long long ws_bytes, void* stream) {
     launch_fn f = find_class(la, lb, lc, ld);
     if (!f) return GS_ERR_CLASS;
-    if (ntask < 0 || nk < 0 || nk > 1 || !pair_rec || !prim64 || !prim32 || !comp_scale ||
+    const int pf64 = decode_precision(la, lb, lc, ld, form64 < 0 ? -1 : 64 | form64 << 8);
+    const int pf32 = decode_precision(la, lb, lc, ld, form32 < 0 ? -1 : 32 | form32 << 8);
+    if (pf64 < 0 || pf32 < 0 || ntask < 0 || nk < 0 || nk > 1 || !pair_rec || !prim64 || !prim32 || !comp_scale ||
         !func_off || !shell_mol || !mol_base || !mol_n || !mol_dmax || (ntask > 0 && !tasks) ||
         (!!pj != !!j) || (nk > 0 && (!pk || !k)) || mat_stride <= 0 || !workspace ||
         (!!mol_sbase != !!mol_shell0) || (!!mol_sbase != !!mol_nshell))
@@ -769,12 +788,42 @@ int gs_fock_jk_batched_mixed(int la, int lb, int lc, int ld, const void* pair_re
     a.prims = prim64;
     a.tasks = l64;
     a.ntask_dev = counts;
-    int rc = f(GS_KIND_JK, pv(la, lb, lc, ld, 64), &a, S(stream));
+    int rc = f(GS_KIND_JK, pf64, &a, S(stream));
     if (rc) return rc;
     a.prims = prim32;
     a.tasks = l32;
     a.ntask_dev = counts + 1;
-    return f(GS_KIND_JK, pv(la, lb, lc, ld, 32), &a, S(stream));
+    return f(GS_KIND_JK, pf32, &a, S(stream));
+}
+}  // namespace
+
+int gs_fock_jk_batched_mixed(int la, int lb, int lc, int ld, const void* pair_rec,
+                             const void* prim64, const void* prim32, const double* comp_scale,
+                             const int* func_off, const int* shell_mol, const long long* mol_base,
+                             const int* mol_n, const double* mol_dmax, const int* mol_shell0,
+                             const int* mol_nshell, const long long* mol_sbase,
+                             long long mat_stride, int ntask, const int* tasks, const double* pj,
+                             double* j, int nk, const double* pk, double* k, double screen_thr,
+                             double mixed_cut, void* workspace, long long ws_bytes, void* stream) {
+    return fock_jk_batched_mixed_impl(la, lb, lc, ld, 0, 0, pair_rec, prim64, prim32, comp_scale,
+                                      func_off, shell_mol, mol_base, mol_n, mol_dmax, mol_shell0,
+                                      mol_nshell, mol_sbase, mat_stride, ntask, tasks, pj, j, nk, pk,
+                                      k, screen_thr, mixed_cut, workspace, ws_bytes, stream);
+}
+
+int gs_fock_jk_batched_mixed_forms(int la, int lb, int lc, int ld, int form64, int form32,
+                             const void* pair_rec,
+                             const void* prim64, const void* prim32, const double* comp_scale,
+                             const int* func_off, const int* shell_mol, const long long* mol_base,
+                             const int* mol_n, const double* mol_dmax, const int* mol_shell0,
+                             const int* mol_nshell, const long long* mol_sbase,
+                             long long mat_stride, int ntask, const int* tasks, const double* pj,
+                             double* j, int nk, const double* pk, double* k, double screen_thr,
+                             double mixed_cut, void* workspace, long long ws_bytes, void* stream) {
+    return fock_jk_batched_mixed_impl(la, lb, lc, ld, form64, form32, pair_rec, prim64, prim32, comp_scale,
+                                      func_off, shell_mol, mol_base, mol_n, mol_dmax, mol_shell0,
+                                      mol_nshell, mol_sbase, mat_stride, ntask, tasks, pj, j, nk, pk,
+                                      k, screen_thr, mixed_cut, workspace, ws_bytes, stream);
 }
 
 int gs_boys_eval(int m, int precision, int n, const double* t, double* F, void* stream) {

@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(32 * kSplitWarps) k_eri_jk_split(const JKArgs 
     using G = ClassGen<LA, LB, LC, LD>;
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * kSplitWarps + (threadIdx.x >> 5);
-    if (t >= a.ntask) return;                      // warp-uniform
+    if (t >= (a.ntask_dev ? *a.ntask_dev : a.ntask)) return;       // warp-uniform
     const int2 task = a.tasks[t];
     const PairRec B = a.pairs[task.x];
     const PairRec K = a.pairs[task.y];
@@ -328,9 +328,8 @@ __global__ void __launch_bounds__(kBlock) k_schwarz(const SchwarzArgs a) {
     a.q[p] = sqrt(m);
 }
 
-// The split form (one warp per quartet over its primitive quartets, thread-form code).
-// Task counts on the device (partitioned lists) are not supported; those launches use the
-// thread form.
+// The split form (one warp per quartet over its primitive quartets, thread-form code).  A task
+// count on the device (a partitioned list) ends the warps beyond it; the grid covers its bound.
 template <int LA, int LB, int LC, int LD, int PREC>
 int launch_class_split(int kind, const void* args, cudaStream_t st) {
     using T = typename std::conditional<PREC == 64, double, float>::type;
@@ -342,7 +341,6 @@ int launch_class_split(int kind, const void* args, cudaStream_t st) {
     } else if (kind == GS_KIND_JK) {
         const JKArgs& a = *(const JKArgs*)args;
         if (a.ntask <= 0) return 0;
-        if (a.ntask_dev) return GS_ERR_ARG;
         k_eri_jk_split<LA, LB, LC, LD, T><<<(a.ntask + kSplitWarps - 1) / kSplitWarps, TPB, 0, st>>>(a);
     } else {
         return GS_ERR_ARG;

@@ -121,12 +121,8 @@ int launch_prec(int kind, int variant, int per, const void* args, cudaStream_t s
         return thread ? 1 : (wide ? 2 : 0);
     }
     if constexpr (thread) {
-        if (v == 4 && kind != GS_KIND_SCHWARZ) {
-            // task counts that live on the device run in the thread form
-            if (kind == GS_KIND_JK && ((const JKArgs*)args)->ntask_dev)
-                return launch_class<LA, LB, LC, LD, PREC>(kind, args, st);
+        if (v == 4 && kind != GS_KIND_SCHWARZ)
             return launch_class_split<LA, LB, LC, LD, PREC>(kind, args, st);
-        }
     }
     if (v == 4) v = 1;
     if constexpr (wide) {

@@ -740,8 +740,8 @@ __global__ void __launch_bounds__(32 * kWideWarps) k_wide_schwarz(const SchwarzA
 // own accumulators; the partial sums meet in shared memory, added in
 // warp order (the result does not depend on timing), and warp 0 runs the HRR and the
 // epilogue.  A class's tasks are sorted by descending primitive work, so its heavy prefix
-// is a contiguous range with a host count; this form takes that range and leaves the rest
-// of the segment to the one-warp form.
+// is a contiguous range; this form takes that range and leaves the rest of the segment to
+// the one-warp form.
 //
 // Warp w takes primitive quartets w, w + warps, ..., so the warps' shares differ by one at
 // most and none waits long at the reduction.
@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(32 * kCoopMaxWarps) k_wide_jk_coop(const JKArg
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     T* base = reinterpret_cast<T*>(smem_raw);
     const int t = blockIdx.x;
-    if (t >= a.ntask) return;                      // block-uniform
+    if (t >= (a.ntask_dev ? *a.ntask_dev : a.ntask)) return;       // block-uniform
     const int2 task = a.tasks[t];
     const PairRec B = a.pairs[task.x];
     const PairRec K = a.pairs[task.y];
@@ -922,6 +922,7 @@ k_wide_jk_cluster(const JKArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     T* base = reinterpret_cast<T*>(smem_raw);
+    if (a.ntask_dev && (int)blockIdx.x / kClusterBlocks >= *a.ntask_dev) return;   // cluster-uniform
     const int2 task = a.tasks[blockIdx.x / kClusterBlocks];
     const PairRec B = a.pairs[task.x];
     const PairRec K = a.pairs[task.y];
@@ -986,7 +987,8 @@ int launch_wide(int kind, const void* args, cudaStream_t st, int per) {
     return cudaGetLastError() == cudaSuccess ? 0 : GS_ERR_CUDA;
 }
 
-// The cooperative form (host task counts only: the heavy prefix of a class segment).
+// The cooperative form (the heavy prefix of a class segment; a task count on the device ends
+// the blocks beyond it).
 template <int LA, int LB, int LC, int LD, int PREC>
 int launch_wide_coop(int kind, const void* args, cudaStream_t st) {
     using T = typename std::conditional<PREC == 64, double, float>::type;
@@ -1000,7 +1002,6 @@ int launch_wide_coop(int kind, const void* args, cudaStream_t st) {
         using CL = CoopLayout<LA, LB, LC, LD, T, true>;
         const JKArgs& a = *(const JKArgs*)args;
         if (a.ntask <= 0) return 0;
-        if (a.ntask_dev) return GS_ERR_ARG;
         if (set_smem<k_wide_jk_coop<LA, LB, LC, LD, T>>(CL::BYTES)) return GS_ERR_CUDA;
         k_wide_jk_coop<LA, LB, LC, LD, T><<<a.ntask, 32 * CL::WARPS, CL::BYTES, st>>>(a);
     } else {
@@ -1009,7 +1010,7 @@ int launch_wide_coop(int kind, const void* args, cudaStream_t st) {
     return cudaGetLastError() == cudaSuccess ? 0 : GS_ERR_CUDA;
 }
 
-// The cluster form (host task counts only).
+// The cluster form.
 template <int LA, int LB, int LC, int LD, int PREC>
 int launch_wide_cluster(int kind, const void* args, cudaStream_t st) {
     using T = typename std::conditional<PREC == 64, double, float>::type;
@@ -1024,7 +1025,6 @@ int launch_wide_cluster(int kind, const void* args, cudaStream_t st) {
         using CL = CoopLayout<LA, LB, LC, LD, T, true>;
         const JKArgs& a = *(const JKArgs*)args;
         if (a.ntask <= 0) return 0;
-        if (a.ntask_dev) return GS_ERR_ARG;
         if (set_smem<k_wide_jk_cluster<LA, LB, LC, LD, T>>(CL::BYTES)) return GS_ERR_CUDA;
         k_wide_jk_cluster<LA, LB, LC, LD, T>
             <<<a.ntask * kClusterBlocks, 32 * CL::WARPS, CL::BYTES, st>>>(a);

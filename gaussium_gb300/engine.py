@@ -246,24 +246,32 @@ def launch_plan(engine_like, precision, kind, classes=None, share=1.0):
     return sorted(out, key=lambda x: -x[4])
 
 
-def mixed_plan(engine_like, cls, s, t, heavy, prof, mixed_cut):
-    """mixed_prefix for a class segment whose forms were not chosen: the tiers above the
-    lightest of either precision's plan (class_plan) as banded launches over the same
-    prefix, the partitioned launch taking the rest."""
+def mixed_plan(engine_like, classes, mixed_cut):
+    """(banded, tiers) of a mixed-precision build.  banded: [(class, first task, precision,
+    form, count, lo, hi)], the heavy prefixes (mixed_prefix) of the classes whose form was
+    chosen.  tiers: [(class, first task, count, form64, form32)], longest latency first, for
+    one partitioned launch each: a class segment cut wherever either precision's plan
+    (class_plan) changes its form."""
     e = engine_like
     L = _lib.lib()
-    if any(L.gs_class_variant(*cls, p) or (cls, p) in SPLIT_OFF for p in (64, 32)):
-        return mixed_prefix(cls, heavy, mixed_cut)
-    plans = {p: [(form, first - s, count) for c, first, count, form, _ in
-                 launch_plan(e, p, "jk", [cls], 0.5)] for p in (64, 32)}
-    h = max((first for p in plans.values() for _, first, _ in p), default=0)
-    out = []
-    for p, lo, hi in ((64, mixed_cut, float("inf")), (32, 0.0, mixed_cut)):
-        for form, first, count in plans[p]:
-            c = min(count, h - first)
-            if c > 0 and hi > 0.0:
-                out.append((p, form, first, c, lo, hi))
-    return h, out
+    banded, tiers = [], []
+    for (cls, s, t), heavy in zip(e.segments, e.heavy):
+        if classes is not None and cls not in classes:
+            continue
+        if any(L.gs_class_variant(*cls, p) or (cls, p) in SPLIT_OFF for p in (64, 32)):
+            h, launches = mixed_prefix(cls, heavy, mixed_cut)
+            banded += [(cls, s + first, p, form, n, lo, hi) for p, form, first, n, lo, hi in launches]
+            if s + h < t:
+                tiers.append((0.0, cls, s + h, t - s - h, 0, 0))
+            continue
+        plans = [launch_plan(e, p, "jk", [cls], 0.5) for p in (64, 32)]
+        cuts = sorted({first for plan in plans for _, first, _, _, _ in plan} | {t})
+        for x, y in zip(cuts[:-1], cuts[1:]):
+            (f64, l64), (f32, l32) = [next((form, lat) for _, first, n, form, lat in plan
+                                           if first <= x < first + n) for plan in plans]
+            tiers.append((max(l64, l32), cls, x, y - x, f64, f32))
+    tiers.sort(key=lambda x: -x[0])
+    return banded, [x[1:] for x in tiers]
 
 
 def mixed_prefix(cls, heavy, mixed_cut):
@@ -882,21 +890,20 @@ def eri_blocks(sb: ShellBasis, quartets, precision=64, device="cuda"):
 
 
 # ---------------------------------------------------------------------- Fock (J/K) engine
-# streams of the partitioned launches of a mixed-precision build, each with its own workspace
-# (one class's lists at a time); the heavy tiers take the remaining side streams
-MIXED_LANES = 4
-
-
 class MixedWorkspace:
-    """The partition workspace of an engine with ``segments``: one region per stream of the
-    partitioned launches."""
+    """The partition workspace of an engine: one region per stream of the partitioned launches
+    (one launch's lists at a time)."""
 
-    def mixed_workspace(self, dev):
-        need = max(_lib.lib().gs_fock_jk_mixed_workspace(e - s) for _, s, e in self.segments)
+    def mixed_workspace(self, dev, tiers):
+        need = _lib.lib().gs_fock_jk_mixed_workspace(max((x[2] for x in tiers), default=0))
         need = -(-int(need) // 256) * 256
         if getattr(self, "_ws", None) is None or self._ws.numel() < MIXED_LANES * need:
             self._ws = torch.empty(MIXED_LANES * need, dtype=torch.uint8, device=dev)
         return self._ws.data_ptr(), need
+
+
+# streams of a mixed-precision build's partitioned launches
+MIXED_LANES = SIDE_STREAMS + 1
 
 
 def task_keys(pairs, bra, ket):
@@ -1049,30 +1056,25 @@ class JKEngine(MixedWorkspace):
         lane = HeavyLane(dev, stream)
         base = self.tasks.data_ptr()
         if mixed_cut is not None:
-            ws, each = self.mixed_workspace(dev)
-            segs = [x for x in zip(self.segments, self.heavy, self.profiles)
-                    if classes is None or x[0][0] in classes]
-            for i, ((cls, s, e), heavy, prof) in enumerate(segs):
-                # the heavy prefix in the heavy forms: banded launches per precision (the
-                # same density-weighted bound and cut as the partition)
-                h, launches = mixed_plan(self, cls, s, e, heavy, prof, mixed_cut)
-                for j, (prec, form, first, count, lo, hi) in enumerate(launches):
-                    rc = L.gs_fock_jk(*cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
-                                      _lib.ptr(self.pairs.prims(prec)),
-                                      _lib.ptr(self.ds.comp_scale), _lib.ptr(self.ds.func_off),
-                                      self.sb.nshell, n, count, base + (s + first) * 8,
-                                      _lib.ptr(pj_c), _lib.ptr(jbuf), nk, _lib.ptr(pk_c),
-                                      _lib.ptr(kbuf), _lib.ptr(dmax), thr, lo, hi,
-                                      lane.stream(MIXED_LANES - 1 + j % (SIDE_STREAMS + 1 - MIXED_LANES)))
-                    _lib.check(rc, f"gs_fock_jk{cls}")
-                rc = L.gs_fock_jk_mixed(*cls, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
-                                        _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale),
-                                        _lib.ptr(self.ds.func_off), self.sb.nshell, n, e - s - h,
-                                        base + (s + h) * 8, _lib.ptr(pj_c), _lib.ptr(jbuf), nk,
-                                        _lib.ptr(pk_c), _lib.ptr(kbuf), _lib.ptr(dmax), thr,
-                                        mixed_cut, ws + (i % MIXED_LANES) * each, each,
-                                        lane.lane(i, MIXED_LANES))
-                _lib.check(rc, f"gs_fock_jk_mixed{cls}")
+            banded, tiers = mixed_plan(self, classes, mixed_cut)
+            ws, each = self.mixed_workspace(dev, tiers)
+            for i, (cls, first, prec, form, count, lo, hi) in enumerate(banded):
+                rc = L.gs_fock_jk(*cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
+                                  _lib.ptr(self.pairs.prims(prec)), _lib.ptr(self.ds.comp_scale),
+                                  _lib.ptr(self.ds.func_off), self.sb.nshell, n, count,
+                                  base + first * 8, _lib.ptr(pj_c), _lib.ptr(jbuf), nk,
+                                  _lib.ptr(pk_c), _lib.ptr(kbuf), _lib.ptr(dmax), thr, lo, hi,
+                                  lane.lane(i + 1))
+                _lib.check(rc, f"gs_fock_jk{cls}")
+            for i, (cls, first, count, f64, f32) in enumerate(tiers):
+                rc = L.gs_fock_jk_mixed_forms(
+                    *cls, f64, f32, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
+                    _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale),
+                    _lib.ptr(self.ds.func_off), self.sb.nshell, n, count, base + first * 8,
+                    _lib.ptr(pj_c), _lib.ptr(jbuf), nk, _lib.ptr(pk_c), _lib.ptr(kbuf),
+                    _lib.ptr(dmax), thr, mixed_cut, ws + (i % MIXED_LANES) * each, each,
+                    lane.lane(i, MIXED_LANES))
+                _lib.check(rc, f"gs_fock_jk_mixed_forms{cls}")
             runs = []
         for prec, lo, hi in runs:
             prims = self.pairs.prims(prec)

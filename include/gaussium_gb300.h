@@ -83,7 +83,7 @@ int gs_class_variant(int la, int lb, int lc, int ld, int precision);
  * quartets (the heavy prefix of a class's task list, sorted by descending primitive work)
  * in the split form where the class runs one thread per quartet, and in the cooperative
  * form where it runs one warp per quartet (warp, grouped or stacked), the heaviest in the
- * cluster form.  The cooperative and cluster forms take host task counts only.  Bits 16.. give
+ * cluster form.  Bits 16.. give
  * the number of consecutive tasks a warp of the warp, grouped and stacked forms takes (1-8, 0 =
  * one; classes of total angular momentum above 6 always one): for tasks of few primitive
  * quartets, whose set-up then fills the warp's lanes.  Negative status on a bad class or precision.  No reference counterpart. */
@@ -213,6 +213,26 @@ int gs_fock_jk_batched(int la, int lb, int lc, int ld, int precision, const void
  * mol_shell0[m]); with those three arrays null, mol_dmax[m] is one value per molecule.
  * Same replaced reference functions as gs_fock_jk. */
 int gs_fock_jk_batched_mixed(int la, int lb, int lc, int ld, const void* pair_rec,
+                             const void* prim64, const void* prim32, const double* comp_scale,
+                             const int* func_off, const int* shell_mol, const long long* mol_base,
+                             const int* mol_n, const double* mol_dmax, const int* mol_shell0,
+                             const int* mol_nshell, const long long* mol_sbase,
+                             long long mat_stride, int ntask, const int* tasks, const double* pj,
+                             double* j, int nk, const double* pk, double* k, double screen_thr,
+                             double mixed_cut, void* workspace, long long ws_bytes, void* stream);
+
+/* gs_fock_jk_mixed and gs_fock_jk_batched_mixed with the kernel forms of the two launches (0 =
+ * the class's configured form; any form of gs_class_variants, with the tasks a warp takes in
+ * bits 8.., as in gs_eri_blocks' precision argument): the heavy tiers of a task list, whose
+ * FP64 and FP32 tasks each run in their own form on full warps. */
+int gs_fock_jk_mixed_forms(int la, int lb, int lc, int ld, int form64, int form32, const void* pair_rec, const void* prim64,
+                     const void* prim32, const double* comp_scale, const int* func_off,
+                     int nshell, int nbf, int ntask, const int* tasks, const double* pj, double* j,
+                     int nk, const double* pk, double* k, const double* shell_dmax,
+                     double screen_thr, double mixed_cut, void* workspace, long long ws_bytes,
+                     void* stream);
+int gs_fock_jk_batched_mixed_forms(int la, int lb, int lc, int ld, int form64, int form32,
+                             const void* pair_rec,
                              const void* prim64, const void* prim32, const double* comp_scale,
                              const int* func_off, const int* shell_mol, const long long* mol_base,
                              const int* mol_n, const double* mol_dmax, const int* mol_shell0,

@@ -44,23 +44,29 @@ def test_segment_profiles_match_host():
         assert prof == engine.work_profile(w)
 
 
-def test_mixed_plan_bands(monkeypatch):
-    """Both precisions' heavy tiers cover the same prefix, FP64 at or above the cut and FP32
-    below it; without a cut (screening only) there is no FP32 band."""
-    plans = {64: [((2, 2, 2, 2), 10, 2, 7, 9.0), ((2, 2, 2, 2), 12, 5, 5, 5.0), ((2, 2, 2, 2), 17, 83, 6, 1.0)],
-             32: [((2, 2, 2, 2), 10, 3, 5, 2.0), ((2, 2, 2, 2), 13, 87, 1, 1.0)]}
+def test_mixed_plan_tiers(monkeypatch):
+    """A segment is cut wherever either precision's form changes, each part in both plans'
+    forms; a class whose form was chosen keeps its banded prefix and one partitioned rest."""
+    import types
+    c1, c2 = (2, 2, 2, 2), (1, 0, 0, 0)
+    plans = {64: [(c1, 10, 2, 7, 9.0), (c1, 12, 5, 5, 5.0), (c1, 17, 83, 6, 1.0)],
+             32: [(c1, 10, 3, 5, 2.0), (c1, 13, 87, 1, 1.0)]}
 
     class Stub:
         def gs_class_variant(self, *a):
-            return 0
+            return int(a[:4] == c2)
+
+        def gs_class_form(self, *a):
+            return engine.THREAD_FORM
     monkeypatch.setattr(engine._lib, "lib", lambda: Stub())
     monkeypatch.setattr(engine, "launch_plan", lambda e, p, *a: plans[p])
+    eng = types.SimpleNamespace(segments=[(c1, 10, 100), (c2, 100, 130)], heavy=[(0, 0), (7, 2)])
+    banded, tiers = engine.mixed_plan(eng, None, 1e-3)
+    assert tiers == [(c1, 10, 2, 7, 5), (c1, 12, 1, 5, 5), (c1, 13, 4, 5, 1), (c1, 17, 83, 6, 1),
+                     (c2, 107, 23, 0, 0)]
     inf = float("inf")
-    h, out = engine.mixed_plan(None, (2, 2, 2, 2), 10, 100, None, None, 1e-3)
-    assert h == 7 and out == [(64, 7, 0, 2, 1e-3, inf), (64, 5, 2, 5, 1e-3, inf),
-                              (32, 5, 0, 3, 0.0, 1e-3), (32, 1, 3, 4, 0.0, 1e-3)]
-    h, out = engine.mixed_plan(None, (2, 2, 2, 2), 10, 100, None, None, 0.0)
-    assert h == 7 and [x[0] for x in out] == [64, 64]
+    assert banded == [(c2, 100, 64, 4, 7, 1e-3, inf), (c2, 100, 32, 4, 7, 0.0, 1e-3)]
+    assert engine.mixed_plan(eng, [c2], 1e-3)[1] == [(c2, 107, 23, 0, 0)]
 
 
 @pytest.mark.gpu
@@ -311,3 +317,41 @@ def test_upload_views():
     for a, t in zip(arrays, got):
         assert t.numpy().dtype == a.dtype and np.array_equal(t.numpy(), a)
         assert t.data_ptr() % 8 == 0
+
+
+@pytest.mark.gpu
+def test_mixed_forms_match(gpu_lib):
+    """The partitioned launch gives the same J/K in every pair of forms, the heavy forms with
+    their counts on the device among them; an unknown form is refused."""
+    from gaussium_gb300 import _lib
+    from gaussium_gb300.workloads import random_shell_quartets
+    sb, _, _ = random_shell_quartets(4, seed=5, box_angstrom=3.0, kmax=4)
+    eng = engine.JKEngine(sb, schwarz_thr=0.0)
+    n = sb.nbf
+    p = np.random.default_rng(6).standard_normal((n, n))
+    pt = torch.as_tensor(p + p.T).cuda()
+    dmax = eng.shell_dmax([pt])
+    ws = torch.empty(gpu_lib.gs_fock_jk_mixed_workspace(eng.ntasks), dtype=torch.uint8, device="cuda")
+    for cls, s, e in eng.segments:
+        forms = {q: [f for f in range(1, 8) if gpu_lib.gs_class_variants(*cls, q) & (1 << (f - 1))]
+                 for q in (64, 32)}
+        ref = None
+        for i in range(max(len(x) for x in forms.values())):
+            f64, f32 = (x[i % len(x)] for x in forms.values())
+            j = torch.zeros((n, n), dtype=torch.float64, device="cuda")
+            k = torch.zeros_like(j)
+
+            def call(f64, f32):
+                return gpu_lib.gs_fock_jk_mixed_forms(
+                    *cls, f64, f32, _lib.ptr(eng.pairs.rec), _lib.ptr(eng.pairs.p64),
+                    _lib.ptr(eng.pairs.p32), _lib.ptr(eng.ds.comp_scale),
+                    _lib.ptr(eng.ds.func_off), sb.nshell, n, e - s, eng.tasks.data_ptr() + 8 * s,
+                    _lib.ptr(pt), _lib.ptr(j), 1, _lib.ptr(pt), _lib.ptr(k), _lib.ptr(dmax), 1e-12,
+                    1e-4, _lib.ptr(ws), ws.numel(), _lib.stream())
+            _lib.check(call(f64, f32), "gs_fock_jk_mixed_forms")
+            ref = (j, k) if ref is None else ref
+            # FP32 quartets are below 1e-4: their rounding, 1e-5 of it, on up to 1e4 of them
+            for x, y in zip((j, k), ref):
+                assert float((x - y).abs().max()) <= 1e-5 * 1e-4 * 1e4 * 1e-2 + \
+                    1e-12 * float(y.abs().max()), (cls, f64, f32)
+            assert call(8, 0) == 1 and call(0, -1) == 1
