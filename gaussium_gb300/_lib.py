@@ -46,6 +46,14 @@ _SIGS = {
     "gs_class_form": (I, [I, I, I, I, I]),
     "gs_class_variant": (I, [I, I, I, I, I]),
     "gs_set_class_variant": (I, [I, I, I, I, I, I]),
+    "gs_class_variant_stamp": (ctypes.c_longlong, []),
+    "gs_eri_blocks_list": (I, [I, P, I, P, P, P, P, P, I, P]),
+    "gs_fock_jk_list": (I, [I, P, I, P, P, P, P, I, I, P, P, P, I, P, P, P, D, D, D, I, P]),
+    "gs_fock_jk_mixed_list": (I, [I, P, P, P, P, P, P, I, I, P, P, P, I, P, P, P, D, D, P,
+                                  ctypes.c_longlong, I, P]),
+    "gs_fock_jk_batched_mixed_list": (I, [I, P, P, P, P, P, P, P, P, P, P, P, P, P,
+                                          ctypes.c_longlong, P, P, P, I, P, P, D, D, P,
+                                          ctypes.c_longlong, I, P]),
     "gs_boys_eval": (I, [I, I, I, P, P, P]),
     "gs_product_tasks": (I, [ctypes.c_longlong, I, P, P, P, P, P, P]),
     "gs_task_keys": (I, [ctypes.c_longlong, P, P, P, P, P, P, P]),

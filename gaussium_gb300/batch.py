@@ -16,7 +16,7 @@ import torch
 from . import _lib
 from .basis import ShellBasis
 from .engine import (MIXED_LANES, PAIR_ORDER, PRIM_SCREEN, DeviceShells, HeavyLane,
-                     MixedWorkspace, PairSet, _pc_lut, launch_plan, mixed_plan, segment_profiles,
+                     MixedWorkspace, PairSet, _pc_lut, launch_plan, mixed_list, segment_profiles,
                      task_keys)
 from .hamiltonian import one_electron
 from .molecules import shell_basis
@@ -190,7 +190,7 @@ class BatchedRHF(MixedWorkspace):
             # kernel runs, FP64/FP32 by the density-weighted bound
             cut = mixed_cut if mixed_cut is not None else 0.0
             thr = screen_thr if screen_thr > 0 else 1e-300
-            banded, tiers = mixed_plan(self, classes, cut)
+            banded, tiers = mixed_list(self, classes, cut)
             ws, each = self.mixed_workspace(self.dev, tiers)
             # the bound of the banded launches takes each molecule's largest |P| (at least the
             # block value the partition uses, so no quartet is screened or demoted that the
@@ -207,16 +207,14 @@ class BatchedRHF(MixedWorkspace):
                     base + first * 8, _lib.ptr(P), _lib.ptr(J), 1, _lib.ptr(P), _lib.ptr(K), thr,
                     lo, hi, lane.lane(i + 1))
                 _lib.check(rc, f"gs_fock_jk_batched{cls}")
-            for i, (cls, first, count, f64, f32) in enumerate(tiers):
-                rc = L.gs_fock_jk_batched_mixed_forms(
-                    *cls, f64, f32, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
-                    _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale), _lib.ptr(self.local_fo),
-                    _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base), _lib.ptr(self.mol_n),
-                    _lib.ptr(dmax), _lib.ptr(self.mol_shell0), _lib.ptr(self.mol_nshell),
-                    _lib.ptr(self.mol_sbase), self.mat_stride, count, base + first * 8,
-                    _lib.ptr(P), _lib.ptr(J), 1, _lib.ptr(P), _lib.ptr(K), thr, cut,
-                    ws + (i % MIXED_LANES) * each, each, lane.lane(i, MIXED_LANES))
-                _lib.check(rc, f"gs_fock_jk_batched_mixed_forms{cls}")
+            rc = L.gs_fock_jk_batched_mixed_list(
+                len(tiers), tiers.ctypes.data, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
+                _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale), _lib.ptr(self.local_fo),
+                _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base), _lib.ptr(self.mol_n),
+                _lib.ptr(dmax), _lib.ptr(self.mol_shell0), _lib.ptr(self.mol_nshell),
+                _lib.ptr(self.mol_sbase), self.mat_stride, base, _lib.ptr(P), _lib.ptr(J), 1,
+                _lib.ptr(P), _lib.ptr(K), thr, cut, ws, each, *lane.streams(MIXED_LANES))
+            _lib.check(rc, "gs_fock_jk_batched_mixed_list")
             lane.join()
             return
         thr = 0.0

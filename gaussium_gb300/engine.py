@@ -13,6 +13,7 @@ Layout in HBM (all owned by torch tensors):
                 longest blocks), equal primitive counts together (a warp's threads run
                 the same loop trip counts).
 """
+import ctypes
 import functools
 
 import numpy as np
@@ -274,6 +275,46 @@ def mixed_plan(engine_like, classes, mixed_cut):
     return banded, [x[1:] for x in tiers]
 
 
+LAUNCH_DTYPE = np.dtype([("cls", "<i4", 4), ("form", "<i4"), ("form32", "<i4"), ("count", "<i4"),
+                         ("pad", "<i4"), ("first", "<i8")])
+
+
+def launch_records(launches):
+    """[(class, first task, count, form, FP32 form)] as the records of the list calls."""
+    out = np.zeros(len(launches), dtype=LAUNCH_DTYPE)
+    for r, (cls, first, count, form, form32) in zip(out, launches):
+        r["cls"], r["first"], r["count"], r["form"], r["form32"] = cls, first, count, form, form32
+    return out
+
+
+def kept_plan(engine_like, key, build, *more):
+    """``build()``, kept on the engine under ``key`` until a class's form is chosen anew (or
+    ``more`` changes): task segments, profiles and the device are the engine's for good."""
+    stamp = (_lib.lib().gs_class_variant_stamp(), frozenset(SPLIT_OFF), *more)
+    kept = engine_like.__dict__.setdefault("_kept_plans", {})
+    if key not in kept or kept[key][0] != stamp:
+        kept[key] = (stamp, build())
+    return kept[key][1]
+
+
+def launch_list(engine_like, precision, kind, classes=None):
+    """launch_plan as the records of a list call."""
+    key = (precision, kind, None if classes is None else tuple(classes))
+    return kept_plan(engine_like, key, lambda: launch_records(
+        [(cls, first, n, form, 0) for cls, first, n, form, _ in
+         launch_plan(engine_like, precision, kind, classes)]))
+
+
+def mixed_list(engine_like, classes, mixed_cut):
+    """mixed_plan with the tiers as the records of a list call."""
+    key = ("mixed", None if classes is None else tuple(classes))
+
+    def build():
+        banded, tiers = mixed_plan(engine_like, classes, mixed_cut)
+        return banded, launch_records(tiers)
+    return kept_plan(engine_like, key, build, mixed_cut)
+
+
 def mixed_prefix(cls, heavy, mixed_cut):
     """The heavy prefix of a class segment in a mixed-precision build, whose partitioned
     launch (gs_fock_jk_mixed) evaluates every quartet in the class's configured form.
@@ -333,6 +374,11 @@ class HeavyLane:
         ((H2O)24 mixed 16.3 -> 15.0 ms, one batch of 24 molecules 14.6 -> 14.1)."""
         i %= lanes
         return _lib.stream(self.main) if i == lanes - 1 else self.stream(i)
+
+    def streams(self, lanes=SIDE_STREAMS + 1):
+        """(count, handles) of a list call's streams, which forks and joins them itself."""
+        handles = [x.cuda_stream for x in self.sides[:lanes - 1]] + [self.main.cuda_stream]
+        return lanes, (ctypes.c_void_p * lanes)(*handles)
 
     def join(self):
         for k in range(SIDE_STREAMS):
@@ -782,15 +828,12 @@ class QuartetBatch:
         if out.numel() < self.total:
             raise ValueError(f"output buffer holds {out.numel()} doubles, the blocks need {self.total}")
         L = _lib.lib()
-        lane = HeavyLane(self.ds.device, stream)
-        base = self.tasks.data_ptr()
-        prims = self.pairs.prims(precision)
-        for i, (cls, first, n, form, _) in enumerate(launch_plan(self, precision, "write", classes)):
-            rc = L.gs_eri_blocks(*cls, precision | (form << 8), _lib.ptr(self.pairs.rec),
-                                 _lib.ptr(prims), _lib.ptr(self.ds.comp_scale), n,
-                                 base + first * WRITE_TASK, _lib.ptr(out), lane.lane(i))
-            _lib.check(rc, f"gs_eri_blocks{cls}")
-        lane.join()
+        plan = launch_list(self, precision, "write", classes)
+        rc = L.gs_eri_blocks_list(len(plan), plan.ctypes.data, precision, _lib.ptr(self.pairs.rec),
+                                  _lib.ptr(self.pairs.prims(precision)),
+                                  _lib.ptr(self.ds.comp_scale), self.tasks.data_ptr(),
+                                  _lib.ptr(out), *HeavyLane(self.ds.device, stream).streams())
+        _lib.check(rc, "gs_eri_blocks_list")
         return out
 
 
@@ -901,7 +944,7 @@ class MixedWorkspace:
     (one launch's lists at a time)."""
 
     def mixed_workspace(self, dev, tiers):
-        need = _lib.lib().gs_fock_jk_mixed_workspace(max((x[2] for x in tiers), default=0))
+        need = _lib.lib().gs_fock_jk_mixed_workspace(int(tiers["count"].max(initial=0)))
         need = -(-int(need) // 256) * 256
         if getattr(self, "_ws", None) is None or self._ws.numel() < MIXED_LANES * need:
             self._ws = torch.empty(MIXED_LANES * need, dtype=torch.uint8, device=dev)
@@ -1063,7 +1106,7 @@ class JKEngine(MixedWorkspace):
         lane = HeavyLane(dev, stream)
         base = self.tasks.data_ptr()
         if mixed_cut is not None:
-            banded, tiers = mixed_plan(self, classes, mixed_cut)
+            banded, tiers = mixed_list(self, classes, mixed_cut)
             ws, each = self.mixed_workspace(dev, tiers)
             for i, (cls, first, prec, form, count, lo, hi) in enumerate(banded):
                 rc = L.gs_fock_jk(*cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
@@ -1073,26 +1116,23 @@ class JKEngine(MixedWorkspace):
                                   _lib.ptr(pk_c), _lib.ptr(kbuf), _lib.ptr(dmax), thr, lo, hi,
                                   lane.lane(i + 1))
                 _lib.check(rc, f"gs_fock_jk{cls}")
-            for i, (cls, first, count, f64, f32) in enumerate(tiers):
-                rc = L.gs_fock_jk_mixed_forms(
-                    *cls, f64, f32, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
-                    _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale),
-                    _lib.ptr(self.ds.func_off), self.sb.nshell, n, count, base + first * 8,
-                    _lib.ptr(pj_c), _lib.ptr(jbuf), nk, _lib.ptr(pk_c), _lib.ptr(kbuf),
-                    _lib.ptr(dmax), thr, mixed_cut, ws + (i % MIXED_LANES) * each, each,
-                    lane.lane(i, MIXED_LANES))
-                _lib.check(rc, f"gs_fock_jk_mixed_forms{cls}")
+            rc = L.gs_fock_jk_mixed_list(
+                len(tiers), tiers.ctypes.data, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
+                _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale), _lib.ptr(self.ds.func_off),
+                self.sb.nshell, n, base, _lib.ptr(pj_c), _lib.ptr(jbuf), nk, _lib.ptr(pk_c),
+                _lib.ptr(kbuf), _lib.ptr(dmax), thr, mixed_cut, ws, each,
+                *lane.streams(MIXED_LANES))
+            _lib.check(rc, "gs_fock_jk_mixed_list")
             runs = []
         for prec, lo, hi in runs:
-            prims = self.pairs.prims(prec)
-            for i, (cls, first, m, form, _) in enumerate(launch_plan(self, prec, "jk", classes)):
-                rc = L.gs_fock_jk(*cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
-                                  _lib.ptr(prims), _lib.ptr(self.ds.comp_scale),
-                                  _lib.ptr(self.ds.func_off), self.sb.nshell, n, m,
-                                  base + first * 8, _lib.ptr(pj_c), _lib.ptr(jbuf), nk,
-                                  _lib.ptr(pk_c), _lib.ptr(kbuf), _lib.ptr(dmax), thr, lo, hi,
-                                  lane.lane(i))
-                _lib.check(rc, f"gs_fock_jk{cls}")
+            plan = launch_list(self, prec, "jk", classes)
+            rc = L.gs_fock_jk_list(
+                len(plan), plan.ctypes.data, prec, _lib.ptr(self.pairs.rec),
+                _lib.ptr(self.pairs.prims(prec)), _lib.ptr(self.ds.comp_scale),
+                _lib.ptr(self.ds.func_off), self.sb.nshell, n, base, _lib.ptr(pj_c),
+                _lib.ptr(jbuf), nk, _lib.ptr(pk_c), _lib.ptr(kbuf), _lib.ptr(dmax), thr, lo, hi,
+                *lane.streams())
+            _lib.check(rc, "gs_fock_jk_list")
         lane.join()
         J = (jbuf + jbuf.T) if jbuf is not None else None
         K = [kbuf[s] + kbuf[s].T for s in range(nk)]

@@ -74,6 +74,10 @@ int gs_set_class_variant(int la, int lb, int lc, int ld, int precision, int vari
  * or precision.  No reference counterpart. */
 int gs_class_variant(int la, int lb, int lc, int ld, int precision);
 
+/* Grows with every form chosen (gs_set_class_variant): launch lists made for one value hold as
+ * long as it stays. */
+long long gs_class_variant_stamp(void);
+
 /* The kernel form (1 thread, 2 warp, 3 grouped warp, 4 split, 6 stacked) a launch of
  * (la lb|lc ld) in that precision uses with no explicit form: the configured variant, or
  * the built-in default of a long Fock list.
@@ -240,6 +244,44 @@ int gs_fock_jk_batched_mixed_forms(int la, int lb, int lc, int ld, int form64, i
                              long long mat_stride, int ntask, const int* tasks, const double* pj,
                              double* j, int nk, const double* pk, double* k, double screen_thr,
                              double mixed_cut, void* workspace, long long ws_bytes, void* stream);
+
+/* One launch of a list call: count tasks of class (la lb|lc ld) from task `first` of the call's
+ * task array on, in the given kernel form (as in the precision argument's bits 8.. and up; form32
+ * is the FP32 launch's of a mixed-precision list, else 0).  */
+typedef struct gs_launch {
+    int la, lb, lc, ld, form, form32, count, pad;
+    long long first;
+} gs_launch;
+
+/* The launches of one build from one call, in order over streams[0 .. nstreams-1] round and
+ * round: the last stream is the caller's, the others fork from it before the first launch and
+ * join it after the last one.  Other arguments as in the call of the same name without _list;
+ * the mixed ones take stream_bytes of workspace a stream (at least
+ * gs_fock_jk_mixed_workspace(largest count)).  A launch's error ends the list and is returned;
+ * what was launched before it is joined. */
+int gs_eri_blocks_list(int nlaunch, const gs_launch* list, int precision, const void* pair_rec,
+                       const void* prim, const double* comp_scale, const void* tasks, double* out,
+                       int nstreams, void* const* streams);
+int gs_fock_jk_list(int nlaunch, const gs_launch* list, int precision, const void* pair_rec,
+                    const void* prim, const double* comp_scale, const int* func_off, int nshell,
+                    int nbf, const int* tasks, const double* pj, double* j, int nk,
+                    const double* pk, double* k, const double* shell_dmax, double screen_thr,
+                    double prec_lo, double prec_hi, int nstreams, void* const* streams);
+int gs_fock_jk_mixed_list(int nlaunch, const gs_launch* list, const void* pair_rec,
+                          const void* prim64, const void* prim32, const double* comp_scale,
+                          const int* func_off, int nshell, int nbf, const int* tasks,
+                          const double* pj, double* j, int nk, const double* pk, double* k,
+                          const double* shell_dmax, double screen_thr, double mixed_cut,
+                          void* workspace, long long stream_bytes, int nstreams,
+                          void* const* streams);
+int gs_fock_jk_batched_mixed_list(
+    int nlaunch, const gs_launch* list, const void* pair_rec, const void* prim64,
+    const void* prim32, const double* comp_scale, const int* func_off, const int* shell_mol,
+    const long long* mol_base, const int* mol_n, const double* mol_dmax, const int* mol_shell0,
+    const int* mol_nshell, const long long* mol_sbase, long long mat_stride, const int* tasks,
+    const double* pj, double* j, int nk, const double* pk, double* k, double screen_thr,
+    double mixed_cut, void* workspace, long long stream_bytes, int nstreams,
+    void* const* streams);
 
 /* K2 Boys function F_0..F_m(t) (m <= 10) of n arguments t[] into F[n*(m+1)], in FP64 or
  * FP32 (results widened to FP64).  Replaces boys_function / boys_function_recursion

@@ -355,3 +355,96 @@ def test_mixed_forms_match(gpu_lib):
                 assert float((x - y).abs().max()) <= 1e-5 * 1e-4 * 1e4 * 1e-2 + \
                     1e-12 * float(y.abs().max()), (cls, f64, f32)
             assert call(8, 0) == 1 and call(0, -1) == 1
+
+
+def test_kept_plans_follow_the_forms(monkeypatch):
+    """A kept plan is built again once a class's form is chosen, a class leaves or joins
+    SPLIT_OFF, or the precision cut changes, and only then; records have the C ABI's layout."""
+    stamp, built = [0], []
+
+    class Stub:
+        def gs_class_variant_stamp(self):
+            return stamp[0]
+
+    class Eng:
+        pass
+
+    monkeypatch.setattr(engine._lib, "lib", lambda: Stub())
+    monkeypatch.setattr(engine, "SPLIT_OFF", set())
+    plan = [((2, 1, 1, 0), 1 << 40, 7, 5 | 3 << 8, 2)]
+    monkeypatch.setattr(engine, "mixed_plan", lambda e, c, cut: (built.append(cut) or [], plan))
+    eng = Eng()
+    get = lambda cut: engine.mixed_list(eng, None, cut)[1]      # noqa: E731
+    r = get(1e-3)
+    assert engine.LAUNCH_DTYPE.itemsize == 40 and r.tobytes() == np.array(
+        [2, 1, 1, 0, 5 | 3 << 8, 2, 7, 0, 0, 1 << 8], dtype="<i4").tobytes()
+    assert get(1e-3) is r and len(built) == 1
+    stamp[0] += 1
+    assert get(1e-3) is not r and len(built) == 2
+    engine.SPLIT_OFF.add(((1, 0, 0, 0), 64))
+    get(1e-3), get(1e-3)
+    assert len(built) == 3
+    get(1e-4), get(1e-4)
+    assert built == [1e-3, 1e-3, 1e-3, 1e-4]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nstreams", [1, 3, 8])
+def test_list_calls_match_single_launches(gpu_lib, nstreams):
+    """A list of launches over several streams gives what the launches one by one give (sums in
+    another order: 1e-13 of the largest element); no launch is an empty list; a class that is not
+    built, a negative form and a missing stream array are refused, and what ran before is joined."""
+    import ctypes
+    from gaussium_gb300 import _lib
+    from gaussium_gb300.workloads import random_shell_quartets
+    sb, _, _ = random_shell_quartets(4, seed=5, box_angstrom=3.0, kmax=4)
+    eng = engine.JKEngine(sb, schwarz_thr=0.0)
+    n = sb.nbf
+    p = np.random.default_rng(9).standard_normal((n, n))
+    pt = torch.as_tensor(p + p.T).cuda()
+    dmax = eng.shell_dmax([pt])
+    plan = engine.launch_list(eng, 64, "jk")
+    sides = [torch.cuda.Stream() for _ in range(nstreams - 1)]
+    handles = (ctypes.c_void_p * nstreams)(*[x.cuda_stream for x in sides],
+                                           torch.cuda.current_stream().cuda_stream)
+
+    def fock(records, streams=handles, count=nstreams):
+        j = torch.zeros((n, n), dtype=torch.float64, device="cuda")
+        k = torch.zeros_like(j)
+        rc = gpu_lib.gs_fock_jk_list(
+            len(records), records.ctypes.data, 64, _lib.ptr(eng.pairs.rec), _lib.ptr(eng.pairs.p64),
+            _lib.ptr(eng.ds.comp_scale), _lib.ptr(eng.ds.func_off), sb.nshell, n,
+            eng.tasks.data_ptr(), _lib.ptr(pt), _lib.ptr(j), 1, _lib.ptr(pt), _lib.ptr(k),
+            _lib.ptr(dmax), 1e-12, 0.0, float("inf"), count, streams)
+        return rc, j, k
+
+    parts = [fock(plan[i:i + 1]) for i in range(len(plan))]
+    assert len(plan) > 8 and all(rc == 0 for rc, _, _ in parts)
+    rc, j, k = fock(plan)
+    assert rc == 0
+    for i, x in ((1, j), (2, k)):
+        ref = sum(part[i] for part in parts)
+        assert float((x - ref).abs().max()) <= 1e-13 * float(ref.abs().max())
+    rc, j, k = fock(plan[:0])
+    assert rc == 0 and not j.any() and not k.any()
+    bad = plan[:3].copy()
+    bad["form"][2] = -1
+    rc, j, _ = fock(bad)
+    assert rc == 1 and not j.any()
+    assert fock(plan, None)[0] == 1 and fock(plan, handles, 0)[0] == 1
+    bad = plan[:3].copy()
+    bad["cls"][2] = (3, 3, 3, 3)
+    rc, j, _ = fock(bad)
+    ref = parts[0][1] + parts[1][1]
+    assert rc == 3 and float((j - ref).abs().max()) <= 1e-13 * float(ref.abs().max())
+    # blocks: each has one writer, so the values are the same bit for bit
+    sb, quartets, _ = random_shell_quartets(300, seed=8, box_angstrom=3.0, kmax=3)
+    b = engine.QuartetBatch(engine.DeviceShells(sb, "cuda"), quartets)
+    recs = engine.launch_list(b, 64, "write")
+    outs = [torch.zeros(b.total, dtype=torch.float64, device="cuda") for _ in range(2)]
+    for r, out in ([(recs, outs[0])] + [(recs[i:i + 1], outs[1]) for i in range(len(recs))]):
+        _lib.check(gpu_lib.gs_eri_blocks_list(
+            len(r), r.ctypes.data, 64, _lib.ptr(b.pairs.rec), _lib.ptr(b.pairs.p64),
+            _lib.ptr(b.ds.comp_scale), b.tasks.data_ptr(), _lib.ptr(out), nstreams, handles),
+            "gs_eri_blocks_list")
+    assert torch.equal(*outs)
