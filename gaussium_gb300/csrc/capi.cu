@@ -77,8 +77,8 @@ __device__ __forceinline__ void build_pair(const gs::ShellView& sv, long long pi
     const int sa = pair_shells[2 * pi], sb = pair_shells[2 * pi + 1];
     const double* A = sv.centre + 3 * sa;
     const double* B = sv.centre + 3 * sb;
-    const double ABx = A[0] - B[0], ABy = A[1] - B[1], ABz = A[2] - B[2];
-    const double ab2 = ABx * ABx + ABy * ABy + ABz * ABz;
+    const double ABx = gs::gs_sub(A[0], B[0]), ABy = gs::gs_sub(A[1], B[1]),
+                 ABz = gs::gs_sub(A[2], B[2]);
     const int a0 = sv.prim_off[sa], b0 = sv.prim_off[sb];
     const int nb = sv.prim_off[sb + 1] - b0;
     const int ntot = (sv.prim_off[sa + 1] - a0) * nb;
@@ -94,12 +94,13 @@ __device__ __forceinline__ void build_pair(const gs::ShellView& sv, long long pi
             j = b0 + k % nb;
             a = sv.expo[i];
             b = sv.expo[j];
-            keep = gs::prim_pair_kept(a, b, ab2, max_exp);
+            keep = gs::prim_pair_kept(a, b, ABx, ABy, ABz, max_exp);
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         if (keep) {
             const int r = base + n + __popc(m & ((1u << lane) - 1u));
-            const gs::PrimRec<double> rec = gs::prim_pair(A, B, a, b, ab2, sv.coef[i], sv.coef[j]);
+            const gs::PrimRec<double> rec =
+                gs::prim_pair(A, B, ABx, ABy, ABz, a, b, sv.coef[i], sv.coef[j]);
             p64[r] = rec;
             if (p32) p32[r] = gs::prim_pair32(rec);
         }
@@ -135,11 +136,14 @@ __global__ void __launch_bounds__(256) k_pairs_build(gs::ShellView sv, int npair
 // groups but only tests the primitive-pair screen per lane there; the kept primitive
 // pairs (about a third on a K = 1-6 basis with exponents over five decades) go to a
 // per-warp queue in shared memory with their record positions, and are evaluated 32 at a
-// time, so the FP64 division and exponential of prim_pair run on full warps.  Records
+// time, so the reciprocal and the exponential of prim_pair run on full warps.  The FP64 pipe bounds
+// it (84 % busy): 36 FP64 instructions a primitive pair, where the screen in FP64, the library's
+// division, exponential and conversions came to some 60; 4.2 M primitive pairs of 800,000 pairs
+// 451 -> 299 us.  Records
 // and counts are those of k_pairs_build (each record goes to the position its ballot
 // rank fixed).
 struct PairCand {
-    double ab2;
+    double ABx, ABy, ABz;
     int pi, i, j, r;
 };
 constexpr int kPairGroupsPerWarp = 8;
@@ -153,7 +157,8 @@ __device__ __forceinline__ void pair_eval(const gs::ShellView& sv,
     const double* A = sv.centre + 3 * pair_shells[2 * c.pi];
     const double* B = sv.centre + 3 * pair_shells[2 * c.pi + 1];
     const gs::PrimRec<double> rec =
-        gs::prim_pair(A, B, sv.expo[c.i], sv.expo[c.j], c.ab2, sv.coef[c.i], sv.coef[c.j]);
+        gs::prim_pair(A, B, c.ABx, c.ABy, c.ABz, sv.expo[c.i], sv.expo[c.j], sv.coef[c.i],
+                      sv.coef[c.j]);
     p64[c.r] = rec;
     if (p32) p32[c.r] = gs::prim_pair32(rec);
 }
@@ -194,8 +199,8 @@ __global__ void __launch_bounds__(32 * kPairWarps) k_pairs_build_compact(
             const int sa = pair_shells[2 * pi], sb = pair_shells[2 * pi + 1];
             const double* A = sv.centre + 3 * sa;
             const double* B = sv.centre + 3 * sb;
-            const double ABx = A[0] - B[0], ABy = A[1] - B[1], ABz = A[2] - B[2];
-            const double ab2 = ABx * ABx + ABy * ABy + ABz * ABz;
+            const double ABx = gs::gs_sub(A[0], B[0]), ABy = gs::gs_sub(A[1], B[1]),
+                         ABz = gs::gs_sub(A[2], B[2]);
             const int a0 = sv.prim_off[sa], b0 = sv.prim_off[sb];
             const int nb = sv.prim_off[sb + 1] - b0;
             const int ntot = (sv.prim_off[sa + 1] - a0) * nb;
@@ -208,10 +213,10 @@ __global__ void __launch_bounds__(32 * kPairWarps) k_pairs_build_compact(
                 if (k < ntot) {
                     i = a0 + k / nb;
                     j = b0 + k % nb;
-                    keep = gs::prim_pair_kept(sv.expo[i], sv.expo[j], ab2, max_exp);
+                    keep = gs::prim_pair_kept(sv.expo[i], sv.expo[j], ABx, ABy, ABz, max_exp);
                 }
                 const unsigned m = __ballot_sync(0xffffffffu, keep);
-                const PairCand c{ab2, pi, i, j, base + n + __popc(m & ((1u << lane) - 1u))};
+                const PairCand c{ABx, ABy, ABz, pi, i, j, base + n + __popc(m & ((1u << lane) - 1u))};
                 pair_push(q, len, keep, c, m, lane, sv, pair_shells, p64, p32);
                 n += __popc(m);
             }
@@ -250,8 +255,8 @@ __global__ void __launch_bounds__(32 * kPairWarps) k_pairs_build_compact(
         const int sa = pair_shells[2 * pi], sb = pair_shells[2 * pi + 1];
         const double* A = sv.centre + 3 * sa;
         const double* B = sv.centre + 3 * sb;
-        const double ABx = A[0] - B[0], ABy = A[1] - B[1], ABz = A[2] - B[2];
-        const double ab2 = ABx * ABx + ABy * ABy + ABz * ABz;
+        const double ABx = gs::gs_sub(A[0], B[0]), ABy = gs::gs_sub(A[1], B[1]),
+                     ABz = gs::gs_sub(A[2], B[2]);
         const int a0 = sv.prim_off[sa], b0 = sv.prim_off[sb];
         const int nb = sv.prim_off[sb + 1] - b0;
         const int k = lane - my_off;
@@ -260,13 +265,13 @@ __global__ void __launch_bounds__(32 * kPairWarps) k_pairs_build_compact(
         if (in) {
             i = a0 + k / nb;
             jj = b0 + k % nb;
-            keep = gs::prim_pair_kept(sv.expo[i], sv.expo[jj], ab2, max_exp);
+            keep = gs::prim_pair_kept(sv.expo[i], sv.expo[jj], ABx, ABy, ABz, max_exp);
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         const unsigned pair_mask = (my_size >= 32 ? 0xffffffffu : ((1u << my_size) - 1u)) << my_off;
         const unsigned mine = m & pair_mask;
         const int base = pair_prim_off[pi];
-        const PairCand c{ab2, pi, i, jj, base + __popc(mine & ((1u << lane) - 1u))};
+        const PairCand c{ABx, ABy, ABz, pi, i, jj, base + __popc(mine & ((1u << lane) - 1u))};
         pair_push(q, len, keep, c, m, lane, sv, pair_shells, p64, p32);
         if (in && lane == my_off) {
             gs::PairRec pr;

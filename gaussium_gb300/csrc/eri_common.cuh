@@ -134,13 +134,20 @@ GS_HD GS_INLINE float gs_rsqrt(float x) {
     return 1.0f / std::sqrt(x);
 #endif
 }
-GS_HD GS_INLINE double gs_exp(double x) { return exp(x); }
-GS_HD GS_INLINE float gs_exp(float x) {
+
+// 1 / x: the hardware's approximation y and y (1 + e + e^2) with e = 1 - x y, whose error is
+// e^3 < 2^-57 before rounding; three FP64 instructions.  Zero, subnormal, non-finite and
+// negative x, and those whose reciprocal is subnormal, go to the division.
+GS_HD GS_INLINE double gs_rcp(double x) {
 #if defined(__CUDA_ARCH__)
-    return expf(x);
-#else
-    return std::exp(x);
+    if ((unsigned)__double2hiint(x) - 0x00100000u < 0x7fc00000u) {
+        double y;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+        const double e = fma(-x, y, 1.0);
+        return fma(y, fma(e, e, e), y);
+    }
 #endif
+    return 1.0 / x;
 }
 
 // ------------------------------------------------------------------ Boys function
@@ -213,6 +220,7 @@ GS_HD GS_INLINE float narrow(double x) {
         const unsigned up = rest > 0x10000000u - (f & 1u) ? 1u : 0u;
         return __uint_as_float((hi & 0x80000000u) | (f + up));
     }
+    if (((hi << 1) | lo) == 0) return __uint_as_float(hi);
 #endif
     return (float)x;
 }
@@ -251,6 +259,15 @@ GS_HD GS_INLINE double max_nonneg(double a, double b) {
 #endif
 }
 
+// a >= b for values that are not negative.
+GS_HD GS_INLINE bool not_less(double a, double b) {
+#if defined(__CUDA_ARCH__)
+    return __double_as_longlong(a) >= __double_as_longlong(b);
+#else
+    return a >= b;
+#endif
+}
+
 // High word of a whole number n, 1 <= n < 2^20, as a double.
 GS_HD constexpr unsigned whole_hiword(unsigned n) {
     unsigned e = 0;
@@ -267,6 +284,49 @@ template <unsigned N> GS_HD GS_INLINE bool below(double t) {
 #endif
 }
 template <unsigned N> GS_HD GS_INLINE bool below(float t) { return t < (float)N; }
+
+// x / 2 for normal x with a normal half.
+GS_HD GS_INLINE double halve(double x) {
+#if defined(__CUDA_ARCH__)
+    const int hi = __double2hiint(x);
+    if ((((unsigned)hi >> 20) & 0x7ffu) - 2u < 0x7fdu)
+        return __hiloint2double(hi - 0x00100000, __double2loint(x));
+#endif
+    return 0.5 * x;
+}
+
+// exp(x): x = k ln 2 + r by Cody and Waite's two-part ln 2, the Taylor sum of exp(r) to r^13
+// (|r| <= ln 2 / 2: the rest is below 2^-57) with its terms from r^9 on, under 2^-32 of the sum,
+// in float, and k added to the exponent; twelve FP64 instructions where the library's function
+// takes the time of 19.  |x| >= 700 and NaN go to the library's.
+GS_HD GS_INLINE double gs_exp(double x) {
+#if defined(__CUDA_ARCH__)
+    if (((unsigned)__double2hiint(x) & 0x7fffffffu) < 0x4085e000u) {
+        const double magic = 6755399441055744.0;
+        const double kf = gs_fma(x, 1.4426950408889634074, magic);
+        const double kd = gs_sub(kf, magic);
+        const double r = gs_fma(kd, -2.3190468138462996e-17, gs_fma(kd, -0.69314718055994530942, x));
+        const float f = narrow(r);
+        float t = fmaf(f, 1.0f / 6227020800.0f, 1.0f / 479001600.0f);
+        t = fmaf(f, t, 1.0f / 39916800.0f);
+        t = fmaf(f, t, 1.0f / 3628800.0f);
+        t = fmaf(f, t, 1.0f / 362880.0f);
+        double y = gs_fma(widen(t), r, 1.0 / 40320.0);
+        y = gs_fma(y, r, 1.0 / 5040.0);
+        y = gs_fma(y, r, 1.0 / 720.0);
+        y = gs_fma(y, r, 1.0 / 120.0);
+        y = gs_fma(y, r, 1.0 / 24.0);
+        y = gs_fma(y, r, 1.0 / 6.0);
+        y = gs_fma(y, r, 0.5);
+        y = gs_fma(y, r, 1.0);
+        y = gs_fma(y, r, 1.0);
+        return __hiloint2double(__double2hiint(y) + (__double2loint(kf) << 20), __double2loint(y));
+    }
+    return exp(x);
+#else
+    return std::exp(x);
+#endif
+}
 
 // Nearest row k of the half-step grid of t >= 0 and T_k - t (exact), the rounding by the sum
 // with 1.5 2^52, whose last bit is worth one.  k is held to the table whatever t is.
@@ -552,29 +612,39 @@ struct ShellView {
 
 constexpr double kSqrt2Pi52 = 5.914967172795613;  // sqrt(2 pi^(5/2))
 
-// Record of the primitive pair (a at A, b at B) with contraction coefficients ca, cb.
-GS_HD GS_INLINE PrimRec<double> prim_pair(const double* A, const double* B, double a, double b,
-                                          double ab2, double ca, double cb) {
-    const double p = a + b, ip = 1.0 / p;
+// Record of the primitive pair (a at A, b at B, AB = A - B) with contraction coefficients ca, cb.
+// P - A = -b/p AB is formed as such, not as a difference of centres (no cancellation), and P from
+// the centre of the larger exponent, its nearer one: seven FP64 instructions for the six where
+// (aA + bB)/p and P - A took twelve.  Over random shells (rms, units of 2^-53) P is off by 0.44,
+// P - A by 0.88 and Kp by 31.3, most of it its exponent's rounding; the other way it was 0.90,
+// 10^6 (from pairs of centres close to each other or of very different exponents) and 31.5.
+GS_HD GS_INLINE PrimRec<double> prim_pair(const double* A, const double* B, double ABx, double ABy,
+                                          double ABz, double a, double b, double ca, double cb) {
     PrimRec<double> r;
+    const double p = gs_add(a, b);
+    const double ip = gs_rcp(p);
+    const double bp = gs_mul(b, ip);
     r.p = p;
-    r.i2p = 0.5 * ip;
-    r.Px = (a * A[0] + b * B[0]) * ip;
-    r.Py = (a * A[1] + b * B[1]) * ip;
-    r.Pz = (a * A[2] + b * B[2]) * ip;
-    r.PAx = r.Px - A[0]; r.PAy = r.Py - A[1]; r.PAz = r.Pz - A[2];
-    r.Kp = kSqrt2Pi52 * ca * cb * exp(-a * b * ip * ab2) * ip;
+    r.i2p = halve(ip);
+    r.PAx = gs_mul(-bp, ABx); r.PAy = gs_mul(-bp, ABy); r.PAz = gs_mul(-bp, ABz);
+    const double ap = gs_mul(a, ip);
+    const bool near = not_less(a, b);
+    const double w = near ? -bp : ap;
+    const double* C = near ? A : B;
+    r.Px = gs_fma(w, ABx, C[0]); r.Py = gs_fma(w, ABy, C[1]); r.Pz = gs_fma(w, ABz, C[2]);
+    const double x = gs_mul(gs_mul(-a, bp), norm2(ABx, ABy, ABz));
+    r.Kp = gs_mul(gs_mul(gs_mul(kSqrt2Pi52, ca), gs_mul(cb, ip)), gs_exp(x));
     r.pad = a;          // exponent of the first shell (derivative weights)
     return r;
 }
 
 GS_HD GS_INLINE PrimRec<float> prim_pair32(const PrimRec<double>& r) {
     PrimRec<float> f;
-    f.p = (float)r.p; f.i2p = (float)r.i2p;
-    f.Px = (float)r.Px; f.Py = (float)r.Py; f.Pz = (float)r.Pz;
-    f.PAx = (float)r.PAx; f.PAy = (float)r.PAy; f.PAz = (float)r.PAz;
-    f.Kp = (float)r.Kp;
-    f.pad0 = (float)r.pad;      // exponent of the first shell (FP32 derivative weights)
+    f.p = narrow(r.p); f.i2p = narrow(r.i2p);
+    f.Px = narrow(r.Px); f.Py = narrow(r.Py); f.Pz = narrow(r.Pz);
+    f.PAx = narrow(r.PAx); f.PAy = narrow(r.PAy); f.PAz = narrow(r.PAz);
+    f.Kp = narrow(r.Kp);
+    f.pad0 = narrow(r.pad);      // exponent of the first shell (FP32 derivative weights)
     f.pad1 = f.pad2 = 0.0f;
     return f;
 }
@@ -584,6 +654,22 @@ GS_HD GS_INLINE PrimRec<float> prim_pair32(const PrimRec<double>& r) {
 // max_exp p), which on this part costs more FP64 issue slots than the rest of the test.
 GS_HD GS_INLINE bool prim_pair_kept(double a, double b, double ab2, double max_exp) {
     return !(max_exp > 0.0 && a * b * ab2 > max_exp * (a + b));
+}
+
+// The same decision from the centres' difference, in float where float's rounding (under 2e-6 of
+// either side together) cannot change it, so that the test stays off the FP64 pipe.
+GS_HD GS_INLINE bool prim_pair_kept(double a, double b, double ABx, double ABy, double ABz,
+                                    double max_exp) {
+#if defined(__CUDA_ARCH__)
+    if (!(max_exp > 0.0)) return true;
+    const float x = narrow(ABx), y = narrow(ABy), z = narrow(ABz), af = narrow(a), bf = narrow(b);
+    const float t = af * bf * (x * x + y * y + z * z), lim = narrow(max_exp) * (af + bf);
+    if (lim > 1e-30f) {
+        if (t < lim * 0.99999f) return true;
+        if (t > lim * 1.00001f) return false;
+    }
+#endif
+    return prim_pair_kept(a, b, ABx * ABx + ABy * ABy + ABz * ABz, max_exp);
 }
 
 // Fill the PairRec and the primitive-pair records of shell pair (sa, sb); la >= lb.
@@ -608,7 +694,7 @@ GS_HD GS_INLINE void make_pair(const ShellView& S, int sa, int sb, int prim_off,
         for (int j = b0; j < b1; ++j) {
             const double a = S.expo[i], b = S.expo[j];
             if (!prim_pair_kept(a, b, ab2, max_exp)) continue;
-            const PrimRec<double> r = prim_pair(A, B, a, b, ab2, S.coef[i], S.coef[j]);
+            const PrimRec<double> r = prim_pair(A, B, ABx, ABy, ABz, a, b, S.coef[i], S.coef[j]);
             pd[n] = r;
             if (pf) pf[n] = prim_pair32(r);
             ++n;

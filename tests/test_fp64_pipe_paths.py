@@ -121,3 +121,63 @@ def test_rsqrt(gpu_lib):
     got = torch.empty_like(odd)
     _lib.check(gpu_lib.gs_rsqrt_eval(7, _lib.ptr(odd), _lib.ptr(got), _lib.stream()), "rsqrt")
     assert torch.allclose(got, torch.rsqrt(odd), rtol=1e-15, equal_nan=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("max_exp", [0.0, 55.0, 3.0])
+@pytest.mark.parametrize("count", [False, True])
+def test_pair_records_against_extended_precision(gpu_lib, max_exp, count):
+    """Primitive-pair records of exponents over 17 decades and centres on, near and far from each
+    other: p exact, 1/2p to 1 ulp, P - A = -b/p AB to five roundings, P to one more, the Gaussian
+    product prefactor to ten roundings and ten of its exponent; the kept
+    pairs are those of the screen's double-precision test, in both kernels."""
+    from gaussium_gb300 import _lib
+    rng = np.random.default_rng(3)
+    shells = []
+    for i in range(24):
+        c = rng.standard_normal(3) * (0.0, 1e-9, 0.3, 2.0, 40.0)[i % 5]
+        k = (1, 3, 6)[i % 3]
+        expo = 10.0 ** (rng.uniform(-8, 9, k) if i % 2 else rng.uniform(-1, 2, k))
+        shells.append(dict(l=0, centre=c, expo=expo, coef=rng.uniform(0.1, 1.0, k)))
+    sb = ShellBasis.from_shell_dicts(shells)
+    ds = engine.DeviceShells(sb, "cuda")
+    pairs = np.stack(np.tril_indices(sb.nshell), 1)
+    ps = engine.PairSet(ds, pairs, max_exp=max_exp)
+    if count:        # one warp a pair instead of several
+        ps.ngroups = 0
+        ps.build()
+    rec = np.frombuffer(ps.p64.cpu().numpy().tobytes(), dtype="<f8").reshape(-1, 10)
+    rec32 = np.frombuffer(ps.p32.cpu().numpy().tobytes(), dtype="<f4").reshape(-1, 12)
+    kept = ps.kept.cpu().numpy()
+    start = ps.prim_start.cpu().numpy()
+    expo, coef, off = (x.cpu().numpy() for x in (ds.expo, ds.coef, ds.prim_off))
+    q, eps = np.longdouble, 2.0 ** -53
+    for n, (sa, s_b) in enumerate(pairs):
+        AB = sb.centre[sa] - sb.centre[s_b]
+        a, b = (x.ravel() for x in np.meshgrid(expo[off[sa]:off[sa + 1]], expo[off[s_b]:off[s_b + 1]],
+                                               indexing="ij"))
+        ca, cb = (x.ravel() for x in np.meshgrid(coef[off[sa]:off[sa + 1]],
+                                                 coef[off[s_b]:off[s_b + 1]], indexing="ij"))
+        ratio = a * b * float(AB @ AB) / (a + b)
+        keep = ratio <= max_exp if max_exp > 0 else np.ones(len(a), bool)
+        assert not np.any((np.abs(ratio - max_exp) < 1e-9 * max_exp) & (max_exp > 0))
+        assert kept[n] == keep.sum()
+        r = rec[start[n]:start[n] + kept[n]]
+        a, b, ca, cb = (x[keep] for x in (a, b, ca, cb))
+        assert np.array_equal(r[:, 0], a + b)
+        ip = 1 / (q(1) * a + b)
+        assert np.all(np.abs(r[:, 1] - ip / 2) <= 2 * eps * ip / 2 + eps * ip / 2)
+        PA = -(b * ip)[:, None] * AB[None].astype(q)
+        exact = sb.centre[sa].astype(q) - sb.centre[s_b].astype(q)     # AB before its rounding
+        P = sb.centre[sa].astype(q)[None] - (b * ip)[:, None] * exact[None]
+        # from the nearer centre: its step is at most half of AB
+        step = np.minimum(a, b)[:, None] * ip[:, None] * np.abs(AB)[None]
+        assert np.all(np.abs(r[:, 5:8] - PA) <= 5 * eps * np.abs(PA))
+        assert np.all(np.abs(r[:, 2:5] - P) <= 5 * eps * step + eps * np.abs(P))
+        x = a * (b * ip) * (AB.astype(q) @ AB.astype(q))
+        K = q("5.914967172795612987") * ca * cb * ip * np.exp(-x)
+        tiny = np.finfo(float).tiny
+        assert np.all(np.abs(r[:, 8] - K) <= (10 + 10 * x) * eps * K + tiny)
+        with np.errstate(under="ignore", over="ignore"):
+            f = rec32[start[n]:start[n] + kept[n]]
+            assert np.array_equal(f[:, :9], r[:, :9].astype(np.float32))
