@@ -3,6 +3,7 @@
 // void*, and returns a status code (0 = success); nothing here allocates device memory.
 #include <cuda_runtime.h>
 #include <atomic>
+#include <cstddef>
 #include <cstdint>
 #include "eri_common.cuh"
 #include "gs_args.h"
@@ -323,6 +324,45 @@ __device__ __forceinline__ double block_dmax(const double* __restrict__ d, int n
     return dm;
 }
 
+// The partition's limits with their float brackets: outside [lo, hi] a bound formed in float
+// (three roundings, under 2e-7 of it) decides as the one in double does.
+struct Limits {
+    double thr, cut;
+    float thr_lo, thr_hi, cut_lo, cut_hi;
+};
+Limits limits(double thr, double cut) {
+    const float t = (float)thr, c = (float)cut;
+    return {thr, cut, t * 0.999999f, t * 1.000001f, c * 0.999999f, c * 1.000001f};
+}
+
+// 0 dropped, 1 FP64, 2 FP32.  Bounds near a limit or out of float's range are formed in double,
+// which for all of them held the FP64 pipe 46 % of the kernel's time, beside the class kernels
+// that need it (24 molecules in one batch 13.67 -> 13.47 ms).
+__device__ __forceinline__ int partition_kind(float qb, float qk, double dm, const Limits& l) {
+    const float est = qb * qk * gs::narrow(dm);
+    if (est > 1e-30f && est < 1e30f) {
+        if (est < l.thr_lo) return 0;
+        if (est > l.thr_hi) {
+            if (est > l.cut_hi) return 1;
+            if (est < l.cut_lo) return 2;
+        }
+    }
+    const double exact = gs::widen(qb) * gs::widen(qk) * dm;
+    return exact < l.thr ? 0 : (exact >= l.cut ? 1 : 2);
+}
+
+// The last 16 bytes of a pair record, in one load.
+struct PairTail {
+    int sa, sb;
+    float qmax;
+};
+__device__ __forceinline__ PairTail pair_tail(const gs::PairRec* __restrict__ pairs, int i) {
+    static_assert(sizeof(gs::PairRec) == 48 && offsetof(gs::PairRec, sa) == 32 &&
+                      offsetof(gs::PairRec, qmax) == 40, "pair record layout");
+    const int4 v = reinterpret_cast<const int4*>(pairs + i)[2];
+    return {v.x, v.y, __int_as_float(v.z)};
+}
+
 // dmax: per (shell, shell) block of one molecule (nshell x nshell); with shell_mol, per
 // molecule: either one value per molecule (mol_sbase null) or molecule m's own block table
 // at dmax + mol_sbase[m] over its mol_nshell[m] shells, numbered from mol_shell0[m].
@@ -331,7 +371,7 @@ __global__ void k_partition(int ntask, const int2* __restrict__ tasks,
                             const double* __restrict__ dmax, int nshell,
                             const int* __restrict__ shell_mol,
                             const int* __restrict__ mol_shell0, const int* __restrict__ mol_nshell,
-                            const long long* __restrict__ mol_sbase, double thr, double cut,
+                            const long long* __restrict__ mol_sbase, Limits lim,
                             int2* __restrict__ out64, int2* __restrict__ out32,
                             int* __restrict__ counts) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -339,8 +379,7 @@ __global__ void k_partition(int ntask, const int2* __restrict__ tasks,
     int2 task = make_int2(0, 0);
     if (t < ntask) {
         task = tasks[t];
-        const gs::PairRec B = pairs[task.x];
-        const gs::PairRec K = pairs[task.y];
+        const PairTail B = pair_tail(pairs, task.x), K = pair_tail(pairs, task.y);
         double dm;
         if (shell_mol && mol_sbase) {
             const int m = shell_mol[B.sa], s0 = mol_shell0[m];
@@ -351,8 +390,7 @@ __global__ void k_partition(int ntask, const int2* __restrict__ tasks,
         } else {
             dm = block_dmax(dmax, nshell, B.sa, B.sb, K.sa, K.sb);
         }
-        const double est = gs::widen(B.qmax) * gs::widen(K.qmax) * dm;
-        kind = est < thr ? 0 : (est >= cut ? 1 : 2);
+        kind = partition_kind(B.qmax, K.qmax, dm, lim);
     }
     const unsigned lane = threadIdx.x & 31;
     for (int which = 1; which <= 2; ++which) {
@@ -422,8 +460,8 @@ int gs::partition_tasks(int ntask, const int2* tasks, const PairRec* pairs,
                         int2* l32, int* counts, cudaStream_t st) {
     if (cudaMemsetAsync(counts, 0, 2 * sizeof(int), st) != cudaSuccess) return GS_ERR_CUDA;
     k_partition<<<(ntask + 255) / 256, 256, 0, st>>>(ntask, tasks, pairs, shell_dmax, nshell, nullptr,
-                                                     nullptr, nullptr, nullptr, thr, cut, l64, l32,
-                                                     counts);
+                                                     nullptr, nullptr, nullptr, limits(thr, cut), l64,
+                                                     l32, counts);
     return check_launch();
 }
 
@@ -815,7 +853,7 @@ int fock_jk_batched_mixed_impl(int la, int lb, int lc, int ld, int form64, int f
     if (cudaMemsetAsync(counts, 0, 2 * sizeof(int), S(stream)) != cudaSuccess) return GS_ERR_CUDA;
     k_partition<<<(ntask + 255) / 256, 256, 0, S(stream)>>>(
         ntask, (const int2*)tasks, (const gs::PairRec*)pair_rec, mol_dmax, 0, shell_mol,
-        mol_shell0, mol_nshell, mol_sbase, screen_thr, mixed_cut, l64, l32, counts);
+        mol_shell0, mol_nshell, mol_sbase, limits(screen_thr, mixed_cut), l64, l32, counts);
     if (check_launch()) return GS_ERR_CUDA;
     gs::JKArgs a;
     a.pairs = (const gs::PairRec*)pair_rec;

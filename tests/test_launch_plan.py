@@ -448,3 +448,55 @@ def test_list_calls_match_single_launches(gpu_lib, nstreams):
             _lib.ptr(b.ds.comp_scale), b.tasks.data_ptr(), _lib.ptr(out), nstreams, handles),
             "gs_eri_blocks_list")
     assert torch.equal(*outs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("thr,cut", [(1e-12, 1e-3), (1e-300, 1e-4), (0.25, 0.25), (3e-13, float("inf")),
+                                     (0.0, 0.0)])
+def test_partition_decides_as_the_double_bound(gpu_lib, thr, cut):
+    """The lists of a partition are those of the bound in double, for bounds at, one step beside
+    and far from either limit, and too small or large for float."""
+    from gaussium_gb300 import _lib
+    from gaussium_gb300.workloads import random_shell_quartets
+    sb, _, _ = random_shell_quartets(4, seed=5, box_angstrom=3.0, kmax=2)
+    eng = engine.JKEngine(sb, schwarz_thr=0.0)
+    rng = np.random.default_rng(11)
+    n, ns = sb.nbf, sb.nshell
+    rec = np.frombuffer(eng.pairs.rec.cpu().numpy().tobytes(), dtype=np.dtype(
+        [("ab", "<f8", 3), ("i", "<i4", 4), ("q", "<f4"), ("pad", "<i4")])).copy()
+    rec["q"] = 2.0 ** rng.integers(-3, 3, len(rec))
+    rec["q"][:4] = 0.0, 1e-38, 3e38, 1e-20
+    eng.pairs.rec.copy_(torch.as_tensor(np.frombuffer(rec.tobytes(), dtype=np.uint8).copy()))
+    near = [x for x in (thr, cut) if 0.0 < x < 1e30] or [1.0]
+    near = np.array([f(x * 2.0 ** k) for x in near for k in range(-6, 7) for f in
+                     (lambda y: y, lambda y: np.nextafter(y, 0), lambda y: np.nextafter(y, 9),
+                      lambda y: y * (1 + 1e-7), lambda y: y * (1 - 3e-7))])
+    d = near[rng.integers(0, len(near), (ns, ns))]
+    d[rng.random((ns, ns)) < 0.05] = 0.0
+    d[rng.random((ns, ns)) < 0.5] *= 1e-9            # so that the largest of six varies
+    dmax = torch.as_tensor(np.maximum(d, d.T)).cuda()
+    d = dmax.cpu().numpy()
+    pt = torch.zeros((n, n), dtype=torch.float64, device="cuda")
+    tasks = eng.tasks[:eng.ntasks].cpu().numpy()
+    seen = set()
+    for cls, s, e in eng.segments:
+        j, k = torch.zeros_like(pt), torch.zeros_like(pt)
+        ws = torch.zeros(gpu_lib.gs_fock_jk_mixed_workspace(e - s), dtype=torch.uint8, device="cuda")
+        _lib.check(gpu_lib.gs_fock_jk_mixed(
+            *cls, _lib.ptr(eng.pairs.rec), _lib.ptr(eng.pairs.p64), _lib.ptr(eng.pairs.p32),
+            _lib.ptr(eng.ds.comp_scale), _lib.ptr(eng.ds.func_off), ns, n, e - s,
+            eng.tasks.data_ptr() + 8 * s, _lib.ptr(pt), _lib.ptr(j), 1, _lib.ptr(pt), _lib.ptr(k),
+            _lib.ptr(dmax), thr, cut, _lib.ptr(ws), ws.numel(), _lib.stream()), "gs_fock_jk_mixed")
+        raw = np.frombuffer(ws.cpu().numpy().tobytes(), dtype="<i4")
+        t = tasks[s:e]
+        B, K = rec[t[:, 0]], rec[t[:, 1]]
+        (a, b), (c, f) = B["i"][:, 2:].T, K["i"][:, 2:].T
+        dm = np.max([d[a, b], d[c, f], d[a, c], d[a, f], d[b, c], d[b, f]], axis=0)
+        est = B["q"].astype(float) * K["q"].astype(float) * dm
+        kind = np.where(est < thr, 0, np.where(est >= cut, 1, 2))
+        lists = raw[64:64 + 2 * (e - s)], raw[64 + 2 * (e - s):64 + 4 * (e - s)]
+        for which in (1, 2):
+            got = lists[which - 1].reshape(-1, 2)[:raw[which - 1]]
+            assert sorted(map(tuple, got.tolist())) == sorted(map(tuple, t[kind == which].tolist()))
+        seen |= set(kind.tolist())
+    assert len(seen) >= (1 if thr == cut == 0.0 else 2)
