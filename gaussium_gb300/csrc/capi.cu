@@ -366,7 +366,8 @@ __device__ __forceinline__ PairTail pair_tail(const gs::PairRec* __restrict__ pa
 // dmax: per (shell, shell) block of one molecule (nshell x nshell); with shell_mol, per
 // molecule: either one value per molecule (mol_sbase null) or molecule m's own block table
 // at dmax + mol_sbase[m] over its mol_nshell[m] shells, numbered from mol_shell0[m].
-constexpr int kPartitionThreads = 256;
+// 1,024: the longest runs in order (24 molecules in one batch 11.4 ms, with 256 11.7 ms)
+constexpr int kPartitionThreads = 1024;
 __global__ void __launch_bounds__(kPartitionThreads) k_partition(int ntask, const int2* __restrict__ tasks,
                             const gs::PairRec* __restrict__ pairs,
                             const double* __restrict__ dmax, int nshell,
