@@ -191,7 +191,7 @@ class BatchedRHF(MixedWorkspace):
             cut = mixed_cut if mixed_cut is not None else 0.0
             thr = screen_thr if screen_thr > 0 else 1e-300
             banded, tiers = mixed_list(self, classes, cut)
-            ws, each = self.mixed_workspace(self.dev, tiers)
+            ws, each = self.mixed_workspace(self.dev)
             # the bound of the banded launches takes each molecule's largest |P| (at least the
             # block value the partition uses, so no quartet is screened or demoted that the
             # partition would keep).  It is ready before any side stream forks.

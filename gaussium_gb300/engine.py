@@ -941,14 +941,17 @@ def eri_blocks(sb: ShellBasis, quartets, precision=64, device="cuda"):
 # ---------------------------------------------------------------------- Fock (J/K) engine
 class MixedWorkspace:
     """The partition workspace of an engine: one region per stream of the partitioned launches
-    (one launch's lists at a time)."""
+    (one launch's lists at a time).  It is allocated once and never moves: its size follows from
+    the task segments, which are the engine's for good, and not from the launch plan, which changes
+    with the chosen forms, so that a captured graph's addresses stay the engine's."""
 
-    def mixed_workspace(self, dev, tiers):
-        need = _lib.lib().gs_fock_jk_mixed_workspace(int(tiers["count"].max(initial=0)))
-        need = -(-int(need) // 256) * 256
-        if getattr(self, "_ws", None) is None or self._ws.numel() < MIXED_LANES * need:
+    def mixed_workspace(self, dev):
+        """(address, bytes of a region)."""
+        if getattr(self, "_ws", None) is None:
+            longest = max((e - s for _, s, e in self.segments), default=0)
+            need = -(-int(_lib.lib().gs_fock_jk_mixed_workspace(longest)) // 256) * 256
             self._ws = torch.empty(MIXED_LANES * need, dtype=torch.uint8, device=dev)
-        return self._ws.data_ptr(), need
+        return self._ws.data_ptr(), self._ws.numel() // MIXED_LANES
 
 
 # streams of a mixed-precision build's partitioned launches, each with a workspace region (of
@@ -1107,7 +1110,7 @@ class JKEngine(MixedWorkspace):
         base = self.tasks.data_ptr()
         if mixed_cut is not None:
             banded, tiers = mixed_list(self, classes, mixed_cut)
-            ws, each = self.mixed_workspace(dev, tiers)
+            ws, each = self.mixed_workspace(dev)
             for i, (cls, first, prec, form, count, lo, hi) in enumerate(banded):
                 rc = L.gs_fock_jk(*cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
                                   _lib.ptr(self.pairs.prims(prec)), _lib.ptr(self.ds.comp_scale),
