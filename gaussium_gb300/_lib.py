@@ -49,6 +49,7 @@ _SIGS = {
     "gs_class_variant_stamp": (ctypes.c_longlong, []),
     "gs_eri_blocks_list": (I, [I, P, I, P, P, P, P, P, I, P]),
     "gs_fock_jk_list": (I, [I, P, I, P, P, P, P, I, I, P, P, P, I, P, P, P, D, D, D, I, P]),
+    "gs_fock_jk_mixed_list_workspace": (ctypes.c_longlong, [I, P, I]),
     "gs_fock_jk_mixed_list": (I, [I, P, P, P, P, P, P, I, I, P, P, P, I, P, P, P, D, D, P,
                                   ctypes.c_longlong, I, P]),
     "gs_fock_jk_batched_mixed_list": (I, [I, P, P, P, P, P, P, P, P, P, P, P, P, P,

@@ -15,9 +15,8 @@ import torch
 
 from . import _lib
 from .basis import ShellBasis
-from .engine import (MIXED_LANES, PAIR_ORDER, PRIM_SCREEN, DeviceShells, HeavyLane,
-                     MixedWorkspace, PairSet, _pc_lut, launch_plan, mixed_list, segment_profiles,
-                     task_keys)
+from .engine import (PAIR_ORDER, PRIM_SCREEN, DeviceShells, HeavyLane, MixedWorkspace, PairSet,
+                     _pc_lut, launch_plan, mixed_list, segment_profiles, task_keys)
 from .hamiltonian import one_electron
 from .molecules import shell_basis
 
@@ -191,7 +190,7 @@ class BatchedRHF(MixedWorkspace):
             cut = mixed_cut if mixed_cut is not None else 0.0
             thr = screen_thr if screen_thr > 0 else 1e-300
             banded, tiers = mixed_list(self, classes, cut)
-            ws, each = self.mixed_workspace(self.dev)
+            ws, size, lanes = self.mixed_workspace(self.dev, tiers)
             # the bound of the banded launches takes each molecule's largest |P| (at least the
             # block value the partition uses, so no quartet is screened or demoted that the
             # partition would keep).  It is ready before any side stream forks.
@@ -213,7 +212,7 @@ class BatchedRHF(MixedWorkspace):
                 _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base), _lib.ptr(self.mol_n),
                 _lib.ptr(dmax), _lib.ptr(self.mol_shell0), _lib.ptr(self.mol_nshell),
                 _lib.ptr(self.mol_sbase), self.mat_stride, base, _lib.ptr(P), _lib.ptr(J), 1,
-                _lib.ptr(P), _lib.ptr(K), thr, cut, ws, each, *lane.streams(MIXED_LANES))
+                _lib.ptr(P), _lib.ptr(K), thr, cut, ws, -size, *lane.streams(lanes))
             _lib.check(rc, "gs_fock_jk_batched_mixed_list")
             lane.join()
             return

@@ -483,6 +483,8 @@ int gs::partition_tasks(int ntask, const int2* tasks, const PairRec* pairs,
 // first and join it at the end, whatever a launch returns.  From an interpreter each launch and
 // each fork or join cost about 10 us: with one call, the Fock matrix of (H2O)2 (47 launches of
 // 10-100 us) takes 578 us instead of 745.
+extern "C" long long gs_fock_jk_mixed_workspace(int ntask);
+
 struct gs_launch {        // as the header declares it
     int la, lb, lc, ld, form, form32, count, pad;
     long long first;
@@ -519,6 +521,31 @@ int run_list(int n, const gs_launch* list, int nstreams, void* const* streams, F
     if (e) cudaEventDestroy(e);
     return rc;
 }
+
+// Workspace regions of a mixed list's streams, in bytes from the workspace's start: stream k's is
+// [at[k], at[k + 1]).  each >= 0: that many bytes a stream.  each < 0: every region as long as its
+// own stream's longest launch needs, -each bytes in all; the longest tier of a list, which may be
+// most of it, then counts once and not for every stream.
+constexpr int kPackedStreams = 64;
+struct Regions {
+    long long at[kPackedStreams + 1];
+    long long each;
+    int rc;
+    Regions(int n, const gs_launch* list, int nstreams, long long bytes) : each(bytes), rc(GS_OK) {
+        if (bytes >= 0 || n < 1 || !list || nstreams < 1) return;
+        const int m = n < nstreams ? n : nstreams;
+        if (m > kPackedStreams) { rc = GS_ERR_ARG; return; }
+        at[0] = 0;
+        for (int k = 0; k < m; ++k) {
+            int longest = 0;
+            for (int i = k; i < n; i += m) longest = list[i].count > longest ? list[i].count : longest;
+            at[k + 1] = at[k] + (gs_fock_jk_mixed_workspace(longest) + 255) / 256 * 256;
+        }
+        if (at[m] > -bytes) rc = GS_ERR_NOMEM;
+    }
+    long long first(int k) const { return each >= 0 ? k * each : at[k]; }
+    long long size(int k) const { return each >= 0 ? each : at[k + 1] - at[k]; }
+};
 }  // namespace
 
 extern "C" {
@@ -952,6 +979,12 @@ int gs_fock_jk_list(int nlaunch, const gs_launch* list, int precision, const voi
     });
 }
 
+long long gs_fock_jk_mixed_list_workspace(int nlaunch, const gs_launch* list, int nstreams) {
+    if (nlaunch < 1 || !list || nstreams < 1) return 0;
+    const Regions ws(nlaunch, list, nstreams, -1);
+    return ws.rc == GS_ERR_ARG ? 0 : ws.at[nlaunch < nstreams ? nlaunch : nstreams];
+}
+
 int gs_fock_jk_mixed_list(int nlaunch, const gs_launch* list, const void* pair_rec,
                           const void* prim64, const void* prim32, const double* comp_scale,
                           const int* func_off, int nshell, int nbf, const int* tasks,
@@ -959,11 +992,13 @@ int gs_fock_jk_mixed_list(int nlaunch, const gs_launch* list, const void* pair_r
                           const double* shell_dmax, double screen_thr, double mixed_cut,
                           void* workspace, long long stream_bytes, int nstreams,
                           void* const* streams) {
+    const Regions ws(nlaunch, list, nstreams, stream_bytes);
+    if (ws.rc) return ws.rc;
     return run_list(nlaunch, list, nstreams, streams, [&](const gs_launch& x, int lane, void* st) {
         return gs_fock_jk_mixed_forms(
             x.la, x.lb, x.lc, x.ld, x.form, x.form32, pair_rec, prim64, prim32, comp_scale,
             func_off, nshell, nbf, x.count, tasks + 2 * x.first, pj, j, nk, pk, k, shell_dmax,
-            screen_thr, mixed_cut, (char*)workspace + lane * stream_bytes, stream_bytes, st);
+            screen_thr, mixed_cut, (char*)workspace + ws.first(lane), ws.size(lane), st);
     });
 }
 
@@ -975,12 +1010,14 @@ int gs_fock_jk_batched_mixed_list(
     const double* pj, double* j, int nk, const double* pk, double* k, double screen_thr,
     double mixed_cut, void* workspace, long long stream_bytes, int nstreams,
     void* const* streams) {
+    const Regions ws(nlaunch, list, nstreams, stream_bytes);
+    if (ws.rc) return ws.rc;
     return run_list(nlaunch, list, nstreams, streams, [&](const gs_launch& x, int lane, void* st) {
         return gs_fock_jk_batched_mixed_forms(
             x.la, x.lb, x.lc, x.ld, x.form, x.form32, pair_rec, prim64, prim32, comp_scale,
             func_off, shell_mol, mol_base, mol_n, mol_dmax, mol_shell0, mol_nshell, mol_sbase,
             mat_stride, x.count, tasks + 2 * x.first, pj, j, nk, pk, k, screen_thr, mixed_cut,
-            (char*)workspace + lane * stream_bytes, stream_bytes, st);
+            (char*)workspace + ws.first(lane), ws.size(lane), st);
     });
 }
 

@@ -939,24 +939,34 @@ def eri_blocks(sb: ShellBasis, quartets, precision=64, device="cuda"):
 
 
 # ---------------------------------------------------------------------- Fock (J/K) engine
-class MixedWorkspace:
-    """The partition workspace of an engine: one region per stream of the partitioned launches
-    (one launch's lists at a time).  It is allocated once and never moves: its size follows from
-    the task segments, which are the engine's for good, and not from the launch plan, which changes
-    with the chosen forms, so that a captured graph's addresses stay the engine's."""
-
-    def mixed_workspace(self, dev):
-        """(address, bytes of a region)."""
-        if getattr(self, "_ws", None) is None:
-            longest = max((e - s for _, s, e in self.segments), default=0)
-            need = -(-int(_lib.lib().gs_fock_jk_mixed_workspace(longest)) // 256) * 256
-            self._ws = torch.empty(MIXED_LANES * need, dtype=torch.uint8, device=dev)
-        return self._ws.data_ptr(), self._ws.numel() // MIXED_LANES
-
-
-# streams of a mixed-precision build's partitioned launches, each with a workspace region (of
-# 16 bytes a task of the longest tier); with eight (H2O)24 takes 14.93 ms, with six 14.95
+# streams of a mixed-precision build's partitioned launches; with eight (H2O)24 takes 14.93 ms,
+# with six 14.95
 MIXED_LANES = 6
+# bytes of partition workspace above which a build takes fewer streams rather than more memory
+MIXED_BYTES = 2 << 30
+
+
+class MixedWorkspace:
+    """The partition workspace of an engine: one region per stream of the partitioned launches,
+    each as long as the stream's longest launch needs (16 bytes a task).  It is allocated once and
+    never moves: its size follows from the task segments, which are the engine's for good, and not
+    from the launch plan, which changes with the chosen forms, so that a captured graph's addresses
+    stay the engine's.  The streams' longest launches are different tiers, so together they have at
+    most the tasks of the MIXED_LANES longest segments."""
+
+    def mixed_workspace(self, dev, tiers):
+        """(address, bytes, streams) for the launch records ``tiers``."""
+        L = _lib.lib()
+        if getattr(self, "_ws", None) is None:
+            need = [int(L.gs_fock_jk_mixed_workspace(n)) + 256 for n in
+                    sorted((e - s for _, s, e in self.segments), reverse=True)[:MIXED_LANES] or [0]]
+            size = max(need[0], min(sum(need) + MIXED_LANES * 512, MIXED_BYTES))
+            self._ws = torch.empty(size, dtype=torch.uint8, device=dev)
+        lanes = MIXED_LANES
+        while lanes > 1 and L.gs_fock_jk_mixed_list_workspace(len(tiers), tiers.ctypes.data,
+                                                              lanes) > self._ws.numel():
+            lanes -= 1
+        return self._ws.data_ptr(), self._ws.numel(), lanes
 
 
 def task_keys(pairs, bra, ket):
@@ -1110,7 +1120,7 @@ class JKEngine(MixedWorkspace):
         base = self.tasks.data_ptr()
         if mixed_cut is not None:
             banded, tiers = mixed_list(self, classes, mixed_cut)
-            ws, each = self.mixed_workspace(dev)
+            ws, size, lanes = self.mixed_workspace(dev, tiers)
             for i, (cls, first, prec, form, count, lo, hi) in enumerate(banded):
                 rc = L.gs_fock_jk(*cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
                                   _lib.ptr(self.pairs.prims(prec)), _lib.ptr(self.ds.comp_scale),
@@ -1123,8 +1133,7 @@ class JKEngine(MixedWorkspace):
                 len(tiers), tiers.ctypes.data, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
                 _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale), _lib.ptr(self.ds.func_off),
                 self.sb.nshell, n, base, _lib.ptr(pj_c), _lib.ptr(jbuf), nk, _lib.ptr(pk_c),
-                _lib.ptr(kbuf), _lib.ptr(dmax), thr, mixed_cut, ws, each,
-                *lane.streams(MIXED_LANES))
+                _lib.ptr(kbuf), _lib.ptr(dmax), thr, mixed_cut, ws, -size, *lane.streams(lanes))
             _lib.check(rc, "gs_fock_jk_mixed_list")
             runs = []
         for prec, lo, hi in runs:

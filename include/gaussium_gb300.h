@@ -257,8 +257,11 @@ typedef struct gs_launch {
  * round: the last stream is the caller's, the others fork from it before the first launch and
  * join it after the last one.  Other arguments as in the call of the same name without _list;
  * the mixed ones take stream_bytes of workspace a stream (at least
- * gs_fock_jk_mixed_workspace(largest count)).  A launch's error ends the list and is returned;
- * what was launched before it is joined. */
+ * gs_fock_jk_mixed_workspace(largest count)) or, below zero, one workspace of -stream_bytes for
+ * all streams, each with as much of it as its own longest launch needs (at most 64 streams; the
+ * list's sum of them is gs_fock_jk_mixed_list_workspace, 0 for an empty list).  A launch's error
+ * ends the list and is returned; what was launched before it is joined. */
+long long gs_fock_jk_mixed_list_workspace(int nlaunch, const gs_launch* list, int nstreams);
 int gs_eri_blocks_list(int nlaunch, const gs_launch* list, int precision, const void* pair_rec,
                        const void* prim, const double* comp_scale, const void* tasks, double* out,
                        int nstreams, void* const* streams);

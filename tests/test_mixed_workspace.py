@@ -1,5 +1,7 @@
 """The partition workspace of mixed-precision builds: it never moves while the engine lives,
-whatever forms are chosen between two builds, since a captured graph holds its address."""
+whatever forms are chosen between two builds, since a captured graph holds its address; each
+stream has as much of it as its own longest launch needs."""
+import shutil
 import types
 
 import numpy as np
@@ -9,6 +11,17 @@ import torch
 from gaussium_gb300 import batch, engine
 
 CLASSES = [(2, 2, 2, 2), (1, 1, 1, 1), (1, 0, 0, 0), (0, 0, 0, 0)]
+
+
+def read(n, address):
+    raw = (engine.ctypes.c_char * (n * engine.LAUNCH_DTYPE.itemsize)).from_address(address)
+    return np.frombuffer(bytes(raw), dtype=engine.LAUNCH_DTYPE)
+
+
+def regions(counts, lanes):
+    """Bytes that each of the streams in use needs, launch i on stream i % streams."""
+    m = min(len(counts), lanes)
+    return [-(-(256 + 16 * int(max(counts[k::m]))) // 256) * 256 for k in range(m)]
 
 
 class Library:
@@ -37,13 +50,14 @@ class Library:
     def gs_fock_jk_mixed_workspace(self, n):
         return 256 + 16 * n
 
+    def gs_fock_jk_mixed_list_workspace(self, n, list_, lanes):
+        return sum(regions(read(n, list_)["count"], lanes))
+
     def gs_fock_jk_batched(self, *a):
         return 0
 
     def gs_fock_jk_batched_mixed_list(self, n, list_, *a):
-        raw = (engine.ctypes.c_char * (n * engine.LAUNCH_DTYPE.itemsize)).from_address(list_)
-        records = np.frombuffer(bytes(raw), dtype=engine.LAUNCH_DTYPE)
-        self.calls.append((records, *a[-4:-1]))
+        self.calls.append((read(n, list_), *a[-4:-1]))
         return 0
 
 
@@ -105,9 +119,46 @@ def test_workspace_stays_when_forms_change(build):
     run(1e-4)
     assert L.calls[-1][0]["count"].max() == 50000
     assert b._ws is first and len({c[1] for c in L.calls}) == 1
-    for records, ws, each, lanes in L.calls:
-        assert ws == first.data_ptr() and lanes * each <= first.numel()
-        assert L.gs_fock_jk_mixed_workspace(int(records["count"].max())) <= each
+    for records, ws, size, lanes in L.calls:
+        assert ws == first.data_ptr() and -size == first.numel() and lanes == engine.MIXED_LANES
+        assert sum(regions(records["count"], lanes)) <= first.numel()
+    # the longest tier is paid for once
+    assert first.numel() <= 16 * b.tasks.shape[0] + 8192
+
+
+def test_fewer_streams_rather_than_more_memory(build, monkeypatch):
+    b, L, run = build
+    monkeypatch.setattr(engine, "MIXED_BYTES", 1 << 20)
+    run(1e-3)
+    records, _, size, lanes = L.calls[-1]
+    assert b._ws.numel() == -size == 1 << 20 and 1 < lanes < engine.MIXED_LANES
+    assert sum(regions(records["count"], lanes)) <= 1 << 20 < \
+        sum(regions(records["count"], lanes + 1))
+    monkeypatch.setattr(engine, "MIXED_BYTES", 0)
+    del b._ws
+    run(1e-3)
+    assert L.calls[-1][3] == 1 and b._ws.numel() < 16 * 50000 + 1024
+
+
+@pytest.mark.skipif(shutil.which("nvcc") is None, reason="nvcc not available")
+def test_packed_regions_of_a_list():
+    """The library's sum of the streams' needs, and its refusal of a workspace below it before
+    anything is launched."""
+    from gaussium_gb300 import _lib, build
+    L = _lib.load_library(build.build())
+    counts = [7, 50000, 0, 16, 300, 12, 1]
+    records = engine.launch_records([((1, 0, 0, 0), 0, c, 0, 0) for c in counts])
+    for lanes in (1, 2, 3, 6, 8, 64):
+        need = sum(regions(counts, lanes))
+        got = L.gs_fock_jk_mixed_list_workspace(len(records), records.ctypes.data, lanes)
+        assert got == need
+        streams = (engine.ctypes.c_void_p * lanes)()
+        rc = L.gs_fock_jk_mixed_list(len(records), records.ctypes.data, 8, 8, 8, 8, 8, 1, 1, 8, None,
+                                     None, 0, None, None, 8, 1e-12, 1e-3, 8, 1 - need, lanes, streams)
+        assert rc == 5                                     # GS_ERR_NOMEM
+    assert L.gs_fock_jk_mixed_list_workspace(0, None, 6) == 0
+    many = np.repeat(records, 16)
+    assert L.gs_fock_jk_mixed_list_workspace(len(many), many.ctypes.data, 65) == 0
 
 
 @pytest.mark.gpu
