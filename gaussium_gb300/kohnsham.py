@@ -130,10 +130,12 @@ class ExchangeCorrelationGPU:
         phi = self.phi()
         n = self.sb.nbf
         L = _lib.lib()
-        if isinstance(p, torch.Tensor) and p.shape == (n, n) and p.dtype == torch.float64 and \
-                p.device == phi.device and 0 < n <= L.gs_xc_lda_max_functions():
+        plain = isinstance(p, torch.Tensor) and p.layout == torch.strided and not p.is_neg() and \
+            p.shape == (n, n) and p.dtype == torch.float64 and p.device == phi.device
+        if plain and phi.is_contiguous() and phi.shape[0] > 0 and 0 < n <= L.gs_xc_lda_max_functions():
             # the library's build (half the multiply-adds of the two GEMMs); a larger basis,
-            # whose tiles exceed the shared memory, and anything torch would refuse go below
+            # whose tiles exceed the shared memory, a grid without points, a density that is no
+            # plain array and anything torch would refuse go below
             p = p.detach().contiguous()
             npts = phi.shape[0]
             need = L.gs_xc_lda_workspace(npts, n)
