@@ -22,8 +22,9 @@
  * (1/64)^4 / 4! = 2^-28.6 of the value, so their rounding to float is 2^-52.6 of it.
  *
  * For FP32 quartets (T below BOYS_TMAX32, their largest asymptotic threshold) it writes
- * GS_BOYS_F32_<M>: row k = eight floats {hi, lo of F_M(T_k); F_{M+j}(T_k) / j!, j = 1..4;
- * hi, lo of exp(-T_k)}, hi + lo being the value to twice a float's precision.
+ * GS_BOYS_F32_<M>: row k = twelve floats {hi, lo of F_M(T_k); hi, lo of F_{M+1}(T_k);
+ * F_{M+j}(T_k) / j!, j = 2..4; 0; hi, lo of exp(-T_k); 0, 0}, hi + lo being the value to twice a
+ * float's precision.
  *
  * usage: boys_table_gen OUT.h
  */
@@ -105,9 +106,11 @@ int main(int argc, char **argv)
         fprintf(f, "#define GS_BOYS_F32_%d \\\n", M);
         for (int k = 0; k <= BOYS_TMAX32 * BOYS_INV_H; ++k) {
             pair32(f, F[k][M]);
-            for (int j = 1; j <= 4; ++j) fprintf(f, "%af,", (float)(F[k][M + j] / fact[j]));
+            pair32(f, F[k][M + 1]);
+            for (int j = 2; j <= 4; ++j) fprintf(f, "%af,", (float)(F[k][M + j] / fact[j]));
+            fprintf(f, "0.0f,");
             pair32(f, F[k][BOYS_NCOL - 1]);
-            fprintf(f, " \\\n");
+            fprintf(f, "0.0f,0.0f, \\\n");
         }
         fprintf(f, "\n");
     }

@@ -188,7 +188,7 @@ template <int M> constexpr int kBoysRows64 = (int)(kBoysAsym64[M] + 1) * BOYS_IN
 #define GS_BOYS_CAT2(a, b) a##b
 #define GS_BOYS_CAT(a, b) GS_BOYS_CAT2(a, b)
 __device__ const BoysRow64 g_boys_row64[] = {GS_BOYS_CAT(GS_BOYS_ROW64_, GS_BOYS_ORDER)};
-__device__ __align__(16) const float g_boys_f32[BOYS_ROWS32 * 8] = {
+__device__ __align__(16) const float g_boys_f32[BOYS_ROWS32 * 12] = {
     GS_BOYS_CAT(GS_BOYS_F32_, GS_BOYS_ORDER)};
 constexpr int kBoysOrder = GS_BOYS_ORDER;
 static_assert(kBoysOrder >= 0 && kBoysOrder <= BOYS_TAYLOR_MMAX, "Boys order without rows");
@@ -413,26 +413,34 @@ GS_HD GS_INLINE void boys_small(double t, double pref, double* __restrict__ F) {
 }
 
 // The same below an FP32 quartet's threshold, without the FP64 pipe: F_M and exp(-t) as
-// unevaluated sums of two floats.  row: eight floats of grid point T_k (see
+// unevaluated sums of two floats.  row: twelve floats of grid point T_k (see
 // boys_table_gen.c), d = T_k - t, exact in float (both are multiples of t's last place and
-// |d| <= 1/32).  The leading term of each expansion is a pair, so the float rounding of the
-// rest, |d| of it at most, is 2^-29 of the result; the downward recursion carries pairs with
-// error-free sums and products (Dekker, Numer. Math. 18, 224 (1971)); each F_m is rounded to
-// float once, as from FP64, and scaled.  About 17 FP32 instructions an order, against two
-// FP64 ones and a conversion at 64 and 82 cycles a warp.
+// |d| <= 1/32).  The leading term of each expansion and the linear one are pairs, so the float
+// rounding of the rest, d^2 / 2 of it at most, is 2^-35 of the result; the downward recursion
+// carries pairs with error-free sums and products (Dekker, Numer. Math. 18, 224 (1971)); each F_m
+// is rounded to float once, as from FP64 (within 0.505 units in the last place, 0.2886 rms; with
+// the linear term in one float 0.53 to 0.56 at most), and scaled.  About 17 FP32 instructions an
+// order, against two FP64 ones and a conversion at 64 and 82 cycles a warp.
 template <int M>
 GS_HD GS_INLINE void boys_pair32(const float* __restrict__ r, float t, float d, float pref,
                                  float* __restrict__ F) {
-    const float tail = d * fmaf(d, fmaf(d, fmaf(d, r[5], r[4]), r[3]), r[2]);
-    const float fl0 = r[1] + tail;
-    float h = r[0] + fl0;
-    float l = fl0 - (h - r[0]);                          // |r[0]| >= |fl0|
+    const float d2 = d * d;
+    const float fp = d * r[2];                           // the linear term: fp + (fma + d lo)
+    const float fr = fmaf(d, r[3], fmaf(d, r[2], -fp)) + d2 * fmaf(d, fmaf(d, r[6], r[5]), r[4]);
+    float s0 = r[0] + fp;
+    float z0 = (fp - (s0 - r[0])) + (r[1] + fr);         // |r[0]| >= |fp|
+    float h = s0 + z0;
+    float l = z0 - (h - s0);
     F[M] = h * pref;
     if (M > 0) {
-        const float q = d * fmaf(d, fmaf(d, fmaf(d, 1.0f / 24, 1.0f / 6), 0.5f), 1.0f);
-        const float el0 = fmaf(r[6], q, r[7]);
-        const float eh = r[6] + el0;
-        const float el = el0 - (eh - r[6]);
+        // exp(-t) = exp(-T_k) (1 + d + d^2 / 2 + ...)
+        const float ep = r[8] * d;
+        const float er = fmaf(r[9], d, fmaf(r[8], d, -ep)) +
+                         r[8] * (d2 * fmaf(d, fmaf(d, 1.0f / 24, 1.0f / 6), 0.5f));
+        s0 = r[8] + ep;
+        z0 = (ep - (s0 - r[8])) + (r[9] + er);
+        const float eh = s0 + z0;
+        const float el = z0 - (eh - s0);
         const float t2 = t + t;
         GS_UNROLL for (int m = M; m >= 1; --m) {
             const float ph = t2 * h;
@@ -468,9 +476,9 @@ GS_HD GS_INLINE void boys_small32(float t, float pref, float* __restrict__ F) {
         const float kf = fmaf(t, float(BOYS_INV_H), 12582912.0f);    // 1.5 2^23: rounds
         const unsigned k = min(__float_as_uint(kf) & 0x3fffffu, (unsigned)(BOYS_ROWS32 - 1));
         const float d = (kf - 12582912.0f) * (1.0f / BOYS_INV_H) - t;
-        const float4* g = reinterpret_cast<const float4*>(g_boys_f32) + 2 * k;
-        const float4 g0 = __ldg(g), g1 = __ldg(g + 1);
-        const float r[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+        const float4* g = reinterpret_cast<const float4*>(g_boys_f32) + 3 * k;
+        const float4 g0 = __ldg(g), g1 = __ldg(g + 1), g2 = __ldg(g + 2);
+        const float r[10] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w, g2.x, g2.y};
         boys_pair32<M>(r, t, d, pref, F);
         return;
     }

@@ -33,12 +33,15 @@ extern "C" int hc_boys_pair32(int M, double t, double* F) {
     double fact = 1.0;
     const float tf = (float)t, kf = std::nearbyint(tf * float(BOYS_INV_H));
     const double* g = h_boys_d + (int)kf * BOYS_NCOL;
-    float r[8];
-    r[0] = (float)g[M];
-    r[1] = (float)(g[M] - (double)r[0]);
-    for (int j = 1; j <= 4; ++j) r[1 + j] = (float)(g[M + j] / (fact *= j));
-    r[6] = (float)g[BOYS_NCOL - 1];
-    r[7] = (float)(g[BOYS_NCOL - 1] - (double)r[6]);
+    float r[10];
+    for (int j = 0; j <= 1; ++j) {
+        r[2 * j] = (float)g[M + j];
+        r[2 * j + 1] = (float)(g[M + j] - (double)r[2 * j]);
+    }
+    for (int j = 2; j <= 4; ++j) r[2 + j] = (float)(g[M + j] / (fact *= j));
+    r[7] = 0.0f;
+    r[8] = (float)g[BOYS_NCOL - 1];
+    r[9] = (float)(g[BOYS_NCOL - 1] - (double)r[8]);
     const float d = kf * (1.0f / BOYS_INV_H) - tf;
 #define GS_B(MM) case MM: { float f[MM + 1]; boys_pair32<MM>(r, tf, d, 1.0f, f); \
         for (int i = 0; i <= MM; ++i) F[i] = f[i]; return 0; }
