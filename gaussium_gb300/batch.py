@@ -77,7 +77,9 @@ class BatchedRHF(MixedWorkspace):
         # ns_m x ns_m table starts at sbase[m]; every packed density element maps to its block
         ns = np.array([sb.nshell for sb in sbs], dtype=np.int64)
         sbase = np.concatenate([[0], np.cumsum(ns * ns)])
-        self.nblocks = int(sbase[-1])
+        # blocks of shells of all molecules, and where one bound per molecule follows theirs
+        # (engine.mixed_plan)
+        self.nblocks = self.heavy_bound = int(sbase[-1])
         self.mol_shell0 = t(np.array(shell0[:-1]), np.int32)
         self.mol_nshell = t(ns, np.int32)
         self.mol_sbase = t(sbase[:-1], np.int64)
@@ -191,12 +193,15 @@ class BatchedRHF(MixedWorkspace):
             thr = screen_thr if screen_thr > 0 else 1e-300
             banded, tiers = mixed_list(self, classes, cut)
             ws, size, lanes = self.mixed_workspace(self.dev, tiers)
-            # the bound of the banded launches takes each molecule's largest |P| (at least the
-            # block value the partition uses, so no quartet is screened or demoted that the
-            # partition would keep).  It is ready before any side stream forks.
-            mol_dmax = torch.zeros(len(self.mol_n), dtype=torch.float64, device=self.dev)
-            if banded:
-                mol_dmax.scatter_reduce_(0, self.block_mol, dmax, "amax", include_self=True)
+            # the bound of the heavy prefixes takes each molecule's largest |P| (at least the block
+            # value of the other tasks, so no heavy quartet is screened or demoted by a smaller
+            # one): one value a molecule after the block tables.  It is ready before any side
+            # stream forks.
+            nmol = len(self.mol_n)
+            both = torch.zeros(self.heavy_bound + nmol, dtype=torch.float64, device=self.dev)
+            both[:self.heavy_bound] = dmax
+            mol_dmax = both[self.heavy_bound:]
+            mol_dmax.scatter_reduce_(0, self.block_mol, dmax, "amax", include_self=True)
             for i, (cls, first, prec, form, count, lo, hi) in enumerate(banded):
                 rc = L.gs_fock_jk_batched(
                     *cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
@@ -210,7 +215,7 @@ class BatchedRHF(MixedWorkspace):
                 len(tiers), tiers.ctypes.data, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
                 _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale), _lib.ptr(self.local_fo),
                 _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base), _lib.ptr(self.mol_n),
-                _lib.ptr(dmax), _lib.ptr(self.mol_shell0), _lib.ptr(self.mol_nshell),
+                _lib.ptr(both), _lib.ptr(self.mol_shell0), _lib.ptr(self.mol_nshell),
                 _lib.ptr(self.mol_sbase), self.mat_stride, base, _lib.ptr(P), _lib.ptr(J), 1,
                 _lib.ptr(P), _lib.ptr(K), thr, cut, ws, -size, *lane.streams(lanes))
             _lib.check(rc, "gs_fock_jk_batched_mixed_list")

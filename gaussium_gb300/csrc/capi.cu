@@ -486,7 +486,7 @@ int gs::partition_tasks(int ntask, const int2* tasks, const PairRec* pairs,
 extern "C" long long gs_fock_jk_mixed_workspace(int ntask);
 
 struct gs_launch {        // as the header declares it
-    int la, lb, lc, ld, form, form32, count, pad;
+    int la, lb, lc, ld, form, form32, count, bound;
     long long first;
 };
 
@@ -1013,9 +1013,12 @@ int gs_fock_jk_batched_mixed_list(
     const Regions ws(nlaunch, list, nstreams, stream_bytes);
     if (ws.rc) return ws.rc;
     return run_list(nlaunch, list, nstreams, streams, [&](const gs_launch& x, int lane, void* st) {
+        // its own bound: one value a molecule instead of the block tables
+        const bool own = x.bound > 0;
         return gs_fock_jk_batched_mixed_forms(
             x.la, x.lb, x.lc, x.ld, x.form, x.form32, pair_rec, prim64, prim32, comp_scale,
-            func_off, shell_mol, mol_base, mol_n, mol_dmax, mol_shell0, mol_nshell, mol_sbase,
+            func_off, shell_mol, mol_base, mol_n, own ? mol_dmax + x.bound : mol_dmax,
+            own ? nullptr : mol_shell0, own ? nullptr : mol_nshell, own ? nullptr : mol_sbase,
             mat_stride, x.count, tasks + 2 * x.first, pj, j, nk, pk, k, screen_thr, mixed_cut,
             (char*)workspace + ws.first(lane), ws.size(lane), st);
     });

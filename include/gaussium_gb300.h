@@ -247,9 +247,11 @@ int gs_fock_jk_batched_mixed_forms(int la, int lb, int lc, int ld, int form64, i
 
 /* One launch of a list call: count tasks of class (la lb|lc ld) from task `first` of the call's
  * task array on, in the given kernel form (as in the precision argument's bits 8.. and up; form32
- * is the FP32 launch's of a mixed-precision list, else 0).  */
+ * is the FP32 launch's of a mixed-precision list, else 0).  bound: 0, or for a launch of
+ * gs_fock_jk_batched_mixed_list that is to take one bound per molecule where the others take
+ * block tables, the bounds' offset from mol_dmax in doubles. */
 typedef struct gs_launch {
-    int la, lb, lc, ld, form, form32, count, pad;
+    int la, lb, lc, ld, form, form32, count, bound;
     long long first;
 } gs_launch;
 
