@@ -404,8 +404,8 @@ def batched_task_list(q, pair_class, pair_mol, nprim, thr, nclass, nmol, pairs=N
             if bra.numel() == 0:
                 continue
             # most primitive quartets first, equal (K_bra, K_ket) together
-            key = (nprim[bra] * nprim[ket]) * 4096 + nprim[bra] * 64 + nprim[ket] \
-                if pairs is None else task_keys(pairs, bra, ket)
+            key = (nprim[bra] * nprim[ket]) * 4096 + nprim[bra].clamp(max=63) * 64 + \
+                nprim[ket].clamp(max=63) if pairs is None else task_keys(pairs, bra, ket)
             perm = torch.argsort(key, descending=True, stable=True)
             tk = torch.stack([bra[perm], ket[perm]], 1).to(torch.int32)
             (la, lb), (lc, ld) = PAIR_ORDER[cb], PAIR_ORDER[ck]

@@ -445,7 +445,10 @@ __global__ void k_task_keys(long long n, const long long* __restrict__ bra,
         const int f = __float_as_int(x * x + y * y + z * z + 0.25f) >> shift;
         bin = min(max(f - (125 << (23 - shift)), 0), 63);
     }
-    keys[i] = ((nb * nk * 4096 + nb * 64 + nk) << 6) | bin;
+    // the pairs' own counts only order equal products: held to their six bits, so that the product
+    // above them stays whole whatever the contractions
+    const long long fb = nb < 63 ? nb : 63, fk = nk < 63 ? nk : 63;
+    keys[i] = ((nb * nk * 4096 + fb * 64 + fk) << 6) | bin;
 }
 
 // Peak-rate probe: each thread runs `iters` rounds of 8 independent FMA chains.

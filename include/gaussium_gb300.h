@@ -515,7 +515,8 @@ int gs_dense_expand(long long nq, const int* quartets, const long long* offsets,
 /* Sort keys (to be sorted descending) of n Fock tasks (bra[i], ket[i]): primitive-quartet count,
  * the pairs' primitive counts, and the pairs' distance in coarse steps, so that neighbouring
  * tasks take the same loop counts and the same branch of the Boys function.  nprim: kept
- * primitive pairs per pair; key >> 18 is the primitive-quartet count.  Device arrays.  No
+ * primitive pairs per pair; key >> 18 is the primitive-quartet count, below it the pairs' counts
+ * (63 for more).  Device arrays.  No
  * reference counterpart. */
 int gs_task_keys(long long n, const long long* bra, const long long* ket, const int* nprim,
                  const void* pair_rec, const void* prim64, long long* keys, void* stream);
