@@ -184,7 +184,6 @@ class BatchedRHF(MixedWorkspace):
     def _jk_launch(self, P, J, K, precision=64, mixed_cut=None, dmax=None, screen_thr=0.0,
                    classes=None):
         L = _lib.lib()
-        lane = HeavyLane(self.dev)
         base = self.tasks.data_ptr()
         if mixed_cut is not None or screen_thr > 0:
             # partitioned path: screened tasks are dropped on the device before any class
@@ -202,40 +201,35 @@ class BatchedRHF(MixedWorkspace):
             both[:self.heavy_bound] = dmax
             mol_dmax = both[self.heavy_bound:]
             mol_dmax.scatter_reduce_(0, self.block_mol, dmax, "amax", include_self=True)
-            for i, (cls, first, prec, form, count, lo, hi) in enumerate(banded):
-                rc = L.gs_fock_jk_batched(
-                    *cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
-                    _lib.ptr(self.pairs.prims(prec)), _lib.ptr(self.ds.comp_scale),
-                    _lib.ptr(self.local_fo), _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base),
-                    _lib.ptr(self.mol_n), _lib.ptr(mol_dmax), self.mat_stride, count,
-                    base + first * 8, _lib.ptr(P), _lib.ptr(J), 1, _lib.ptr(P), _lib.ptr(K), thr,
-                    lo, hi, lane.lane(i + 1))
-                _lib.check(rc, f"gs_fock_jk_batched{cls}")
-            rc = L.gs_fock_jk_batched_mixed_list(
-                len(tiers), tiers.ctypes.data, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
-                _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale), _lib.ptr(self.local_fo),
-                _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base), _lib.ptr(self.mol_n),
-                _lib.ptr(both), _lib.ptr(self.mol_shell0), _lib.ptr(self.mol_nshell),
-                _lib.ptr(self.mol_sbase), self.mat_stride, base, _lib.ptr(P), _lib.ptr(J), 1,
-                _lib.ptr(P), _lib.ptr(K), thr, cut, ws, -size, *lane.streams(lanes))
-            _lib.check(rc, "gs_fock_jk_batched_mixed_list")
-            lane.join()
+            with HeavyLane(self.dev) as lane:
+                for i, (cls, first, prec, form, count, lo, hi) in enumerate(banded):
+                    rc = L.gs_fock_jk_batched(
+                        *cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
+                        _lib.ptr(self.pairs.prims(prec)), _lib.ptr(self.ds.comp_scale),
+                        _lib.ptr(self.local_fo), _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base),
+                        _lib.ptr(self.mol_n), _lib.ptr(mol_dmax), self.mat_stride, count,
+                        base + first * 8, _lib.ptr(P), _lib.ptr(J), 1, _lib.ptr(P), _lib.ptr(K), thr,
+                        lo, hi, lane.lane(i + 1))
+                    _lib.check(rc, f"gs_fock_jk_batched{cls}")
+                rc = L.gs_fock_jk_batched_mixed_list(
+                    len(tiers), tiers.ctypes.data, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
+                    _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale), _lib.ptr(self.local_fo),
+                    _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base), _lib.ptr(self.mol_n),
+                    _lib.ptr(both), _lib.ptr(self.mol_shell0), _lib.ptr(self.mol_nshell),
+                    _lib.ptr(self.mol_sbase), self.mat_stride, base, _lib.ptr(P), _lib.ptr(J), 1,
+                    _lib.ptr(P), _lib.ptr(K), thr, cut, ws, -size, *lane.streams(lanes))
+                _lib.check(rc, "gs_fock_jk_batched_mixed_list")
             return
-        thr = 0.0
-        runs = [(precision, 0.0, float("inf"))]
-        if mixed_cut is not None:
-            runs = [(64, mixed_cut, float("inf")), (32, 0.0, mixed_cut)]
-        for prec, lo, hi in runs:
-            prims = self.pairs.prims(prec)
-            for i, (cls, first, m, form, _) in enumerate(launch_plan(self, prec, "jk", classes)):
+        prims = self.pairs.prims(precision)
+        with HeavyLane(self.dev) as lane:
+            for i, (cls, first, m, form, _) in enumerate(launch_plan(self, precision, "jk", classes)):
                 rc = L.gs_fock_jk_batched(
-                    *cls, prec | (form << 8), _lib.ptr(self.pairs.rec), _lib.ptr(prims),
+                    *cls, precision | (form << 8), _lib.ptr(self.pairs.rec), _lib.ptr(prims),
                     _lib.ptr(self.ds.comp_scale), _lib.ptr(self.local_fo),
                     _lib.ptr(self.shell_mol), _lib.ptr(self.mol_base), _lib.ptr(self.mol_n),
                     _lib.ptr(dmax), self.mat_stride, m, base + first * 8, _lib.ptr(P),
-                    _lib.ptr(J), 1, _lib.ptr(P), _lib.ptr(K), thr, lo, hi, lane.lane(i))
+                    _lib.ptr(J), 1, _lib.ptr(P), _lib.ptr(K), 0.0, 0.0, float("inf"), lane.lane(i))
                 _lib.check(rc, f"gs_fock_jk_batched{cls}")
-        lane.join()
 
     def tune(self, precisions=(64, 32), reps=3):
         """Choose the kernel form of every class with two on this batch's task lists."""

@@ -356,7 +356,8 @@ _SIDE = {}
 
 class HeavyLane:
     """Side streams of a build, forked from the caller's stream before their first launch
-    and joined back by ``join``.  A build's launches go round the caller's stream and the
+    and joined back by ``join`` or at the end of a ``with``, also where a launch raised: the
+    buffers of what runs on a side are free for others' use only behind it.  A build's launches go round the caller's stream and the
     sides (``lane``): the few long blocks of the heavy tiers then run beside the class
     launches instead of leaving most SMs idle while they finish, and one class's last
     partial wave overlaps the next class's first."""
@@ -388,6 +389,12 @@ class HeavyLane:
         """(count, handles) of a list call's streams, which forks and joins them itself."""
         handles = [x.cuda_stream for x in self.sides[:lanes - 1]] + [self.main.cuda_stream]
         return lanes, (ctypes.c_void_p * lanes)(*handles)
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        self.join()
 
     def join(self):
         for k in range(SIDE_STREAMS):
@@ -1112,49 +1119,40 @@ class JKEngine(MixedWorkspace):
         kbuf = torch.zeros((max(nk, 1), n, n), dtype=torch.float64, device=dev) if nk else None
         pj_c = pj.contiguous() if pj is not None else None
         pk_c = torch.stack(pk).contiguous() if nk else None
-        dmax = None
-        runs = [(precision, 0.0, float("inf"))]
+        dmax, thr = None, 0.0
         if mixed_cut is not None or screen_thr > 0:
             mats = ([pj] if pj is not None else []) + pk
             dmax = self.shell_dmax(mats)
             thr = screen_thr if screen_thr > 0 else 1e-300
-            if mixed_cut is not None:
-                runs = [(64, mixed_cut, float("inf")), (32, 0.0, mixed_cut)]
-            else:
-                runs = [(precision, 0.0, float("inf"))]
-        else:
-            thr = 0.0
         L = _lib.lib()
-        lane = HeavyLane(dev, stream)
         base = self.tasks.data_ptr()
-        if mixed_cut is not None:
-            banded, tiers = mixed_list(self, classes, mixed_cut)
-            ws, size, lanes = self.mixed_workspace(dev, tiers)
-            for i, (cls, first, prec, form, count, lo, hi) in enumerate(banded):
-                rc = L.gs_fock_jk(*cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
-                                  _lib.ptr(self.pairs.prims(prec)), _lib.ptr(self.ds.comp_scale),
-                                  _lib.ptr(self.ds.func_off), self.sb.nshell, n, count,
-                                  base + first * 8, _lib.ptr(pj_c), _lib.ptr(jbuf), nk,
-                                  _lib.ptr(pk_c), _lib.ptr(kbuf), _lib.ptr(dmax), thr, lo, hi,
-                                  lane.lane(i + 1))
-                _lib.check(rc, f"gs_fock_jk{cls}")
-            rc = L.gs_fock_jk_mixed_list(
-                len(tiers), tiers.ctypes.data, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
-                _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale), _lib.ptr(self.ds.func_off),
-                self.sb.nshell, n, base, _lib.ptr(pj_c), _lib.ptr(jbuf), nk, _lib.ptr(pk_c),
-                _lib.ptr(kbuf), _lib.ptr(dmax), thr, mixed_cut, ws, -size, *lane.streams(lanes))
-            _lib.check(rc, "gs_fock_jk_mixed_list")
-            runs = []
-        for prec, lo, hi in runs:
-            plan = launch_list(self, prec, "jk", classes)
-            rc = L.gs_fock_jk_list(
-                len(plan), plan.ctypes.data, prec, _lib.ptr(self.pairs.rec),
-                _lib.ptr(self.pairs.prims(prec)), _lib.ptr(self.ds.comp_scale),
-                _lib.ptr(self.ds.func_off), self.sb.nshell, n, base, _lib.ptr(pj_c),
-                _lib.ptr(jbuf), nk, _lib.ptr(pk_c), _lib.ptr(kbuf), _lib.ptr(dmax), thr, lo, hi,
-                *lane.streams())
-            _lib.check(rc, "gs_fock_jk_list")
-        lane.join()
+        with HeavyLane(dev, stream) as lane:
+            if mixed_cut is not None:
+                banded, tiers = mixed_list(self, classes, mixed_cut)
+                ws, size, lanes = self.mixed_workspace(dev, tiers)
+                for i, (cls, first, prec, form, count, lo, hi) in enumerate(banded):
+                    rc = L.gs_fock_jk(*cls, prec | (form << 8), _lib.ptr(self.pairs.rec),
+                                      _lib.ptr(self.pairs.prims(prec)), _lib.ptr(self.ds.comp_scale),
+                                      _lib.ptr(self.ds.func_off), self.sb.nshell, n, count,
+                                      base + first * 8, _lib.ptr(pj_c), _lib.ptr(jbuf), nk,
+                                      _lib.ptr(pk_c), _lib.ptr(kbuf), _lib.ptr(dmax), thr, lo, hi,
+                                      lane.lane(i + 1))
+                    _lib.check(rc, f"gs_fock_jk{cls}")
+                rc = L.gs_fock_jk_mixed_list(
+                    len(tiers), tiers.ctypes.data, _lib.ptr(self.pairs.rec), _lib.ptr(self.pairs.p64),
+                    _lib.ptr(self.pairs.p32), _lib.ptr(self.ds.comp_scale), _lib.ptr(self.ds.func_off),
+                    self.sb.nshell, n, base, _lib.ptr(pj_c), _lib.ptr(jbuf), nk, _lib.ptr(pk_c),
+                    _lib.ptr(kbuf), _lib.ptr(dmax), thr, mixed_cut, ws, -size, *lane.streams(lanes))
+                _lib.check(rc, "gs_fock_jk_mixed_list")
+            else:
+                plan = launch_list(self, precision, "jk", classes)
+                rc = L.gs_fock_jk_list(
+                    len(plan), plan.ctypes.data, precision, _lib.ptr(self.pairs.rec),
+                    _lib.ptr(self.pairs.prims(precision)), _lib.ptr(self.ds.comp_scale),
+                    _lib.ptr(self.ds.func_off), self.sb.nshell, n, base, _lib.ptr(pj_c),
+                    _lib.ptr(jbuf), nk, _lib.ptr(pk_c), _lib.ptr(kbuf), _lib.ptr(dmax), thr, 0.0,
+                    float("inf"), *lane.streams())
+                _lib.check(rc, "gs_fock_jk_list")
         J = (jbuf + jbuf.T) if jbuf is not None else None
         K = [kbuf[s] + kbuf[s].T for s in range(nk)]
         return J, K

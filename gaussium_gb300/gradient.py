@@ -202,7 +202,6 @@ def eri_gradient(sb, engine: JKEngine, shell_atom, P, natom, classes=None, host=
         thr = screen_thr if screen_thr > 0 else 1e-300
     L = _lib.lib()
     base = engine.tasks.data_ptr()
-    lane = HeavyLane(dev)
     inf = float("inf")
     launches = []
     schedulers = 4 * torch.cuda.get_device_properties(dev).multi_processor_count
@@ -238,23 +237,23 @@ def eri_gradient(sb, engine: JKEngine, shell_atom, P, natom, classes=None, host=
         if x[2] == 0:
             need[i % lanes] = max(need[i % lanes], int(L.gs_fock_jk_mixed_workspace(x[4])))
     ws = [torch.empty(b, dtype=torch.uint8, device=dev) for b in need]
-    for i, (cls, form, prec, first, count, lo, hi) in enumerate(launches):
-        if prec == 0:
-            w = ws[i % lanes]
-            rc = L.gs_eri_grad_mixed(
-                *cls, form, _lib.ptr(engine.pairs.rec), _lib.ptr(engine.pairs.p64),
-                _lib.ptr(engine.pairs.p32), _lib.ptr(engine.ds.comp_scale),
-                _lib.ptr(engine.ds.func_off), _lib.ptr(sa), count, base + first * 8, sb.nbf, natom,
-                _lib.ptr(pt), sb.nshell, _lib.ptr(dmax), thr, lo, _lib.ptr(grad), _lib.ptr(w),
-                w.numel(), lane.lane(i, lanes))
-        else:
-            rc = L.gs_eri_grad_band(
-                *cls, form, prec, _lib.ptr(engine.pairs.rec), _lib.ptr(engine.pairs.p64),
-                _lib.ptr(engine.ds.comp_scale), _lib.ptr(engine.ds.func_off), _lib.ptr(sa),
-                count, base + first * 8, sb.nbf, natom, _lib.ptr(pt), sb.nshell,
-                _lib.ptr(dmax), thr, lo, hi, _lib.ptr(grad), lane.lane(i, lanes))
-        _lib.check(rc, f"eri_gradient{cls}")
-    lane.join()
+    with HeavyLane(dev) as lane:
+        for i, (cls, form, prec, first, count, lo, hi) in enumerate(launches):
+            if prec == 0:
+                w = ws[i % lanes]
+                rc = L.gs_eri_grad_mixed(
+                    *cls, form, _lib.ptr(engine.pairs.rec), _lib.ptr(engine.pairs.p64),
+                    _lib.ptr(engine.pairs.p32), _lib.ptr(engine.ds.comp_scale),
+                    _lib.ptr(engine.ds.func_off), _lib.ptr(sa), count, base + first * 8, sb.nbf, natom,
+                    _lib.ptr(pt), sb.nshell, _lib.ptr(dmax), thr, lo, _lib.ptr(grad), _lib.ptr(w),
+                    w.numel(), lane.lane(i, lanes))
+            else:
+                rc = L.gs_eri_grad_band(
+                    *cls, form, prec, _lib.ptr(engine.pairs.rec), _lib.ptr(engine.pairs.p64),
+                    _lib.ptr(engine.ds.comp_scale), _lib.ptr(engine.ds.func_off), _lib.ptr(sa),
+                    count, base + first * 8, sb.nbf, natom, _lib.ptr(pt), sb.nshell,
+                    _lib.ptr(dmax), thr, lo, hi, _lib.ptr(grad), lane.lane(i, lanes))
+            _lib.check(rc, f"eri_gradient{cls}")
     return grad.view(natom, 3).cpu().numpy() if host else grad.view(natom, 3)
 
 
@@ -353,12 +352,11 @@ def gradient_from_state(st: RHFState, screen_thr=GRAD_SCREEN_THR, mixed_cut=GRAD
     ``screen_thr`` / ``mixed_cut``: density screening and FP32 recursions for the quartets
     with small density-weighted bounds (eri_gradient; 0.0 / None: every quartet in FP64)."""
     sa = shell_atoms(st.mol, st.sb)
-    lane = HeavyLane(st.engine.dev)
-    # the one-electron kernel on a side stream, beside the adjoint kernels
-    one, held = _one_electron_launch(st.engine.ds, st.mol, sa, st.P, st.W, lane)
-    g = eri_gradient(st.sb, st.engine, sa, st.P, len(st.mol.symbols), host=False,
-                     screen_thr=screen_thr, mixed_cut=mixed_cut)
-    lane.join()
+    # the one-electron kernel on a side stream, beside the adjoint kernels; ``held`` until the join
+    with HeavyLane(st.engine.dev) as lane:
+        one, held = _one_electron_launch(st.engine.ds, st.mol, sa, st.P, st.W, lane)
+        g = eri_gradient(st.sb, st.engine, sa, st.P, len(st.mol.symbols), host=False,
+                         screen_thr=screen_thr, mixed_cut=mixed_cut)
     del held
     return (one.view(-1, 3) + g).cpu().numpy() + nuclear_repulsion_gradient(st.mol)
 

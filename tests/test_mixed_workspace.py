@@ -71,7 +71,10 @@ class Lane:
     def streams(self, lanes):
         return lanes, None
 
-    def join(self):
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
         pass
 
 
