@@ -78,7 +78,7 @@ def dense_eri(sb: ShellBasis, device="cuda", precision=64):
     try:
         batch = engine.UniqueQuartets(ds, want32=precision == 32)
         nq, qt, offs = batch.n, batch.quartets, batch.block_offsets
-    except ValueError:
+    except engine.TooManyRanges:
         # very many different contractions: a task per quartet, planned on the host
         q = unique_shell_quartets(sb.nshell)
         batch = engine.QuartetBatch(ds, q, want32=precision == 32)

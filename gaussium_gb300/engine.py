@@ -895,6 +895,11 @@ def unique_pair_ranges(pair_class, nprim):
     return np.array(rows, dtype=RANGE_DTYPE), work, segments
 
 
+class TooManyRanges(ValueError):
+    """A basis of so many different contractions that its unique quartets are no short list of
+    ranges (UniqueQuartets)."""
+
+
 class UniqueQuartets:
     """Blocks of every unique shell quartet of a basis, each in canonical shell order (bra
     pair class >= ket pair class, la >= lb), for the dense tensor: one record per shell pair,
@@ -911,7 +916,7 @@ class UniqueQuartets:
         order = np.lexsort((-npp, pc))                 # every primitive pair is kept (no screen)
         plan = unique_pair_ranges(pc[order], npp[order])
         if plan is None:
-            raise ValueError("too many ranges")
+            raise TooManyRanges("too many ranges of equal primitive counts")
         ranges, work, self.segments = plan
         self.ds = ds
         self.pairs = PairSet(ds, np.stack([a, b], 1)[order], want32=want32, count=False)
