@@ -675,7 +675,7 @@ GS_HD GS_INLINE bool prim_pair_kept(double a, double b, double ABx, double ABy, 
     if (!(max_exp > 0.0)) return true;
     const float x = narrow(ABx), y = narrow(ABy), z = narrow(ABz), af = narrow(a), bf = narrow(b);
     const float t = af * bf * (x * x + y * y + z * z), lim = narrow(max_exp) * (af + bf);
-    if (lim > 1e-30f) {
+    if (lim > 1e-30f && t < 1e38f) {              // no product beyond float's range
         if (t < lim * 0.99999f) return true;
         if (t > lim * 1.00001f) return false;
     }
