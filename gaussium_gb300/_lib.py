@@ -59,6 +59,8 @@ _SIGS = {
     "gs_product_tasks": (I, [ctypes.c_longlong, I, P, P, P, P, P, P]),
     "gs_task_keys": (I, [ctypes.c_longlong, P, P, P, P, P, P, P]),
     "gs_rsqrt_eval": (I, [I, P, P, P]),
+    "gs_rcp_eval": (I, [I, P, P, P]),
+    "gs_exp_eval": (I, [I, P, P, P]),
     "gs_fma_probe": (I, [I, I, I, I, P, P]),
     "gs_fma_probe_lanes": (I, [I, I, I, I, I, P, P]),
     "gs_one_electron": (I, [P, P, P, P, P, P, P, I, P, I, I, P, P, P, P, P, P]),

@@ -302,9 +302,18 @@ __global__ void k_boys(int n, const double* __restrict__ t, double* __restrict__
     for (int m = 0; m <= M; ++m) F[(size_t)i * (M + 1) + m] = (double)f[m];
 }
 
-__global__ void k_rsqrt(int n, const double* __restrict__ x, double* __restrict__ y) {
+// One of the kernels' own elementary functions (test hooks): 0 rsqrt, 1 reciprocal, 2 exponential.
+template <int WHICH>
+__global__ void k_elementary(int n, const double* __restrict__ x, double* __restrict__ y) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = gs::gs_rsqrt(x[i]);
+    if (i < n) y[i] = WHICH == 0 ? gs::gs_rsqrt(x[i]) : WHICH == 1 ? gs::gs_rcp(x[i]) : gs::gs_exp(x[i]);
+}
+template <int WHICH>
+int elementary(int n, const double* x, double* y, void* stream) {
+    if (n < 0 || !x || !y) return GS_ERR_ARG;
+    if (n == 0) return GS_OK;
+    k_elementary<WHICH><<<(n + 127) / 128, 128, 0, S(stream)>>>(n, x, y);
+    return check_launch();
 }
 
 // Split a class's quartet tasks by their density-weighted Schwarz estimate
@@ -1057,10 +1066,15 @@ int gs_task_keys(long long n, const long long* bra, const long long* ket, const 
 }
 
 int gs_rsqrt_eval(int n, const double* x, double* y, void* stream) {
-    if (n < 0 || !x || !y) return GS_ERR_ARG;
-    if (n == 0) return GS_OK;
-    k_rsqrt<<<(n + 127) / 128, 128, 0, S(stream)>>>(n, x, y);
-    return check_launch();
+    return elementary<0>(n, x, y, stream);
+}
+
+int gs_rcp_eval(int n, const double* x, double* y, void* stream) {
+    return elementary<1>(n, x, y, stream);
+}
+
+int gs_exp_eval(int n, const double* x, double* y, void* stream) {
+    return elementary<2>(n, x, y, stream);
 }
 
 int gs_fma_probe_lanes(int precision, int blocks, int threads, int iters, int lanes, void* sink,

@@ -525,6 +525,12 @@ int gs_task_keys(long long n, const long long* bra, const long long* ket, const 
  * units in the last place over the normal range.  No reference counterpart. */
 int gs_rsqrt_eval(int n, const double* x, double* y, void* stream);
 
+/* y[i] = 1 / x[i] and exp(x[i]) as the pair records' kernels evaluate them (test hooks; device
+ * arrays): rounded to 0.51 and 1.3 units in the last place, the library's values outside their
+ * ranges (normal positive x with a normal reciprocal; |x| < 700).  No reference counterpart. */
+int gs_rcp_eval(int n, const double* x, double* y, void* stream);
+int gs_exp_eval(int n, const double* x, double* y, void* stream);
+
 /* FMA throughput probe (FP64 or FP32) used to measure the roofline peaks; sink must hold
  * blocks*threads elements of the chosen type.  No reference counterpart. */
 int gs_fma_probe(int precision, int blocks, int threads, int iters, void* sink, void* stream);
