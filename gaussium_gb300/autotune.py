@@ -7,11 +7,14 @@ primitive quartets through each pass, and as the stacked warp kernel whose lanes
 their node record on several primitive quartets (``gs_class_variants``).  Which is faster
 depends on the workload, chiefly on the primitive counts of the quartets and on how much
 shared memory the grouped buffers take from occupancy.  The
-tuner times both forms of every such class on the caller's own task lists (CUDA events on
-the launching stream, after a warm-up launch, median of ``reps``) and selects the faster
+tuner times every form of every such class on the caller's own task lists (CUDA events on
+the launching stream, after a warm-up launch, median of ``reps``) and selects the fastest
 with ``gs_set_class_variant``; then, for every class, it times the class with and without
 its heavy form (split or cooperative, for the quartets with many primitive quartets) and
-keeps the faster.  The choices are process-wide and stay until changed.
+keeps the faster.  A class without a chosen form follows the engine's launch plan
+(``engine.class_plan``: tiers of several forms by primitive work); ``tune_jk``, ``tune_blocks``
+and ``BatchedRHF.tune`` time that too and choose forms only where they beat the plan.  The
+choices are process-wide and stay until changed.
 """
 import json
 
@@ -37,7 +40,9 @@ def forms(cls, precision):
 
 def describe(row):
     """Name of a tuned class's forms: its form, with the heavy form where the tuner kept
-    its heavy quartets in the split or cooperative form."""
+    its heavy quartets in the split or cooperative form, or the launch plan."""
+    if row.get("plan"):
+        return "plan"
     name = NAMES[row["form"]]
     if row.get("heavy_form"):
         name += "+split" if row["form"] == THREAD else "+cooperative"
@@ -47,6 +52,17 @@ def describe(row):
 def set_form(cls, precision, variant):
     _lib.check(_lib.lib().gs_set_class_variant(*cls, precision, variant),
                f"gs_set_class_variant{cls}")
+
+
+def _apply(cls, precision, row):
+    """Set what a tuned row chose: its form, with or without the heavy form, or the launch plan."""
+    from . import engine
+    plan = row.get("plan", False)
+    set_form(cls, precision, 0 if plan else row["form"])
+    if plan or row.get("heavy_form", True):
+        engine.SPLIT_OFF.discard((cls, precision))
+    else:
+        engine.SPLIT_OFF.add((cls, precision))
 
 
 def _time(fn, reps):
@@ -64,10 +80,23 @@ def _time(fn, reps):
     return out[len(out) // 2]
 
 
-def tune(segments, run_class, precisions=(64, 32), reps=3, min_tasks=1):
+# forms are chosen over the launch plan where their time is below this share of the plan's: timings
+# differ by a few per cent, and a chosen form also takes its class out of the mixed builds'
+# partition by tiers ((H2O)24 14.6 -> 15.1 ms with forms for three of 42, 24 molecules in one batch
+# 12.0 -> 12.5 ms with eleven, whose plain builds they had made 0 to 1 % faster)
+FORM_OVER_PLAN = 0.95
+
+
+def tune(segments, run_class, precisions=(64, 32), reps=3, min_tasks=1, whole=None):
     """Choose the faster form for every class of ``segments`` ([(cls, start, end)]) that
     has two; ``run_class(cls, precision)`` launches that class's work once on the current
-    stream.  Returns {(cls, precision): {"form": v, "ms": {v: t}}}."""
+    stream.  With ``whole(precision)``, which launches every class's, a class keeps the
+    engine's launch plan, which it follows when it has no form, unless a form is faster (rows
+    then have "plan" and its time "ms_plan"; "form" is the fastest form all the same), and all
+    classes keep it unless the whole call is faster with the forms: the plan's tiers overlap
+    across classes, which the times of one class do not show ((H2O)7 unrestricted 4.38 ms by the
+    plan, 4.63 with a form for each class where one was faster alone).  Returns
+    {(cls, precision): {"form": v, "ms": {v: t}}}."""
     chosen = {}
     from . import engine
     for prec in precisions:
@@ -76,7 +105,11 @@ def tune(segments, run_class, precisions=(64, 32), reps=3, min_tasks=1):
                 continue
             fs = forms(cls, prec)
             times = {}
-            if len(fs) >= 2:
+            if whole:
+                set_form(cls, prec, 0)
+                engine.SPLIT_OFF.discard((cls, prec))
+                t_plan = _time(lambda: run_class(cls, prec), reps)
+            if len(fs) >= 2 or whole:
                 for v in fs:
                     set_form(cls, prec, v)
                     times[v] = _time(lambda: run_class(cls, prec), reps)
@@ -97,21 +130,34 @@ def tune(segments, run_class, precisions=(64, 32), reps=3, min_tasks=1):
             row["ms_without_heavy_form"] = off
             if not row["heavy_form"]:
                 engine.SPLIT_OFF.add((cls, prec))
+            if whole:
+                row["ms_plan"] = t_plan
+                row["plan"] = min(t_best, off) >= FORM_OVER_PLAN * t_plan
+                _apply(cls, prec, row)
             chosen[(cls, prec)] = row
+        formed = {k: r for k, r in chosen.items() if k[1] == prec and not r.get("plan")}
+        if whole and formed:
+            t_forms = _time(lambda: whole(prec), reps)
+            for (cls, _), row in formed.items():
+                _apply(cls, prec, dict(row, plan=True))
+            keep = t_forms < FORM_OVER_PLAN * _time(lambda: whole(prec), reps)
+            for (cls, _), row in formed.items():
+                row["plan"] = not keep
+                _apply(cls, prec, row)
     return chosen
 
 
 def tune_jk(engine, density, precisions=(64, 32), reps=3):
     """Tune the J/K class launches of a JKEngine on its task list with one density."""
     P = density if torch.is_tensor(density) else torch.as_tensor(density).to(engine.dev)
-    return tune(engine.segments, lambda cls, prec: engine.jk(P, [P], precision=prec, classes=[cls]),
-                precisions, reps)
+    run = lambda prec, classes=None: engine.jk(P, [P], precision=prec, classes=classes)  # noqa: E731
+    return tune(engine.segments, lambda cls, prec: run(prec, [cls]), precisions, reps, whole=run)
 
 
 def tune_blocks(batch, out, precisions=(64, 32), reps=3):
     """Tune the integral-block class launches of a QuartetBatch writing into ``out``."""
-    return tune(batch.segments, lambda cls, prec: batch.run(out, prec, classes=[cls]),
-                precisions, reps)
+    run = lambda prec, classes=None: batch.run(out, prec, classes=classes)    # noqa: E731
+    return tune(batch.segments, lambda cls, prec: run(prec, [cls]), precisions, reps, whole=run)
 
 
 def grad_forms(cls):
@@ -156,29 +202,24 @@ def reset(segments, precisions=(64, 32)):
 
 def save(chosen, path):
     rows = [{"class": list(cls), "precision": prec, "form": r["form"],
-             "heavy_form": r.get("heavy_form", True),
+             "heavy_form": r.get("heavy_form", True), "plan": r.get("plan", False),
              "ms": {str(k): v for k, v in r["ms"].items()}} for (cls, prec), r in chosen.items()]
     with open(path, "w") as f:
         json.dump(rows, f, indent=1)
 
 
 def load(path):
-    """Apply a saved choice (form and heavy form of every class); returns it in the form
-    ``tune`` returns."""
-    from . import engine
+    """Apply a saved choice (form and heavy form of every class, or the launch plan); returns
+    it in the form ``tune`` returns."""
     with open(path) as f:
         rows = json.load(f)
     chosen = {}
     for r in rows:
         cls, prec = tuple(r["class"]), r["precision"]
-        set_form(cls, prec, r["form"])
-        heavy = r.get("heavy_form", True)
-        if heavy:
-            engine.SPLIT_OFF.discard((cls, prec))
-        else:
-            engine.SPLIT_OFF.add((cls, prec))
-        chosen[(cls, prec)] = {"form": r["form"], "heavy_form": heavy,
-                               "ms": {int(k): v for k, v in r["ms"].items()}}
+        row = {"form": r["form"], "heavy_form": r.get("heavy_form", True),
+               "plan": r.get("plan", False), "ms": {int(k): v for k, v in r["ms"].items()}}
+        _apply(cls, prec, row)
+        chosen[(cls, prec)] = row
     return chosen
 
 

@@ -236,9 +236,9 @@ class BatchedRHF(MixedWorkspace):
         from . import autotune
         P = torch.zeros(self.mat_stride, dtype=torch.float64, device=self.dev)
         J, K = torch.zeros_like(P), torch.zeros_like(P)
-        return autotune.tune(self.segments,
-                             lambda cls, prec: self._jk_launch(P, J, K, prec, classes=[cls]),
-                             precisions, reps)
+        run = lambda prec, classes=None: self._jk_launch(P, J, K, prec, classes=classes)  # noqa: E731
+        return autotune.tune(self.segments, lambda cls, prec: run(prec, [cls]), precisions, reps,
+                             whole=run)
 
     def density(self, m):
         """Converged density of molecule m (host nbf_m x nbf_m) after ``run``."""
