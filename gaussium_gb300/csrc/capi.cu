@@ -614,7 +614,8 @@ int gs_class_variant(int la, int lb, int lc, int ld, int precision) {
 
 int gs_set_class_variant(int la, int lb, int lc, int ld, int precision, int variant) {
     if (!find_class(la, lb, lc, ld)) return GS_ERR_CLASS;
-    // the cooperative form (5) takes host task counts only, so it is per call, not per class
+    // the cooperative (5) and cluster (7) forms are for heavy quartets: a block or eight on every
+    // light one would leave most warps idle, so they are chosen per call, not per class
     if ((precision != 64 && precision != 32) || variant < 0 || variant > 6 || variant == 5)
         return GS_ERR_ARG;
     if (variant && !(find_variants(la, lb, lc, ld, precision) & (1 << (variant - 1))))

@@ -183,6 +183,8 @@ __device__ __forceinline__ void jk_digest(const JKArgs& a, const int2 task, cons
         GS_UNROLL for (int i = 0; i < NC; ++i)
             GS_UNROLL for (int j = 0; j < ND; ++j) pcd[i * ND + j] = narrow_to(T(0), P[(fc + i) * n + fd + j]);
         T jab[NA * NB], jcd[NC * ND];
+        // a zero that the compiler does not know: with a known one it makes the first multiply-add
+        // of each sum a product, which holds the FP64 pipe longer
         const T nil = gs_mul(T(0), T(0));
         GS_UNROLL for (int i = 0; i < NA * NB; ++i) jab[i] = nil;
         GS_UNROLL for (int i = 0; i < NC * ND; ++i) jcd[i] = T(0);

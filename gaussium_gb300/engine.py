@@ -349,7 +349,8 @@ def mixed_prefix(cls, heavy, mixed_cut):
 
 # Eight streams with the caller's, the hardware queues of a default context (CUDA_DEVICE_MAX_
 # CONNECTIONS): 4,096 random cc-pVTZ-shaped quartets 831 us with four streams, 695 with six, 594
-# with eight, 587 with twelve, which share queues; 2 x (H2O)7 3.15, 3.06, 2.99, 2.99 ms.
+# with eight, 587 with twelve, which share queues; the unrestricted build of one (H2O)7 geometry
+# 3.15, 3.06, 2.99, 2.99 ms (others take up to 4.4).
 SIDE_STREAMS = 7
 _SIDE = {}
 
@@ -629,17 +630,14 @@ _DEVICE_LUTS = {}
 
 
 def _device_luts(dev):
-    """The canonicalisation and block-size tables (and each pair-class combination's
-    heavy threshold) on a device."""
+    """The canonicalisation and block-size tables on a device."""
     if dev not in _DEVICE_LUTS:
         pos, code, pcb, pck = _CANON_LUT
-        thr = [heavy_threshold(PAIR_ORDER[c // 6] + PAIR_ORDER[c % 6]) for c in range(36)]
         _DEVICE_LUTS[dev] = {
             "pos": torch.as_tensor(np.asarray(pos, dtype=np.int64)).to(dev),
             "code": torch.as_tensor(np.asarray(code, dtype=np.int32)).to(dev),
             "cls": torch.as_tensor(np.asarray(pcb * 6 + pck, dtype=np.int64)).to(dev),
             "size": torch.as_tensor(np.asarray(_SIZE_LUT, dtype=np.int64)).to(dev),
-            "thr": torch.as_tensor(np.asarray(thr, dtype=np.int64)).to(dev),
         }
     return _DEVICE_LUTS[dev]
 
