@@ -109,6 +109,11 @@ COOP_LEVEL = COOP_PRIM_QUARTETS.bit_length() - 1     # one warp alone takes fewe
 _LEVELS = 1 << np.arange(WORK_LEVELS, dtype=np.int64)
 MIN_LATENCY = 600.0       # slots (20 us) below which a long quartet is not worth splitting
 LATENCY_SHARE = 0.15      # of a call's whole work that one lane or warp may take alone
+# and of a call's own work where it is for some of the classes only, in FP64: 21 classes of 300,000
+# random quartets' blocks one by one 13.4 ms (1: 13.3, 4: 13.9, without: 18.4), of 2,000,000 71.2
+# (69.9, 74.5, 86.7), Fock classes of (H2O)8 6.1 ms (6.7, 6.2, 6.2).  FP32's estimate of the work is
+# too low for it (its kernels are not bound by their pipe).
+ALONE_SHARE = 2.0
 
 
 def work_profile(work_desc):
@@ -230,6 +235,11 @@ def launch_plan(engine_like, precision, kind, classes=None, share=1.0):
         plans[key] = (slots, sch, {})
     slots, sch, cached = plans[key]
     limit = max(MIN_LATENCY, LATENCY_SHARE * share * slots[precision])
+    if classes is not None and share == 1.0 and precision == 64:
+        # a call for some classes alone: nothing runs beside their long tiers
+        mine = [(seg, prof) for seg, prof in zip(e.segments, e.profiles) if seg[0] in classes]
+        alone = total_slots(*zip(*mine), precision, kind, sch) if mine else 0.0
+        limit = min(limit, max(MIN_LATENCY, ALONE_SHARE * alone))
     out = []
     for (cls, s, t), heavy, prof in zip(e.segments, e.heavy, e.profiles):
         if classes is not None and cls not in classes:
