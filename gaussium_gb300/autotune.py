@@ -80,11 +80,12 @@ def _time(fn, reps):
     return out[len(out) // 2]
 
 
-# forms are chosen over the launch plan where their time is below this share of the plan's: timings
-# differ by a few per cent, and a chosen form also takes its class out of the mixed builds'
-# partition by tiers ((H2O)24 14.6 -> 15.1 ms with forms for three of 42, 24 molecules in one batch
-# 12.0 -> 12.5 ms with eleven, whose plain builds they had made 0 to 1 % faster)
-FORM_OVER_PLAN = 0.95
+# forms are chosen over the launch plan where their time is below this share of the plan's, for the
+# class alone and for the whole call: timings of one class differ by a few per cent, and a chosen
+# form also takes its class out of the mixed builds' partition by tiers ((H2O)24 14.6 -> 15.1 ms
+# with forms for three of 42, 24 molecules in one batch 12.0 -> 12.5 ms with eleven, whose plain
+# builds they had made 0 to 1 % faster).  2,000,000 random quartets' FP64 blocks gain 4 % by forms
+FORM_OVER_PLAN, FORMS_OVER_PLANS = 0.95, 0.98
 
 
 def tune(segments, run_class, precisions=(64, 32), reps=3, min_tasks=1, whole=None):
@@ -140,7 +141,7 @@ def tune(segments, run_class, precisions=(64, 32), reps=3, min_tasks=1, whole=No
             t_forms = _time(lambda: whole(prec), reps)
             for (cls, _), row in formed.items():
                 _apply(cls, prec, dict(row, plan=True))
-            keep = t_forms < FORM_OVER_PLAN * _time(lambda: whole(prec), reps)
+            keep = t_forms < FORMS_OVER_PLANS * _time(lambda: whole(prec), reps)
             for (cls, _), row in formed.items():
                 row["plan"] = not keep
                 _apply(cls, prec, row)
