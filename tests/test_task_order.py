@@ -34,3 +34,21 @@ def test_task_keys_of_long_contractions(gpu_lib):
     assert np.array_equal(keys // engine.KEY_WORK, work) and np.array_equal(keys >> 18, work)
     assert np.all(np.diff(work) <= 0)
     assert eng.profiles[0] == engine.work_profile(work)
+
+
+@pytest.mark.parametrize("at_once", [1 << 26, 10])
+@pytest.mark.parametrize("first", [0, 7])
+def test_segment_profiles_of_uneven_segments(monkeypatch, at_once, first):
+    """Empty and one-task segments, counts of zero and far beyond the levels, a list that starts
+    behind others, and lists taken segment by segment: the host's counts."""
+    from gaussium_gb300 import engine
+    monkeypatch.setattr(engine, "SEARCH_AT_ONCE", at_once)
+    rng = np.random.default_rng(6)
+    segs = [np.sort(rng.integers(0, t, n))[::-1] for t, n in
+            ((1, 5), (1300, 400), (2, 0), (1 << 45, 30), (5, 1), (129, 200), (1, 0))]
+    cls = [(0, 0, 0, 0), (2, 2, 2, 2), (1, 0, 0, 0), (1, 1, 1, 1), (2, 0, 0, 0), (2, 1, 1, 0), (1, 1, 0, 0)]
+    w = torch.as_tensor(np.concatenate([np.full(first, 99), *segs]))
+    bounds = (first + np.concatenate([[0], np.cumsum([len(x) for x in segs])])).tolist()
+    got = engine.segment_profiles(cls, w, bounds)
+    assert got == [(engine.heavy_counts(c, x), engine.work_profile(x)) for c, x in zip(cls, segs)]
+    assert engine.segment_profiles([], w, [0]) == []
