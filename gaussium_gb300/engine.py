@@ -108,7 +108,7 @@ MANY_WARPS = {"jk": 4, "write": 16}
 COOP_LEVEL = COOP_PRIM_QUARTETS.bit_length() - 1     # one warp alone takes fewer than that
 _LEVELS = 1 << np.arange(WORK_LEVELS, dtype=np.int64)
 KEY_STEP = 1 << 57        # more than any quartet's primitive quartets; times 36 classes within int64
-SEARCH_AT_ONCE = 1 << 26  # tasks
+SEARCH_AT_ONCE = 1 << 20  # tasks
 MIN_LATENCY = 600.0       # slots (20 us) below which a long quartet is not worth splitting
 LATENCY_SHARE = 0.15      # of a call's whole work that one lane or warp may take alone
 # and of a call's own work where it is for some of the classes only, in FP64: 21 classes of 300,000
@@ -127,29 +127,33 @@ def work_profile(work_desc):
 
 def segment_profiles(cls_list, work_desc, bounds):
     """(heavy_counts, work_profile) of every segment [bounds[i], bounds[i+1]) of a device
-    tensor of primitive-quartet counts, descending within each segment, in one transfer.  One
-    search finds every segment's thresholds: segment i's counts, negated and moved up by i
-    times KEY_STEP, are one ascending list (a search a segment cost 2 ms for 21 of them, most of
-    a small batch's device planning).  Lists beyond SEARCH_AT_ONCE go segment by segment, without
-    copies of the whole."""
+    tensor of primitive-quartet counts, descending within each segment, in one transfer.  Up to
+    SEARCH_AT_ONCE tasks one search finds every segment's thresholds: segment i's counts, negated
+    and moved up by i times KEY_STEP, are one ascending list.  Longer lists go segment by segment,
+    without copies of the whole (device planning of 4,096 quartets 2.4 ms, segment by segment 3.9;
+    the task lists of (H2O)24 31.7 and, in one search, 36.5)."""
     dev = work_desc.device
     n = len(cls_list)
     if n == 0:
         return []
     first = np.asarray(bounds, dtype=np.int64)
-    if n > 1 and first[-1] - first[0] > SEARCH_AT_ONCE:
-        return [segment_profiles([c], work_desc[s:e], [0, e - s])[0]
-                for c, s, e in zip(cls_list, bounds[:-1], bounds[1:])]
     levels = np.array([[heavy_threshold(c), COOP_PRIM_QUARTETS, *_LEVELS.tolist()] for c in cls_list],
                       dtype=np.int64)
     step = np.arange(n, dtype=np.int64) * KEY_STEP
-    at, length, query = upload(dev, first - first[0], np.diff(first), step[:, None] - levels)
     w = work_desc[int(first[0]):int(first[-1])]
-    key = torch.repeat_interleave(torch.arange(n, device=dev) * KEY_STEP, length,
-                                  output_size=w.numel()) - w
-    found = torch.searchsorted(key, query, right=True) - at[:-1, None]
-    upto = torch.cat([w.new_zeros(1), torch.cumsum(w, 0)])
-    rows = torch.cat([(upto[at[1:]] - upto[at[:-1]])[:, None], found], 1).tolist()
+    if w.numel() > SEARCH_AT_ONCE:
+        (query,) = upload(dev, -levels)
+        parts = [work_desc[s:e] for s, e in zip(bounds[:-1], bounds[1:])]
+        found = torch.stack([torch.searchsorted(-x, q, right=True) for x, q in zip(parts, query)])
+        total = torch.stack([x.sum() for x in parts])
+    else:
+        at, length, query = upload(dev, first - first[0], np.diff(first), step[:, None] - levels)
+        key = torch.repeat_interleave(torch.arange(n, device=dev) * KEY_STEP, length,
+                                      output_size=w.numel()) - w
+        found = torch.searchsorted(key, query, right=True) - at[:-1, None]
+        upto = torch.cat([w.new_zeros(1), torch.cumsum(w, 0)])
+        total = upto[at[1:]] - upto[at[:-1]]
+    rows = torch.cat([total[:, None], found], 1).tolist()
     return [((r[1], r[2]), (r[0], r[3:])) for r in rows]
 
 
