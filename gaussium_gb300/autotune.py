@@ -13,8 +13,8 @@ with ``gs_set_class_variant``; then, for every class, it times the class with an
 its heavy form (split or cooperative, for the quartets with many primitive quartets) and
 keeps the faster.  A class without a chosen form follows the engine's launch plan
 (``engine.class_plan``: tiers of several forms by primitive work); ``tune_jk``, ``tune_blocks``
-and ``BatchedRHF.tune`` time that too and choose forms only where they beat the plan.  The
-choices are process-wide and stay until changed.
+and ``BatchedRHF.tune`` time that too and leave unpartitioned calls on it where it is the
+faster (``engine.PLAN_ON``).  The choices are process-wide and stay until changed.
 """
 import json
 
@@ -40,7 +40,8 @@ def forms(cls, precision):
 
 def describe(row):
     """Name of a tuned class's forms: its form, with the heavy form where the tuner kept
-    its heavy quartets in the split or cooperative form, or the launch plan."""
+    its heavy quartets in the split or cooperative form; "plan" where unpartitioned calls
+    follow the launch plan."""
     if row.get("plan"):
         return "plan"
     name = NAMES[row["form"]]
@@ -50,19 +51,24 @@ def describe(row):
 
 
 def set_form(cls, precision, variant):
+    from . import engine
     _lib.check(_lib.lib().gs_set_class_variant(*cls, precision, variant),
                f"gs_set_class_variant{cls}")
+    engine.PLAN_ON.pop((cls, precision), None)
 
 
-def _apply(cls, precision, row):
-    """Set what a tuned row chose: its form, with or without the heavy form, or the launch plan."""
+def _apply(cls, precision, row, variant):
+    """Set what a tuned row chose: ``variant``, with or without the heavy form, and the launch
+    plan for unpartitioned calls."""
     from . import engine
-    plan = row.get("plan", False)
-    set_form(cls, precision, 0 if plan else row["form"])
-    if plan or row.get("heavy_form", True):
+    set_form(cls, precision, variant)
+    engine.PLAN_ON.pop((cls, precision), None)
+    if row.get("heavy_form", True):
         engine.SPLIT_OFF.discard((cls, precision))
     else:
         engine.SPLIT_OFF.add((cls, precision))
+    if row.get("plan", False):
+        engine.PLAN_ON[cls, precision] = variant
 
 
 def _time(fn, reps):
@@ -80,27 +86,25 @@ def _time(fn, reps):
     return out[len(out) // 2]
 
 
-# forms are chosen over the launch plan where their time is below this share of the plan's, for the
-# class alone and for the whole call: timings of one class differ by a few per cent, and a chosen
-# form also takes its class out of the mixed builds' partition by tiers ((H2O)24 14.6 -> 15.1 ms
-# with forms for three of 42, 24 molecules in one batch 12.0 -> 12.5 ms with eleven, whose plain
-# builds they had made 0 to 1 % faster).  2,000,000 random quartets' FP64 blocks gain 4 % by forms
-FORM_OVER_PLAN, FORMS_OVER_PLANS = 0.95, 0.98
+# unpartitioned calls leave the launch plan for the forms where the whole call's time is below this
+# share of the plan's.  2,000,000 random quartets' FP64 blocks gain 4 % by forms, FP32 35 %
+FORMS_OVER_PLANS = 0.98
 
 
 def tune(segments, run_class, precisions=(64, 32), reps=3, min_tasks=1, whole=None):
     """Choose the faster form for every class of ``segments`` ([(cls, start, end)]) that
     has two; ``run_class(cls, precision)`` launches that class's work once on the current
-    stream.  With ``whole(precision)``, which launches every class's, a class keeps the
-    engine's launch plan, which it follows when it has no form, unless a form is faster (rows
-    then have "plan" and its time "ms_plan"; "form" is the fastest form all the same), and all
-    classes keep it unless the whole call is faster with the forms: the plan's tiers overlap
-    across classes, which the times of one class do not show ((H2O)7 unrestricted 4.38 ms by the
-    plan, 4.63 with a form for each class where one was faster alone).  Returns
-    {(cls, precision): {"form": v, "ms": {v: t}}}."""
+    stream.  With ``whole(precision)``, which launches every class's, unpartitioned calls keep
+    the engine's launch plan for a class unless its form is faster, and for all classes unless
+    the whole call is faster with the forms: the plan's tiers overlap across classes, which the
+    times of one class do not show (rows then have "plan" and its time "ms_plan").
+    Mixed-precision builds take the forms either way: by forms for all classes or by the plan for
+    all they are within some per cent of each other, small ones up to 45 % faster by forms, and by
+    some of each slower than by either.  Returns {(cls, precision): {"form": v, "ms": {v: t}}}."""
     chosen = {}
     from . import engine
     for prec in precisions:
+        variants = {}
         for cls, s, e in segments:
             if e - s < min_tasks:
                 continue
@@ -110,7 +114,7 @@ def tune(segments, run_class, precisions=(64, 32), reps=3, min_tasks=1, whole=No
                 set_form(cls, prec, 0)
                 engine.SPLIT_OFF.discard((cls, prec))
                 t_plan = _time(lambda: run_class(cls, prec), reps)
-            if len(fs) >= 2 or whole:
+            if len(fs) >= 2:
                 for v in fs:
                     set_form(cls, prec, v)
                     times[v] = _time(lambda: run_class(cls, prec), reps)
@@ -133,18 +137,19 @@ def tune(segments, run_class, precisions=(64, 32), reps=3, min_tasks=1, whole=No
                 engine.SPLIT_OFF.add((cls, prec))
             if whole:
                 row["ms_plan"] = t_plan
-                row["plan"] = min(t_best, off) >= FORM_OVER_PLAN * t_plan
-                _apply(cls, prec, row)
+                row["plan"] = min(t_best, off) >= t_plan
+                variants[cls] = best if len(fs) >= 2 else 0
+                _apply(cls, prec, row, variants[cls])
             chosen[(cls, prec)] = row
         formed = {k: r for k, r in chosen.items() if k[1] == prec and not r.get("plan")}
         if whole and formed:
             t_forms = _time(lambda: whole(prec), reps)
             for (cls, _), row in formed.items():
-                _apply(cls, prec, dict(row, plan=True))
+                _apply(cls, prec, dict(row, plan=True), variants[cls])
             keep = t_forms < FORMS_OVER_PLANS * _time(lambda: whole(prec), reps)
             for (cls, _), row in formed.items():
                 row["plan"] = not keep
-                _apply(cls, prec, row)
+                _apply(cls, prec, row, variants[cls])
     return chosen
 
 
@@ -219,7 +224,7 @@ def load(path):
         cls, prec = tuple(r["class"]), r["precision"]
         row = {"form": r["form"], "heavy_form": r.get("heavy_form", True),
                "plan": r.get("plan", False), "ms": {int(k): v for k, v in r["ms"].items()}}
-        _apply(cls, prec, row)
+        _apply(cls, prec, row, row["form"])
         chosen[(cls, prec)] = row
     return chosen
 

@@ -49,6 +49,10 @@ THREAD_FORM, WARP_FORM, GROUPED_FORM, SPLIT_FORM, COOP_FORM, STACKED_FORM, CLUST
 # (class, precision) pairs whose heavy quartets stay on the class's own form (set by the
 # autotuner where that measured faster)
 SPLIT_OFF = set()
+# (class, precision): form, where the autotuner measured the launch plan (class_plan) faster than
+# that form, the class's chosen one: unpartitioned calls follow the plan as long as the form stays
+# chosen, mixed-precision builds the form (mixed_plan)
+PLAN_ON = {}
 
 
 @functools.lru_cache(maxsize=None)
@@ -242,7 +246,8 @@ def class_plan(cls, precision, kind, n, profile, limit, built, schedulers=608):
 def launch_plan(engine_like, precision, kind, classes=None, share=1.0):
     """[(class, first task, count, form, latency)] of one call, longest latency first: the
     launches go to several streams, so the few long blocks run beside the rest.  Classes
-    with a chosen form (gs_set_class_variant, the autotuner) follow split_forms."""
+    with a chosen form (gs_set_class_variant, the autotuner) follow split_forms, unless the
+    autotuner left them to the plan (PLAN_ON)."""
     e = engine_like
     L = _lib.lib()
     key = (precision, kind)
@@ -262,7 +267,8 @@ def launch_plan(engine_like, precision, kind, classes=None, share=1.0):
     for (cls, s, t), heavy, prof in zip(e.segments, e.heavy, e.profiles):
         if classes is not None and cls not in classes:
             continue
-        if L.gs_class_variant(*cls, precision) or (cls, precision) in SPLIT_OFF:
+        variant = L.gs_class_variant(*cls, precision)
+        if (variant or (cls, precision) in SPLIT_OFF) and PLAN_ON.get((cls, precision)) != variant:
             parts = [(form, first, (t - s - first) if count is None else count,
                       float("inf") if count is not None else 0.0)
                      for form, first, count in split_forms(cls, precision, heavy)]
@@ -327,7 +333,8 @@ def launch_records(launches):
 def kept_plan(engine_like, key, build, *more):
     """``build()``, kept on the engine under ``key`` until a class's form is chosen anew (or
     ``more`` changes): task segments, profiles and the device are the engine's for good."""
-    stamp = (_lib.lib().gs_class_variant_stamp(), frozenset(SPLIT_OFF), *more)
+    stamp = (_lib.lib().gs_class_variant_stamp(), frozenset(SPLIT_OFF), frozenset(PLAN_ON.items()),
+             *more)
     kept = engine_like.__dict__.setdefault("_kept_plans", {})
     if key not in kept or kept[key][0] != stamp:
         kept[key] = (stamp, build())
