@@ -867,10 +867,10 @@ class QuartetBatch:
     def class_counts(self):
         return {cls: e - s for cls, s, e in self.segments}
 
-    def launch_count(self, precision=64):
+    def launch_count(self, precision=64, classes=None):
         """Kernel launches one ``run`` makes with the current kernel forms: one per class
         and tier of primitive work."""
-        return len(launch_plan(self, precision, "write"))
+        return len(launch_plan(self, precision, "write", classes))
 
     def run(self, out, precision=64, stream=None, classes=None):
         _check_device_tensor(out, self.ds.device, "output buffer")
